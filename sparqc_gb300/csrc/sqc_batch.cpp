@@ -43,7 +43,7 @@ TableDev slice_table(unsigned char* base, unsigned long long nb, bool dbl) {
     t.amps = base + off;
     off += align256(nb * kSlots * (dbl ? 16 : 8));
     t.list = reinterpret_cast<unsigned*>(base + off);
-    t.mask = nb - 1;
+    t.mask = nb - 1;   // (map_on stays 0: the caller stores the circuit's map)
     return t;
 }
 

@@ -77,10 +77,25 @@ __device__ __forceinline__ Header cas_hdr(Header* p, const Header& expect, const
     return o;
 }
 
+// Bucket where group G lives (mapped table) or where its probe chain starts (hashed table).
+__device__ __forceinline__ unsigned long long home_bucket(const TableDev& t, unsigned long long G) {
+    if (!t.map_on) return mix64(G) & t.mask;
+    unsigned b = 0;
+    for (uint32_t i = 0; i < t.map_n; ++i) b |= (unsigned)((G >> t.map_q[i]) & 1ULL) << i;
+    return b;
+}
+
+// Group of bucket b of a mapped table.
+__device__ __forceinline__ unsigned long long group_of_bucket(const TableDev& t, unsigned b) {
+    unsigned long long G = 0;
+    for (uint32_t i = 0; i < t.map_n; ++i) G |= (unsigned long long)((b >> i) & 1u) << t.map_q[i];
+    return G;
+}
+
 // Find the live bucket of group G, or -1. Correct while other threads claim buckets: a
 // claim only turns a non-live bucket live, and G's probe chain has no non-live bucket.
 __device__ __forceinline__ long long lookup_group(const TableDev& t, unsigned ep, unsigned long long G) {
-    unsigned long long b = mix64(G) & t.mask;
+    unsigned long long b = home_bucket(t, G);
     for (uint32_t i = 0; i < kMaxProbe; ++i) {
         const Header h = load_hdr_cg(t.hdr + b);
         if (h.epoch != ep) return -1;
@@ -96,7 +111,7 @@ __device__ __forceinline__ long long lookup_group(const TableDev& t, unsigned ep
 __device__ __forceinline__ long long claim_group(const TableDev& t, unsigned ep, unsigned long long G,
                                                  unsigned int* status, bool* created) {
     *created = false;
-    unsigned long long b = mix64(G) & t.mask;
+    unsigned long long b = home_bucket(t, G);
     Header cur = load_hdr_cg(t.hdr + b);
     uint32_t probes = 0, attempts = 0;
     while (probes < kMaxProbe && attempts < 4 * kMaxProbe) {

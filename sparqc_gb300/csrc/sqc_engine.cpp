@@ -21,6 +21,19 @@ constexpr unsigned long long kTinyMaxList = 256;   // live buckets up to which a
 constexpr size_t kDescInitial = 1 << 14;   // descriptors held between verified syncs
 constexpr unsigned long long kEpochRestart = 0xFFFFFF00ULL;   // epochs before the headers are cleared
 constexpr double kMaxLoad = 0.9;           // live buckets a pair pass may leave behind
+// A mapped table grows with the span of its keys, not with their number: past this many buckets
+// it is kept only while its mapped bits span at most kMapSpan times its live buckets (one pass
+// adds at most three bits); a thinner state moves to a hashed table.
+constexpr unsigned long long kMapFree = 1ULL << 12;
+constexpr unsigned long long kMapSpan = 16;
+// Buckets a grown mapped table has beyond its span: eight times as many while that is under a
+// gigabyte, so that a state growing one qubit at a time is not rebuilt at every one; then twice.
+constexpr unsigned long long kMapRoomy = 1ULL << 21;
+constexpr uint32_t kNoMap = 63;            // Span::dn of a pass whose bits no table maps: always refused
+
+bool map_worth(uint32_t dn, unsigned long long groups) {
+    return dn < kNoMap && ((1ULL << dn) <= kMapFree || (1ULL << dn) <= kMapSpan * groups);
+}
 
 unsigned long long pow2_at_least(unsigned long long x) {
     unsigned long long p = 1;
@@ -39,6 +52,7 @@ Engine::~Engine() {
     if (ev_copied_) cudaEventDestroy(ev_copied_);
     if (h_async_n_) cudaFreeHost(h_async_n_);
     free_table(&tab_);
+    free_table(&spare_);
     if (ctl_) cudaFree(ctl_);
     if (ctl_host_) cudaFreeHost(ctl_host_);
     if (sums_) cudaFree(sums_);
@@ -153,6 +167,17 @@ int Engine::alloc_table(unsigned long long nb, HostTable* out) {
     HostTable t;
     t.nb = nb;
     int rc;
+    if (spare_.nb == nb) {
+        t = spare_;
+        spare_ = HostTable();
+        if ((rc = cuda(cudaMemsetAsync(t.hdr, 0, nb * sizeof(Header), stream_), "cudaMemset(hdr)"))) {
+            free_table(&t);
+            return rc;
+        }
+        *out = t;
+        return SQC_OK;
+    }
+    free_table(&spare_);   // of another size: its memory may be needed
     if ((rc = cuda(cudaMalloc(&t.hdr, nb * sizeof(Header)), "cudaMalloc(hdr)")) ||
         (rc = cuda(cudaMalloc(&t.keys, nb * kSlots * sizeof(unsigned long long)), "cudaMalloc(keys)")) ||
         (rc = cuda(cudaMalloc(&t.amps, nb * kSlots * (dbl_ ? 16 : 8)), "cudaMalloc(amps)")) ||
@@ -183,6 +208,9 @@ TableDev Engine::dev() const {
     d.list = tab_.list;
     d.units = tab_.units;
     d.mask = tab_.nb - 1;
+    d.map_on = 0;
+    d.map_n = 0;
+    if (mapped_) map_.store(&d);
     return d;
 }
 
@@ -241,6 +269,8 @@ int Engine::set_zero() {
     snap_log_ = 0;
     host_upd_ = 0;
     list_hint_ = 1;
+    mapped_ = true;
+    map_.clear();
     int rc;
     if ((rc = next_epoch())) return rc;
     rc = cuda(launch_set_zero(dev(), ctl_, dbl_, stream_), "set_zero");
@@ -312,14 +342,17 @@ int Engine::set_state(const uint64_t* keys, const double* re, const double* im, 
     if (n) {
         plan_.kmask = ~(all_and ^ all_or);
         plan_.kval = all_and & plan_.kmask;
+        plan_.frame = plan_.kval;   // bits every key has set are stored as 0, as a mapped table needs
     }
     snap_plan_ = plan_;
     snap_log_ = 0;
     host_upd_ = 0;
     list_hint_ = std::max<unsigned long long>(n, 1);
+    map_.clear();
+    mapped_ = map_.extend(plan_.kmask, nq_) && map_worth(map_.n, groups) && (1ULL << map_.n) <= max_groups();
     if ((rc = next_epoch())) return rc;
-    rc = cuda(launch_set_state(d_rk_, d_rr_, d_ri_, n, dev(), ctl_, dbl_, sms_, stream_), "set_state");
-    launches_ += n ? 5 : 2;
+    rc = cuda(launch_set_state(d_rk_, d_rr_, d_ri_, n, plan_.frame, dev(), ctl_, dbl_, sms_, stream_), "set_state");
+    launches_ += n ? (mapped_ ? 6 : 5) : 2;
     if (rc) return rc;
     if ((rc = read_ctl())) return rc;
     if (ctl_host_->status != ST_OK) {
@@ -396,12 +429,12 @@ int Engine::flush(bool hold_last) {
         size_t g0, g1;
         uint32_t nx, q1, q2, q3;
         bool fixed;
+        uint32_t map0, dn, dim[3];   // mapped tables: mapped bits before and after, the units' dimensions
     };
     std::vector<Span> spans;
     split_passes(hd, nd, max_run_, max_nx_,
                  [&](size_t g0, size_t g1, uint32_t nx, uint32_t q1, uint32_t q2, uint32_t q3, bool fixed) {
-                     spans.push_back(Span{g0, g1, nx, q1, q2, q3, fixed});
-                     encode_pass(hd, g0, g1, q1, q3);
+                     spans.push_back(Span{g0, g1, nx, q1, q2, q3, fixed, 0, 0, {0, 0, 0}});
                  });
     if (hold_last && spans.size() >= 2) {
         // the last pass's gates, and the host-resolved gates around them, go back to the queue;
@@ -414,6 +447,21 @@ int Engine::flush(bool hold_last) {
         plan_ = after[spans.back().g0 - 1];
         spans.pop_back();
     }
+    // how each pass applies its gates: by place in its units (mapped tables; the map grows with
+    // the bits its gates make differ) or by key (hashed ones)
+    const uint32_t dims = dbl_ && max_nx_ < 3 ? 2u : 3u;
+    for (Span& sp : spans) {
+        const uint32_t q[3] = {sp.q1, sp.q2, sp.q3};
+        encode_pass(hd, sp.g0, sp.g1, sp.q1, sp.q3);
+        if (!mapped_) continue;
+        sp.map0 = map_.n;
+        sp.dn = kNoMap;   // more bits than a table maps: the pass refuses, and the state is hashed then
+        if (!map_.extend(after[sp.g1 - 1].kmask, nq_)) continue;
+        sp.dn = map_.n;
+        encode_unit_pass(hd, sp.g0, sp.g1, q, map_, dims, sp.dim);
+    }
+    if (mapped_) map_.store(&a.t);   // a pass uses the first dn of the mapped bits
+    a.dims = dims;
     if ((rc = cuda(cudaMemcpyAsync(d_desc_ + desc_used_, hd, nd * sizeof(GateDesc), cudaMemcpyHostToDevice, stream_),
                    "H2D gate descriptors")))
         return rc;
@@ -426,6 +474,10 @@ int Engine::flush(bool hold_last) {
         for (const Span& sp : spans) {
             if (sp.nx) h = std::min<unsigned long long>(tab_.nb, std::min(h << sp.nx, group_bound(after[sp.g1 - 1], nq_)));
             hmax = std::max(hmax, h);
+        }
+        if (mapped_) {   // unit passes enumerate the mapped bits' span
+            hmax = 1;
+            for (const Span& sp : spans) hmax = std::max(hmax, 1ULL << sp.dn);
         }
         if (spans.size() >= 2 && tiny_table(tab_.nb) && hmax <= kTinyMaxList) {
             TinyPass* ht = h_tiny_ + desc_used_;
@@ -440,14 +492,17 @@ int Engine::flush(bool hold_last) {
                 q.q2 = sp.q2;
                 q.q3 = sp.q3;
                 q.keys_fixed = sp.fixed ? 1u : 0u;
-                q.pad = 0;
+                q.dn = sp.dn;
+                for (int i = 0; i < 3; ++i) q.dim[i] = sp.dim[i];
+                q.dim[3] = 0;
                 q.grow_bound = group_bound(after[sp.g1 - 1], nq_);
                 any_pair = any_pair || sp.nx > 0;
             }
             if ((rc = cuda(cudaMemcpyAsync(d_tiny_ + desc_used_, ht, spans.size() * sizeof(TinyPass),
                                            cudaMemcpyHostToDevice, stream_), "H2D tiny passes")))
                 return rc;
-            if (launch_tiny(a, d_tiny_ + desc_used_, (uint32_t)spans.size(), dbl_, stream_) < 0)
+            if ((mapped_ ? launch_tiny_units(a, d_tiny_ + desc_used_, (uint32_t)spans.size(), dbl_, stream_)
+                         : launch_tiny(a, d_tiny_ + desc_used_, (uint32_t)spans.size(), dbl_, stream_)) < 0)
                 return launch_failed("tiny passes");
             if (time_passes_) {
                 cudaEvent_t ev = nullptr;
@@ -456,7 +511,7 @@ int Engine::flush(bool hold_last) {
             }
             for (const Span& sp : spans) {
                 passes_pair_ += sp.nx > 0 ? 1 : 0;
-                passes_.push_back(PassRec{snap_log_, snap_plan_});
+                passes_.push_back(PassRec{snap_log_, snap_plan_, sp.map0, sp.dn, sp.nx});
                 snap_log_ = src[sp.g1 - 1] + 1;
                 snap_plan_ = after[sp.g1 - 1];
                 ++passes_run_;
@@ -477,9 +532,17 @@ int Engine::flush(bool hold_last) {
         a.q3 = sp.q3;
         a.keys_fixed = sp.fixed ? 1u : 0u;
         a.grow_bound = group_bound(after[i - 1], nq_);
+        if (!mapped_ && sp.nx && std::min(list_hint_ << sp.nx, a.grow_bound) > a.max_groups) {
+            if ((rc = make_room(sp.nx, a.grow_bound))) return rc;
+            a.t = dev();
+            a.max_groups = max_groups();
+        }
         if (sp.nx)
             list_hint_ = std::min<unsigned long long>(tab_.nb, std::min(list_hint_ << sp.nx, a.grow_bound));
-        const int nl = launch_pass(a, list_hint_, dbl_, sms_, stream_);
+        a.dn = sp.dn;
+        for (int d = 0; d < 3; ++d) a.dim[d] = sp.dim[d];
+        const int nl = mapped_ ? launch_unit_pass(a, dbl_, sms_, stream_)
+                               : launch_pass(a, list_hint_, dbl_, sms_, stream_);
         if (nl < 0) return launch_failed("gate pass");
         const bool pair = sp.nx > 0;
         if (time_passes_) {
@@ -489,13 +552,41 @@ int Engine::flush(bool hold_last) {
             ev_prev = ev;
         }
         passes_pair_ += pair ? 1 : 0;
-        passes_.push_back(PassRec{snap_log_, snap_plan_});
+        passes_.push_back(PassRec{snap_log_, snap_plan_, sp.map0, sp.dn, sp.nx});
         snap_log_ = src[i - 1] + 1;
         snap_plan_ = after[i - 1];
         launches_ += (uint64_t)nl;
         ++passes_run_;
+        // a mapped pass the table is too small for refuses, and so would every later one: they
+        // are queued again, with it, when the table has grown
+        if (mapped_ && (1ULL << sp.dn) > a.max_groups) break;
     }
     desc_used_ += nd;
+    return SQC_OK;
+}
+
+// Buckets of a hashed table of `groups` groups: room for a pass with nx cross-group qubits, and
+// for several that empty as many groups as they make (keys that move leave their groups behind,
+// live and empty, until the table is rebuilt).
+unsigned long long Engine::hashed_size(unsigned long long groups, uint32_t nx) {
+    const double factor = std::max(8.0, (double)(1u << nx));
+    return std::max(kMinBuckets, pow2_at_least((unsigned long long)std::ceil(factor * (double)groups / kMaxLoad)));
+}
+
+// Before a pass that might not fit a hashed table by what the host knows: look at the exact list
+// length, and rebuild the table if the pass really might not fit. Waiting costs about 20 us; a pass
+// that refuses costs the launches of every pass queued behind it as well.
+int Engine::make_room(uint32_t nx, unsigned long long bound) {
+    int rc;
+    if ((rc = read_ctl())) return rc;
+    if (ctl_host_->status != ST_OK) return SQC_OK;   // an earlier pass refused or failed: sync() deals with it
+    list_hint_ = std::max<unsigned long long>(ctl_host_->list_n, 1);
+    if (std::min(list_hint_ << nx, bound) <= max_groups()) return SQC_OK;
+    const unsigned long long groups = ctl_host_->list_n - std::min(ctl_host_->list_n, ctl_host_->empty_groups);
+    const unsigned long long nb = std::max(tab_.nb, hashed_size(groups, nx));
+    if ((double)nb * bucket_bytes() > (double)budget_) return SQC_OK;   // the pass refuses; sync() decides
+    if ((rc = rebuild(nb, false))) return rc;
+    passes_.clear();   // all verified: later ones count from here
     return SQC_OK;
 }
 
@@ -615,7 +706,7 @@ int Engine::sync() {
             list_hint_ = std::max<unsigned long long>(ctl_host_->list_n, 1);
             // many groups left without keys (pruned away): rebuild without them
             if (ctl_host_->list_n > 4096 && ctl_host_->empty_groups * 2 > ctl_host_->list_n) {
-                if ((rc = rebuild(tab_.nb))) return rc;
+                if ((rc = rebuild(tab_.nb, mapped_))) return rc;
             }
             return SQC_OK;
         }
@@ -632,7 +723,7 @@ int Engine::sync() {
 
 // Copy the live, non-empty buckets into a new table of nb_new buckets. The control block
 // must be in sync with the device (read_ctl) and no pass may be in flight.
-int Engine::rebuild(unsigned long long nb_new) {
+int Engine::rebuild(unsigned long long nb_new, bool mapped) {
     HostTable nt;
     int rc;
     if ((rc = alloc_table(nb_new, &nt))) return rc;
@@ -655,6 +746,9 @@ int Engine::rebuild(unsigned long long nb_new) {
     TableDev nd;
     nd.hdr = nt.hdr; nd.keys = nt.keys; nd.amps = nt.amps; nd.list = nt.list; nd.units = nt.units;
     nd.mask = nt.nb - 1;
+    nd.map_on = 0;
+    nd.map_n = 0;
+    if (mapped) map_.store(&nd);
     if ((rc = cuda(launch_rehash(dev(), n_old, nd, 1u, dbl_ ? 16 : 8, ctl_, sms_, stream_), "rehash"))) return rc;
     ++launches_;
     if ((rc = read_ctl())) return rc;
@@ -667,8 +761,14 @@ int Engine::rebuild(unsigned long long nb_new) {
                                    cudaMemcpyHostToDevice, stream_), "H2D list_n")) ||
         (rc = cuda(cudaStreamSynchronize(stream_), "sync")))
         return rc;
+    if (!mapped && !mapped_ && (double)(tab_.nb + nb_new) * bucket_bytes() <= (double)budget_) {
+        free_table(&spare_);
+        spare_ = tab_;
+        tab_ = HostTable();
+    }
     free_table(&tab_);
     tab_ = nt;
+    mapped_ = mapped;
     seq_verified_ = 0;
     list_hint_ = std::max<unsigned long long>(ctl_host_->list_n, 1);
     ++rebuilds_;
@@ -680,14 +780,32 @@ int Engine::rebuild(unsigned long long nb_new) {
 // again, from the planner state saved with pass k.
 int Engine::repair(size_t k) {
     const PassRec pr = passes_[k];
-    const unsigned long long groups = ctl_host_->list_n;
-    unsigned long long nb = std::max(tab_.nb * 2, pow2_at_least((unsigned long long)std::ceil(4.0 * (double)groups / kMaxLoad)));
-    // near the budget, take the largest table that still fits (the pass may refuse again)
-    unsigned long long fit = tab_.nb;
-    while ((double)(fit * 2) * bucket_bytes() <= (double)budget_) fit *= 2;
-    if (nb > fit && fit > tab_.nb) nb = fit;
+    // groups that still hold keys: the rebuild drops the others
+    const unsigned long long groups = ctl_host_->list_n - std::min(ctl_host_->list_n, ctl_host_->empty_groups);
+    auto fits = [&](unsigned long long b) { return (double)b * bucket_bytes() <= (double)budget_; };
+    unsigned long long nb = 0;
+    bool mapped = false;
+    if (mapped_) {
+        map_.n = pr.map_n;
+        if (map_worth(pr.dn, groups)) {
+            const unsigned long long span = 1ULL << pr.dn;
+            nb = std::max(span * 8 <= kMapRoomy ? span * 8 : std::max(span * 2, kMapRoomy), kMinBuckets);
+            while (nb > 2 * span && !fits(nb)) nb /= 2;   // at most 0.9 full, like a hashed table
+            mapped = fits(nb);
+        }
+    }
+    if (!mapped) {
+        nb = hashed_size(groups, pr.nx);
+        // a hashed table mostly of emptied groups has room once they are dropped; else it doubles
+        if (!mapped_ && (nb > tab_.nb || groups * 2 > ctl_host_->list_n)) nb = std::max(nb, tab_.nb * 2);
+        // near the budget, take the largest table that still fits (the pass may refuse again)
+        unsigned long long fit = tab_.nb;
+        while (fits(fit * 2)) fit *= 2;
+        if (nb > fit && (fit > tab_.nb || mapped_)) nb = fit;
+        if ((double)groups > kMaxLoad * (double)nb) return fail(SQC_ERR_BUDGET, "table memory would exceed the HBM budget");
+    }
     int rc;
-    if ((rc = rebuild(nb))) return rc;
+    if ((rc = rebuild(nb, mapped))) return rc;
     std::vector<sqc_gate> again(log_.begin() + (long)pr.log_begin, log_.end());
     replays_ += passes_.size() - k;
     passes_run_ -= passes_.size() - k;
@@ -722,6 +840,7 @@ int Engine::take_unapplied(std::vector<sqc_gate>* rest) {
         (rc = cuda(cudaStreamSynchronize(stream_), "sync")))
         return rc;
     plan_ = pr.snap;
+    if (mapped_) map_.n = pr.map_n;
     snap_plan_ = plan_;
     snap_log_ = 0;
     log_.clear();
@@ -962,6 +1081,10 @@ int Engine::measure(uint32_t qubit, double u, int* outcome, double* p1) {
                    "collapse")))
         return rc;
     launches_ += 2;
+    if (mapped_) {   // the kept keys are the buckets' presence masks now
+        if ((rc = cuda(launch_refresh_masks(dev(), ctl_, list_hint_, sms_, stream_), "refresh masks"))) return rc;
+        ++launches_;
+    }
     if ((rc = read_ctl())) return rc;
     plan_.kmask |= bit;
     plan_.kval = (plan_.kval & ~bit) | val;

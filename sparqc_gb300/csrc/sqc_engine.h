@@ -26,7 +26,9 @@ struct HostTable {
 
 struct PassRec {
     size_t log_begin;   // replay of this pass starts at this log index...
-    Planner snap;       // ...with this planner state
+    Planner snap;       // ...with this planner state...
+    uint32_t map_n;     // ...and this many mapped group bits
+    uint32_t dn, nx;    // mapped bits the pass needs (0: hashed table) and its cross-group qubits
 };
 
 class Engine {
@@ -99,7 +101,9 @@ private:
     int alloc_table(unsigned long long nb, HostTable* out);
     void free_table(HostTable* t);
     TableDev dev() const;
-    int rebuild(unsigned long long nb_new);
+    int rebuild(unsigned long long nb_new, bool mapped);
+    int make_room(uint32_t nx, unsigned long long bound);   // hashed tables: room for the next pass
+    unsigned long long hashed_size(unsigned long long groups, uint32_t nx);
     int repair(size_t failed_pass);
     int ensure_desc(size_t n);
     int ensure_readout(size_t n);
@@ -138,6 +142,9 @@ private:
     bool own_stream_ = false;
 
     HostTable tab_;
+    HostTable spare_;           // the table the last rebuild left, for the next one (hashed tables)
+    GroupMap map_;              // mapped group bits, when mapped_
+    bool mapped_ = true;        // the table is mapped (sqc_types.h, TableDev), else hashed
     Ctl* ctl_ = nullptr;        // device
     Ctl* ctl_host_ = nullptr;   // pinned mirror
     ExactSums* sums_ = nullptr;       // device: exact sums of norm, probability and compare

@@ -128,6 +128,8 @@ extern "C" int sqc_apply_fixed(uint32_t nq, const uint64_t* keys_in, const doubl
     t.list = reinterpret_cast<unsigned*>(b + kOffList);
     t.units = nullptr;    // small tables take the direct pass, which needs neither
     t.mask = kFixedBuckets - 1;
+    t.map_on = 0;         // the scratch table is hashed
+    t.map_n = 0;
     Ctl* ctl = reinterpret_cast<Ctl*>(b + kOffCtl);
     GateDesc* d_desc = reinterpret_cast<GateDesc*>(b + kOffDesc);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -142,8 +144,8 @@ extern "C" int sqc_apply_fixed(uint32_t nq, const uint64_t* keys_in, const doubl
         }
     }
     // load the caller's state (the kernels read its device arrays; the epoch bump frees the table)
-    if (launch_set_state(reinterpret_cast<const unsigned long long*>(keys_in), re_in, im_in, n_in, t, ctl, true,
-                         sms, st) != cudaSuccess)
+    if (launch_set_state(reinterpret_cast<const unsigned long long*>(keys_in), re_in, im_in, n_in, 0ULL, t, ctl,
+                         true, sms, st) != cudaSuccess)
         return SQC_ERR_CUDA;
     if (nq < 64 && n_in) {
         const unsigned long long outside = ~((1ULL << nq) - 1);

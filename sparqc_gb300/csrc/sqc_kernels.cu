@@ -69,6 +69,7 @@ __global__ void set_zero_kernel(TableDev t, Ctl* ctl, int dbl) {
         const size_t s = (size_t)b * kSlots + lane;
         t.keys[s] = lane == 0 ? 0ULL : empty_key(lane);
         if (lane == 0) {
+            if (t.map_on) t.hdr[b].aux = 1u;   // presence mask: slot 0
             if (dbl) reinterpret_cast<double2*>(t.amps)[s] = make_double2(1.0, 0.0);
             else reinterpret_cast<float2*>(t.amps)[s] = make_float2(1.0f, 0.0f);
         }
@@ -102,12 +103,12 @@ __global__ void set_state_begin_kernel(Ctl* ctl) {
 
 // set_state step 1: claim the bucket of every entry's group; the claimer appends it to the list.
 __global__ void set_state_claim_kernel(const unsigned long long* __restrict__ keys, unsigned long long n,
-                                       TableDev t, Ctl* ctl) {
+                                       unsigned long long frame, TableDev t, Ctl* ctl) {
     const unsigned ep = ctl->epoch;
     for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x) {
         bool created;
-        const long long b = claim_group(t, ep, keys[i] >> kSlotBits, &ctl->status, &created);
+        const long long b = claim_group(t, ep, (keys[i] ^ frame) >> kSlotBits, &ctl->status, &created);
         if (created) t.list[atomicAdd(&ctl->list_tail, 1ULL)] = (unsigned)b;
     }
 }
@@ -124,12 +125,12 @@ __global__ void set_state_clear_kernel(TableDev t, Ctl* ctl) {
 
 // set_state step 3: store every entry in its slot; a second store to a slot is a duplicate key.
 __global__ void set_state_fill_kernel(const unsigned long long* __restrict__ keys, const double* __restrict__ re,
-                                      const double* __restrict__ im, unsigned long long n, TableDev t, Ctl* ctl,
-                                      int dbl) {
+                                      const double* __restrict__ im, unsigned long long n,
+                                      unsigned long long frame, TableDev t, Ctl* ctl, int dbl) {
     const unsigned ep = ctl->epoch;
     for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x) {
-        const unsigned long long k = keys[i];
+        const unsigned long long k = keys[i] ^ frame;
         const long long b = lookup_group(t, ep, k >> kSlotBits);
         if (b < 0) { atomicCAS(&ctl->status, 0u, (unsigned)ST_TABLE_FULL); continue; }
         const int j = (int)(k & 15ULL);
@@ -145,6 +146,21 @@ __global__ void set_state_fill_kernel(const unsigned long long* __restrict__ key
 __global__ void set_state_end_kernel(Ctl* ctl, unsigned long long n) {
     ctl->list_n = ctl->list_tail;
     ctl->nnz = n;
+}
+
+// Presence masks of a mapped table's listed buckets, from their keys (a half-warp per bucket).
+__global__ void refresh_masks_kernel(TableDev t, Ctl* ctl) {
+    const unsigned long long n = ctl->list_tail;
+    const int lane = threadIdx.x & 31, j = lane & 15;
+    const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+    for (unsigned long long e0 = warp * 2; e0 < n; e0 += nwarps * 2) {
+        const unsigned long long e = e0 + (lane >> 4);
+        const unsigned b = e < n ? t.list[e] : 0u;
+        const bool p = e < n && slot_present(t.keys[(size_t)b * kSlots + j], j);
+        const unsigned bal = __ballot_sync(kFull, p);
+        if (e < n && j == 0) t.hdr[b].aux = lane >= 16 ? bal >> 16 : bal & 0xFFFFu;
+    }
 }
 
 // Present keys and empty live buckets over the list, into ctl->acc_nnz / acc_empty (adds).
@@ -338,12 +354,14 @@ __global__ void rehash_kernel(TableDev told, unsigned long long n_old, TableDev 
         const unsigned long long k = in ? told.keys[s] : 0ULL;
         const bool p = in && slot_present(k, j);
         const unsigned bal = __ballot_sync(kFull, p);
-        const bool keep = in && ((half ? (bal >> 16) : (bal & 0xFFFFu)) != 0);
+        const unsigned mine = half ? (bal >> 16) : (bal & 0xFFFFu);
+        const bool keep = in && mine != 0;
         long long nbk = -1;
         bool created = false;
         if (keep && j == 0) nbk = claim_group(tnew, ep_new, load_hdr(told.hdr + b).group, &ctl->status, &created);
         nbk = (long long)shfl64((unsigned long long)nbk, half << 4);
         const long long fresh = (keep && j == 0 && nbk >= 0) ? nbk : -1;
+        if (fresh >= 0 && tnew.map_on) tnew.hdr[fresh].aux = mine;
         if (keep && nbk >= 0) {
             const size_t d = (size_t)nbk * kSlots + j;
             tnew.keys[d] = k;
@@ -378,16 +396,22 @@ cudaError_t launch_set_zero(const TableDev& t, Ctl* ctl, bool dbl, cudaStream_t 
 }
 
 cudaError_t launch_set_state(const unsigned long long* keys, const double* re, const double* im,
-                             unsigned long long n, const TableDev& t, Ctl* ctl, bool dbl, int sms,
-                             cudaStream_t st) {
+                             unsigned long long n, unsigned long long frame, const TableDev& t, Ctl* ctl, bool dbl,
+                             int sms, cudaStream_t st) {
     set_state_begin_kernel<<<1, 1, 0, st>>>(ctl);
     const int ge = grid_for(n, kThreads, sms);
     if (n) {
-        set_state_claim_kernel<<<ge, kThreads, 0, st>>>(keys, n, t, ctl);
+        set_state_claim_kernel<<<ge, kThreads, 0, st>>>(keys, n, frame, t, ctl);
         set_state_clear_kernel<<<grid_for(n * kSlots, kThreads, sms), kThreads, 0, st>>>(t, ctl);
-        set_state_fill_kernel<<<ge, kThreads, 0, st>>>(keys, re, im, n, t, ctl, dbl ? 1 : 0);
+        set_state_fill_kernel<<<ge, kThreads, 0, st>>>(keys, re, im, n, frame, t, ctl, dbl ? 1 : 0);
+        if (t.map_on) refresh_masks_kernel<<<grid_for(n, kThreads / 16, sms), kThreads, 0, st>>>(t, ctl);
     }
     set_state_end_kernel<<<1, 1, 0, st>>>(ctl, n);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_refresh_masks(const TableDev& t, Ctl* ctl, unsigned long long list_hint, int sms, cudaStream_t st) {
+    refresh_masks_kernel<<<grid_for(list_hint, kThreads / 16, sms), kThreads, 0, st>>>(t, ctl);
     return cudaGetLastError();
 }
 

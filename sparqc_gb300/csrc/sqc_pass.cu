@@ -24,6 +24,7 @@
 // and diagonal gates keep every key.
 #include "sqc_kernels.h"
 #include "sqc_pass_dev.cuh"
+#include "sqc_unit.cuh"
 
 #include <algorithm>
 
@@ -184,6 +185,90 @@ __global__ void __launch_bounds__(kThreads, DirectOcc<T, NX>::kMin) direct_kerne
     };
     direct_work<T, NX, kSmem>(a, sg, ep, n, next4, cnt_nnz, cnt_empty, upd);
     finish_pass(ctl, cnt_nnz, cnt_empty, upd, nnz_in, a.keys_fixed != 0, NX > 0, a.amp_bytes);
+}
+
+// ---- unit pass (mapped tables) ---------------------------------------------------------------
+// Units are dealt out round robin to the warps (they cost the same); a table whose live buckets
+// are few among the mapped ones is walked by its list instead, 32 entries per warp at a time.
+template <class T, int DIMS> struct UnitOcc {
+    static constexpr int kMin = sizeof(T) == 4 ? 4 : DIMS == 2 ? 3 : 2;
+};
+
+template <class T, int DIMS>
+__global__ void __launch_bounds__(kThreads, UnitOcc<T, DIMS>::kMin) unit_kernel(PassArgs a) {
+    __shared__ UGates<T> sg;
+    stage_ugates<T>(sg, a.gates, a.g0, a.g1);   // no kernel writes the gates: staged while the previous pass drains
+    wait_prior_grid();
+    allow_next_grid();
+    Ctl* ctl = a.ctl;
+    if (*(volatile unsigned int*)&ctl->status) return;
+    if ((1ULL << a.dn) > a.max_groups) {   // the mapped bits outgrow the table: refuse before touching the state
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(&ctl->status, 0u, (unsigned)ST_GROW);
+        return;
+    }
+    const unsigned long long n = ctl->list_n;
+    const unsigned ep = ctl->epoch;
+    const unsigned long long nnz_in = ctl->nnz;
+    const int lane = threadIdx.x & 31;
+    const UnitPass up = unit_pass<DIMS>(a.dn, a.dim[0], a.dim[1], a.dim[2]);
+    const unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned long long nw = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+    const uint32_t ng = a.g1 - a.g0;
+    const GateDesc* gates = a.gates + a.g0;
+    unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
+    if (walk_list(n, a.dn)) {
+        for (unsigned long long e0 = w * 32; e0 < n; e0 += nw * 32)
+            walk_entries<T, DIMS>(a.t, ctl, ep, up, e0, n, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+    } else {
+        walk_units<T, DIMS>(a.t, ctl, ep, up, w, up.units, nw, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+    }
+    finish_pass(ctl, cnt_nnz, cnt_empty, upd, nnz_in, a.keys_fixed != 0, a.nx > 0, a.amp_bytes);
+}
+
+// The passes of a flush on a tiny mapped table, one block, one launch (as tiny_kernel below).
+template <class T, int DIMS>
+__global__ void __launch_bounds__(kThreads) tiny_unit_kernel(PassArgs a, const TinyPass* __restrict__ tp, uint32_t np) {
+    __shared__ UGates<T> sg;
+    __shared__ unsigned long long red[3][kThreads / 32];
+    Ctl* ctl = a.ctl;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (*(volatile unsigned int*)&ctl->status) return;
+    const unsigned ep = *(volatile unsigned int*)&ctl->epoch;
+    unsigned long long nnz_in = *(volatile unsigned long long*)&ctl->nnz;
+    for (uint32_t p = 0; p < np; ++p) {
+        const TinyPass q = tp[p];
+        if ((1ULL << q.dn) > a.max_groups) {   // refuse before touching the state
+            if (threadIdx.x == 0) atomicCAS(&ctl->status, 0u, (unsigned)ST_GROW);
+            return;
+        }
+        stage_ugates<T>(sg, a.gates, q.g0, q.g1);
+        const UnitPass up = unit_pass<DIMS>(q.dn, q.dim[0], q.dim[1], q.dim[2]);
+        unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
+        walk_units<T, DIMS>(a.t, ctl, ep, up, w, up.units, kThreads / 32, sg, a.gates + q.g0, q.g1 - q.g0, lane, a.prune,
+                            cnt_nnz, cnt_empty, upd);
+        cnt_nnz = warp_sum(cnt_nnz);
+        cnt_empty = warp_sum(cnt_empty);
+        upd = warp_sum(upd);
+        if (lane == 0) { red[0][w] = cnt_nnz; red[1][w] = cnt_empty; red[2][w] = upd; }
+        __syncthreads();
+        unsigned long long tn = 0;   // every thread knows the pass's key count
+        for (int i = 0; i < kThreads / 32; ++i) tn += red[0][i];
+        if (threadIdx.x == 0) {
+            unsigned long long te = 0, tu = 0;
+            for (int i = 0; i < kThreads / 32; ++i) { te += red[1][i]; tu += red[2][i]; }
+            ctl->nnz = tn;
+            ctl->empty_groups = te;
+            ctl->list_n = *(volatile unsigned long long*)&ctl->list_tail;
+            ctl->amp_updates += tu;
+            const unsigned long long ab = q.keys_fixed ? nnz_in * (8ULL + 2ULL * a.amp_bytes)
+                                                       : (nnz_in + tn) * (8ULL + a.amp_bytes);
+            ctl->alg_bytes += ab;
+            if (q.nx > 0) ctl->alg_bytes_pair += ab;
+            ctl->seq += 1;
+        }
+        nnz_in = tn;
+        __syncthreads();   // the pass is published, and red and sg are free, before the next one
+    }
 }
 
 // ---- tiny states: every pass of a flush in one single-block launch --------------------------
@@ -622,6 +707,13 @@ int direct_residency(bool dbl, int nx) {
 
 constexpr unsigned long long kTinyMaxBuckets = 4096;
 
+template <class T, int DIMS>
+int unit_residency() {
+    static int cache = 0;
+    if (!cache) cache = occupancy(unit_kernel<T, DIMS>, kThreads, 0);
+    return cache;
+}
+
 // Launch a direct pass with programmatic stream serialization: its blocks may be scheduled
 // once the previous kernel in the stream has let them (allow_next_grid), and they wait for
 // that kernel's completion in wait_prior_grid before touching the state. Direct passes take
@@ -648,6 +740,15 @@ cudaError_t launch_direct(const PassArgs& a, int grid, cudaStream_t st) {
     return launch_dep(direct_kernel<T, NX>, grid, kThreads, 0, a, st);
 }
 
+template <class T, int DIMS>
+cudaError_t launch_unit(const PassArgs& a, int sms, cudaStream_t st) {
+    // at most one resident wave; a warp per unit (or per 32 list entries) below that
+    const unsigned long long units = std::max<unsigned long long>(1, (1ULL << a.dn) >> DIMS);
+    const unsigned long long wave = (unsigned long long)sms * unit_residency<T, DIMS>();
+    const int grid = (int)std::max<unsigned long long>(1, std::min(wave, (units + kThreads / 32 - 1) / (kThreads / 32)));
+    return launch_dep(unit_kernel<T, DIMS>, grid, kThreads, 0, a, st);
+}
+
 template <class T, int NX>
 cudaError_t launch_staged(const PassArgs& a, int grid, cudaStream_t st) {
     staged_kernel<T, NX><<<grid, kStagedThreads, staged_smem<T, NX>(), st>>>(a);
@@ -663,6 +764,20 @@ int launch_tiny(const PassArgs& a, const TinyPass* passes, uint32_t np, bool dbl
     if (dbl) tiny_kernel<double><<<1, kThreads, 0, st>>>(a, passes, np);
     else tiny_kernel<float><<<1, kThreads, 0, st>>>(a, passes, np);
     return cudaGetLastError() == cudaSuccess ? 1 : -1;
+}
+
+int launch_tiny_units(const PassArgs& a, const TinyPass* passes, uint32_t np, bool dbl, cudaStream_t st) {
+    if (a.t.mask + 1 > kTinyMaxBuckets) return -1;
+    if (!dbl) tiny_unit_kernel<float, 3><<<1, kThreads, 0, st>>>(a, passes, np);
+    else if (a.dims == 3) tiny_unit_kernel<double, 3><<<1, kThreads, 0, st>>>(a, passes, np);
+    else tiny_unit_kernel<double, 2><<<1, kThreads, 0, st>>>(a, passes, np);
+    return cudaGetLastError() == cudaSuccess ? 1 : -1;
+}
+
+int launch_unit_pass(const PassArgs& a, bool dbl, int sms, cudaStream_t st) {
+    const cudaError_t e = !dbl ? launch_unit<float, 3>(a, sms, st)
+                          : a.dims == 3 ? launch_unit<double, 3>(a, sms, st) : launch_unit<double, 2>(a, sms, st);
+    return e == cudaSuccess ? 1 : -1;
 }
 
 int launch_pass(const PassArgs& a, unsigned long long list_hint, bool dbl, int sms, cudaStream_t st) {

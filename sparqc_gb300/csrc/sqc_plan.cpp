@@ -98,6 +98,115 @@ void encode_pass(GateDesc* d, size_t g0, size_t g1, uint32_t q1, uint32_t q3) {
     }
 }
 
+bool GroupMap::extend(unsigned long long kmask, uint32_t nq) {
+    const unsigned long long reg = nq >= 64 ? ~0ULL : ((1ULL << nq) - 1);
+    unsigned long long add = ~kmask & reg & ~15ULL;
+    for (uint32_t i = 0; i < n; ++i) add &= ~(1ULL << (q[i] + kSlotBits));
+    if (n + (uint32_t)__builtin_popcountll(add) > kMaxMapBits) return false;
+    for (; add; add &= add - 1) q[n++] = (uint8_t)(__builtin_ctzll(add) - kSlotBits);
+    return true;
+}
+
+void encode_unit_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[3], const GroupMap& map, uint32_t dims,
+                      uint32_t dim[3]) {
+    // the cross-group qubit with the fewest gates goes to the lane dimension (1), whose gates
+    // shuffle; the others pair slots of one lane, the most used in dimension 0 (dimension 2 costs
+    // an exchange of slots around each gate)
+    uint32_t order[3] = {q[0], q[1], q[2]}, uses[3] = {0, 0, 0};
+    for (size_t k = g0; k < g1; ++k)
+        for (int i = 0; i < 3; ++i)
+            if (!streamable(d[k]) && d[k].target == q[i]) ++uses[i];
+    int nx = 0;
+    while (nx < 3 && q[nx] != kNoQubit) ++nx;
+    if ((uint32_t)nx == dims) {
+        int least = 0;
+        for (int i = 1; i < nx; ++i)
+            if (uses[i] < uses[least]) least = i;
+        std::swap(order[1], order[least]);
+        std::swap(uses[1], uses[least]);
+    } else if (nx == 2) {   // three dimensions, two qubits: both pair slots
+        order[2] = order[1];
+        uses[2] = uses[1];
+        order[1] = kNoQubit;
+    }
+    if (dims == 3 && nx >= 2 && uses[2] > uses[0]) std::swap(order[0], order[2]);
+    unsigned long long taken = 0;
+    int bit[3] = {-1, -1, -1};
+    for (uint32_t i = 0; i < dims; ++i) {
+        if (order[i] == kNoQubit) continue;
+        bit[i] = map.bit_of(order[i]);
+        taken |= 1ULL << bit[i];
+    }
+    for (uint32_t i = 0; i < 3; ++i) {
+        if (i < dims && bit[i] < 0) {
+            int b = 0;
+            while ((taken >> b) & 1ULL) ++b;
+            bit[i] = b;
+            taken |= 1ULL << b;
+        }
+        dim[i] = i < dims ? (uint32_t)bit[i] : 31u;
+    }
+    for (size_t k = g0; k < g1; ++k) {
+        GateDesc& g = d[k];
+        g.om = g.ov = 0;
+        uint32_t lmask = 0, lval = 0, smask = 0, sval = 0;
+        for (unsigned long long c = g.ctrl; c; c &= c - 1) {
+            const uint32_t qb = (uint32_t)__builtin_ctzll(c);
+            const uint32_t v = (uint32_t)((g.cval >> qb) & 1ULL);
+            if (qb < (uint32_t)kSlotBits) {
+                lmask |= 1u << qb;
+                lval |= v << qb;
+                continue;
+            }
+            const uint32_t b = (uint32_t)map.bit_of(qb);
+            if (b == dim[0]) { smask |= 1u; sval |= v; }
+            else if (b == dim[1]) { lmask |= 16u; lval |= v << 4; }
+            else if (b == dim[2]) { smask |= 2u; sval |= v << 1; }
+            else { g.om |= 1u << b; g.ov |= v << b; }
+        }
+        // the target: a lane bit, a slot bit (0 or 1), or a bit of the unit's base; a diagonal gate
+        // on a bit that never differed reads stored 0 (no bit of the base)
+        uint32_t lane_bit = kNoQubit, slot_bit = kNoQubit, outer = kMaxMapBits;
+        if (g.target < (uint32_t)kSlotBits) {
+            lane_bit = g.target;
+        } else {
+            const int b = map.bit_of(g.target);
+            if (b >= 0 && (uint32_t)b == dim[0]) slot_bit = 0;
+            else if (b >= 0 && (uint32_t)b == dim[1]) lane_bit = 4;
+            else if (b >= 0 && (uint32_t)b == dim[2]) slot_bit = 1;
+            else if (b >= 0) outer = (uint32_t)b;
+        }
+        const bool flip = (g.flip & kOpFlip) != 0, pairs = is_branch_kind(g.kind) || is_swap_kind(g.kind);
+        const bool pair3 = pairs && slot_bit == 1;
+        uint32_t slots = 0, bits = 0;
+        for (uint32_t s = 0; s < 4; ++s) {
+            const uint32_t at = pair3 ? ((s & 1u) << 1) | (s >> 1) : s;   // the slot at place s of the exchanged order
+            if (((at ^ sval) & smask) == 0) slots |= 1u << s;
+            if ((slot_bit != kNoQubit && ((at >> slot_bit) & 1u)) != flip) bits |= 1u << s;
+        }
+        uint32_t op;
+        const uint32_t shfl = lane_bit != kNoQubit ? 1u : 0u;
+        switch (g.kind) {
+        case KX: op = UO_X_PAIR + shfl; break;
+        case KY: op = UO_Y_PAIR + shfl; break;
+        case KH: op = UO_H_PAIR + shfl; break;
+        case KRX: op = UO_RX_PAIR + shfl; break;
+        case KRY: op = UO_RY_PAIR + shfl; break;
+        case KU: op = UO_U_PAIR + shfl; break;
+        case KZ: op = UO_Z; break;
+        case KS: op = UO_S; break;
+        case KSDG: op = UO_SDG; break;
+        case KYPH: op = UO_YPH; break;
+        case KRZ: op = UO_RZ; break;
+        default: op = UO_PHASE; break;   // Phase, T, Tdg
+        }
+        const uint32_t tb = lane_bit != kNoQubit ? lane_bit : slot_bit != kNoQubit ? kMaxMapBits : outer;
+        g.loc = lmask | (lval << kLocLaneVal) | (slots << kLocSlots) | (bits << kLocSlotBit) | (tb << kLocBit) |
+                (shfl ? kLocLane : 0u) | (flip ? kLocFlip : 0u) | (is_branch_kind(g.kind) ? kLocBranch : 0u) |
+                (pair3 ? kLocPair3 : 0u) | (op << kLocOp);
+    }
+}
+
 namespace {
 
 // The gates of a scheduling window, as the scheduler sees them: the qubits each touches (target

@@ -78,6 +78,35 @@ void split_passes(const GateDesc* d, size_t n, size_t max_run, uint32_t max_nx, 
 // pair lanes (shuffles).
 void encode_pass(GateDesc* d, size_t g0, size_t g1, uint32_t q1, uint32_t q3 = kNoQubit);
 
+// The group bits a mapped table addresses its buckets by (TableDev::map_q): bucket bit i is group
+// bit q[i]. Bits join in the order they begin to differ between keys, so a table that gains a bit
+// keeps every bucket where it is.
+struct GroupMap {
+    uint32_t n = 0;
+    uint8_t q[kMaxMapBits + 1] = {};
+    void clear() { n = 0; }
+    // Add the qubits >= 4 that may differ between keys (not in kmask, below nq) and are not mapped
+    // yet, lowest first. False when they would not fit.
+    bool extend(unsigned long long kmask, uint32_t nq);
+    int bit_of(uint32_t qubit) const {   // bucket bit of a qubit >= 4, or -1
+        for (uint32_t i = 0; i < n; ++i)
+            if (q[i] + (uint32_t)kSlotBits == qubit) return (int)i;
+        return -1;
+    }
+    void store(TableDev* t) const {
+        t->map_on = 1;
+        t->map_n = n;
+        for (uint32_t i = 0; i < n; ++i) t->map_q[i] = q[i];
+    }
+};
+
+// Choose the bucket bits of a unit pass's dimensions and record in descriptors [g0, g1) (one pass
+// with cross-group qubits q[0..2], kNoQubit when absent, at most dims of them) how the pass
+// applies each gate (GateDesc.om, ov, loc). Every qubit >= 4 a gate tests or changes must be
+// mapped. Dimensions without a cross-group qubit take the lowest free bucket bits.
+void encode_unit_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[3], const GroupMap& map, uint32_t dims,
+                      uint32_t dim[3]);
+
 // An order of gates g[0..n) that passes fuse better, as a permutation: perm[i] is the index of
 // the i-th gate to apply. Passes are built greedily from the first gate not yet placed: a gate
 // within the next `window` joins the pass when it commutes with every gate it moves ahead of

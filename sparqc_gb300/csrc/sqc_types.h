@@ -41,6 +41,13 @@ struct alignas(16) Unit {
     unsigned int b[8];
 };
 
+// Where a group's bucket is. A *mapped* table addresses groups directly: bucket bit i is group
+// bit map_q[i], for the map_n group bits that may differ between keys (in the order they began
+// to); every other bit of a stored group is 0, so the address is exact and no probing is needed.
+// Header.aux then holds the bucket's presence mask. A *hashed* table (map_on 0) probes linearly
+// from a hash of the group, and Header.aux is 0.
+constexpr uint32_t kMaxMapBits = 31;
+
 struct TableDev {
     Header* hdr;
     unsigned long long* keys;
@@ -48,6 +55,9 @@ struct TableDev {
     unsigned int* list;         // live buckets, in claim order
     Unit* units;                // owned units of a pair or quad pass, compacted by the resolve kernel
     unsigned long long mask;    // nb - 1
+    uint32_t map_on;            // 1: mapped, 0: hashed
+    uint32_t map_n;             // mapped group bits
+    uint8_t map_q[kMaxMapBits + 1];
 };
 
 // Device-resident control block of one state. Per-pass bookkeeping happens here, on the
@@ -87,6 +97,26 @@ struct alignas(16) GateDesc {
     double m[8];          // u: m00, m01, m10, m11 as (re, im)
     float cf, sf;         // float copies for FP32 states
     float mf[8];
+    // how a unit pass (sqc_unit.cuh) applies the gate, set by encode_unit_pass on the host: the
+    // unit's base index u satisfies the controls outside the unit iff (u & om) == ov; loc holds
+    // the rest (kLoc* fields)
+    uint32_t om, ov, loc, pad2;
+};
+
+// GateDesc.loc: what a unit pass does for the gate, by place in the unit. Slot fields are as seen
+// after the exchange of slots 1 and 2 that kLocPair3 asks for.
+constexpr uint32_t kLocLaneVal = 5;        // bits 0..4: controlled lane bits (qubits 0..3, dimension 1), 5..9: their values
+constexpr uint32_t kLocSlots = 10;         // bits 10..13: slots whose controls (dimensions 0 and 2) hold
+constexpr uint32_t kLocSlotBit = 14;       // bits 14..17: diagonal gates: logical target bit per slot, before the next two
+constexpr uint32_t kLocBit = 18;           // bits 18..22: the target's bit of the lane index or of the unit's base (31: none)
+constexpr uint32_t kLocLane = 1u << 23;    // ... of the lane index
+constexpr uint32_t kLocFlip = 1u << 24;    // the stored frame flips the target bit (pairing gates)
+constexpr uint32_t kLocBranch = 1u << 25;  // H, Rx, Ry, U
+constexpr uint32_t kLocPair3 = 1u << 26;   // pairs slots 0-2 and 1-3 (dimension 2)
+constexpr uint32_t kLocOp = 27;            // bits 27..31: UOp
+enum UOp : uint32_t {
+    UO_X_PAIR = 0, UO_X_SHFL, UO_Y_PAIR, UO_Y_SHFL, UO_H_PAIR, UO_H_SHFL, UO_RX_PAIR, UO_RX_SHFL, UO_RY_PAIR,
+    UO_RY_SHFL, UO_U_PAIR, UO_U_SHFL, UO_Z, UO_S, UO_SDG, UO_YPH, UO_RZ, UO_PHASE
 };
 
 // GateDesc.flip bits.
@@ -119,8 +149,9 @@ struct ExactSums {
 
 // One pass of a single-launch run over a tiny table (tiny_kernel): what PassArgs says per pass.
 struct TinyPass {
-    uint32_t g0, g1, nx, q1, q2, q3, keys_fixed, pad;
+    uint32_t g0, g1, nx, q1, q2, q3, keys_fixed, dn;
     unsigned long long grow_bound;
+    uint32_t dim[4];        // unit passes: bucket bits of the unit's dimensions (dim[3] unused)
 };
 
 struct PassArgs {
@@ -138,6 +169,9 @@ struct PassArgs {
     PruneBits prune;
     uint32_t q1, q2, q3;             // the cross-group qubits (kNoQubit when absent)
     unsigned long long grow_bound;   // groups the state can hold after the pass, at most
+    // unit passes (mapped tables): mapped bits in use after the pass, dimensions of a unit (2 or
+    // 3) and the bucket bit of each dimension
+    uint32_t dn, dims, dim[3];
 };
 
 }  // namespace sqc

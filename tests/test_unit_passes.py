@@ -1,0 +1,194 @@
+"""Unit passes over mapped tables, and their FP64 products on the integer pipes.
+
+CPU part: the product code (sparqc_gb300/csrc/sqc_dmul.cuh) compiled for the host gives the
+hardware's product for every operand pair it does not refuse, and refuses only pairs whose product
+is not a normal number by exponent or with an operand that is not a finite normal number or zero.
+GPU part: states at the edges of what a unit pass handles, bit for bit against the oracle.
+"""
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from oracle.sparse import SparseOracle
+from sparqc_gb300 import circuits, gates as G
+from test_oracle import assert_identical
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sparqc_gb300", "csrc")
+
+PROGRAM = r'''
+#include <cmath>
+#include <cstdio>
+#include <cstring>
+#include <random>
+#include "sqc_dmul.cuh"
+using namespace sqc;
+static uint64_t bits(double x) { uint64_t u; std::memcpy(&u, &x, 8); return u; }
+static double from(uint64_t u) { double x; std::memcpy(&x, &u, 8); return x; }
+int main() {
+    std::mt19937_64 r(7);
+    unsigned long long done = 0, refused = 0, bad = 0, wrong_refusal = 0;
+    auto mantissa = [&]() -> uint64_t {
+        uint64_t m = r() & 0xFFFFFFFFFFFFFULL;
+        switch (r() % 8) {
+        case 0: return 0;
+        case 1: return 0xFFFFFFFFFFFFFULL;
+        case 2: return m & ~0x3FFFFFFULL;              // few significant bits: exact products and ties
+        case 3: return 1ULL << (r() % 52);
+        case 4: return m & ~((1ULL << (r() % 52)) - 1);
+        default: return m;
+        }
+    };
+    for (int ci = 0; ci < 4000; ++ci) {
+        double c;
+        switch (ci % 5) {
+        case 0: c = std::cos(0.37 * ci); break;
+        case 1: c = std::ldexp(1.0, -(ci % 40)); break;
+        case 2: c = std::nextafter(1.0, 0.0) * ((ci & 8) ? -1 : 1); break;
+        case 3: c = ci % 7 ? std::sqrt(0.5) : 0.0; break;
+        default: c = from((r() & 0x8000000000000000ULL) | ((600 + r() % 500) << 52) | mantissa()); break;
+        }
+        const DCoef k = dcoef(bits(c));
+        if (!k.ok) {
+            const double a = std::fabs(c);
+            wrong_refusal += a <= 1.0 && a >= 0x1p-400;
+            continue;
+        }
+        for (int i = 0; i < 4000; ++i) {
+            uint64_t e = r() % 4 ? 963 + r() % 64 : r() % 2048;
+            uint64_t u = (r() & 0x8000000000000000ULL) | (e << 52) | mantissa();
+            if (r() % 16 == 0) u &= 0x8000000000000000ULL;
+            const double a = from(u), want = a * c;
+            const DUnpacked x = dunpack((uint32_t)(u >> 32), (uint32_t)u, k.min_exp);
+            if (x.slow) {
+                ++refused;
+                const int pe = (int)e + (int)((bits(c) >> 52) & 0x7FF) - 1023;   // product exponent, or one less
+                wrong_refusal += e > 0 && e < 2047 && pe >= 2;
+                continue;
+            }
+            uint32_t hi, lo;
+            dproduct(x, k.hi, k.lo, k.exp, (uint32_t)(bits(c) >> 32), &hi, &lo);
+            ++done;
+            bad += (((uint64_t)hi << 32) | lo) != bits(want);
+        }
+    }
+    std::printf("%llu %llu %llu %llu\n", done, refused, bad, wrong_refusal);
+    return 0;
+}
+'''
+
+
+def test_integer_products_equal_the_hardware(tmp_path):
+    src = tmp_path / "dmul.cpp"
+    src.write_text(PROGRAM)
+    exe = tmp_path / "dmul"
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-x", "c++", "-I", CSRC, str(src), "-o", str(exe)],
+                   check=True)
+    done, refused, bad, wrong = map(int, subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split())
+    assert bad == 0 and wrong == 0
+    assert done > 5_000_000 and refused > 10_000
+
+
+def _both(nq, gates, precision, init=None, **kw):
+    from sparqc_gb300.engine import State
+    st = State(nq, precision=precision, **kw)
+    o = SparseOracle(precision)
+    if init is not None:
+        st.set_state(*init)
+        o.set_state(*init)
+    st.apply(gates)
+    o.apply(gates)
+    got, want = st.state(sorted=True), o.state(sorted=True)
+    stats = st.stats()
+    st.close()
+    assert_identical(got, want)
+    assert stats["amp_updates"] == o.amp_updates
+    return got
+
+
+KINDS = ((G.Z, G.S, G.SDG, G.T, G.TDG, G.RZ, G.PHASE), (G.X, G.Y), (G.H, G.RX, G.RY, G.U))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("cross", [0, 3])
+@pytest.mark.parametrize("nq", [1, 4, 5, 6, 7, 8, 9, 12, 13])
+def test_small_registers(nq, cross, precision):
+    """Fewer mapped bits than a unit has dimensions, and the first sizes past the single launch."""
+    rng = circuits.SplitMix64(circuits.stream_seed("unit-small", nq, precision))
+    g = circuits.random_circuit(nq, nq, 150, min(3, nq - 1), rng, kinds=KINDS)
+    _both(nq, g, precision, max_cross_qubits=cross)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("seed", range(3))
+def test_loaded_states(seed, precision):
+    """States whose constant bits are set (the stored frame), with thin spans and with empty slots."""
+    rng = np.random.default_rng(seed)
+    nq, free = 40, [2, 3, 5, 11, 17, 18, 30, 39][:6 + seed]
+    sub = rng.choice(1 << len(free), 1 << (len(free) - seed), replace=False)
+    keys = np.full(sub.size, (1 << 4) | (1 << 20) | (1 << 33), np.uint64)
+    for i, q in enumerate(free):
+        keys |= ((sub >> i) & 1).astype(np.uint64) << np.uint64(q)
+    a = rng.standard_normal((2, keys.size))
+    g = circuits.random_circuit(nq, 12, 120, 2, circuits.SplitMix64(seed), prefix_h=False, kinds=KINDS)
+    _both(nq, g, precision, init=(keys, a[0], a[1]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+def test_thin_states_walk_the_list_and_leave_the_map(precision):
+    """Keys that spread over ever more qubits: few live buckets among the mapped ones, then more
+    mapped bits than the table holds (the state moves to a hashed table)."""
+    nq = 60
+    gs = [(G.H, q) for q in range(6)] + [(G.RX, 3, (), 0.3)]
+    for i, t in enumerate(range(6, 50)):
+        gs += [(G.X, t, (i % 6, (i + 1) % 6)[: 1 + i % 2]), (G.RZ, t, (i % 5,), 0.1 * i)]
+        if i % 9 == 4:
+            gs += [(G.RY, i % 6, (t,), 0.7), (G.H, t)]
+    _both(nq, G.gate_array(gs), precision)
+
+
+@pytest.mark.gpu
+def test_fp64_products_beyond_the_integer_path():
+    """Amplitudes and coefficients the integer products leave to the FP64 instruction: subnormal and
+    tiny values, zero and one as coefficients, next to ordinary ones."""
+    rng = np.random.default_rng(5)
+    n = 1 << 9
+    keys = np.arange(n, dtype=np.uint64)
+    scale = 10.0 ** rng.choice([0, -5, -150, -290, -300, -308, -320], (2, n))
+    a = rng.standard_normal((2, n)) * scale
+    a[:, rng.random(n) < 0.2] = 0.0
+    a[1, rng.random(n) < 0.2] = -0.0
+    tiny = [0.0, np.pi, 2 * np.pi, 1e-5, 1e-140, 1e-300, np.pi / 2, 1.234]
+    gs = []
+    for i, th in enumerate(tiny):
+        gs += [(G.RZ, i % 9, (), th), (G.PHASE, (i + 2) % 9, (), th), (G.T, i % 9)]
+    diag = G.gate_array(gs)
+    _both(9, diag, 64, init=(keys, a[0], a[1]))
+    big = a.copy()
+    big[0] += rng.standard_normal(n)   # every key survives the pruning of branching gates
+    gs += [(k, (i + 3 * j) % 9, (), th) for j, k in enumerate((G.RX, G.RY, G.U, G.H)) for i, th in enumerate(tiny)]
+    _both(9, G.gate_array(gs), 64, init=(keys, big[0], big[1]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+def test_measured_bits_keep_the_masks(precision):
+    """A measurement removes keys behind the passes' back: the presence masks follow it."""
+    from sparqc_gb300.engine import State
+    nq = 12
+    g = circuits.random_circuit(nq, 10, 120, 2, circuits.SplitMix64(3), kinds=KINDS)
+    st = State(nq, precision=precision)
+    st.apply(g)
+    for q in (1, 7):
+        st.measure(q, 0.4)
+    k, r, i = st.state(sorted=True)
+    st.apply(g)
+    o = SparseOracle(precision)
+    o.set_state(k, r, i)
+    o.apply(g)
+    assert_identical(st.state(sorted=True), o.state(sorted=True))
+    st.close()
