@@ -43,7 +43,7 @@ TableDev slice_table(unsigned char* base, unsigned long long nb, bool dbl) {
     t.amps = base + off;
     off += align256(nb * kSlots * (dbl ? 16 : 8));
     t.list = reinterpret_cast<unsigned*>(base + off);
-    t.mask = nb - 1;   // (map_on stays 0: the caller stores the circuit's map)
+    t.mask = nb - 1;   // the caller stores the circuit's map
     return t;
 }
 
@@ -54,7 +54,7 @@ unsigned long long slice_buckets(unsigned long long bound, double lf) {
 }
 
 const char* plan_circuit(uint32_t nq, const sqc_gate* gates, uint64_t n, uint32_t max_run, uint32_t max_nx,
-                         CircuitPlan* out) {
+                         uint32_t dims, CircuitPlan* out) {
     if (nq < 1 || nq > 64) return "qubit count must be 1..64";
     if (n && !gates) return "null gate array";
     CircuitPlan& c = *out;
@@ -65,6 +65,8 @@ const char* plan_circuit(uint32_t nq, const sqc_gate* gates, uint64_t n, uint32_
     p.kmask = ~0ULL;   // |0...0>: every bit known to be 0
     p.kval = 0;
     c.desc.reserve(n);
+    std::vector<unsigned long long> after;   // known key bits after each descriptor
+    after.reserve(n);
     for (uint64_t i = 0; i < n; ++i) {
         if (const char* why = check_gate(gates[i], nq)) return why;
         GateDesc d;
@@ -72,20 +74,26 @@ const char* plan_circuit(uint32_t nq, const sqc_gate* gates, uint64_t n, uint32_
         d.pad = p.credit;
         p.credit = 0;
         c.desc.push_back(d);
+        after.push_back(p.kmask);
     }
     c.end = p;
     split_passes(c.desc.data(), c.desc.size(), max_run, max_nx,
-                 [&](size_t g0, size_t g1, uint32_t nx, uint32_t q1, uint32_t q2, uint32_t, bool fixed) {
+                 [&](size_t g0, size_t g1, uint32_t nx, uint32_t q1, uint32_t q2, uint32_t q3, bool fixed) {
                      BPass b;
                      std::memset(&b, 0, sizeof b);
                      b.g0 = (uint32_t)g0;
                      b.g1 = (uint32_t)g1;
                      b.nx = (uint16_t)nx;
                      b.keys_fixed = fixed ? 1 : 0;
-                     b.q1 = (uint8_t)(nx >= 1 ? q1 : 0xFF);
-                     b.q2 = (uint8_t)(nx >= 2 ? q2 : 0xFF);
+                     // more bits than any slice maps: the circuit's slice can never be laid out
+                     if (c.map.extend(after[g1 - 1], nq)) {
+                         const uint32_t q[3] = {q1, q2, q3};
+                         uint32_t dim[3];
+                         encode_unit_pass(c.desc.data(), g0, g1, q, c.map, dims, dim);
+                         b.dn = (uint8_t)c.map.n;
+                         for (int i = 0; i < 3; ++i) b.dim[i] = (uint8_t)dim[i];
+                     }
                      c.passes.push_back(b);
-                     encode_pass(c.desc.data(), g0, g1, q1);
                  });
     if (c.passes.size() > kMaxBatchPasses) return "too many passes for a batch circuit";
     c.bound = group_bound(p, nq);
@@ -131,7 +139,7 @@ int Batch::init(const sqc_batch_options* opt) {
     idle_limit_ns_ = o.idle_limit_us ? 1000ULL * o.idle_limit_us : 2000000000ULL;
     if (o.threads_per_unit != 0 && o.threads_per_unit != 16 && o.threads_per_unit != 32)
         return fail(SQC_ERR_ARG, "threads_per_unit must be 0, 16 or 32");
-    max_nx_ = o.threads_per_unit == 16 ? 1u : 2u;
+    max_nx_ = o.threads_per_unit == 16 ? 1u : 3u;
     sched_ = o.schedule_gates != 0;
     use_graph_ = o.use_graph != 0;
     device_ = (int)o.device;
@@ -197,7 +205,8 @@ int Batch::plan_and_upload() {
     if ((rc = cuda(cudaStreamSynchronize(stream_), "sync"))) return rc;
     std::vector<CircuitPlan> plans(n);
     for (uint32_t i = 0; i < n; ++i) {
-        if (const char* why = plan_circuit(nqs_[i], gates_[i].data(), gates_[i].size(), kMaxRun, max_nx_, &plans[i]))
+        if (const char* why = plan_circuit(nqs_[i], gates_[i].data(), gates_[i].size(), kMaxRun,
+                                           std::min(max_nx_, batch_dims(dbl_)), batch_dims(dbl_), &plans[i]))
             return fail(SQC_ERR_ARG, "circuit " + std::to_string(i) + ": " + why);
     }
     plans_.swap(plans);
@@ -291,6 +300,7 @@ int Batch::layout() {
         const unsigned long long nb = nb_[i];
         TableDev& t = tables_[i];
         t = slice_table(pool_ + off, nb, dbl_);
+        plans_[i].map.store(&t);
         off += slice_bytes(nb, dbl_);
         // free every bucket of the slice (epoch 0 is never used)
         if ((rc = cuda(cudaMemsetAsync(t.hdr, 0, nb * sizeof(Header), stream_), "cudaMemset(hdr)"))) return rc;
@@ -323,8 +333,7 @@ BatchArgs Batch::args() const {
     a.n = (uint32_t)plans_.size();
     a.amp_bytes = dbl_ ? 16u : 8u;
     a.min_chunk = min_chunk_;
-    const unsigned long long warps = (unsigned long long)grid() * 8;
-    a.target_chunks = (uint32_t)std::min<unsigned long long>(kMaxChunks, std::max<unsigned long long>(4 * warps, 1));
+    a.target_chunks = (uint32_t)std::min<unsigned long long>(kMaxChunks, std::max<unsigned long long>(4ULL * grid(), 1));
     a.prune = prune_;
     a.idle_limit_ns = idle_limit_ns_;
     return a;
@@ -602,7 +611,7 @@ int Batch::autotune(sqc_batch_tuning* out) {
     uint32_t best_ch = ch0, best_bps = bps0, best_nx = nx0;
     uint32_t count = 1;
     const int res = std::max(batch_residency(dbl_, 0), batch_residency(dbl_, 2));
-    for (uint32_t nx : {2u, 1u}) {
+    for (uint32_t nx : {3u, 1u}) {
         if (nx != max_nx_) {
             max_nx_ = nx;
             if ((rc = plan_and_upload())) return rc;

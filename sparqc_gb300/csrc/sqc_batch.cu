@@ -1,36 +1,32 @@
 // Many-circuit batch: one persistent kernel runs the passes of every circuit of a batch.
 //
 // Every circuit has its own table slice, control block and gate descriptors, planned on the
-// host exactly as for a single state; the per-slot code (sqc_pass_dev.cuh) is the same, so a
-// circuit's result is bit-identical to running it alone. Scheduling is per circuit: pass p
-// is cut into chunks of list entries, and a warp takes chunk i of pass p with one atomicAdd
-// on the circuit's scheduling word (pass, chunks, issued). The warp that finishes the last
+// host exactly as for a single state; the unit code (sqc_unit.cuh) is the same, so a circuit's
+// result is bit-identical to running it alone (its map is known in advance). Scheduling is per
+// circuit: pass p is cut into chunks of units, and a block takes chunk i of pass p with one atomicAdd
+// on the circuit's scheduling word (pass, chunks, issued). The block that finishes the last
 // chunk of a pass publishes the pass (key count, list length, counters) and opens the next
 // one. Circuits never wait for each other, so short and long circuits share the GPU without
 // lockstep.
 //
 // This file is compiled with global loads defaulting to L2 (-dlcm=cg): a persistent kernel
 // reads, in pass p + 1, buckets that other SMs wrote in pass p, and L1 is not coherent.
-// Gate descriptors and the circuit array never change during a launch and are read through
-// the read-only path (plain non-coherent loads, without the pass kernels' L1 priority hint).
+// Gate descriptors and the circuit array never change during a launch.
 //
-// A warp that finds no work sleeps briefly and retries; after idle_limit_ns without work it
+// A block that finds no work sleeps briefly and retries; after idle_limit_ns without work it
 // records ST_TIMEOUT in the batch control block and returns (the limit is a batch option,
-// 2 s by default); every warp returns at its next check of that status. Parking: when the batch has a
+// 2 s by default); every block returns at its next check of that status. Parking: when the batch has a
 // deadline, a circuit whose pass ends after the deadline parks instead of opening its next
 // pass; a later launch resumes it (used by the serving loop to admit new circuits).
-#define SQC_DESC_EVICT_LAST 0
 #include "sqc_batch.h"
-#include "sqc_pass_dev.cuh"
+#include "sqc_unit.cuh"
 
 namespace sqc {
 namespace {
 
 constexpr int kBatchThreads = 256;
-// FP32 circuits read each pass's gates from a per-warp shared-memory copy (7% faster on the
-// 256-circuit batch); FP64 circuits read them in place (their registers are tighter: the copy
-// cost 4%).
-template <class T> struct BatchStage { static constexpr bool kOn = sizeof(T) == 4; };
+constexpr int kBatchWarps = kBatchThreads / 32;
+constexpr unsigned kBusyChunks = 64;
 constexpr unsigned kIdleSleepNs = 1000;                       // back-off of a warp that found no work
 
 __device__ __forceinline__ unsigned long long sched_word(unsigned long long pass, unsigned long long chunks) {
@@ -43,79 +39,64 @@ __device__ __forceinline__ unsigned long long globaltimer() {
     return t;
 }
 
-// Chunking of a pass over n list entries: entries per chunk (a multiple of 4, at least
-// min_chunk, large enough that the pass has at most target chunks) and the chunk count.
-__device__ __forceinline__ void chunking(unsigned long long n, unsigned min_chunk, unsigned target, unsigned* chunk,
+template <int DIMS>
+__device__ __forceinline__ UnitPass units_of(const BPass& p) {
+    return unit_pass<DIMS>(p.dn, p.dim[0], p.dim[1], p.dim[2]);
+}
+
+// Items of a pass: its units, or the list 32 entries at a time (walk_list).
+template <int DIMS>
+__device__ __forceinline__ unsigned long long pass_items(const BPass& p, unsigned long long list_n) {
+    if (walk_list(list_n, p.dn)) return (list_n + 31) / 32;
+    return units_of<DIMS>(p).units;
+}
+__device__ __forceinline__ unsigned long long pass_items(const BPass& p, unsigned long long list_n, bool dbl) {
+    return dbl ? pass_items<(int)kBatchDims64>(p, list_n) : pass_items<(int)kBatchDims32>(p, list_n);
+}
+
+// Chunking of a pass over n items while `running` circuits share the GPU: items per chunk and the
+// chunk count. A chunk gives every warp of its block at least min_chunk's list entries (four to an
+// item); a pass has at most target_chunks chunks shared among the running circuits, but up to
+// kBusyChunks, so that a large circuit's passes still spread when many run (256 circuits, FP32:
+// 10.7 ms with the smallest chunks for all, 7.3 with four times as many entries).
+__device__ __forceinline__ void chunking(const BatchArgs& a, unsigned long long n, unsigned running, unsigned* chunk,
                                          unsigned* total) {
+    const unsigned share = a.target_chunks / (running ? running : 1u);
+    const unsigned target = share > kBusyChunks ? share : kBusyChunks;
     unsigned long long c = (n + target - 1) / target;
-    c = (c + 3) & ~3ULL;
-    if (c < min_chunk) c = min_chunk;
+    const unsigned least = a.min_chunk / 4 * kBatchWarps;
+    if (c < least) c = least;
     *chunk = (unsigned)c;
     const unsigned long long t = (n + c - 1) / c;
     *total = (unsigned)(t ? t : 1);
 }
 
-// Stream pass over list entries [eb, ee): each warp step holds four entries (two per half).
-template <class T>
-__device__ __forceinline__ void stream_chunk(const TableDev& t, const GateDesc* gates, const SmemGate* sg, uint32_t g0,
-                                             uint32_t g1,
-                                             unsigned ep, Ctl* ctl, unsigned long long eb, unsigned long long ee,
-                                             const PruneBits& pb, unsigned long long& cnt_nnz,
-                                             unsigned long long& cnt_empty, unsigned long long& upd) {
-    const int lane = threadIdx.x & 31, half = lane >> 4, j = lane & 15;
-    Val<T> va, vb;
-    for (unsigned long long e0 = eb; e0 < ee; e0 += 4) {
-        const unsigned long long ea = e0 + 2 * half, ebb = ea + 1;
-        const long long ba = ea < ee ? (long long)t.list[ea] : -1;
-        const long long bb = ebb < ee ? (long long)t.list[ebb] : -1;
-        const unsigned long long Ga = ba >= 0 ? load_hdr(t.hdr + ba).group : 0ULL;
-        const unsigned long long Gb = bb >= 0 ? load_hdr(t.hdr + bb).group : 0ULL;
-        load_val_g<T>(t, va, Ga, ba, j);
-        load_val_g<T>(t, vb, Gb, bb, j);
-        if constexpr (BatchStage<T>::kOn) run_gates_s<T, false>(sg, gates, g0, g1, va, vb, lane, pb, upd);
-        else run_gates<T, false>(gates, g0, g1, va, vb, lane, pb, upd);
-        write_val<T>(t, ep, va, lane, &ctl->status, cnt_nnz, cnt_empty);
-        write_val<T>(t, ep, vb, lane, &ctl->status, cnt_nnz, cnt_empty);
-    }
-}
+// A chunk in hand: circuit, pass, chunk index, chunks of the pass.
+struct Claim {
+    unsigned c, p, i, total;
+};
 
-// Pass that pairs groups over list entries [eb, ee), four entries at a time (units4 and
-// run_units4 of sqc_pass_dev.cuh).
-template <class T, int NX>
-__device__ __forceinline__ void unit_chunk(const TableDev& t, const GateDesc* gates, const SmemGate* sg, uint32_t g0,
-                                           uint32_t g1,
-                                           uint32_t q1, uint32_t q2, unsigned ep, Ctl* ctl, unsigned long long eb,
-                                           unsigned long long ee, const PruneBits& pb, unsigned long long& cnt_nnz,
-                                           unsigned long long& cnt_empty, unsigned long long& upd) {
-    const int lane = threadIdx.x & 31;
-    const unsigned long long m1 = 1ULL << (q1 - kSlotBits);
-    const unsigned long long m2 = NX == 2 ? 1ULL << (q2 - kSlotBits) : 0ULL;
-    Val<T> va, vb;
-    for (unsigned long long e0 = eb; e0 < ee; e0 += 4) {
-        long long mb;
-        unsigned long long G0;
-        const unsigned om = units4<NX>(t, ep, e0, ee, m1, m2, lane, &mb, &G0);
-        run_units4<T, NX, false, BatchStage<T>::kOn>(t, ep, ctl, gates, sg, g0, g1, m1, m2, om, mb, G0, lane, pb, va,
-                                                     vb, cnt_nnz, cnt_empty, upd);
-    }
-}
-
-// Lane 0, after the last chunk of pass p of circuit c: publish the pass and open the next
-// one (or finish / park / fail the circuit).
-__device__ void finish_circuit_pass(const BatchArgs& a, unsigned c, const BCirc& C, unsigned p) {
+// One thread, after the last chunk of pass p of circuit c, with the pass's sums: publish the pass
+// and open the next one (or finish / park / fail the circuit). True when the next pass is open:
+// its chunk 0 is then *next's, without a search.
+__device__ __noinline__ bool finish_circuit_pass(const BatchArgs& a, unsigned c, unsigned p, unsigned long long tn,
+                                                 unsigned long long te, unsigned long long tu, Claim* next_claim) {
+    const BCirc& C = a.circ[c];
     Ctl* ctl = a.ctl + c;
     BSched* s = a.sched + c;
-    __threadfence();
-    const unsigned long long nnz_in = *(volatile unsigned long long*)&ctl->nnz;
-    const unsigned long long tn = atomicExch(&ctl->acc_nnz, 0ULL);
-    const unsigned long long te = atomicExch(&ctl->acc_empty, 0ULL);
-    const unsigned long long tu = atomicExch(&ctl->acc_upd, 0ULL);
+    const unsigned next = p + 1;
+    const unsigned npasses = C.npasses;
     const BPass bp = C.passes[p];
-    bool ok = *(volatile unsigned int*)&ctl->status == 0;
+    const BPass nxp = C.passes[next < npasses ? next : p];
+    const unsigned long long nnz_in = *(volatile unsigned long long*)&ctl->nnz;
+    const unsigned long long n = *(volatile unsigned long long*)&ctl->list_tail;
+    const unsigned long long dl = *(volatile unsigned long long*)&a.bctl->deadline_ns;
+    const unsigned limit = s->limit;
+    const bool ok = *(volatile unsigned int*)&ctl->status == 0;
     if (ok) {
         ctl->nnz = tn;
         ctl->empty_groups = te;
-        ctl->list_n = *(volatile unsigned long long*)&ctl->list_tail;
+        ctl->list_n = n;
         ctl->amp_updates += tu;
         const unsigned long long A = a.amp_bytes;
         const unsigned long long ab = bp.keys_fixed ? nnz_in * (8ULL + 2ULL * A) : (nnz_in + tn) * (8ULL + A);
@@ -123,131 +104,175 @@ __device__ void finish_circuit_pass(const BatchArgs& a, unsigned c, const BCirc&
         if (bp.nx) ctl->alg_bytes_pair += ab;
         ctl->seq += 1;
     }
-    const unsigned next = p + 1;
     unsigned state = BS_RUN;
     unsigned chunk = 0, total = 0;
     if (!ok) {
         state = BS_FAILED;
-    } else if (next >= C.npasses) {
+    } else if (next >= npasses) {
         state = BS_DONE;
+    } else if ((1ULL << nxp.dn) > C.max_groups) {   // the slice could overflow: stop before touching it
+        atomicCAS(&ctl->status, 0u, (unsigned)ST_GROW);
+        state = BS_FAILED;
     } else {
-        const unsigned long long n = ctl->list_n;
-        const BPass nxp = C.passes[next];
-        const unsigned long long grown = umin64(C.bound, n << nxp.nx);
-        if (nxp.nx && grown > C.max_groups) {   // the slice could overflow: stop before touching it
-            atomicCAS(&ctl->status, 0u, (unsigned)ST_GROW);
-            state = BS_FAILED;
-        } else {
-            chunking(n, a.min_chunk, a.target_chunks, &chunk, &total);
-            const unsigned long long dl = *(volatile unsigned long long*)&a.bctl->deadline_ns;
-            if (next >= s->limit || (dl && globaltimer() > dl)) state = BS_PARKED;
-        }
+        chunking(a, pass_items(nxp, n, a.amp_bytes == 16), *(volatile unsigned int*)&a.bctl->left, &chunk, &total);
+        if (next >= limit || (dl && globaltimer() > dl)) state = BS_PARKED;
     }
+    const bool run = state == BS_RUN;
     s->done = 0;
     s->chunk = chunk;
     s->next_total = total;
     s->state = state;
     __threadfence();
-    atomicExch(a.words + c, sched_word(next, state == BS_RUN ? total : 0));
-    if (state != BS_RUN) atomicSub(&a.bctl->left, 1u);
+    atomicExch(a.words + c, sched_word(next, run ? total : 0) + (run ? 1u : 0u));   // chunk 0 is taken
+    if (!run) atomicSub(&a.bctl->left, 1u);
     atomicAdd(&a.bctl->progress, 1ULL);
+    *next_claim = Claim{c, next, 0u, total};
+    return run;
 }
 
-// MINB: blocks per SM the register allocation is sized for (3: 80 registers with a few
-// spills; 2: no spills).
-template <class T, int MINB>
-__global__ void __launch_bounds__(kBatchThreads, MINB) batch_run_kernel(BatchArgs a) {
-    __shared__ SmemGate sgw[kBatchThreads / 32][BatchStage<T>::kOn ? kMaxRun : 1];
-    const int lane = threadIdx.x & 31;
-    const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    unsigned c = a.n ? warp % a.n : 0;
+// Warp 0 of a block: find a chunk, starting at circuit c: the lanes read the scheduling words of
+// 128 circuits at a time; the first one with a chunk left is tried with an atomicAdd by its lane.
+// Waits, with a pause between searches, until there is a chunk (true) or the launch is over.
+__device__ bool find_chunk(const BatchArgs& a, unsigned c, int lane, Claim* out) {
     unsigned long long idle_since = 0;
     while (true) {
-        if (*(volatile unsigned int*)&a.bctl->status) return;
-        if (*(volatile unsigned int*)&a.bctl->left == 0) return;
-        // look for a chunk, starting at the circuit this warp worked on last: the lanes read
-        // the scheduling words of 32 consecutive circuits at a time; the first one with a
-        // chunk left is tried with an atomicAdd by its lane
-        bool found = false;
-        unsigned fc = 0, fp = 0, fi = 0, ftot = 0;
-        for (unsigned base = 0; base < a.n && !found; base += 32) {
-            const unsigned i = base + lane;
-            const unsigned cc = i < a.n ? (c + i) % a.n : 0;
-            bool avail = false;
-            if (i < a.n) {
-                const unsigned long long w = *(volatile unsigned long long*)(a.words + cc);
-                avail = (w & kSchedFieldMask) < ((w >> kSchedFieldBits) & kSchedFieldMask);
+        const unsigned status = *(volatile unsigned int*)&a.bctl->status, left = *(volatile unsigned int*)&a.bctl->left;
+        for (unsigned base = 0; base < a.n; base += 128) {
+            unsigned long long w[4];
+            unsigned cc[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const unsigned i = base + 32 * k + lane;
+                cc[k] = i < a.n ? (c + i) % a.n : 0;
+                w[k] = i < a.n ? *(volatile unsigned long long*)(a.words + cc[k]) : 0ULL;   // 0: no chunks
             }
-            unsigned mask = __ballot_sync(kFull, avail);
-            while (mask && !found) {
-                const int l = __ffs(mask) - 1;
-                mask &= mask - 1;
-                unsigned ok = 0, op = 0, oi = 0, ot = 0;
-                if (lane == l) {
-                    const unsigned long long old = atomicAdd(a.words + cc, 1ULL);
-                    ot = (unsigned)((old >> kSchedFieldBits) & kSchedFieldMask);
-                    oi = (unsigned)(old & kSchedFieldMask);
-                    op = (unsigned)(old >> (2 * kSchedFieldBits));
-                    ok = oi < ot;
-                }
-                if (__shfl_sync(kFull, ok, l)) {
-                    found = true;
-                    fc = __shfl_sync(kFull, cc, l);
-                    fp = __shfl_sync(kFull, op, l);
-                    fi = __shfl_sync(kFull, oi, l);
-                    ftot = __shfl_sync(kFull, ot, l);
+            if (status || !left) return false;   // (read together with the first words)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                unsigned mask = __ballot_sync(kFull, (w[k] & kSchedFieldMask) < ((w[k] >> kSchedFieldBits) & kSchedFieldMask));
+                while (mask) {
+                    const int l = __ffs(mask) - 1;
+                    mask &= mask - 1;
+                    unsigned long long old = 0;
+                    if (lane == l) old = atomicAdd(a.words + cc[k], 1ULL);
+                    old = shfl64(old, l);
+                    const unsigned total = (unsigned)((old >> kSchedFieldBits) & kSchedFieldMask);
+                    const unsigned i = (unsigned)(old & kSchedFieldMask);
+                    if (i < total) {
+                        *out = Claim{__shfl_sync(kFull, cc[k], l), (unsigned)(old >> (2 * kSchedFieldBits)), i, total};
+                        return true;
+                    }
                 }
             }
         }
-        if (!found) {
+        if (status || !left) return false;
+        if (lane == 0) {
+            const unsigned long long now = globaltimer();
+            if (!idle_since) idle_since = now;
+            else if (now - idle_since > a.idle_limit_ns) atomicCAS(&a.bctl->status, 0u, (unsigned)ST_TIMEOUT);
+        }
+        __syncwarp();
+        __nanosleep(kIdleSleepNs);
+    }
+}
+
+// Blocks take chunks: the gates of a pass are staged once per block, its warps run the same code
+// (the instruction cache holds one pass's gates, not one per warp), and the bookkeeping of a chunk
+// -- claim, fence, completion -- is paid once for eight warps. A block whose chunk ends a pass goes
+// on with the next pass's chunk 0, so a circuit that fits one chunk runs like a tiny state, one
+// barrier between passes. (A warp per chunk of two units, each with its own staged copy: 128
+// circuits FP32 9.6 ms, 256 circuits FP64 35 ms.)
+// MINB: blocks per SM the register allocation is sized for.
+template <class T, int MINB>
+__global__ void __launch_bounds__(kBatchThreads, MINB) batch_run_kernel(BatchArgs a) {
+    constexpr int DIMS = (int)(sizeof(T) == 8 ? kBatchDims64 : kBatchDims32);
+    __shared__ UGates<T> sg;
+    __shared__ Claim claim;
+    __shared__ bool have;                      // claim holds a chunk taken with the last publication
+    __shared__ bool stop;
+    __shared__ unsigned long long sums[3];     // keys, empty buckets, amp updates of the chunk
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned last_c = a.n ? blockIdx.x % a.n : 0;
+    unsigned staged_c = ~0u, staged_p = 0;     // the pass in sg
+    if (threadIdx.x == 0) have = false;
+    __syncthreads();
+    while (true) {
+        if (w == 0 && !have) {
+            Claim got{0, 0, 0, 0};
+            const bool ok = find_chunk(a, last_c, lane, &got);
             if (lane == 0) {
-                const unsigned long long now = globaltimer();
-                if (!idle_since) idle_since = now;
-                else if (now - idle_since > a.idle_limit_ns) atomicCAS(&a.bctl->status, 0u, (unsigned)ST_TIMEOUT);
+                claim = got;
+                stop = !ok;
             }
-            __syncwarp();
-            __nanosleep(kIdleSleepNs);
-            continue;
+        } else if (threadIdx.x == 0) {
+            stop = *(volatile unsigned int*)&a.bctl->status != 0;
         }
-        idle_since = 0;
-        c = fc;
-        __threadfence();   // acquire: the previous pass of this circuit is visible
-        const BCirc C = a.circ[fc];
-        Ctl* ctl = a.ctl + fc;
-        const BPass bp = C.passes[fp];
+        if (threadIdx.x == 0) {
+            __threadfence();   // acquire: the previous pass of this circuit is visible
+            sums[0] = sums[1] = sums[2] = 0;
+        }
+        __syncthreads();
+        if (stop) return;
+        const Claim cl = claim;
+        last_c = cl.c;
+        const BCirc& C = a.circ[cl.c];
+        TableDev t;   // all but the map
+        t.hdr = C.t.hdr;
+        t.keys = C.t.keys;
+        t.amps = C.t.amps;
+        t.list = C.t.list;
+        t.map_n = C.t.map_n;
+        const GateDesc* cgates = C.gates;
+        Ctl* ctl = a.ctl + cl.c;
+        const BPass bp = C.passes[cl.p];
         const unsigned long long n = *(volatile unsigned long long*)&ctl->list_n;
-        const unsigned chunk = *(volatile unsigned int*)&a.sched[fc].chunk;
+        const unsigned chunk = *(volatile unsigned int*)&a.sched[cl.c].chunk;
         const unsigned ep = *(volatile unsigned int*)&ctl->epoch;
-        const unsigned long long eb = (unsigned long long)fi * chunk;
-        const unsigned long long ee = umin64(eb + chunk, n);
+        if (staged_c != cl.c || staged_p != cl.p) {   // (a circuit's descriptors do not change during a launch)
+            stage_ugates<T>(sg, cgates, bp.g0, bp.g1);
+            staged_c = cl.c;
+            staged_p = cl.p;
+        }
+        const unsigned long long ib = (unsigned long long)cl.i * chunk, ie = umin64(ib + chunk, pass_items<DIMS>(bp, n));
+        const UnitPass up = units_of<DIMS>(bp);
+        const GateDesc* gates = cgates + bp.g0;
+        const uint32_t ng = bp.g1 - bp.g0;
         unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
-        const unsigned cst = __shfl_sync(kFull, *(volatile unsigned int*)&ctl->status, 0);
-        if (eb < ee && cst == 0) {
-            // FP32: the pass's gates into this warp's shared-memory copy (they are read once per
-            // slot held, and loads default to L2 in this file); FP64 reads them in place
-            SmemGate* sg = BatchStage<T>::kOn ? sgw[threadIdx.x >> 5] : nullptr;
-            if constexpr (BatchStage<T>::kOn) stage_gates_warp(sg, C.gates, bp.g0, bp.g1, lane);
-            if (bp.nx == 1)
-                unit_chunk<T, 1>(C.t, C.gates, sg, bp.g0, bp.g1, bp.q1, kNoQubit, ep, ctl, eb, ee, a.prune, cnt_nnz,
-                                 cnt_empty, upd);
-            else if (bp.nx == 2)
-                unit_chunk<T, 2>(C.t, C.gates, sg, bp.g0, bp.g1, bp.q1, bp.q2, ep, ctl, eb, ee, a.prune, cnt_nnz,
-                                 cnt_empty, upd);
-            else
-                stream_chunk<T>(C.t, C.gates, sg, bp.g0, bp.g1, ep, ctl, eb, ee, a.prune, cnt_nnz, cnt_empty, upd);
+        if (walk_list(n, bp.dn)) {
+            for (unsigned long long i = ib + w; i < ie; i += kBatchWarps)
+                walk_entries<T, DIMS>(t, C.t.map_q, ctl, ep, up, i * 32, n, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+        } else {
+            walk_units<T, DIMS>(t, C.t.map_q, ctl, ep, up, ib + w, ie, kBatchWarps, sg, gates, ng, lane, a.prune, cnt_nnz,
+                             cnt_empty, upd);
         }
         cnt_nnz = warp_sum(cnt_nnz);
         cnt_empty = warp_sum(cnt_empty);
         upd = warp_sum(upd);
         if (lane == 0) {
-            if (cnt_nnz) atomicAdd(&ctl->acc_nnz, cnt_nnz);
-            if (cnt_empty) atomicAdd(&ctl->acc_empty, cnt_empty);
-            if (upd) atomicAdd(&ctl->acc_upd, upd);
-            __threadfence();   // release: this chunk's writes before its completion
-            const unsigned d = atomicAdd(&a.sched[fc].done, 1u);
-            if (d == ftot - 1) finish_circuit_pass(a, fc, C, fp);
+            if (cnt_nnz) atomicAdd(&sums[0], cnt_nnz);
+            if (cnt_empty) atomicAdd(&sums[1], cnt_empty);
+            if (upd) atomicAdd(&sums[2], upd);
         }
-        __syncwarp();
+        __syncthreads();   // the block's writes precede thread 0's fence
+        if (threadIdx.x == 0) {
+            unsigned long long tn = sums[0], te = sums[1], tu = sums[2];
+            bool last = cl.total == 1;
+            if (!last) {
+                if (tn) atomicAdd(&ctl->acc_nnz, tn);
+                if (te) atomicAdd(&ctl->acc_empty, te);
+                if (tu) atomicAdd(&ctl->acc_upd, tu);
+                __threadfence();   // release: this chunk's writes before its completion
+                last = atomicAdd(&a.sched[cl.c].done, 1u) == cl.total - 1;
+                if (last) {
+                    __threadfence();
+                    tn = atomicExch(&ctl->acc_nnz, 0ULL);
+                    te = atomicExch(&ctl->acc_empty, 0ULL);
+                    tu = atomicExch(&ctl->acc_upd, 0ULL);
+                }
+            }
+            have = last && finish_circuit_pass(a, cl.c, cl.p, tn, te, tu, &claim);
+        }
+        __syncthreads();
     }
 }
 
@@ -295,6 +320,7 @@ __global__ void batch_begin_kernel(BatchArgs a, unsigned long long deadline_ns) 
                 const size_t sl = (size_t)b * kSlots + lane;
                 C.t.keys[sl] = lane == 0 ? 0ULL : empty_key(lane);
                 if (lane == 0) {
+                    C.t.hdr[b].aux = 1u;   // presence mask: slot 0
                     if (a.amp_bytes == 16) reinterpret_cast<double2*>(C.t.amps)[sl] = make_double2(1.0, 0.0);
                     else reinterpret_cast<float2*>(C.t.amps)[sl] = make_float2(1.0f, 0.0f);
                 }
@@ -309,7 +335,7 @@ __global__ void batch_begin_kernel(BatchArgs a, unsigned long long deadline_ns) 
                 s->limit = lim;
                 s->done = 0;
                 unsigned chunk, total;
-                chunking(ctl->list_n, a.min_chunk, a.target_chunks, &chunk, &total);
+                chunking(a, C.npasses ? pass_items(C.passes[0], 1, a.amp_bytes == 16) : 1, a.n, &chunk, &total);
                 s->chunk = chunk;
                 s->next_total = total;
                 const bool run = b >= 0 && C.npasses > 0 && lim > 0;
@@ -345,19 +371,26 @@ __global__ void batch_begin_kernel(BatchArgs a, unsigned long long deadline_ns) 
 
 }  // namespace
 
+template <class T, int MINB>
+int batch_occupancy() {
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_run_kernel<T, MINB>, kBatchThreads, 0);
+    return n > 0 ? n : 1;
+}
+
+template <class T, int MINB>
+cudaError_t launch_run(const BatchArgs& a, int grid, cudaStream_t st) {
+    batch_run_kernel<T, MINB><<<grid, kBatchThreads, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
 // Blocks per SM that fit for the variant a launch of `blocks_per_sm` (0: most) would use.
 int batch_residency(bool dbl, int blocks_per_sm) {
     static int cache[2][2] = {{0, 0}, {0, 0}};
     const int v = blocks_per_sm == 0 || blocks_per_sm >= 3 ? 1 : 0;
     int& c = cache[dbl ? 1 : 0][v];
-    if (!c) {
-        int n = 0;
-        if (dbl && v) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_run_kernel<double, 3>, kBatchThreads, 0);
-        else if (dbl) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_run_kernel<double, 2>, kBatchThreads, 0);
-        else if (v) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_run_kernel<float, 3>, kBatchThreads, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_run_kernel<float, 2>, kBatchThreads, 0);
-        c = n > 0 ? n : 1;
-    }
+    if (!c) c = dbl ? (v ? batch_occupancy<double, 3>() : batch_occupancy<double, 2>())
+                    : (v ? batch_occupancy<float, 3>() : batch_occupancy<float, 2>());
     return c;
 }
 
@@ -365,14 +398,8 @@ cudaError_t launch_batch(const BatchArgs& a, bool dbl, int grid, int blocks_per_
                          cudaStream_t st) {
     batch_begin_kernel<<<1, 1024, 0, st>>>(a, deadline_ns);
     const bool v3 = blocks_per_sm == 0 || blocks_per_sm >= 3;
-    if (dbl) {
-        if (v3) batch_run_kernel<double, 3><<<grid, kBatchThreads, 0, st>>>(a);
-        else batch_run_kernel<double, 2><<<grid, kBatchThreads, 0, st>>>(a);
-    } else {
-        if (v3) batch_run_kernel<float, 3><<<grid, kBatchThreads, 0, st>>>(a);
-        else batch_run_kernel<float, 2><<<grid, kBatchThreads, 0, st>>>(a);
-    }
-    return cudaGetLastError();
+    if (dbl) return v3 ? launch_run<double, 3>(a, grid, st) : launch_run<double, 2>(a, grid, st);
+    return v3 ? launch_run<float, 3>(a, grid, st) : launch_run<float, 2>(a, grid, st);
 }
 
 }  // namespace sqc

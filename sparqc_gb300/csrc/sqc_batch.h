@@ -38,13 +38,18 @@ struct CircuitPlan {
     std::vector<GateDesc> desc;
     std::vector<BPass> passes;
     Planner end;                   // planner state after the last gate
+    GroupMap map;                  // group bits its table is mapped by
     unsigned long long bound = 1;  // groups the circuit can ever hold
     uint64_t n_gates = 0;
 };
 
 // Plan a circuit from |0...0>. Returns nullptr or the reason it cannot be batched.
+// max_nx: cross-group qubits of a pass at most; dims: dimensions of the batch kernel's units.
 const char* plan_circuit(uint32_t nq, const sqc_gate* gates, uint64_t n, uint32_t max_run, uint32_t max_nx,
-                         CircuitPlan* out);
+                         uint32_t dims, CircuitPlan* out);
+// Dimensions of the batch kernel's units: three in FP32, two in FP64 (whose slots are twice as large).
+constexpr uint32_t kBatchDims64 = 2, kBatchDims32 = 3;
+inline uint32_t batch_dims(bool dbl) { return dbl ? kBatchDims64 : kBatchDims32; }
 
 class Batch {
 public:

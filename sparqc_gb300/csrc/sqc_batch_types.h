@@ -3,7 +3,7 @@
 // A batch holds up to a few thousand independent circuits, each with its own table slice
 // (the single-state layout of sqc_device.cuh, sized from the circuit's group bound), its own
 // control block (Ctl) and gate descriptors. One persistent kernel runs every circuit's
-// passes: a circuit's pass is cut into chunks of list entries; any warp may take any chunk
+// passes: a circuit's pass is cut into chunks of units (sqc_unit.cuh); any warp may take any chunk
 // of any circuit, and the warp that finishes the last chunk of a pass publishes it and opens
 // the circuit's next pass. Circuits never wait for one another.
 #pragma once
@@ -16,10 +16,10 @@ namespace sqc {
 // One pass of a circuit: gates [g0, g1) of its descriptors.
 struct BPass {
     uint32_t g0, g1;
-    uint16_t nx;          // cross-group qubits: 0, 1 or 2
+    uint16_t nx;          // cross-group qubits: 0 to 3
     uint16_t keys_fixed;  // diagonal gates only
-    uint8_t q1, q2;       // the cross-group qubits (>= 4; unused ones 0xFF)
-    uint8_t pad[2];
+    uint8_t dn;           // mapped group bits after the pass (sqc_types.h, TableDev)
+    uint8_t dim[3];       // bucket bits of its units' dimensions (FP64 units have two)
 };
 
 // A circuit of the batch (read-only while the kernel runs).
@@ -44,7 +44,7 @@ enum BState : unsigned int { BS_IDLE = 0, BS_RUN = 1, BS_DONE = 2, BS_PARKED = 3
 
 struct alignas(32) BSched {
     unsigned int done;         // chunks finished in the current pass
-    unsigned int chunk;        // list entries per chunk in the current pass (a multiple of 4)
+    unsigned int chunk;        // items (units, or 32 list entries each) per chunk in the current pass
     unsigned int next_total;   // chunks of the pass a parked circuit resumes with
     unsigned int state;        // BState
     unsigned int limit;        // the circuit parks before starting this pass

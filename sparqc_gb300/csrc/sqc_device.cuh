@@ -85,10 +85,10 @@ __device__ __forceinline__ unsigned long long home_bucket(const TableDev& t, uns
     return b;
 }
 
-// Group of bucket b of a mapped table.
-__device__ __forceinline__ unsigned long long group_of_bucket(const TableDev& t, unsigned b) {
+// Group of bucket b of a mapped table (map_n bits, mq its map_q).
+__device__ __forceinline__ unsigned long long group_of_bucket(uint32_t map_n, const uint8_t* mq, unsigned b) {
     unsigned long long G = 0;
-    for (uint32_t i = 0; i < t.map_n; ++i) G |= (unsigned long long)((b >> i) & 1u) << t.map_q[i];
+    for (uint32_t i = 0; i < map_n; ++i) G |= (unsigned long long)((b >> i) & 1u) << mq[i];
     return G;
 }
 
@@ -172,40 +172,23 @@ __device__ __forceinline__ float neg(float x) {
 }
 
 // Gate descriptors are read-only for a whole launch and read by every warp for every slot it
-// holds, while the table streams through the same L1: the pass kernels mark descriptor loads
-// to stay in L1 (evict_last), so the table's traffic does not push them out to L2 between
-// uses. The persistent batch kernel, whose loads default to L2 only, keeps the plain
-// non-coherent loads (SQC_DESC_EVICT_LAST 0), which measured faster there.
-#ifndef SQC_DESC_EVICT_LAST
-#define SQC_DESC_EVICT_LAST 1
-#endif
+// holds, while the table streams through the same L1: descriptor loads are marked to stay in L1
+// (evict_last), so the table's traffic does not push them out to L2 between uses.
 __device__ __forceinline__ uint4 ld_desc4(const void* p) {
-#if SQC_DESC_EVICT_LAST
     uint4 v;
     asm("ld.global.nc.L1::evict_last.v4.u32 {%0, %1, %2, %3}, [%4];"
         : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
-#else
-    return __ldg(reinterpret_cast<const uint4*>(p));
-#endif
 }
 __device__ __forceinline__ double ld_desc(const double* p) {
-#if SQC_DESC_EVICT_LAST
     double v;
     asm("ld.global.nc.L1::evict_last.f64 %0, [%1];" : "=d"(v) : "l"(p));
     return v;
-#else
-    return __ldg(p);
-#endif
 }
 __device__ __forceinline__ float ld_desc(const float* p) {
-#if SQC_DESC_EVICT_LAST
     float v;
     asm("ld.global.nc.L1::evict_last.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
-#else
-    return __ldg(p);
-#endif
 }
 
 // Programmatic dependent launch. Direct passes are launched with programmatic stream
@@ -305,37 +288,6 @@ template <class T, uint32_t K>
 __device__ __forceinline__ Cx<T> swap_update(bool bit, Cx<T> b) {
     if constexpr (K == KX) return b;
     else return bit ? Cx<T>{neg(b.i), b.r} : Cx<T>{b.i, neg(b.r)};   // Y
-}
-
-// Kind parameter of the update templates meaning "the kind is only known at run time".
-constexpr uint32_t KANY = 0xFFu;
-
-// Run-time dispatch of the updates (one copy of each kind's code per call site).
-template <class T, class G>
-__device__ __forceinline__ Cx<T> branch_update_rt(uint32_t kind, const G& g, bool bit, Cx<T> a, Cx<T> b) {
-    switch (kind) {
-    case KH: return branch_update<T, KH>(g, bit, a, b);
-    case KRX: return branch_update<T, KRX>(g, bit, a, b);
-    case KRY: return branch_update<T, KRY>(g, bit, a, b);
-    default: return branch_update<T, KU>(g, bit, a, b);
-    }
-}
-
-template <class T, class G>
-__device__ __forceinline__ Cx<T> diag_update_rt(uint32_t kind, const G& g, bool bit, Cx<T> a) {
-    switch (kind) {
-    case KZ: return diag_update<T, KZ>(g, bit, a);
-    case KS: return diag_update<T, KS>(g, bit, a);
-    case KSDG: return diag_update<T, KSDG>(g, bit, a);
-    case KYPH: return diag_update<T, KYPH>(g, bit, a);
-    case KRZ: return diag_update<T, KRZ>(g, bit, a);
-    default: return diag_update<T, KPHASE>(g, bit, a);
-    }
-}
-
-template <class T>
-__device__ __forceinline__ Cx<T> swap_update_rt(uint32_t kind, bool bit, Cx<T> b) {
-    return kind == KX ? swap_update<T, KX>(bit, b) : swap_update<T, KY>(bit, b);
 }
 
 __host__ __device__ constexpr bool branch_kind(uint32_t k) { return k == KH || k == KRX || k == KRY || k == KU; }

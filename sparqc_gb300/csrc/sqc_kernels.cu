@@ -163,28 +163,6 @@ __global__ void refresh_masks_kernel(TableDev t, Ctl* ctl) {
     }
 }
 
-// Present keys and empty live buckets over the list, into ctl->acc_nnz / acc_empty (adds).
-__global__ void count_kernel(TableDev t, Ctl* ctl) {
-    const unsigned long long n = ctl->list_n;
-    unsigned long long c = 0, e = 0;
-    for (unsigned long long s0 = (unsigned long long)blockIdx.x * blockDim.x; s0 < n * kSlots;
-         s0 += (unsigned long long)gridDim.x * blockDim.x) {   // same trip count for the whole block
-        const unsigned long long s = s0 + threadIdx.x;
-        const int j = (int)(s & 15);
-        bool p = false;
-        if (s < n * kSlots) p = slot_present(t.keys[(size_t)t.list[s >> kSlotBits] * kSlots + j], j);
-        c += p;
-        const unsigned grp = __ballot_sync(kFull, p);
-        if (s < n * kSlots && j == 0 && ((grp >> (threadIdx.x & 16)) & 0xFFFFu) == 0) e += 1;
-    }
-    c = warp_sum(c);
-    e = warp_sum(e);
-    if ((threadIdx.x & 31) == 0) {
-        if (c) atomicAdd(&ctl->acc_nnz, c);
-        if (e) atomicAdd(&ctl->acc_empty, e);
-    }
-}
-
 // Compact the present entries whose stored key matches (key & smask) == sval into
 // (keys ^ frame, re, im). Each warp owns a contiguous range of list entries: it counts,
 // reserves its span with one atomic, then writes. Entries beyond cap are counted but not
@@ -412,11 +390,6 @@ cudaError_t launch_set_state(const unsigned long long* keys, const double* re, c
 
 cudaError_t launch_refresh_masks(const TableDev& t, Ctl* ctl, unsigned long long list_hint, int sms, cudaStream_t st) {
     refresh_masks_kernel<<<grid_for(list_hint, kThreads / 16, sms), kThreads, 0, st>>>(t, ctl);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_count(const TableDev& t, Ctl* ctl, unsigned long long list_hint, int sms, cudaStream_t st) {
-    count_kernel<<<grid_for(list_hint * kSlots + 1, kThreads, sms), kThreads, 0, st>>>(t, ctl);
     return cudaGetLastError();
 }
 

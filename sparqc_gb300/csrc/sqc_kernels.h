@@ -29,7 +29,6 @@ cudaError_t launch_set_state(const unsigned long long* keys, const double* re, c
                              int sms, cudaStream_t st);
 // Recompute the presence masks (Header.aux) of a mapped table's listed buckets from their keys.
 cudaError_t launch_refresh_masks(const TableDev& t, Ctl* ctl, unsigned long long list_hint, int sms, cudaStream_t st);
-cudaError_t launch_count(const TableDev& t, Ctl* ctl, unsigned long long list_hint, int sms, cudaStream_t st);
 // Readout of the present entries whose stored key k has (k & smask) == sval (all by default).
 cudaError_t launch_readout(const TableDev& t, Ctl* ctl, unsigned long long list_hint, unsigned long long frame,
                            bool dbl, unsigned long long* okeys, double* ore, double* oim, unsigned long long cap,

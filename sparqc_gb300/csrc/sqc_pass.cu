@@ -152,7 +152,7 @@ __device__ __forceinline__ void direct_work(const PassArgs& a, const SmemGate* s
             long long mb;
             unsigned long long G0;
             const unsigned om = units4<NX>(t, ep, e0, n, m1, m2, lane, &mb, &G0);
-            run_units4<T, NX, true, SMEM>(t, ep, ctl, a.gates, sg, a.g0, a.g1, m1, m2, om, mb, G0, lane, a.prune, va,
+            run_units4<T, NX, SMEM>(t, ep, ctl, a.gates, sg, a.g0, a.g1, m1, m2, om, mb, G0, lane, a.prune, va,
                                           vb, cnt_nnz, cnt_empty, upd);
         }
     }
@@ -218,9 +218,9 @@ __global__ void __launch_bounds__(kThreads, UnitOcc<T, DIMS>::kMin) unit_kernel(
     unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
     if (walk_list(n, a.dn)) {
         for (unsigned long long e0 = w * 32; e0 < n; e0 += nw * 32)
-            walk_entries<T, DIMS>(a.t, ctl, ep, up, e0, n, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+            walk_entries<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, e0, n, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
     } else {
-        walk_units<T, DIMS>(a.t, ctl, ep, up, w, up.units, nw, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+        walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, nw, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
     }
     finish_pass(ctl, cnt_nnz, cnt_empty, upd, nnz_in, a.keys_fixed != 0, a.nx > 0, a.amp_bytes);
 }
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kThreads) tiny_unit_kernel(PassArgs a, const T
         stage_ugates<T>(sg, a.gates, q.g0, q.g1);
         const UnitPass up = unit_pass<DIMS>(q.dn, q.dim[0], q.dim[1], q.dim[2]);
         unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
-        walk_units<T, DIMS>(a.t, ctl, ep, up, w, up.units, kThreads / 32, sg, a.gates + q.g0, q.g1 - q.g0, lane, a.prune,
+        walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, kThreads / 32, sg, a.gates + q.g0, q.g1 - q.g0, lane, a.prune,
                             cnt_nnz, cnt_empty, upd);
         cnt_nnz = warp_sum(cnt_nnz);
         cnt_empty = warp_sum(cnt_empty);

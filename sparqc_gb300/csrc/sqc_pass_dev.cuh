@@ -1,5 +1,4 @@
-// Per-slot device code of a gate pass, shared by the single-state passes (sqc_pass.cu) and
-// the many-circuit persistent kernel (sqc_batch.cu): a warp holds two slots per lane (two
+// Per-slot device code of a gate pass over a hashed table (sqc_pass.cu): a warp holds two slots per lane (two
 // buckets, or both groups of a pair), applies a run of gates in registers and writes the
 // slots back in place.
 #pragma once
@@ -100,11 +99,11 @@ __device__ __forceinline__ void shfl_step(const G& g, const GateHead& h, int off
     Cx<T> pa;
     pa.r = __shfl_xor_sync(kFull, v.amp.r, off);
     pa.i = __shfl_xor_sync(kFull, v.amp.i, off);
-    const bool swap = K == KANY ? (h.op & kOpSwap) != 0 : swap_kind(K);
+    const bool swap = swap_kind(K);
     bool pp = false;
     if (swap || NeedAny<T>::kOn) pp = __shfl_xor_sync(kFull, (int)v.pres, off) != 0;   // warp-uniform
     if (swap) {
-        const Cx<T> o = K == KANY ? swap_update_rt<T>(h.kind, bit, pa) : swap_update<T, K == KANY ? KX : K>(bit, pa);
+        const Cx<T> o = swap_update<T, swap_kind(K) ? K : KX>(bit, pa);
         if constexpr (SelectForm<T>::kOn) {
             v.amp = pick(sat, o, v.amp);
             v.pres = sat ? pp : v.pres;
@@ -117,8 +116,7 @@ __device__ __forceinline__ void shfl_step(const G& g, const GateHead& h, int off
     } else {
         const bool any = !NeedAny<T>::kOn || v.pres || pp;
         if (warp_needs<T>(sat && any)) {
-            const Cx<T> o = K == KANY ? branch_update_rt<T>(h.kind, g, bit, v.amp, pa)
-                                      : branch_update<T, K == KANY ? KH : K>(g, bit, v.amp, pa);
+            const Cx<T> o = branch_update<T, branch_kind(K) ? K : KH>(g, bit, v.amp, pa);
             if constexpr (SelectForm<T>::kOn) {
                 const bool keep = any && !negligible(o, pb);
                 v.amp = pick(sat, pick(keep, o, czero<T>()), v.amp);
@@ -138,11 +136,10 @@ __device__ __forceinline__ void shfl_step(const G& g, const GateHead& h, int off
 template <class T, uint32_t K, class G>
 __device__ __forceinline__ void diag_step(const G& g, const GateHead& h, Val<T>& v) {
     const bool bit = slot_bit(h, v.key);
-    const bool one_sided = K == KANY ? (h.op & kOpOneSided) != 0 : one_sided_kind(K);
+    const bool one_sided = one_sided_kind(K);
     const bool need = v.pres && (!one_sided || bit) && slot_sat(h, v.key);
     if (warp_needs<T>(need)) {
-        Cx<T> o = K == KANY ? diag_update_rt<T>(h.kind, g, bit, v.amp)
-                            : diag_update<T, K == KANY ? KZ : K>(g, bit, v.amp);
+        Cx<T> o = diag_update<T, K>(g, bit, v.amp);
         if constexpr (K == KS) {   // Sdg runs S's code: its result is S's negated (exact)
             if (h.kind == KSDG) o = Cx<T>{neg(o.r), neg(o.i)};
         }
@@ -163,11 +160,11 @@ __device__ __forceinline__ void pair_step(const G& g, const GateHead& h, Val<T>&
                                           const PruneBits& pb) {
     const bool sat = slot_sat(h, a.key);
     const bool bit_a = (h.op & kOpFlip) != 0, bit_b = !bit_a;
-    const bool swap = K == KANY ? (h.op & kOpSwap) != 0 : swap_kind(K);
-    constexpr uint32_t KS_ = K == KANY ? KX : K;
+    const bool swap = swap_kind(K);
+    constexpr uint32_t KS_ = swap_kind(K) ? K : KX;
     if (swap) {
-        const Cx<T> na = K == KANY ? swap_update_rt<T>(h.kind, bit_a, b.amp) : swap_update<T, KS_>(bit_a, b.amp);
-        const Cx<T> nb = K == KANY ? swap_update_rt<T>(h.kind, bit_b, a.amp) : swap_update<T, KS_>(bit_b, a.amp);
+        const Cx<T> na = swap_update<T, KS_>(bit_a, b.amp);
+        const Cx<T> nb = swap_update<T, KS_>(bit_b, a.amp);
         const bool pa = b.pres, pbr = a.pres;
         if constexpr (SelectForm<T>::kOn) {
             a.amp = pick(sat, na, a.amp);
@@ -184,11 +181,9 @@ __device__ __forceinline__ void pair_step(const G& g, const GateHead& h, Val<T>&
     } else {
         const bool any = !NeedAny<T>::kOn || a.pres || b.pres;
         if (warp_needs<T>(sat && any)) {
-            constexpr uint32_t KB_ = K == KANY ? KH : K;
-            const Cx<T> oa = K == KANY ? branch_update_rt<T>(h.kind, g, bit_a, a.amp, b.amp)
-                                       : branch_update<T, KB_>(g, bit_a, a.amp, b.amp);
-            const Cx<T> ob = K == KANY ? branch_update_rt<T>(h.kind, g, bit_b, b.amp, a.amp)
-                                       : branch_update<T, KB_>(g, bit_b, b.amp, a.amp);
+            constexpr uint32_t KB_ = branch_kind(K) ? K : KH;
+            const Cx<T> oa = branch_update<T, KB_>(g, bit_a, a.amp, b.amp);
+            const Cx<T> ob = branch_update<T, KB_>(g, bit_b, b.amp, a.amp);
             if constexpr (SelectForm<T>::kOn) {
                 const bool ka = any && !negligible(oa, pb), kb = any && !negligible(ob, pb);
                 a.amp = pick(sat, pick(ka, oa, czero<T>()), a.amp);
@@ -214,19 +209,7 @@ __device__ __forceinline__ void gate_on(const G& g, const GateHead& h, Val<T>& a
     // A shuffled gate targets a qubit below 4 (a bit of the slot index, shared by a and b) or
     // the quad's second cross-group qubit (whose bit a and b, one unit's groups in one half of
     // the warp, also share): its target bit is computed once for both slots.
-    if constexpr (K == KANY) {   // kind known at run time: category from the encoded op bits
-        if (h.op & kOpPair) {
-            pair_step<T, KANY>(g, h, a, b, pb);
-        } else if (h.op & kOpShfl) {
-            const int off = 1 << ((h.op >> kOpOffShift) & 7u);
-            const bool bit = slot_bit(h, a.key);
-            shfl_step<T, KANY>(g, h, off, bit, a, pb);
-            shfl_step<T, KANY>(g, h, off, bit, b, pb);
-        } else {
-            diag_step<T, KANY>(g, h, a);
-            diag_step<T, KANY>(g, h, b);
-        }
-    } else if constexpr (branch_kind(K) || swap_kind(K)) {
+    if constexpr (branch_kind(K) || swap_kind(K)) {
         if (h.op & kOpPair) {
             pair_step<T, K>(g, h, a, b, pb);
         } else {
@@ -241,18 +224,15 @@ __device__ __forceinline__ void gate_on(const G& g, const GateHead& h, Val<T>& a
     }
 }
 
-// Apply gates [g0, g1) to the two held slots. With SPEC each gate is dispatched once on its
-// (warp-uniform) kind to code specialised for that kind; without, its category is read from
-// the encoded op bits and the kind is switched on inside the arithmetic -- less code, for the
-// persistent batch kernel whose every pass type shares one instruction cache. Each gate is
-// applied as its pass encoded it:
+// Apply gates [g0, g1) to the two held slots. Each gate is dispatched once on its (warp-uniform)
+// kind to code specialised for that kind, and applied as its pass encoded it:
 // branching and swap gates on the pass's first cross-group qubit pair a with b (lane-local),
 // those on qubits 0..3 or on the second cross-group qubit pair each lane with lane ^ off (the
 // other half of the warp holds the groups with the second qubit's bit set), diagonal gates are
 // lane-local. Every lane accumulates the amp-update count of its own slots (the pass sums the
 // lanes): every gate is credited with the present slots it sees, and host-resolved gates
 // recorded in a descriptor's credit with the same count.
-template <class T, bool SPEC = true>
+template <class T>
 __device__ __forceinline__ void run_gates(const GateDesc* __restrict__ gates, uint32_t g0, uint32_t g1, Val<T>& a,
                                           Val<T>& b, int lane, const PruneBits& pb, unsigned long long& upd) {
     // present slots in the warp: only a branching gate changes the count (swap gates permute
@@ -265,10 +245,6 @@ __device__ __forceinline__ void run_gates(const GateDesc* __restrict__ gates, ui
         if (recount) n = (unsigned)a.pres + (unsigned)b.pres;
         recount = (h.op & kOpBranch) != 0;
         upd += (unsigned long long)n * (1ULL + h.credit);
-        if constexpr (!SPEC) {
-            gate_on<T, KANY>(g, h, a, b, pb);
-            continue;
-        }
         switch (h.kind) {
         case KX: gate_on<T, KX>(g, h, a, b, pb); break;
         case KY: gate_on<T, KY>(g, h, a, b, pb); break;
@@ -319,13 +295,6 @@ __device__ __forceinline__ void stage_gates(SmemGate* sg, const GateDesc* __rest
     __syncthreads();
 }
 
-// The same for one warp's own copy (every lane calls it; it ends with a warp barrier).
-__device__ __forceinline__ void stage_gates_warp(SmemGate* sg, const GateDesc* __restrict__ gates, uint32_t g0,
-                                                 uint32_t g1, int lane) {
-    for (uint32_t i = (uint32_t)lane; g0 + i < g1; i += 32) stage_gate(sg + i, gates + g0 + i);
-    __syncwarp();
-}
-
 template <class T> struct SmemPair;
 template <> struct SmemPair<double> {
     __device__ static __forceinline__ SmemCoef<double> of(const SmemGate& x, const GateDesc* g) {
@@ -339,7 +308,7 @@ template <> struct SmemPair<float> {
 };
 
 // run_gates with the pass's gates staged in shared memory (sg[i] is gate g0 + i).
-template <class T, bool SPEC = true>
+template <class T>
 __device__ __forceinline__ void run_gates_s(const SmemGate* sg, const GateDesc* __restrict__ gates, uint32_t g0,
                                             uint32_t g1, Val<T>& a, Val<T>& b, int lane, const PruneBits& pb,
                                             unsigned long long& upd) {
@@ -359,10 +328,6 @@ __device__ __forceinline__ void run_gates_s(const SmemGate* sg, const GateDesc* 
         if (recount) n = (unsigned)a.pres + (unsigned)b.pres;
         recount = (h.op & kOpBranch) != 0;
         upd += (unsigned long long)n * (1ULL + h.credit);
-        if constexpr (!SPEC) {
-            gate_on<T, KANY>(g, h, a, b, pb);
-            continue;
-        }
         switch (h.kind) {
         case KX: gate_on<T, KX>(g, h, a, b, pb); break;
         case KY: gate_on<T, KY>(g, h, a, b, pb); break;
@@ -380,35 +345,6 @@ __device__ __forceinline__ void run_gates_s(const SmemGate* sg, const GateDesc* 
         default: gate_on<T, KYPH>(g, h, a, b, pb); break;
         }
     }
-}
-
-// Ownership of the unit of list entry group G (bucket b) in a pass with nx cross-group qubits
-// (masks m1, m2, m3): the unit's members are G0 | i0*m1 | i1*m2 | i2*m3 (G0 = G with those bits
-// cleared); the owner is the member with the smallest index i0 + 2*i1 + 4*i2 among those live at
-// the start of the pass -- for a pair this is the reference's rule (the bit-0 key owns the pair unless it
-// is absent, emulator/device/device_table_FC.cuh:62-110) lifted to groups. Fills the members'
-// buckets (-1 when absent) and returns whether G owns its unit. Members a pass creates are
-// only ever created by the unit's owner, after its own check, so the lookups are consistent.
-template <int NX>
-__device__ __forceinline__ bool unit_owner(const TableDev& t, unsigned ep, unsigned long long G, long long b,
-                                           unsigned long long m1, unsigned long long m2, unsigned long long m3,
-                                           long long bk[8], unsigned long long* G0) {
-    constexpr int K = 1 << NX;
-    const int idx = ((G & m1) ? 1 : 0) | ((NX >= 2 && (G & m2)) ? 2 : 0) | ((NX == 3 && (G & m3)) ? 4 : 0);
-    *G0 = G & ~(m1 | (NX >= 2 ? m2 : 0ULL) | (NX == 3 ? m3 : 0ULL));
-    auto member = [&](int k) { return *G0 | ((k & 1) ? m1 : 0ULL) | ((k & 2) ? m2 : 0ULL) | ((k & 4) ? m3 : 0ULL); };
-#pragma unroll
-    for (int k = 0; k < 8; ++k) bk[k] = -1;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {   // a live member of smaller index owns the unit
-        if (k < idx && lookup_group(t, ep, member(k)) >= 0) return false;
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        if (k == idx) bk[k] = b;
-        else if (k > idx) bk[k] = lookup_group(t, ep, member(k));
-    }
-    return true;
 }
 
 // Write a held slot back in place. A group absent at the start of the pass gets a bucket
@@ -483,8 +419,10 @@ __device__ __forceinline__ void load_val_g(const TableDev& t, Val<T>& v, unsigne
 
 // Ownership of the units of the (up to) four list entries [e0, e0 + 4) ∩ [0, n) in one round
 // of lookups: with K = 2^NX members per unit (NX <= 3, masks m1, m2, m3), lane l < 4K looks up
-// member k = l % K of the unit of entry l / K. Returns the owner mask (bit e: entry e owns its unit, by unit_owner's
-// rule); afterwards lane e*K + k holds member k's bucket (*mb, -1 when absent) and lane e*K
+// member k = l % K of the unit of entry l / K. Returns the owner mask (bit e: entry e owns its unit: it
+// is the member with the smallest index among those live at the start of the pass -- for a pair this is the
+// reference's rule, emulator/device/device_table_FC.cuh:62-110, lifted to groups; members a pass creates are
+// only ever created by the unit's owner, after its own check, so the lookups are consistent); afterwards lane e*K + k holds member k's bucket (*mb, -1 when absent) and lane e*K
 // the unit's base group (*G0).
 template <int NX>
 __device__ __forceinline__ unsigned units4(const TableDev& t, unsigned ep, unsigned long long e0, unsigned long long n,
@@ -518,7 +456,7 @@ __device__ __forceinline__ unsigned units4(const TableDev& t, unsigned ep, unsig
 // Process the owned units of a units4 round: pairs two per warp step (one per half), quads one
 // per warp step (the half selects the q2 bit); each unit's groups are loaded straight from the
 // table, the gates applied (from shared memory with SMEM), and the slots written back.
-template <class T, int NX, bool SPEC = true, bool SMEM = false>
+template <class T, int NX, bool SMEM = false>
 __device__ __forceinline__ void run_units4(const TableDev& t, unsigned ep, Ctl* ctl, const GateDesc* gates,
                                            const SmemGate* sg, uint32_t g0,
                                            uint32_t g1, unsigned long long m1, unsigned long long m2, unsigned om,
@@ -551,8 +489,8 @@ __device__ __forceinline__ void run_units4(const TableDev& t, unsigned ep, Ctl* 
         const bool act = u >= 0;
         load_val_g<T>(t, va, Ga, act ? xa : -1, j);
         load_val_g<T>(t, vb, Ga | m1, act ? xb : -1, j);
-        if constexpr (SMEM) run_gates_s<T, SPEC>(sg, gates, g0, g1, va, vb, lane, pb, upd);   // gates in shared memory
-        else run_gates<T, SPEC>(gates, g0, g1, va, vb, lane, pb, upd);
+        if constexpr (SMEM) run_gates_s<T>(sg, gates, g0, g1, va, vb, lane, pb, upd);   // gates in shared memory
+        else run_gates<T>(gates, g0, g1, va, vb, lane, pb, upd);
         const long long fa = write_val<T>(t, ep, va, lane, &ctl->status, cnt_nnz, cnt_empty);
         const long long fb = write_val<T>(t, ep, vb, lane, &ctl->status, cnt_nnz, cnt_empty);
         append_new(t, ctl, fa, fb, lane);

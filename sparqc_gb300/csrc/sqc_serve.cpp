@@ -137,7 +137,7 @@ size_t Server::request_bytes(const Request& r) const {
 int Server::submit(const sqc_circuit_desc* c, uint64_t* id) {
     if (!c || !id) return fail(SQC_ERR_ARG, "null argument");
     Request r;
-    if (const char* why = plan_circuit(c->nq, c->gates, c->n_gates, kMaxRun, 2, &r.plan)) return fail(SQC_ERR_ARG, why);
+    if (const char* why = plan_circuit(c->nq, c->gates, c->n_gates, kMaxRun, batch_dims(dbl_), batch_dims(dbl_), &r.plan)) return fail(SQC_ERR_ARG, why);
     r.nb = slice_buckets(r.plan.bound, lf_);
     r.solo = r.plan.bound >= solo_min_groups_ && r.nb && solo_bytes(r) <= solo_cap_;
     // schedule_gates order, for the passes that will run the circuit: the single-state engine's
@@ -151,7 +151,7 @@ int Server::submit(const sqc_circuit_desc* c, uint64_t* id) {
         for (uint64_t j = 0; j < c->n_gates; ++j) sched[j] = c->gates[perm[j]];
         if (!r.solo) {
             r.plan = CircuitPlan();
-            if (const char* why = plan_circuit(c->nq, sched.data(), sched.size(), kMaxRun, 2, &r.plan))
+            if (const char* why = plan_circuit(c->nq, sched.data(), sched.size(), kMaxRun, batch_dims(dbl_), batch_dims(dbl_), &r.plan))
                 return fail(SQC_ERR_ARG, why);
         }
     }
@@ -259,6 +259,7 @@ int Server::admit() {
         r.bytes = bytes;
         unsigned char* base = pool_ + off;
         r.table = slice_table(base, r.nb, dbl_);
+        r.plan.map.store(&r.table);
         GateDesc* dd = reinterpret_cast<GateDesc*>(base + slice_bytes(r.nb, dbl_));
         BPass* dp = reinterpret_cast<BPass*>(reinterpret_cast<unsigned char*>(dd) +
                                              align256(r.plan.desc.size() * sizeof(GateDesc)));
@@ -302,8 +303,7 @@ BatchArgs Server::args(uint32_t n) const {
     a.n = n;
     a.amp_bytes = dbl_ ? 16u : 8u;
     a.min_chunk = min_chunk_;
-    const unsigned long long warps = (unsigned long long)sms_ * batch_residency(dbl_, 0) * 8;
-    a.target_chunks = (uint32_t)std::min<unsigned long long>(kMaxChunks, 4 * warps);
+    a.target_chunks = (uint32_t)std::min<unsigned long long>(kMaxChunks, 4ULL * sms_ * batch_residency(dbl_, 0));
     a.prune = prune_;
     a.idle_limit_ns = 2000000000ULL;   // a warp without work for 2 s ends the slice with ST_TIMEOUT
     return a;

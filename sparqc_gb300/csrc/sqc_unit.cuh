@@ -73,7 +73,7 @@ __device__ __forceinline__ void stage_ugate(UGate<double>* d, const GateDesc* g)
 // What a gate does on one lane, decoded once per pass: bits 0..3 the slots it acts on (its controls
 // on lane and slot bits hold), bits 4..7 the slots among them with logical target bit 1 (diagonal
 // gates; as if the target's bit of the unit's base were 0), bit 31 the logical target bit of the
-// lane (shuffles) or of the first slot of a pair.
+// lane (shuffles) or of the first slot of a pair. Kept as 16 bits, the top one sign-extended.
 __device__ __forceinline__ uint32_t lane_word(uint32_t loc, uint32_t lane) {
     const bool on = (((loc >> kLocLaneVal) ^ lane) & loc & 31u) == 0;
     const uint32_t tb = (loc >> kLocBit) & 31u;
@@ -83,10 +83,12 @@ __device__ __forceinline__ uint32_t lane_word(uint32_t loc, uint32_t lane) {
     return act | (e << 4) | (at != flip ? 0x80000000u : 0u);
 }
 
+__device__ __forceinline__ int16_t short_word(uint32_t w) { return (int16_t)((w & 0xFFu) | ((w >> 16) & 0x8000u)); }
+
 // The gates of a pass in shared memory: the gates, and their lane words.
 template <class T> struct UGates {
     UGate<T> g[kMaxRun];
-    uint32_t lw[kMaxRun][32];
+    int16_t lw[kMaxRun][32];
 };
 
 // Copy gates [g0, g1) (at most kMaxRun) into shared memory; every thread of the block calls it, and it
@@ -95,7 +97,7 @@ template <class T>
 __device__ __forceinline__ void stage_ugates(UGates<T>& sg, const GateDesc* __restrict__ gates, uint32_t g0, uint32_t g1) {
     for (uint32_t i = threadIdx.x; g0 + i < g1; i += blockDim.x) stage_ugate(sg.g + i, gates + g0 + i);
     for (uint32_t i = threadIdx.x; i < (g1 - g0) * 32u; i += blockDim.x)
-        sg.lw[i >> 5][i & 31u] = lane_word(__ldg(&gates[g0 + (i >> 5)].loc), i & 31u);
+        sg.lw[i >> 5][i & 31u] = short_word(lane_word(__ldg(&gates[g0 + (i >> 5)].loc), i & 31u));
     __syncthreads();
 }
 
@@ -349,7 +351,7 @@ __device__ __forceinline__ void run_unit(const UGates<T>& sg, const GateDesc* __
         const uint4 head = *reinterpret_cast<const uint4*>(&g);   // om, ov, loc, weight
         upd += (unsigned long long)n * head.w;
         if ((uid & head.x) != head.y) continue;   // a control outside the unit excludes all of it
-        const uint32_t w = sg.lw[gi][lane];
+        const uint32_t w = (uint32_t)(int)sg.lw[gi][lane];
         const uint32_t loc = head.z;
         const GateDesc* gd = gates + gi;
         touched = true;
@@ -415,10 +417,11 @@ __device__ __forceinline__ UnitPass unit_pass(uint32_t dn, uint32_t d0, uint32_t
     return p;
 }
 
+// (t's map is read through mq: a pass over many circuits leaves it in memory.)
 // One unit: load, apply the gates, write back. Absent buckets are created (header, keys, list
 // entry) when a key of theirs becomes present; the unit is this warp's alone, so plain stores do.
 template <class T, int DIMS>
-__device__ __forceinline__ void do_unit(const TableDev& t, Ctl* ctl, unsigned ep, const UnitPass& up, unsigned base,
+__device__ __forceinline__ void do_unit(const TableDev& t, const uint8_t* mq, Ctl* ctl, unsigned ep, const UnitPass& up, unsigned base,
                                         const UGates<T>& sg, const GateDesc* gates, uint32_t ng, int lane,
                                         const PruneBits& pb, unsigned long long& cnt_nnz, unsigned long long& cnt_empty,
                                         unsigned long long& upd) {
@@ -462,7 +465,7 @@ __device__ __forceinline__ void do_unit(const TableDev& t, Ctl* ctl, unsigned ep
             mk[s] = lane >= 16 ? bal >> 16 : bal & 0xFFFFu;
             const bool live = h[s].x == ep, make = !live && mk[s] != 0;
             if (live ? mk[s] != h[s].y : make) {
-                const unsigned long long G = group_of_bucket(t, bk[s]);
+                const unsigned long long G = group_of_bucket(t.map_n, mq, bk[s]);
                 const bool p = (pm >> s) & 1u;
                 if (make || p != (((pm0 >> s) & 1u) != 0))
                     t.keys[(size_t)bk[s] * kSlots + j] = p ? (G << kSlotBits) | (unsigned)j : empty_key(j);
@@ -495,13 +498,13 @@ __device__ __forceinline__ void do_unit(const TableDev& t, Ctl* ctl, unsigned ep
 
 // Units [u0, u1) step `stride` of a table whose live buckets fill it.
 template <class T, int DIMS>
-__device__ __forceinline__ void walk_units(const TableDev& t, Ctl* ctl, unsigned ep, const UnitPass& up,
+__device__ __forceinline__ void walk_units(const TableDev& t, const uint8_t* mq, Ctl* ctl, unsigned ep, const UnitPass& up,
                                            unsigned long long u0, unsigned long long u1, unsigned long long stride,
                                            const UGates<T>& sg, const GateDesc* gates, uint32_t ng, int lane,
                                            const PruneBits& pb, unsigned long long& cnt_nnz,
                                            unsigned long long& cnt_empty, unsigned long long& upd) {
     for (unsigned long long u = u0; u < u1; u += stride)
-        do_unit<T, DIMS>(t, ctl, ep, up, unit_base<DIMS>((unsigned)u, up.lo), sg, gates, ng, lane, pb, cnt_nnz, cnt_empty,
+        do_unit<T, DIMS>(t, mq, ctl, ep, up, unit_base<DIMS>((unsigned)u, up.lo), sg, gates, ng, lane, pb, cnt_nnz, cnt_empty,
                          upd);
 }
 
@@ -510,7 +513,7 @@ __device__ __forceinline__ void walk_units(const TableDev& t, Ctl* ctl, unsigned
 // (members a pass creates are made by the unit's owner, after its own check), found by reading
 // the headers of the smaller members.
 template <class T, int DIMS>
-__device__ __forceinline__ void walk_entries(const TableDev& t, Ctl* ctl, unsigned ep, const UnitPass& up,
+__device__ __forceinline__ void walk_entries(const TableDev& t, const uint8_t* mq, Ctl* ctl, unsigned ep, const UnitPass& up,
                                              unsigned long long e0, unsigned long long n, const UGates<T>& sg,
                                              const GateDesc* gates, uint32_t ng, int lane, const PruneBits& pb,
                                              unsigned long long& cnt_nnz, unsigned long long& cnt_empty,
@@ -539,7 +542,7 @@ __device__ __forceinline__ void walk_entries(const TableDev& t, Ctl* ctl, unsign
     while (todo) {
         const int l = __ffs(todo) - 1;
         todo &= todo - 1;
-        do_unit<T, DIMS>(t, ctl, ep, up, __shfl_sync(kFull, base, l), sg, gates, ng, lane, pb, cnt_nnz, cnt_empty, upd);
+        do_unit<T, DIMS>(t, mq, ctl, ep, up, __shfl_sync(kFull, base, l), sg, gates, ng, lane, pb, cnt_nnz, cnt_empty, upd);
     }
 }
 

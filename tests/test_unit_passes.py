@@ -192,3 +192,32 @@ def test_measured_bits_keep_the_masks(precision):
     o.apply(g)
     assert_identical(st.state(sorted=True), o.state(sorted=True))
     st.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+def test_batch_of_thin_and_tiny_circuits(precision):
+    """Circuits whose keys are few among their mapped bits (their passes walk the list), circuits
+    smaller than a unit, and one large enough for many chunks, in one launch."""
+    from sparqc_gb300.engine import Batch
+    thin = []
+    for n in (10, 14, 18):
+        gs = [(G.H, q) for q in range(5)] + [(G.X, 5 + i, (i % 5, (i + 2) % 5)[: 1 + i % 2]) for i in range(n)]
+        gs += [(G.RZ, 5 + i, (i % 5,), 0.3 + i) for i in range(0, n, 3)] + [(G.RY, 5 + n - 1, (1,), 0.4), (G.H, 2)]
+        thin.append((40, G.gate_array(gs)))
+    rng = circuits.SplitMix64(circuits.stream_seed("unit-batch", precision))
+    small = [(nq, circuits.random_circuit(nq, nq, 40, min(2, nq - 1), rng, kinds=KINDS)) for nq in (1, 3, 4, 5, 6, 7)]
+    big = [(20, circuits.random_circuit(20, 16, 120, 2, rng, kinds=KINDS))]
+    cs = thin + small + big
+    b = Batch(precision=precision)
+    b.prepare(cs)
+    b.run()
+    b.sync()
+    upd = 0
+    for i, (_, g) in enumerate(cs):
+        o = SparseOracle(precision)
+        o.apply(g)
+        assert_identical(b.state(i), o.state(sorted=True))
+        upd += o.amp_updates
+    assert b.stats()["amp_updates"] == upd
+    b.close()
