@@ -103,6 +103,7 @@ const char* plan_circuit(uint32_t nq, const sqc_gate* gates, uint64_t n, uint32_
 Batch::~Batch() {
     if (stream_) cudaStreamSynchronize(stream_);
     drop_graph();
+    rank_.release();
     for (void* p : {(void*)pool_, (void*)d_desc_, (void*)d_pass_, (void*)d_circ_, (void*)d_ctl_, (void*)d_sched_,
                     (void*)d_words_, (void*)d_cmd_, (void*)d_limit_, (void*)d_bctl_, (void*)d_rk_, (void*)d_rr_, (void*)d_ri_})
         if (p) cudaFree(p);
@@ -447,69 +448,40 @@ int Batch::get_states(uint64_t* keys, double* re, double* im, uint64_t cap, uint
     if (total) *total = off[nc];
     int rc;
     if ((rc = ensure_readout(off[nc]))) return rc;
-    // circuit i's readout lands at offset off[i] (its key count bounds what it writes)
+    // every circuit's entries, in key order, one circuit after the other
+    std::vector<RankJob> jobs(nc);
+    unsigned long long tiles = 0;
     for (size_t i = 0; i < nc; ++i) {
-        Ctl* ctl = d_ctl_ + i;
-        if ((rc = cuda(cudaMemsetAsync(&ctl->out_count, 0, sizeof(unsigned long long), stream_), "memset"))) return rc;
-        if (!h_ctl_[i].nnz) continue;
-        if ((rc = cuda(launch_readout(tables_[i], ctl, std::max<unsigned long long>(h_ctl_[i].list_n, 1),
-                                      plans_[i].end.frame, dbl_, d_rk_ + off[i], d_rr_ + off[i], d_ri_ + off[i],
-                                      h_ctl_[i].nnz, (flags & SQC_READ_DROP_NEGLIGIBLE) != 0, prune_, sms_, stream_),
-                       "readout")))
-            return rc;
-        ++launches_;
+        jobs[i] = rank_job(tables_[i], d_ctl_ + i, plans_[i].end.frame, 0, 0);
+        jobs[i].tile0 = tiles;
+        tiles += jobs[i].tiles();
     }
-    if ((rc = cuda(cudaMemcpyAsync(h_ctl_, d_ctl_, nc * sizeof(Ctl), cudaMemcpyDeviceToHost, stream_), "D2H ctl")) ||
-        (rc = cuda(cudaStreamSynchronize(stream_), "sync")))
-        return rc;
-    uint64_t got = 0;
-    for (size_t i = 0; i < nc; ++i) got += h_ctl_[i].out_count;
+    std::vector<unsigned long long> found(nc + 1, 0);
+    if (nc) {
+        if ((rc = cuda(rank_.need(tiles, nc), "cudaMalloc(readout)")) ||
+            (rc = cuda(cudaMemcpyAsync(rank_.jobs, jobs.data(), nc * sizeof(RankJob), cudaMemcpyHostToDevice, stream_),
+                       "H2D jobs")) ||
+            (rc = cuda(launch_ranked(jobs[0], rank_.jobs, (uint32_t)nc, tiles, rank_.tiles, dbl_, d_rk_, d_rr_, d_ri_, rcap_,
+                                     (flags & SQC_READ_DROP_NEGLIGIBLE) != 0, prune_, rank_.counts + nc, rank_.counts,
+                                     stream_),
+                       "readout")) ||
+            (rc = cuda(cudaMemcpyAsync(found.data(), rank_.counts, (nc + 1) * sizeof(unsigned long long),
+                                       cudaMemcpyDeviceToHost, stream_), "D2H counts")) ||
+            (rc = cuda(cudaStreamSynchronize(stream_), "sync")))
+            return rc;
+        launches_ += 3;
+    }
+    const uint64_t got = found[nc];
     if (total) *total = got;
     if (got > cap) return fail(SQC_ERR_CAPACITY, "output arrays too small");
     if (got && (!keys || !re || !im || !counts)) return fail(SQC_ERR_ARG, "null output array");
     if (!off[nc]) return SQC_OK;
-    // without dropping, the circuits' entries are already contiguous: one copy per array
-    const bool dense = got == off[nc];
-    if (dense) {
-        if ((rc = cuda(cudaMemcpyAsync(keys, d_rk_, got * 8, cudaMemcpyDeviceToHost, stream_), "D2H keys")) ||
-            (rc = cuda(cudaMemcpyAsync(re, d_rr_, got * 8, cudaMemcpyDeviceToHost, stream_), "D2H re")) ||
-            (rc = cuda(cudaMemcpyAsync(im, d_ri_, got * 8, cudaMemcpyDeviceToHost, stream_), "D2H im")))
-            return rc;
-    } else {
-        uint64_t at = 0;
-        for (size_t i = 0; i < nc; ++i) {
-            const uint64_t c = h_ctl_[i].out_count;
-            if (c && ((rc = cuda(cudaMemcpyAsync(keys + at, d_rk_ + off[i], c * 8, cudaMemcpyDeviceToHost, stream_),
-                                 "D2H keys")) ||
-                      (rc = cuda(cudaMemcpyAsync(re + at, d_rr_ + off[i], c * 8, cudaMemcpyDeviceToHost, stream_),
-                                 "D2H re")) ||
-                      (rc = cuda(cudaMemcpyAsync(im + at, d_ri_ + off[i], c * 8, cudaMemcpyDeviceToHost, stream_),
-                                 "D2H im"))))
-                return rc;
-            at += c;
-        }
-    }
-    if ((rc = cuda(cudaStreamSynchronize(stream_), "sync"))) return rc;
-    uint64_t at = 0;
-    for (size_t i = 0; i < nc; ++i) {
-        const uint64_t c = h_ctl_[i].out_count;
-        counts[i] = c;
-        if ((flags & SQC_READ_SORTED) && c > 1) {   // key order within each circuit
-            std::vector<uint64_t> idx(c);
-            std::iota(idx.begin(), idx.end(), 0);
-            uint64_t* k = keys + at;
-            double* r = re + at;
-            double* im_ = im + at;
-            std::sort(idx.begin(), idx.end(), [&](uint64_t a, uint64_t b) { return k[a] < k[b]; });
-            std::vector<uint64_t> k2(c);
-            std::vector<double> r2(c), i2(c);
-            for (uint64_t j = 0; j < c; ++j) { k2[j] = k[idx[j]]; r2[j] = r[idx[j]]; i2[j] = im_[idx[j]]; }
-            std::memcpy(k, k2.data(), c * 8);
-            std::memcpy(r, r2.data(), c * 8);
-            std::memcpy(im_, i2.data(), c * 8);
-        }
-        at += c;
-    }
+    if (got && ((rc = cuda(cudaMemcpyAsync(keys, d_rk_, got * 8, cudaMemcpyDeviceToHost, stream_), "D2H keys")) ||
+                (rc = cuda(cudaMemcpyAsync(re, d_rr_, got * 8, cudaMemcpyDeviceToHost, stream_), "D2H re")) ||
+                (rc = cuda(cudaMemcpyAsync(im, d_ri_, got * 8, cudaMemcpyDeviceToHost, stream_), "D2H im")) ||
+                (rc = cuda(cudaStreamSynchronize(stream_), "sync"))))
+        return rc;
+    for (size_t i = 0; i < nc; ++i) counts[i] = found[i];
     return SQC_OK;
 }
 
@@ -521,13 +493,13 @@ int Batch::get_state(uint32_t i, uint64_t* keys, double* re, double* im, uint64_
     const unsigned long long have = h_ctl_[i].nnz;
     if ((rc = ensure_readout(have))) return rc;
     Ctl* ctl = d_ctl_ + i;
-    if ((rc = cuda(cudaMemsetAsync(&ctl->out_count, 0, sizeof(unsigned long long), stream_), "memset"))) return rc;
-    if ((rc = cuda(launch_readout(tables_[i], ctl, std::max<unsigned long long>(h_ctl_[i].list_n, 1),
-                                  plans_[i].end.frame, dbl_, d_rk_, d_rr_, d_ri_, rcap_,
-                                  (flags & SQC_READ_DROP_NEGLIGIBLE) != 0, prune_, sms_, stream_),
+    const RankJob job = rank_job(tables_[i], ctl, plans_[i].end.frame, 0, 0);
+    if ((rc = cuda(rank_.need(job.tiles(), 0), "cudaMalloc(readout)")) ||
+        (rc = cuda(launch_ranked(job, nullptr, 1, job.tiles(), rank_.tiles, dbl_, d_rk_, d_rr_, d_ri_, rcap_,
+                                 (flags & SQC_READ_DROP_NEGLIGIBLE) != 0, prune_, &ctl->out_count, nullptr, stream_),
                    "readout")))
         return rc;
-    ++launches_;
+    launches_ += 3;
     unsigned long long got = 0;
     if ((rc = cuda(cudaMemcpyAsync(&got, &ctl->out_count, sizeof got, cudaMemcpyDeviceToHost, stream_), "D2H")) ||
         (rc = cuda(cudaStreamSynchronize(stream_), "sync")))
@@ -542,18 +514,7 @@ int Batch::get_state(uint32_t i, uint64_t* keys, double* re, double* im, uint64_
             (rc = cuda(cudaStreamSynchronize(stream_), "sync")))
             return rc;
     }
-    if ((flags & SQC_READ_SORTED) && got > 1) {
-        std::vector<uint64_t> idx(got);
-        std::iota(idx.begin(), idx.end(), 0);
-        std::sort(idx.begin(), idx.end(), [&](uint64_t a, uint64_t b) { return keys[a] < keys[b]; });
-        std::vector<uint64_t> k2(got);
-        std::vector<double> r2(got), i2(got);
-        for (uint64_t j = 0; j < got; ++j) { k2[j] = keys[idx[j]]; r2[j] = re[idx[j]]; i2[j] = im[idx[j]]; }
-        std::memcpy(keys, k2.data(), got * 8);
-        std::memcpy(re, r2.data(), got * 8);
-        std::memcpy(im, i2.data(), got * 8);
-    }
-    return SQC_OK;
+    return SQC_OK;   // in key order, asked for or not
 }
 
 int Batch::table_of(uint32_t i, TableDev* t, const Ctl** ctl, unsigned long long* hint, unsigned long long* frame,

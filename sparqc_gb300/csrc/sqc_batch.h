@@ -15,6 +15,7 @@
 #include "../../include/sparqc.h"
 #include "sqc_batch_types.h"
 #include "sqc_plan.h"
+#include "sqc_rank.h"
 
 namespace sqc {
 
@@ -133,6 +134,7 @@ private:
     double* d_rr_ = nullptr;
     double* d_ri_ = nullptr;
     size_t rcap_ = 0;
+    RankScratch rank_;             // key-ordered readout
 
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t graph_exec_ = nullptr;

@@ -18,7 +18,7 @@ namespace {
 constexpr unsigned long long kMinBuckets = 64;
 constexpr size_t kFlushAt = 1024;          // queued gates that trigger a launch
 constexpr unsigned long long kTinyMaxList = 256;   // live buckets up to which a flush is one launch
-constexpr size_t kDescInitial = 1 << 14;   // descriptors held between verified syncs
+constexpr size_t kDescInitial = 1 << 13;   // descriptors held between verified syncs
 constexpr unsigned long long kEpochRestart = 0xFFFFFF00ULL;   // epochs before the headers are cleared
 constexpr double kMaxLoad = 0.9;           // live buckets a pair pass may leave behind
 // A mapped table grows with the span of its keys, not with their number: past this many buckets
@@ -61,9 +61,10 @@ Engine::~Engine() {
     if (h_desc_) cudaFreeHost(h_desc_);
     if (d_tiny_) cudaFree(d_tiny_);
     if (h_tiny_) cudaFreeHost(h_tiny_);
-    if (d_rk_) cudaFree(d_rk_);
-    if (d_rr_) cudaFree(d_rr_);
-    if (d_ri_) cudaFree(d_ri_);
+    if (d_rk_) cudaFree(d_rk_);   // one allocation with d_rr_ and d_ri_
+    rank_.release();
+    if (d_cum_) cudaFree(d_cum_);
+    if (d_cum_tmp_) cudaFree(d_cum_tmp_);
     for (void* p : {(void*)sort_.keys_out, (void*)sort_.re_out, (void*)sort_.im_out, (void*)sort_.idx_in,
                     (void*)sort_.idx_out, (void*)sort_.cum, sort_.tmp})
         if (p) cudaFree(p);
@@ -178,12 +179,15 @@ int Engine::alloc_table(unsigned long long nb, HostTable* out) {
         return SQC_OK;
     }
     free_table(&spare_);   // of another size: its memory may be needed
-    if ((rc = cuda(cudaMalloc(&t.hdr, nb * sizeof(Header)), "cudaMalloc(hdr)")) ||
-        (rc = cuda(cudaMalloc(&t.keys, nb * kSlots * sizeof(unsigned long long)), "cudaMalloc(keys)")) ||
-        (rc = cuda(cudaMalloc(&t.amps, nb * kSlots * (dbl_ ? 16 : 8)), "cudaMalloc(amps)")) ||
-        (rc = cuda(cudaMalloc(&t.list, nb * sizeof(unsigned)), "cudaMalloc(list)")) ||
-        (rc = cuda(cudaMalloc(&t.units, nb * sizeof(Unit)), "cudaMalloc(units)")) ||
-        (rc = cuda(cudaMemsetAsync(t.hdr, 0, nb * sizeof(Header), stream_), "cudaMemset(hdr)"))) {
+    // one allocation: nb is at least 64, so every array starts on a 256-byte boundary
+    unsigned char* base = nullptr;
+    if ((rc = cuda(cudaMalloc(&base, nb * bucket_bytes()), "cudaMalloc(table)"))) return rc;
+    t.hdr = reinterpret_cast<Header*>(base);
+    t.keys = reinterpret_cast<unsigned long long*>(base += nb * sizeof(Header));
+    t.amps = base += nb * kSlots * sizeof(unsigned long long);
+    t.list = reinterpret_cast<unsigned*>(base += nb * kSlots * (dbl_ ? 16 : 8));
+    t.units = reinterpret_cast<Unit*>(base += nb * sizeof(unsigned));
+    if ((rc = cuda(cudaMemsetAsync(t.hdr, 0, nb * sizeof(Header), stream_), "cudaMemset(hdr)"))) {
         free_table(&t);
         return rc;
     }
@@ -192,11 +196,7 @@ int Engine::alloc_table(unsigned long long nb, HostTable* out) {
 }
 
 void Engine::free_table(HostTable* t) {
-    if (t->hdr) cudaFree(t->hdr);
-    if (t->keys) cudaFree(t->keys);
-    if (t->amps) cudaFree(t->amps);
-    if (t->list) cudaFree(t->list);
-    if (t->units) cudaFree(t->units);
+    if (t->hdr) cudaFree(t->hdr);   // the start of the table's one allocation
     *t = HostTable();
 }
 
@@ -244,14 +244,11 @@ int Engine::ensure_readout(size_t n) {
     }
     const size_t cap = std::max<size_t>(n, 1024);
     if (d_rk_) cudaFree(d_rk_);
-    if (d_rr_) cudaFree(d_rr_);
-    if (d_ri_) cudaFree(d_ri_);
     d_rk_ = nullptr; d_rr_ = nullptr; d_ri_ = nullptr; rcap_ = 0;
     int rc;
-    if ((rc = cuda(cudaMalloc(&d_rk_, cap * 8), "cudaMalloc(readout)")) ||
-        (rc = cuda(cudaMalloc(&d_rr_, cap * 8), "cudaMalloc(readout)")) ||
-        (rc = cuda(cudaMalloc(&d_ri_, cap * 8), "cudaMalloc(readout)")))
-        return rc;
+    if ((rc = cuda(cudaMalloc(&d_rk_, cap * 24), "cudaMalloc(readout)"))) return rc;
+    d_rr_ = reinterpret_cast<double*>(d_rk_ + cap);
+    d_ri_ = d_rr_ + cap;
     rcap_ = cap;
     return SQC_OK;
 }
@@ -948,13 +945,44 @@ int Engine::readout_wait() {
     return SQC_OK;
 }
 
+int Engine::ensure_cum(size_t n) {
+    if (n <= cum_cap_) return SQC_OK;
+    const size_t cap = std::max<size_t>(n, 1024);
+    if (d_cum_) cudaFree(d_cum_);
+    if (d_cum_tmp_) cudaFree(d_cum_tmp_);
+    d_cum_ = nullptr; d_cum_tmp_ = nullptr; cum_cap_ = 0;
+    cum_tmp_bytes_ = cumulate_scratch_bytes(cap);
+    int rc;
+    if ((rc = cuda(cudaMalloc(&d_cum_, cap * 8), "cudaMalloc(cumulative)")) ||
+        (rc = cuda(cudaMalloc(&d_cum_tmp_, cum_tmp_bytes_), "cudaMalloc(cumulative)")))
+        return rc;
+    cum_cap_ = cap;
+    return SQC_OK;
+}
+
 // Compact the present keys with (actual & mask) == value into the device readout arrays
 // (actual keys); *got receives their number (also when it exceeds the arrays).
-int Engine::readout_to_device(uint64_t mask, uint64_t value, bool drop_negl, unsigned long long* got, bool wait) {
+int Engine::readout_to_device(uint64_t mask, uint64_t value, bool drop_negl, unsigned long long* got, bool wait,
+                              bool* ordered) {
     int rc = sync();
     if (rc) return rc;
+    const bool ranked = mapped_ && rank_worth(map_.n, ctl_host_->nnz);
+    if (ordered) *ordered = ranked;
     if ((rc = ensure_readout(ctl_host_->nnz))) return rc;
     if ((rc = readout_buffers_free())) return rc;
+    if (ranked) {
+        const RankJob job = rank_job(dev(), ctl_, plan_.frame, mask, value ^ (plan_.frame & mask));
+        if ((rc = cuda(rank_.need(job.tiles(), 0), "cudaMalloc(tiles)")) ||
+            (rc = cuda(launch_ranked(job, nullptr, 1, job.tiles(), rank_.tiles, dbl_, d_rk_, d_rr_, d_ri_, rcap_, drop_negl,
+                                     prune_, &ctl_->out_count, nullptr, stream_),
+                       "ranked readout")))
+            return rc;
+        launches_ += 3;
+        if (!wait) return SQC_OK;
+        if ((rc = read_ctl())) return rc;
+        *got = ctl_host_->out_count;
+        return SQC_OK;
+    }
     if ((rc = cuda(cudaMemsetAsync(&ctl_->out_count, 0, sizeof(unsigned long long), stream_), "memset"))) return rc;
     if ((rc = cuda(launch_readout(dev(), ctl_, list_hint_, plan_.frame, dbl_, d_rk_, d_rr_, d_ri_, rcap_, drop_negl,
                                   prune_, sms_, stream_, mask, value ^ (plan_.frame & mask)),
@@ -974,7 +1002,8 @@ int Engine::get_state(uint64_t* keys, double* re, double* im, uint64_t cap, uint
 int Engine::get_state_where(uint64_t mask, uint64_t value, uint64_t* keys, double* re, double* im, uint64_t cap,
                             uint64_t* n, uint32_t flags) {
     unsigned long long got = 0;
-    int rc = readout_to_device(mask, value, (flags & SQC_READ_DROP_NEGLIGIBLE) != 0, &got);
+    bool ordered = false;
+    int rc = readout_to_device(mask, value, (flags & SQC_READ_DROP_NEGLIGIBLE) != 0, &got, true, &ordered);
     if (rc) return rc;
     if (n) *n = got;
     if (got > cap) return fail(SQC_ERR_CAPACITY, "output arrays too small");
@@ -983,7 +1012,7 @@ int Engine::get_state_where(uint64_t mask, uint64_t value, uint64_t* keys, doubl
     const unsigned long long* sk = d_rk_;
     const double* sr = d_rr_;
     const double* si = d_ri_;
-    if ((flags & SQC_READ_SORTED) && got > 1) {   // key sort on the device
+    if ((flags & SQC_READ_SORTED) && got > 1 && !ordered) {   // key sort on the device
         if ((rc = ensure_sort(got))) return rc;
         sort_.keys_in = d_rk_;
         sort_.re_in = d_rr_;
@@ -1097,22 +1126,34 @@ int Engine::measure(uint32_t qubit, double u, int* outcome, double* p1) {
 int Engine::sample(uint64_t shots, uint64_t seed, uint64_t* keys) {
     if (shots && !keys) return fail(SQC_ERR_ARG, "null output array");
     unsigned long long got = 0;
-    int rc = readout_to_device(0, 0, false, &got);
+    bool ordered = false;
+    int rc = readout_to_device(0, 0, false, &got, true, &ordered);
     if (rc) return rc;
     if (!shots) return SQC_OK;
     if (!got) return fail(SQC_ERR_STATE, "sampling an empty state");
-    if ((rc = ensure_sort(got))) return rc;
-    sort_.keys_in = d_rk_;
-    sort_.re_in = d_rr_;
-    sort_.im_in = d_ri_;
-    if ((rc = cuda(sort_entries(sort_, got, nq_, true, sms_, stream_), "sort"))) return rc;
+    const unsigned long long* keys_in_order = d_rk_;
+    const double* cum = nullptr;
+    if (ordered) {
+        if ((rc = ensure_cum(got)) ||
+            (rc = cuda(cumulate(d_rr_, d_ri_, d_cum_, got, d_cum_tmp_, cum_tmp_bytes_, sms_, stream_), "cumulate")))
+            return rc;
+        cum = d_cum_;
+    } else {
+        if ((rc = ensure_sort(got))) return rc;
+        sort_.keys_in = d_rk_;
+        sort_.re_in = d_rr_;
+        sort_.im_in = d_ri_;
+        if ((rc = cuda(sort_entries(sort_, got, nq_, true, sms_, stream_), "sort"))) return rc;
+        keys_in_order = sort_.keys_out;
+        cum = sort_.cum;
+    }
     unsigned long long* d_out = nullptr;
     if ((rc = cuda(cudaMallocAsync(&d_out, shots * 8, stream_), "cudaMallocAsync(samples)"))) return rc;
-    rc = cuda(launch_sample(sort_.keys_out, sort_.cum, got, seed, shots, d_out, sms_, stream_), "sample");
+    rc = cuda(launch_sample(keys_in_order, cum, got, seed, shots, d_out, sms_, stream_), "sample");
     if (!rc) rc = cuda(cudaMemcpyAsync(keys, d_out, shots * 8, cudaMemcpyDeviceToHost, stream_), "D2H samples");
     cudaFreeAsync(d_out, stream_);
     if (!rc) rc = cuda(cudaStreamSynchronize(stream_), "sync");
-    launches_ += 5;
+    launches_ += ordered ? 3 : 5;
     return rc;
 }
 

@@ -11,6 +11,7 @@
 #include "../../include/sparqc.h"
 #include "sqc_measure.h"
 #include "sqc_plan.h"
+#include "sqc_rank.h"
 #include "sqc_types.h"
 
 namespace sqc {
@@ -109,8 +110,11 @@ private:
     int ensure_readout(size_t n);
     int readout_buffers_free();   // later users of the readout buffers wait for the async copy
     int ensure_sort(size_t n);
-    // wait = false: only queue the readout (the count stays on the device)
-    int readout_to_device(uint64_t mask, uint64_t value, bool drop_negl, unsigned long long* got, bool wait = true);
+    int ensure_cum(size_t n);
+    // wait = false: only queue the readout (the count stays on the device). *ordered (if given):
+    // whether the entries are in key order (mapped tables)
+    int readout_to_device(uint64_t mask, uint64_t value, bool drop_negl, unsigned long long* got, bool wait = true,
+                          bool* ordered = nullptr);
     bool plan_gate(const sqc_gate& g, GateDesc* out);
     int read_ctl();
     int read_sums();   // copy the exact sums back and wait
@@ -174,6 +178,10 @@ private:
     size_t rcap_ = 0;
     SortBuffers sort_;            // device key sort of readouts (sorted readout, sampling)
     size_t sort_cap_ = 0;
+    RankScratch rank_;            // key-ordered readout of mapped tables
+    double* d_cum_ = nullptr;     // cumulative probabilities of a key-ordered readout, and scan scratch
+    void* d_cum_tmp_ = nullptr;
+    size_t cum_cap_ = 0, cum_tmp_bytes_ = 0;
 
     uint64_t gates_applied_ = 0, passes_run_ = 0, launches_ = 0, replays_ = 0, rebuilds_ = 0;
     uint64_t passes_pair_ = 0;

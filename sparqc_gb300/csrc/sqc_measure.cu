@@ -109,6 +109,15 @@ __global__ void gather_kernel(const unsigned* idx, const double* re_in, const do
     }
 }
 
+// |a|^2 per entry, as gather_kernel forms it.
+__global__ void prob_kernel(const double* re, const double* im, double* prob, unsigned long long n) {
+    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (unsigned long long)gridDim.x * blockDim.x) {
+        const double r = re[i], im_ = im[i];
+        prob[i] = __fma_rn(r, r, __dmul_rn(im_, im_));
+    }
+}
+
 __device__ __forceinline__ unsigned long long splitmix(unsigned long long x) {
     x += 0x9E3779B97F4A7C15ULL;
     x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ULL;
@@ -185,6 +194,19 @@ cudaError_t sort_entries(SortBuffers& sb, unsigned long long n, uint32_t key_bit
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
+}
+
+size_t cumulate_scratch_bytes(unsigned long long n) {
+    size_t b = 0;
+    cub::DeviceScan::InclusiveSum(nullptr, b, (const double*)nullptr, (double*)nullptr, (int)n);
+    return b + 256;
+}
+
+cudaError_t cumulate(const double* re, const double* im, double* cum, unsigned long long n, void* tmp, size_t tmp_bytes,
+                     int sms, cudaStream_t st) {
+    prob_kernel<<<grid_of(n, sms), 256, 0, st>>>(re, im, cum, n);
+    const cudaError_t e = cub::DeviceScan::InclusiveSum(tmp, tmp_bytes, cum, cum, (int)n, st);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_sample(const unsigned long long* keys, const double* cum, unsigned long long n,

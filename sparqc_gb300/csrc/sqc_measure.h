@@ -37,6 +37,10 @@ size_t sort_scratch_bytes(unsigned long long n);
 // Sort n readout entries by their low key_bits bits; with_cum also fills sb.cum.
 cudaError_t sort_entries(SortBuffers& sb, unsigned long long n, uint32_t key_bits, bool with_cum, int sms,
                          cudaStream_t st);
+// Inclusive cumulative |a|^2 of n entries in the order given, and its scratch bytes.
+size_t cumulate_scratch_bytes(unsigned long long n);
+cudaError_t cumulate(const double* re, const double* im, double* cum, unsigned long long n, void* tmp, size_t tmp_bytes,
+                     int sms, cudaStream_t st);
 // shots samples from key-sorted entries with inclusive cumulative probabilities cum.
 cudaError_t launch_sample(const unsigned long long* keys, const double* cum, unsigned long long n,
                           unsigned long long seed, unsigned long long shots, unsigned long long* out, int sms,

@@ -142,6 +142,7 @@ private:
     double* d_rr_ = nullptr;
     double* d_ri_ = nullptr;
     size_t rcap_ = 0;
+    RankScratch rank_;   // key-ordered readout
 
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, ev2_ = nullptr;
     std::vector<cudaEvent_t> solo_ev_;   // end of each large circuit's part of a step

@@ -221,3 +221,31 @@ def test_batch_of_thin_and_tiny_circuits(precision):
         upd += o.amp_updates
     assert b.stats()["amp_updates"] == upd
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("nq,k", [(3, 3), (5, 5), (16, 9), (30, 15), (64, 17)])
+def test_key_ordered_readout(nq, k, precision):
+    """Readouts of mapped tables come in key order without a sort: whole, by pattern (bits in and
+    outside the map, patterns nothing matches), without negligible entries, and sampled."""
+    from sparqc_gb300.engine import State
+    rng = circuits.SplitMix64(circuits.stream_seed("rank", nq, precision))
+    gs = circuits.random_circuit(nq, k, 60 + k, min(2, nq - 1), rng, kinds=KINDS)
+    gs = np.concatenate([gs, G.gate_array([(G.X, q) for q in range(0, nq, 2)])])   # a frame on every other bit
+    st, o = State(nq, precision=precision), SparseOracle(precision)
+    st.apply(gs)
+    o.apply(gs)
+    full = o.state(sorted=True)
+    assert_identical(st.state(sorted=True), full)
+    assert_identical(st.state(sorted=False), full)
+    top, low = 1 << (nq - 1), 1
+    key = int(full[0][full[0].size // 2])
+    for mask, value in ((low, low), (top, key & top), (top, ~key & top), (low | top, key & (low | top)), (2 % (1 << nq), 1),
+                        ((1 << nq) - 1, key), (6, key & 6)):
+        want = (full[0] & np.uint64(mask)) == np.uint64(value)
+        assert_identical(st.state_where(mask, value), tuple(x[want] for x in full))
+    keep = ~((np.abs(full[1]) < 1e-14) & (np.abs(full[2]) < 1e-14))
+    assert_identical(st.state(drop_negligible=True), tuple(x[keep] for x in full))
+    assert np.isin(st.sample(200, seed=3), full[0]).all()
+    st.close()
