@@ -29,6 +29,7 @@ constexpr unsigned long long kMapSpan = 16;
 // Buckets a grown mapped table has beyond its span: eight times as many while that is under a
 // gigabyte, so that a state growing one qubit at a time is not rebuilt at every one; then twice.
 constexpr unsigned long long kMapRoomy = 1ULL << 21;
+constexpr unsigned long long kHashRoomy = 1ULL << 17;   // 55 MB
 constexpr uint32_t kNoMap = 63;            // Span::dn of a pass whose bits no table maps: always refused
 
 bool map_worth(uint32_t dn, unsigned long long groups) {
@@ -266,6 +267,8 @@ int Engine::set_zero() {
     snap_log_ = 0;
     host_upd_ = 0;
     list_hint_ = 1;
+    key_hint_ = 1;
+    fresh_ = true;
     mapped_ = true;
     map_.clear();
     int rc;
@@ -345,6 +348,8 @@ int Engine::set_state(const uint64_t* keys, const double* re, const double* im, 
     snap_log_ = 0;
     host_upd_ = 0;
     list_hint_ = std::max<unsigned long long>(n, 1);
+    key_hint_ = std::max<unsigned long long>(n, 1);
+    fresh_ = false;
     map_.clear();
     mapped_ = map_.extend(plan_.kmask, nq_) && map_worth(map_.n, groups) && (1ULL << map_.n) <= max_groups();
     if ((rc = next_epoch())) return rc;
@@ -427,11 +432,12 @@ int Engine::flush(bool hold_last) {
         uint32_t nx, q1, q2, q3;
         bool fixed;
         uint32_t map0, dn, dim[3];   // mapped tables: mapped bits before and after, the units' dimensions
+        unsigned long long keys;     // keys after the pass, at most
     };
     std::vector<Span> spans;
     split_passes(hd, nd, max_run_, max_nx_,
                  [&](size_t g0, size_t g1, uint32_t nx, uint32_t q1, uint32_t q2, uint32_t q3, bool fixed) {
-                     spans.push_back(Span{g0, g1, nx, q1, q2, q3, fixed, 0, 0, {0, 0, 0}});
+                     spans.push_back(Span{g0, g1, nx, q1, q2, q3, fixed, 0, 0, {0, 0, 0}, 0});
                  });
     if (hold_last && spans.size() >= 2) {
         // the last pass's gates, and the host-resolved gates around them, go back to the queue;
@@ -447,6 +453,25 @@ int Engine::flush(bool hold_last) {
     // how each pass applies its gates: by place in its units (mapped tables; the map grows with
     // the bits its gates make differ) or by key (hashed ones)
     const uint32_t dims = dbl_ && max_nx_ < 3 ? 2u : 3u;
+    unsigned long long keys = key_hint_;   // a branching gate at most doubles them
+    for (Span& sp : spans) {
+        for (size_t i = sp.g0; i < sp.g1; ++i)
+            if (is_branch_kind(hd[i].kind)) keys = std::min(keys * 2, kKeysUnknown);
+        sp.keys = keys;
+    }
+    if (fresh_ && mapped_) {
+        // a state that will spread too thinly for any map starts hashed: |0...0> lies in bucket 0
+        // either way, so nothing moves
+        GroupMap m;
+        for (const Span& sp : spans) {
+            const bool fits = m.extend(after[sp.g1 - 1].kmask, nq_);
+            if (fits && ((1ULL << m.n) <= max_groups() || map_worth(m.n, sp.keys))) continue;
+            mapped_ = false;
+            a.t = dev();
+            break;
+        }
+    }
+    fresh_ = fresh_ && spans.empty();
     for (Span& sp : spans) {
         const uint32_t q[3] = {sp.q1, sp.q2, sp.q3};
         encode_pass(hd, sp.g0, sp.g1, sp.q1, sp.q3);
@@ -469,7 +494,8 @@ int Engine::flush(bool hold_last) {
     {
         unsigned long long h = list_hint_, hmax = list_hint_;
         for (const Span& sp : spans) {
-            if (sp.nx) h = std::min<unsigned long long>(tab_.nb, std::min(h << sp.nx, group_bound(after[sp.g1 - 1], nq_)));
+            if (sp.nx)
+                h = std::min<unsigned long long>({tab_.nb, h << sp.nx, h + sp.keys, group_bound(after[sp.g1 - 1], nq_)});
             hmax = std::max(hmax, h);
         }
         if (mapped_) {   // unit passes enumerate the mapped bits' span
@@ -493,6 +519,7 @@ int Engine::flush(bool hold_last) {
                 for (int i = 0; i < 3; ++i) q.dim[i] = sp.dim[i];
                 q.dim[3] = 0;
                 q.grow_bound = group_bound(after[sp.g1 - 1], nq_);
+                q.key_bound = sp.keys;
                 any_pair = any_pair || sp.nx > 0;
             }
             if ((rc = cuda(cudaMemcpyAsync(d_tiny_ + desc_used_, ht, spans.size() * sizeof(TinyPass),
@@ -508,13 +535,14 @@ int Engine::flush(bool hold_last) {
             }
             for (const Span& sp : spans) {
                 passes_pair_ += sp.nx > 0 ? 1 : 0;
-                passes_.push_back(PassRec{snap_log_, snap_plan_, sp.map0, sp.dn, sp.nx});
+                passes_.push_back(PassRec{snap_log_, snap_plan_, sp.map0, sp.dn, sp.nx, sp.keys});
                 snap_log_ = src[sp.g1 - 1] + 1;
                 snap_plan_ = after[sp.g1 - 1];
                 ++passes_run_;
             }
             ++launches_;
             list_hint_ = h;
+            key_hint_ = keys;
             desc_used_ += nd;
             return SQC_OK;
         }
@@ -529,13 +557,14 @@ int Engine::flush(bool hold_last) {
         a.q3 = sp.q3;
         a.keys_fixed = sp.fixed ? 1u : 0u;
         a.grow_bound = group_bound(after[i - 1], nq_);
-        if (!mapped_ && sp.nx && std::min(list_hint_ << sp.nx, a.grow_bound) > a.max_groups) {
-            if ((rc = make_room(sp.nx, a.grow_bound))) return rc;
+        a.key_bound = sp.keys;
+        if (!mapped_ && sp.nx && grown(sp.nx, a.grow_bound, sp.keys) > a.max_groups) {
+            if ((rc = make_room(sp.nx, a.grow_bound, sp.keys))) return rc;
             a.t = dev();
             a.max_groups = max_groups();
         }
-        if (sp.nx)
-            list_hint_ = std::min<unsigned long long>(tab_.nb, std::min(list_hint_ << sp.nx, a.grow_bound));
+        if (sp.nx) list_hint_ = std::min(tab_.nb, grown(sp.nx, a.grow_bound, sp.keys));
+        key_hint_ = sp.keys;
         a.dn = sp.dn;
         for (int d = 0; d < 3; ++d) a.dim[d] = sp.dim[d];
         const int nl = mapped_ ? launch_unit_pass(a, dbl_, sms_, stream_)
@@ -549,7 +578,7 @@ int Engine::flush(bool hold_last) {
             ev_prev = ev;
         }
         passes_pair_ += pair ? 1 : 0;
-        passes_.push_back(PassRec{snap_log_, snap_plan_, sp.map0, sp.dn, sp.nx});
+        passes_.push_back(PassRec{snap_log_, snap_plan_, sp.map0, sp.dn, sp.nx, sp.keys});
         snap_log_ = src[i - 1] + 1;
         snap_plan_ = after[i - 1];
         launches_ += (uint64_t)nl;
@@ -562,25 +591,36 @@ int Engine::flush(bool hold_last) {
     return SQC_OK;
 }
 
-// Buckets of a hashed table of `groups` groups: room for a pass with nx cross-group qubits, and
-// for several that empty as many groups as they make (keys that move leave their groups behind,
-// live and empty, until the table is rebuilt).
-unsigned long long Engine::hashed_size(unsigned long long groups, uint32_t nx) {
-    const double factor = std::max(8.0, (double)(1u << nx));
-    return std::max(kMinBuckets, pow2_at_least((unsigned long long)std::ceil(factor * (double)groups / kMaxLoad)));
+// Groups after a pass with nx cross-group qubits, at most: a unit has 2^nx groups, and a pass makes
+// no more groups than the state has keys after it.
+unsigned long long Engine::grown(uint32_t nx, unsigned long long bound, unsigned long long keys) const {
+    return std::min({bound, list_hint_ << nx, list_hint_ + keys});
+}
+
+// Buckets of a hashed table of `groups` groups: room for a pass, and for several that empty as many
+// groups as they make (keys that move leave their groups behind, live and empty, until the table is
+// rebuilt): eight times the groups, or every group the keys could make in four passes; small tables
+// far more, so that a short circuit needs no rebuild at all.
+unsigned long long Engine::hashed_size(unsigned long long groups, uint32_t nx, unsigned long long keys) {
+    const double room = std::max((double)groups * (double)std::max(8u, 1u << nx), 0.0);
+    const double by_keys = (double)groups + 4.0 * (double)keys;
+    const double one_pass = std::min((double)groups * (double)(1u << nx), (double)groups + (double)keys);
+    const double want = std::max(one_pass, std::min(room, by_keys));
+    const unsigned long long nb = std::max(kMinBuckets, pow2_at_least((unsigned long long)std::ceil(want / kMaxLoad)));
+    return std::max(nb, std::min(nb * 32, kHashRoomy));
 }
 
 // Before a pass that might not fit a hashed table by what the host knows: look at the exact list
 // length, and rebuild the table if the pass really might not fit. Waiting costs about 20 us; a pass
 // that refuses costs the launches of every pass queued behind it as well.
-int Engine::make_room(uint32_t nx, unsigned long long bound) {
+int Engine::make_room(uint32_t nx, unsigned long long bound, unsigned long long keys) {
     int rc;
     if ((rc = read_ctl())) return rc;
     if (ctl_host_->status != ST_OK) return SQC_OK;   // an earlier pass refused or failed: sync() deals with it
     list_hint_ = std::max<unsigned long long>(ctl_host_->list_n, 1);
-    if (std::min(list_hint_ << nx, bound) <= max_groups()) return SQC_OK;
+    if (grown(nx, bound, keys) <= max_groups()) return SQC_OK;
     const unsigned long long groups = ctl_host_->list_n - std::min(ctl_host_->list_n, ctl_host_->empty_groups);
-    const unsigned long long nb = std::max(tab_.nb, hashed_size(groups, nx));
+    const unsigned long long nb = std::max(tab_.nb, hashed_size(groups, nx, keys));
     if ((double)nb * bucket_bytes() > (double)budget_) return SQC_OK;   // the pass refuses; sync() decides
     if ((rc = rebuild(nb, false))) return rc;
     passes_.clear();   // all verified: later ones count from here
@@ -701,6 +741,7 @@ int Engine::sync() {
             snap_log_ = 0;
             snap_plan_ = plan_;
             list_hint_ = std::max<unsigned long long>(ctl_host_->list_n, 1);
+            key_hint_ = std::max<unsigned long long>(ctl_host_->nnz, 1);
             // many groups left without keys (pruned away): rebuild without them
             if (ctl_host_->list_n > 4096 && ctl_host_->empty_groups * 2 > ctl_host_->list_n) {
                 if ((rc = rebuild(tab_.nb, mapped_))) return rc;
@@ -768,6 +809,7 @@ int Engine::rebuild(unsigned long long nb_new, bool mapped) {
     mapped_ = mapped;
     seq_verified_ = 0;
     list_hint_ = std::max<unsigned long long>(ctl_host_->list_n, 1);
+    key_hint_ = std::max<unsigned long long>(ctl_host_->nnz, 1);
     ++rebuilds_;
     return SQC_OK;
 }
@@ -792,7 +834,7 @@ int Engine::repair(size_t k) {
         }
     }
     if (!mapped) {
-        nb = hashed_size(groups, pr.nx);
+        nb = hashed_size(groups, pr.nx, pr.keys);
         // a hashed table mostly of emptied groups has room once they are dropped; else it doubles
         if (!mapped_ && (nb > tab_.nb || groups * 2 > ctl_host_->list_n)) nb = std::max(nb, tab_.nb * 2);
         // near the budget, take the largest table that still fits (the pass may refuse again)
@@ -846,6 +888,7 @@ int Engine::take_unapplied(std::vector<sqc_gate>* rest) {
     desc_used_ = 0;
     seq_verified_ = ctl_host_->seq;
     list_hint_ = std::max<unsigned long long>(ctl_host_->list_n, 1);
+    key_hint_ = std::max<unsigned long long>(ctl_host_->nnz, 1);
     err.clear();
     return SQC_OK;
 }

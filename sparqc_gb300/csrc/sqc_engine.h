@@ -30,6 +30,7 @@ struct PassRec {
     Planner snap;       // ...with this planner state...
     uint32_t map_n;     // ...and this many mapped group bits
     uint32_t dn, nx;    // mapped bits the pass needs (0: hashed table) and its cross-group qubits
+    unsigned long long keys;   // keys the state can hold after it, at most
 };
 
 class Engine {
@@ -103,8 +104,10 @@ private:
     void free_table(HostTable* t);
     TableDev dev() const;
     int rebuild(unsigned long long nb_new, bool mapped);
-    int make_room(uint32_t nx, unsigned long long bound);   // hashed tables: room for the next pass
-    unsigned long long hashed_size(unsigned long long groups, uint32_t nx);
+    // hashed tables: groups after a pass, at most; buckets for a state; room for the next pass
+    unsigned long long grown(uint32_t nx, unsigned long long bound, unsigned long long keys) const;
+    unsigned long long hashed_size(unsigned long long groups, uint32_t nx, unsigned long long keys);
+    int make_room(uint32_t nx, unsigned long long bound, unsigned long long keys);
     int repair(size_t failed_pass);
     int ensure_desc(size_t n);
     int ensure_readout(size_t n);
@@ -155,6 +158,8 @@ private:
     ExactSums* sums_host_ = nullptr;  // pinned mirror
     unsigned long long seq_verified_ = 0;
     unsigned long long list_hint_ = 1;
+    unsigned long long key_hint_ = 1;   // keys the state holds after the launched passes, at most
+    bool fresh_ = true;                 // |0...0>, no pass launched yet
     PruneBits prune_{};
 
     Planner plan_;              // after every queued gate

@@ -85,7 +85,7 @@ __device__ void finish_pass(Ctl* ctl, unsigned long long n, unsigned long long e
 // registers.
 // True when a pass with nx cross-group qubits could leave more groups than the table takes.
 __device__ __forceinline__ bool could_overflow(const PassArgs& a, unsigned long long n) {
-    const unsigned long long grown = umin64(a.grow_bound, n << a.nx);
+    const unsigned long long grown = umin64(umin64(a.grow_bound, n << a.nx), n + a.key_bound);
     return grown > a.max_groups;
 }
 
@@ -303,6 +303,7 @@ __global__ void __launch_bounds__(kThreads) tiny_kernel(PassArgs a, const TinyPa
         b.q3 = q.q3;
         b.keys_fixed = q.keys_fixed;
         b.grow_bound = q.grow_bound;
+        b.key_bound = q.key_bound;
         const unsigned long long n = *(volatile unsigned long long*)&ctl->list_n;
         if (b.nx > 0 && could_overflow(b, n)) {   // refuse before touching the state
             if (threadIdx.x == 0) atomicCAS(&ctl->status, 0u, (unsigned)ST_GROW);

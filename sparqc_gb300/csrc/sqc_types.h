@@ -137,6 +137,7 @@ struct PruneBits {
 };
 
 constexpr uint32_t kNoQubit = 0xFFFFFFFFu;
+constexpr unsigned long long kKeysUnknown = 1ULL << 62;
 
 // Exact sums of products (sqc_exact.cuh): fixed-point numbers with their least significant bit
 // at 2^kSumLsb, kSumChunks 32-bit pieces each held in a 64-bit counter.
@@ -152,6 +153,7 @@ struct TinyPass {
     uint32_t g0, g1, nx, q1, q2, q3, keys_fixed, dn;
     unsigned long long grow_bound;
     uint32_t dim[4];        // unit passes: bucket bits of the unit's dimensions (dim[3] unused)
+    unsigned long long key_bound;
 };
 
 struct PassArgs {
@@ -164,11 +166,13 @@ struct PassArgs {
     uint32_t amp_bytes;     // 16 (FP64) or 8 (FP32)
     uint32_t credit;        // gates resolved on the host just before this pass (identity or
                             // relabel): each is credited with this pass's input key count
-    unsigned long long max_groups;   // a pass that pairs groups refuses to start when its groups
-                                     // could exceed this: min(grow_bound, n << nx) > max_groups
+    unsigned long long max_groups;   // a pass that pairs groups refuses to start when its groups could
+                                     // exceed this: min(grow_bound, n << nx, n + key_bound) > max_groups
     PruneBits prune;
     uint32_t q1, q2, q3;             // the cross-group qubits (kNoQubit when absent)
     unsigned long long grow_bound;   // groups the state can hold after the pass, at most
+    unsigned long long key_bound;    // keys it can hold after the pass, at most: a pass makes no more
+                                     // groups than that (hashed tables; at most kKeysUnknown)
     // unit passes (mapped tables): mapped bits in use after the pass, dimensions of a unit (2 or
     // 3) and the bucket bit of each dimension
     uint32_t dn, dims, dim[3];
