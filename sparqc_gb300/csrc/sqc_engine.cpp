@@ -33,7 +33,7 @@ constexpr unsigned long long kHashRoomy = 1ULL << 17;   // 55 MB
 constexpr uint32_t kNoMap = 63;            // Span::dn of a pass whose bits no table maps: always refused
 
 bool map_worth(uint32_t dn, unsigned long long groups) {
-    return dn < kNoMap && ((1ULL << dn) <= kMapFree || (1ULL << dn) <= kMapSpan * groups);
+    return dn < kNoMap && ((1ULL << dn) <= kMapFree || (1ULL << dn) / kMapSpan <= groups);   // (no overflow)
 }
 
 unsigned long long pow2_at_least(unsigned long long x) {
