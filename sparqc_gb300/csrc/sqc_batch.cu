@@ -240,9 +240,9 @@ __global__ void __launch_bounds__(kBatchThreads, MINB) batch_run_kernel(BatchArg
         unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
         if (walk_list(n, bp.dn)) {
             for (unsigned long long i = ib + w; i < ie; i += kBatchWarps)
-                walk_entries<T, DIMS>(t, C.t.map_q, ctl, ep, up, i * 32, n, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+                walk_entries<T, DIMS>(t, C.t.map_q, ctl, ep, up, i * 32, n, SharedHeads<T>{sg.g}, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
         } else {
-            walk_units<T, DIMS>(t, C.t.map_q, ctl, ep, up, ib + w, ie, kBatchWarps, sg, gates, ng, lane, a.prune, cnt_nnz,
+            walk_units<T, DIMS>(t, C.t.map_q, ctl, ep, up, (unsigned)(ib + w), (unsigned)ie, kBatchWarps, SharedHeads<T>{sg.g}, sg, gates, ng, lane, a.prune, cnt_nnz,
                              cnt_empty, upd);
         }
         cnt_nnz = warp_sum(cnt_nnz);

@@ -567,6 +567,8 @@ int Engine::flush(bool hold_last) {
         key_hint_ = sp.keys;
         a.dn = sp.dn;
         for (int d = 0; d < 3; ++d) a.dim[d] = sp.dim[d];
+        if (mapped_)
+            for (size_t k = sp.g0; k < sp.g1; ++k) a.heads[k - sp.g0] = UnitHead{hd[k].om, hd[k].ov, hd[k].loc, hd[k].pad + 1u};
         const int nl = mapped_ ? launch_unit_pass(a, dbl_, sms_, stream_)
                                : launch_pass(a, list_hint_, dbl_, sms_, stream_);
         if (nl < 0) return launch_failed("gate pass");

@@ -195,7 +195,7 @@ template <class T, int DIMS> struct UnitOcc {
 };
 
 template <class T, int DIMS>
-__global__ void __launch_bounds__(kThreads, UnitOcc<T, DIMS>::kMin) unit_kernel(PassArgs a) {
+__global__ void __launch_bounds__(kThreads, UnitOcc<T, DIMS>::kMin) unit_kernel(const __grid_constant__ PassArgs a) {
     __shared__ UGates<T> sg;
     stage_ugates<T>(sg, a.gates, a.g0, a.g1);   // no kernel writes the gates: staged while the previous pass drains
     wait_prior_grid();
@@ -211,16 +211,18 @@ __global__ void __launch_bounds__(kThreads, UnitOcc<T, DIMS>::kMin) unit_kernel(
     const unsigned long long nnz_in = ctl->nnz;
     const int lane = threadIdx.x & 31;
     const UnitPass up = unit_pass<DIMS>(a.dn, a.dim[0], a.dim[1], a.dim[2]);
-    const unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned long long nw = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+    // the warp's index as one value for the whole warp: unit addresses and control tests are then
+    // uniform, as the heads in the parameter bank are
+    const unsigned w = blockIdx.x * (kThreads / 32) + __shfl_sync(kFull, threadIdx.x >> 5, 0);
+    const unsigned nw = gridDim.x * (kThreads / 32);
     const uint32_t ng = a.g1 - a.g0;
     const GateDesc* gates = a.gates + a.g0;
     unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
     if (walk_list(n, a.dn)) {
-        for (unsigned long long e0 = w * 32; e0 < n; e0 += nw * 32)
-            walk_entries<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, e0, n, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+        for (unsigned long long e0 = w * 32ULL; e0 < n; e0 += nw * 32ULL)
+            walk_entries<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, e0, n, a.heads, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
     } else {
-        walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, nw, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+        walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, nw, a.heads, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
     }
     finish_pass(ctl, cnt_nnz, cnt_empty, upd, nnz_in, a.keys_fixed != 0, a.nx > 0, a.amp_bytes);
 }
@@ -244,7 +246,7 @@ __global__ void __launch_bounds__(kThreads) tiny_unit_kernel(PassArgs a, const T
         stage_ugates<T>(sg, a.gates, q.g0, q.g1);
         const UnitPass up = unit_pass<DIMS>(q.dn, q.dim[0], q.dim[1], q.dim[2]);
         unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
-        walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, kThreads / 32, sg, a.gates + q.g0, q.g1 - q.g0, lane, a.prune,
+        walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, kThreads / 32, SharedHeads<T>{sg.g}, sg, a.gates + q.g0, q.g1 - q.g0, lane, a.prune,
                             cnt_nnz, cnt_empty, upd);
         cnt_nnz = warp_sum(cnt_nnz);
         cnt_empty = warp_sum(cnt_empty);

@@ -180,9 +180,8 @@ void encode_unit_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[3], co
         const bool pair3 = pairs && slot_bit == 1;
         uint32_t slots = 0, bits = 0;
         for (uint32_t s = 0; s < 4; ++s) {
-            const uint32_t at = pair3 ? ((s & 1u) << 1) | (s >> 1) : s;   // the slot at place s of the exchanged order
-            if (((at ^ sval) & smask) == 0) slots |= 1u << s;
-            if ((slot_bit != kNoQubit && ((at >> slot_bit) & 1u)) != flip) bits |= 1u << s;
+            if (((s ^ sval) & smask) == 0) slots |= 1u << s;
+            if ((slot_bit != kNoQubit && ((s >> slot_bit) & 1u)) != flip) bits |= 1u << s;
         }
         uint32_t op;
         const uint32_t shfl = lane_bit != kNoQubit ? 1u : 0u;
@@ -200,10 +199,12 @@ void encode_unit_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[3], co
         case KRZ: op = UO_RZ; break;
         default: op = UO_PHASE; break;   // Phase, T, Tdg
         }
+        const bool all = pairs && !lmask && !smask;   // no controls inside the unit
+        if (pairs && (all || pair3)) op += all ? (pair3 ? UO_ALL3 : UO_ALL) : UO_PAIR3;
         const uint32_t tb = lane_bit != kNoQubit ? lane_bit : slot_bit != kNoQubit ? kMaxMapBits : outer;
         g.loc = lmask | (lval << kLocLaneVal) | (slots << kLocSlots) | (bits << kLocSlotBit) | (tb << kLocBit) |
-                (shfl ? kLocLane : 0u) | (flip ? kLocFlip : 0u) | (is_branch_kind(g.kind) ? kLocBranch : 0u) |
-                (pair3 ? kLocPair3 : 0u) | (op << kLocOp);
+                (shfl ? kLocLane : 0u) | (flip ? kLocFlip : 0u) |
+                (op << kLocOp);
     }
 }
 

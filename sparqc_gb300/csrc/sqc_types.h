@@ -103,20 +103,23 @@ struct alignas(16) GateDesc {
     uint32_t om, ov, loc, pad2;
 };
 
-// GateDesc.loc: what a unit pass does for the gate, by place in the unit. Slot fields are as seen
-// after the exchange of slots 1 and 2 that kLocPair3 asks for.
+// GateDesc.loc: what a unit pass does for the gate, by place in the unit.
 constexpr uint32_t kLocLaneVal = 5;        // bits 0..4: controlled lane bits (qubits 0..3, dimension 1), 5..9: their values
 constexpr uint32_t kLocSlots = 10;         // bits 10..13: slots whose controls (dimensions 0 and 2) hold
 constexpr uint32_t kLocSlotBit = 14;       // bits 14..17: diagonal gates: logical target bit per slot, before the next two
 constexpr uint32_t kLocBit = 18;           // bits 18..22: the target's bit of the lane index or of the unit's base (31: none)
 constexpr uint32_t kLocLane = 1u << 23;    // ... of the lane index
 constexpr uint32_t kLocFlip = 1u << 24;    // the stored frame flips the target bit (pairing gates)
-constexpr uint32_t kLocBranch = 1u << 25;  // H, Rx, Ry, U
-constexpr uint32_t kLocPair3 = 1u << 26;   // pairs slots 0-2 and 1-3 (dimension 2)
-constexpr uint32_t kLocOp = 27;            // bits 27..31: UOp
+constexpr uint32_t kLocOp = 26;            // bits 26..31: UOp
+// Pairing gates come as their controls inside the unit ask, on slots 0-1 and 2-3 or (UO_PAIR3) 0-2 and
+// 1-3, and, when they have none there (every lane and slot takes part), straight through (UO_ALL,
+// UO_ALL3).
 enum UOp : uint32_t {
     UO_X_PAIR = 0, UO_X_SHFL, UO_Y_PAIR, UO_Y_SHFL, UO_H_PAIR, UO_H_SHFL, UO_RX_PAIR, UO_RX_SHFL, UO_RY_PAIR,
-    UO_RY_SHFL, UO_U_PAIR, UO_U_SHFL, UO_Z, UO_S, UO_SDG, UO_YPH, UO_RZ, UO_PHASE
+    UO_RY_SHFL, UO_U_PAIR, UO_U_SHFL, UO_Z, UO_S, UO_SDG, UO_YPH, UO_RZ, UO_PHASE,
+    UO_ALL = 18,    // + 0..11: the forms above
+    UO_ALL3 = 30,   // + 0, 2, .., 10: UO_X_PAIR .. UO_U_PAIR on dimension 2
+    UO_PAIR3 = 31   // + 0, 2, .., 10: the same with controls inside the unit
 };
 
 // GateDesc.flip bits.
@@ -148,6 +151,11 @@ struct ExactSums {
     unsigned long long c[kSums][kSumChunks];
 };
 
+// Where a gate of a unit pass acts: GateDesc.om, ov, loc, and the amp updates a present key counts.
+struct alignas(16) UnitHead {
+    uint32_t om, ov, loc, weight;
+};
+
 // One pass of a single-launch run over a tiny table (tiny_kernel): what PassArgs says per pass.
 struct TinyPass {
     uint32_t g0, g1, nx, q1, q2, q3, keys_fixed, dn;
@@ -176,6 +184,7 @@ struct PassArgs {
     // unit passes (mapped tables): mapped bits in use after the pass, dimensions of a unit (2 or
     // 3) and the bucket bit of each dimension
     uint32_t dn, dims, dim[3];
+    UnitHead heads[kMaxRun];   // unit passes: those of the pass's gates (read from the parameter bank)
 };
 
 }  // namespace sqc

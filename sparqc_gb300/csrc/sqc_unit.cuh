@@ -61,7 +61,8 @@ __device__ __forceinline__ void stage_ugate(UGate<double>* d, const GateDesc* g)
     x.s = __ldg(&g->s);
     const DCoef c = dcoef((uint64_t)__double_as_longlong(x.c));
     const uint32_t op = x.loc >> kLocOp;
-    const bool two = op >= UO_RX_PAIR;   // H has one coefficient
+    const uint32_t form = op >= UO_ALL3 ? (op - UO_ALL3) & ~1u : op >= UO_ALL ? op - UO_ALL : op;
+    const bool two = form >= UO_RX_PAIR;   // H has one coefficient
     const DCoef s = dcoef((uint64_t)__double_as_longlong(two ? x.s : x.c));
     x.exact = c.ok && s.ok;
     x.ch = c.hi; x.cl = c.lo; x.ce = c.exp;
@@ -84,6 +85,15 @@ __device__ __forceinline__ uint32_t lane_word(uint32_t loc, uint32_t lane) {
 }
 
 __device__ __forceinline__ int16_t short_word(uint32_t w) { return (int16_t)((w & 0xFFu) | ((w >> 16) & 0x8000u)); }
+
+// A pass's heads read from its gates in shared memory.
+template <class T> struct SharedHeads {
+    const UGate<T>* g;
+    __device__ __forceinline__ UnitHead operator[](uint32_t i) const {
+        const uint4 h = *reinterpret_cast<const uint4*>(g + i);   // om, ov, loc, weight
+        return UnitHead{h.x, h.y, h.z, h.w};
+    }
+};
 
 // The gates of a pass in shared memory: the gates, and their lane words.
 template <class T> struct UGates {
@@ -129,14 +139,35 @@ __device__ __forceinline__ void products(const UGate<double>& g, Cx<double> x, C
         }
     }
 }
-template <bool TWO>
-__device__ __forceinline__ void products(const UGate<float>& g, Cx<float> x, Cx<float>& C, Cx<float>& P) {
-    C.r = __fmul_rn(g.c, x.r);
-    C.i = __fmul_rn(g.c, x.i);
-    if (TWO) {
-        P.r = __fmul_rn(g.s, x.r);
-        P.i = __fmul_rn(g.s, x.i);
-    }
+// FP32 arithmetic on an amplitude's two components at once (one instruction each; every component is
+// rounded as by the scalar instruction).
+__device__ __forceinline__ unsigned long long pack2(float r, float i) {
+    unsigned long long p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(r), "f"(i));
+    return p;
+}
+__device__ __forceinline__ unsigned long long pack2(Cx<float> v) { return pack2(v.r, v.i); }
+__device__ __forceinline__ Cx<float> unpack2(unsigned long long p) {
+    Cx<float> v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.r), "=f"(v.i) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// Sums of two products go through scalar additions: the assembler fuses a packed product into a
+// packed sum (found by comparing with the oracle), which rounds once instead of twice.
+__device__ __forceinline__ Cx<float> add_parts(unsigned long long a, unsigned long long b) {
+    const Cx<float> x = unpack2(a), y = unpack2(b);
+    return Cx<float>{__fadd_rn(x.r, y.r), __fadd_rn(x.i, y.i)};
 }
 
 // x with its sign flipped where m has bit 31 set. The xor is opaque: written in C++ the compiler
@@ -165,226 +196,366 @@ __device__ __forceinline__ Cx<T> shfl_cx(Cx<T> a, int off) {
     return Cx<T>{__shfl_xor_sync(kFull, a.r, off), __shfl_xor_sync(kFull, a.i, off)};
 }
 
-// U's fused multiply-add chain (branch_update), `uniform`: the own bit is the warp's. The bit-0 row's own coefficient is real: its imaginary terms add +-0, which changes
-// nothing unless the sum so far is itself 0.
-__device__ __forceinline__ float u_coef(const UGate<float>& g, const GateDesc*, int i) { return g.m[i]; }
-__device__ __forceinline__ double u_coef(const UGate<double>&, const GateDesc* gd, int i) { return __ldg(&gd->m[i]); }
-__device__ __forceinline__ bool is_zero(float x) { return x == 0.f; }
-__device__ __forceinline__ bool is_zero(double x) {   // no FP64 compare
-    return (((uint32_t)__double2hiint(x) & 0x7FFFFFFFu) | (uint32_t)__double2loint(x)) == 0;
-}
-template <class T>
-__device__ __forceinline__ Cx<T> u_update(const UGate<T>& g, const GateDesc* gd, bool bit, bool uniform, Cx<T> a,
-                                          Cx<T> b) {
-    using A = Arith<T>;
-    auto m = [&](int i) { return u_coef(g, gd, i); };
-    const T msr = bit ? m(6) : m(0), mor = bit ? m(4) : m(2), moi = bit ? m(5) : m(3);
-    T r = A::mul(msr, a.r), i = A::mul(msr, a.i);
-    if (!uniform || bit || is_zero(r) || is_zero(i)) {
-        const T msi = bit ? m(7) : m(1);
-        r = A::fma(neg(msi), a.i, r);
-        i = A::fma(msi, a.r, i);
-    }
-    return Cx<T>{A::fma(neg(moi), b.i, A::fma(mor, b.r, r)), A::fma(moi, b.r, A::fma(mor, b.i, i))};
-}
-
 // ---- one gate on the slots a lane holds ---------------------------------------------------------
 // Formulas and rounding are branch_update's, swap_update's and diag_update's (sqc_device.cuh): an
 // Rx, Ry, Rz or Phase result is C + P', C = c * own, P' the s-product of the own or the partner
 // amplitude with its sign flipped and its components exchanged as the kind asks (a - b and a + (-b),
-// and (-s) * x and -(s * x), round alike).
+// (-s) * x and -(s * x), and (-1) * a + b and b - a, round alike).
 template <class T, int S> struct Slots {
     Cx<T> v[S];
     unsigned pm;   // presence bits
+    unsigned n;    // their number
 };
 
-// Store branching results into slots (s the lane word's slots to change). Results below the prune
-// threshold are rare in the slots that hold keys: every result is stored as present, and the few
-// that are not kept are cleared on a branch.
-template <class T, int S>
-__device__ __forceinline__ void put(Slots<T, S>& x, int s, Cx<T> o, const PruneBits& pb) {
-    x.v[s] = o;
-    if (!kept(o, pb)) {
-        x.v[s] = czero<T>();
-        x.pm &= ~(1u << s);
+// Both results of a branching gate on a lane-local pair: a the slot whose logical target bit is w's
+// bit 31, b its partner.
+template <uint32_t K>
+__device__ __forceinline__ void pair_results(const UGate<float>& g, const GateDesc*, uint32_t w, Cx<float>& a, Cx<float>& b) {
+    const unsigned long long pa = pack2(a), pb = pack2(b);
+    if constexpr (K == KH) {   // logical bit 0: v0 + v1, bit 1: v0 - v1
+        const float one = __int_as_float(0x3F800000 | (int)(w & 0x80000000u));   // -1 where a has bit 1
+        const unsigned long long f = pack2(g.c, g.c);
+        a = unpack2(mul2(f, fma2(pa, pack2(one, one), pb)));
+        b = unpack2(mul2(f, fma2(pb, pack2(-one, -one), pa)));
+    } else if constexpr (K == KRX) {
+        const unsigned long long c = pack2(g.c, g.c), s = pack2(g.s, g.s);
+        const Cx<float> ca = unpack2(mul2(c, pa)), cb = unpack2(mul2(c, pb));
+        const Cx<float> sa = unpack2(mul2(s, pa)), sb = unpack2(mul2(s, pb));
+        a = Cx<float>{__fadd_rn(ca.r, sb.i), __fsub_rn(ca.i, sb.r)};
+        b = Cx<float>{__fadd_rn(cb.r, sa.i), __fsub_rn(cb.i, sa.r)};
+    } else if constexpr (K == KRY) {   // bit 0: c*own - s*partner, bit 1: c*own + s*partner
+        const float sa = flip_sign(g.s, ~w);
+        const unsigned long long c = pack2(g.c, g.c);
+        a = add_parts(mul2(c, pa), mul2(pack2(sa, sa), pb));
+        b = add_parts(mul2(c, pb), mul2(pack2(-sa, -sa), pa));
+    } else {   // U: fused multiply-add chains, the self terms first
+        const bool bit = (w >> 31) != 0;
+        const unsigned long long xa = pack2(a.i, a.r), xb = pack2(b.i, b.r);
+        const int own = bit ? 6 : 0, mix = bit ? 4 : 2;   // a's row; b's row is the other one
+        const float ar = g.m[own], ai = g.m[own + 1], br = g.m[6 - own], bi = g.m[7 - own];
+        const float amr = g.m[mix], ami = g.m[mix + 1], bmr = g.m[6 - mix], bmi = g.m[7 - mix];
+        unsigned long long oa = mul2(pack2(ar, ar), pa), ob = mul2(pack2(br, br), pb);
+        oa = fma2(pack2(-ai, ai), xa, oa);
+        ob = fma2(pack2(-bi, bi), xb, ob);
+        oa = fma2(pack2(amr, amr), pb, oa);
+        ob = fma2(pack2(bmr, bmr), pa, ob);
+        a = unpack2(fma2(pack2(-ami, ami), xb, oa));
+        b = unpack2(fma2(pack2(-bmi, bmi), xa, ob));
     }
 }
 
-template <class T, uint32_t K, int S>
+__device__ __forceinline__ bool is_zero(double x) {   // no FP64 compare
+    return (((uint32_t)__double2hiint(x) & 0x7FFFFFFFu) | (uint32_t)__double2loint(x)) == 0;
+}
+// U's chain for one member. `uniform`: its logical bit is the whole warp's; the bit-0 row's own
+// coefficient is real, and its imaginary terms add +-0, which changes nothing unless the sum so far
+// is itself 0: two of the chain's eight FP64 instructions are spared.
+__device__ __forceinline__ Cx<double> u_update(const GateDesc* gd, bool bit, bool uniform, Cx<double> a, Cx<double> b) {
+    auto m = [&](int i) { return __ldg(&gd->m[i]); };
+    const double msr = bit ? m(6) : m(0), mor = bit ? m(4) : m(2), moi = bit ? m(5) : m(3);
+    double r = __dmul_rn(msr, a.r), i = __dmul_rn(msr, a.i);
+    if (!uniform || bit || is_zero(r) || is_zero(i)) {
+        const double msi = bit ? m(7) : m(1);
+        r = __fma_rn(neg(msi), a.i, r);
+        i = __fma_rn(msi, a.r, i);
+    }
+    return Cx<double>{__fma_rn(neg(moi), b.i, __fma_rn(mor, b.r, r)), __fma_rn(moi, b.r, __fma_rn(mor, b.i, i))};
+}
+template <uint32_t K>
+__device__ __forceinline__ void pair_results(const UGate<double>& g, const GateDesc* gd, uint32_t w, Cx<double>& a,
+                                             Cx<double>& b) {
+    using A = Arith<double>;
+    if constexpr (K == KH) {
+        const Cx<double> y0{A::add(b.r, flip_sign(a.r, w)), A::add(b.i, flip_sign(a.i, w))};
+        const Cx<double> y1{A::add(a.r, flip_sign(b.r, ~w)), A::add(a.i, flip_sign(b.i, ~w))};
+        Cx<double> none;
+        products<false>(g, y0, a, none);
+        products<false>(g, y1, b, none);
+    } else if constexpr (K == KU) {
+        const Cx<double> o = u_update(gd, (w >> 31) != 0, true, a, b);
+        b = u_update(gd, (w >> 31) == 0, true, b, a);
+        a = o;
+    } else {
+        Cx<double> C0, C1, P0, P1;
+        products<true>(g, a, C0, P0);
+        products<true>(g, b, C1, P1);
+        if constexpr (K == KRX) {
+            a = Cx<double>{A::add(C0.r, P1.i), A::sub(C0.i, P1.r)};
+            b = Cx<double>{A::add(C1.r, P0.i), A::sub(C1.i, P0.r)};
+        } else {
+            a = Cx<double>{A::add(C0.r, flip_sign(P1.r, ~w)), A::add(C0.i, flip_sign(P1.i, ~w))};
+            b = Cx<double>{A::add(C1.r, flip_sign(P0.r, w)), A::add(C1.i, flip_sign(P0.i, w))};
+        }
+    }
+}
+
+// A branching gate's result for a slot whose partner is in lane ^ off; every lane calls it.
+template <uint32_t K>
+__device__ __forceinline__ Cx<float> shfl_result(const UGate<float>& g, const GateDesc*, uint32_t w, int off, Cx<float> a) {
+    const unsigned long long pa = pack2(a);
+    if constexpr (K == KH) {
+        const float one = __int_as_float(0x3F800000 | (int)(w & 0x80000000u));
+        return unpack2(mul2(pack2(g.c, g.c), fma2(pa, pack2(one, one), pack2(shfl_cx(a, off)))));
+    } else if constexpr (K == KRX) {
+        const Cx<float> b = shfl_cx(a, off);
+        const Cx<float> c = unpack2(mul2(pack2(g.c, g.c), pa)), s = unpack2(mul2(pack2(g.s, g.s), pack2(b)));
+        return Cx<float>{__fadd_rn(c.r, s.i), __fsub_rn(c.i, s.r)};
+    } else if constexpr (K == KRY) {
+        const float s = flip_sign(g.s, ~w);
+        return add_parts(mul2(pack2(g.c, g.c), pa), mul2(pack2(s, s), pack2(shfl_cx(a, off))));
+    } else {
+        const Cx<float> b = shfl_cx(a, off);
+        const bool bit = (w >> 31) != 0;
+        const float sr = bit ? g.m[6] : g.m[0], si = bit ? g.m[7] : g.m[1];
+        const float mr = bit ? g.m[4] : g.m[2], mi = bit ? g.m[5] : g.m[3];
+        unsigned long long o = mul2(pack2(sr, sr), pa);
+        o = fma2(pack2(-si, si), pack2(a.i, a.r), o);
+        o = fma2(pack2(mr, mr), pack2(b), o);
+        return unpack2(fma2(pack2(-mi, mi), pack2(b.i, b.r), o));
+    }
+}
+template <uint32_t K>
+__device__ __forceinline__ Cx<double> shfl_result(const UGate<double>& g, const GateDesc* gd, uint32_t w, int off,
+                                                  Cx<double> a) {
+    using A = Arith<double>;
+    Cx<double> o, P;
+    if constexpr (K == KH) {
+        const Cx<double> b = shfl_cx(a, off);
+        const Cx<double> y{A::add(b.r, flip_sign(a.r, w)), A::add(b.i, flip_sign(a.i, w))};
+        products<false>(g, y, o, P);
+        return o;
+    } else if constexpr (K == KU) {
+        return u_update(gd, (w >> 31) != 0, false, a, shfl_cx(a, off));
+    } else {
+        products<true>(g, a, o, P);   // the partner lane needs this lane's s-product
+        P = shfl_cx(P, off);
+        if constexpr (K == KRX) return Cx<double>{A::add(o.r, P.i), A::sub(o.i, P.r)};
+        else return Cx<double>{A::add(o.r, flip_sign(P.r, ~w)), A::add(o.i, flip_sign(P.i, ~w))};
+    }
+}
+
+// After a branching gate on the slots of `act`: they are present, but for results below the prune
+// threshold, which are rare in slots that hold keys: one test over all slots, and a branch that
+// looks at each.
+template <int S>
+__device__ __forceinline__ bool may_prune(const Slots<float, S>& x, const PruneBits& pb) {
+    float m = fmaxf(fabsf(x.v[0].r), fabsf(x.v[0].i));
+#pragma unroll
+    for (int s = 1; s < S; ++s) m = fminf(m, fmaxf(fabsf(x.v[s].r), fabsf(x.v[s].i)));
+    return !(m > __int_as_float((int)pb.f));
+}
+template <int S>
+__device__ __forceinline__ bool may_prune(const Slots<double, S>& x, const PruneBits& pb) {
+    uint32_t m = ~0u;
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const uint32_t r = (uint32_t)__double2hiint(x.v[s].r) & 0x7FFFFFFFu, i = (uint32_t)__double2hiint(x.v[s].i) & 0x7FFFFFFFu;
+        m = min(m, max(r, i));
+    }
+    return m <= (uint32_t)(pb.d >> 32);
+}
+template <class T, int S>
+__device__ __forceinline__ void settle(Slots<T, S>& x, uint32_t act, const PruneBits& pb) {
+    x.pm |= act;
+    if (!may_prune<S>(x, pb)) {
+        x.n = __popc(x.pm);
+        return;
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        if ((act & (1u << s)) && negligible(x.v[s], pb)) {
+            x.v[s] = czero<T>();
+            x.pm &= ~(1u << s);
+        }
+    }
+    x.n = __popc(x.pm);
+}
+
+// The first slot of pair p of stride ST: (0, 1), (2, 3) or (0, 2), (1, 3).
+template <int ST> __device__ constexpr int pair_slot(int p) { return ST == 1 ? 2 * p : p; }
+
+template <class T, uint32_t K, int S, int ST, bool ALL>
+__device__ __forceinline__ void branch_pair(const UGate<T>& g, const GateDesc* gd, uint32_t w, Slots<T, S>& x,
+                                            const PruneBits& pb) {
+#pragma unroll
+    for (int p = 0; p < S / 2; ++p) {
+        constexpr int kStep = S == 2 ? 1 : ST;
+        const int s = S == 2 ? 0 : pair_slot<ST>(p);
+        if (ALL || (w & (1u << s))) pair_results<K>(g, gd, w, x.v[s], x.v[s + kStep]);
+    }
+    settle<T, S>(x, ALL ? (1u << S) - 1u : w & ((1u << S) - 1u), pb);
+}
+
+template <class T, uint32_t K, int S, bool ALL>
+__device__ __forceinline__ void branch_shfl(const UGate<T>& g, const GateDesc* gd, uint32_t loc, uint32_t w, Slots<T, S>& x,
+                                            const PruneBits& pb) {
+    const int off = 1 << ((loc >> kLocBit) & 31u);
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        if (!ALL && !(loc & (1u << (kLocSlots + s)))) continue;
+        const Cx<T> o = shfl_result<K>(g, gd, w, off, x.v[s]);
+        if (ALL || (w & (1u << s))) x.v[s] = o;
+    }
+    settle<T, S>(x, ALL ? (1u << S) - 1u : w & ((1u << S) - 1u), pb);
+}
+
+template <class T, uint32_t K, int S, int ST, bool ALL>
 __device__ __forceinline__ void swap_pair(uint32_t w, Slots<T, S>& x) {
     const bool flip = (w >> 31) != 0;
 #pragma unroll
-    for (int s = 0; s < S; s += 2) {
-        if (!(w & (1u << s))) continue;
-        const Cx<T> a = x.v[s], b = x.v[s + 1];
+    for (int p = 0; p < S / 2; ++p) {
+        constexpr int kStep = S == 2 ? 1 : ST;
+        const int s = S == 2 ? 0 : pair_slot<ST>(p);
+        if (!ALL && !(w & (1u << s))) continue;
+        const Cx<T> a = x.v[s], b = x.v[s + kStep];
         x.v[s] = swap_update<T, K>(flip, b);
-        x.v[s + 1] = swap_update<T, K>(!flip, a);
-        x.pm = (x.pm & ~(3u << s)) | ((x.pm >> 1) & (1u << s)) | ((x.pm << 1) & (2u << s));
+        x.v[s + kStep] = swap_update<T, K>(!flip, a);
+        const unsigned lo = 1u << s, hi = lo << kStep;
+        x.pm = (x.pm & ~(lo | hi)) | ((x.pm >> kStep) & lo) | ((x.pm << kStep) & hi);
     }
 }
 
-template <class T, uint32_t K, int S>
+template <class T, uint32_t K, int S, bool ALL>
 __device__ __forceinline__ void swap_shfl(uint32_t loc, uint32_t w, Slots<T, S>& x) {
     const int off = 1 << ((loc >> kLocBit) & 31u);
     const unsigned pp = __shfl_xor_sync(kFull, x.pm, off);
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-        if (!(loc & (1u << (kLocSlots + s)))) continue;
+        if (!ALL && !(loc & (1u << (kLocSlots + s)))) continue;
         const Cx<T> b = shfl_cx(x.v[s], off);
-        if (w & (1u << s)) x.v[s] = swap_update<T, K>((w >> 31) != 0, b);
+        if (ALL || (w & (1u << s))) x.v[s] = swap_update<T, K>((w >> 31) != 0, b);
     }
-    x.pm = (x.pm & ~(w & 15u)) | (pp & w & 15u);
+    x.pm = ALL ? pp : (x.pm & ~(w & 15u)) | (pp & w & 15u);
+    x.n = __popc(x.pm);   // (a lane's, not the unit's, changes)
 }
 
-// Rx, Ry: results of the two members from their products (C: c * own, P: s * partner); Ry subtracts
-// where minus has bit 31 set.
-template <class T, uint32_t K>
-__device__ __forceinline__ Cx<T> rot(Cx<T> C, Cx<T> P, uint32_t minus) {
-    using A = Arith<T>;
-    if constexpr (K == KRX) return Cx<T>{A::add(C.r, P.i), A::sub(C.i, P.r)};
-    else return Cx<T>{A::add(C.r, flip_sign(P.r, minus)), A::add(C.i, flip_sign(P.i, minus))};
+// Rz (every bit; minus: bit 31 set where the logical bit is 1) and Phase (bit 1 only) on one slot.
+template <bool RZ>
+__device__ __forceinline__ Cx<float> turn(const UGate<float>& g, uint32_t minus, Cx<float> v) {
+    const float sg = RZ ? flip_sign(g.s, ~minus) : g.s;   // bit 0 turns the other way
+    const Cx<float> C = unpack2(mul2(pack2(g.c, g.c), pack2(v))), P = unpack2(mul2(pack2(sg, sg), pack2(v)));
+    return Cx<float>{__fsub_rn(C.r, P.i), __fadd_rn(C.i, P.r)};
 }
-
-template <class T, uint32_t K, int S, class G>
-__device__ __forceinline__ void branch_pair(const G& g, const GateDesc* gd, uint32_t w, Slots<T, S>& x,
-                                            const PruneBits& pb) {
-    using A = Arith<T>;
-    x.pm |= w & ((1u << S) - 1u);
-#pragma unroll
-    for (int s = 0; s < S; s += 2) {
-        if (!(w & (1u << s))) continue;
-        Cx<T> a = x.v[s], b = x.v[s + 1], o0, o1;
-        if constexpr (K == KH) {   // logical bit 0: v0 + v1, bit 1: v0 - v1
-            const Cx<T> y0{A::add(b.r, flip_sign(a.r, w)), A::add(b.i, flip_sign(a.i, w))};
-            const Cx<T> y1{A::add(a.r, flip_sign(b.r, ~w)), A::add(a.i, flip_sign(b.i, ~w))};
-            Cx<T> none;
-            products<false>(g, y0, o0, none);
-            products<false>(g, y1, o1, none);
-        } else if constexpr (K == KU) {
-            o0 = u_update<T>(g, gd, (w >> 31) != 0, true, a, b);
-            o1 = u_update<T>(g, gd, (w >> 31) == 0, true, b, a);
-        } else {
-            Cx<T> C0, C1, P0, P1;
-            products<true>(g, a, C0, P0);
-            products<true>(g, b, C1, P1);
-            o0 = rot<T, K>(C0, P1, ~w);
-            o1 = rot<T, K>(C1, P0, w);
-        }
-        put<T, S>(x, s, o0, pb);
-        put<T, S>(x, s + 1, o1, pb);
-    }
-}
-
-template <class T, uint32_t K, int S, class G>
-__device__ __forceinline__ void branch_shfl(const G& g, const GateDesc* gd, uint32_t loc, uint32_t w, Slots<T, S>& x,
-                                            const PruneBits& pb) {
-    using A = Arith<T>;
-    const int off = 1 << ((loc >> kLocBit) & 31u);
-    x.pm |= w & ((1u << S) - 1u);
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-        if (!(loc & (1u << (kLocSlots + s)))) continue;
-        const Cx<T> a = x.v[s];
-        Cx<T> o;
-        if constexpr (K == KH) {
-            const Cx<T> b = shfl_cx(a, off);
-            const Cx<T> y{A::add(b.r, flip_sign(a.r, w)), A::add(b.i, flip_sign(a.i, w))};
-            Cx<T> none;
-            products<false>(g, y, o, none);
-        } else if constexpr (K == KU) {
-            o = u_update<T>(g, gd, (w >> 31) != 0, false, a, shfl_cx(a, off));
-        } else {
-            Cx<T> C, P;
-            products<true>(g, a, C, P);   // the partner lane needs this lane's s-product
-            o = rot<T, K>(C, shfl_cx(P, off), ~w);
-        }
-        if (w & (1u << s)) put<T, S>(x, s, o, pb);
-    }
+template <bool RZ>
+__device__ __forceinline__ Cx<double> turn(const UGate<double>& g, uint32_t minus, Cx<double> v) {
+    using A = Arith<double>;
+    Cx<double> C, P;
+    products<true>(g, v, C, P);
+    if constexpr (RZ) return Cx<double>{A::add(C.r, flip_sign(P.i, minus)), A::add(C.i, flip_sign(P.r, ~minus))};
+    else return Cx<double>{A::sub(C.r, P.i), A::add(C.i, P.r)};
 }
 
 // Diagonal gates: e has bit s set where the gate acts on slot s and its logical target bit is 1.
-template <class T, uint32_t K, int S, class G>
-__device__ __forceinline__ void diag(const G& g, unsigned e, unsigned act, Slots<T, S>& x) {
-    using A = Arith<T>;
+template <class T, uint32_t K, int S>
+__device__ __forceinline__ void diag(const UGate<T>& g, unsigned e, unsigned act, Slots<T, S>& x) {
+    if (K != KZ && !(K == KYPH || K == KRZ ? act : e)) return;
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         Cx<T>& v = x.v[s];
+        const uint32_t m = e << (31 - s);   // bit 31: logical target bit 1
         if constexpr (K == KZ) {
-            const uint32_t m = e << (31 - s);
             v = Cx<T>{flip_sign(v.r, m), flip_sign(v.i, m)};
         } else if constexpr (K == KS || K == KSDG) {   // S: i * v, Sdg: -i * v
             if (e & (1u << s)) v = K == KSDG ? Cx<T>{v.i, neg(v.r)} : Cx<T>{neg(v.i), v.r};
         } else if constexpr (K == KYPH) {              // bit 1: i * v, bit 0: -i * v
-            const uint32_t m = e << (31 - s);
             if (act & (1u << s)) v = Cx<T>{flip_sign(v.i, m), flip_sign(v.r, ~m)};
         } else if (K == KRZ ? (act & (1u << s)) : (e & (1u << s))) {
-            Cx<T> C, P;
-            products<true>(g, v, C, P);
-            if constexpr (K == KRZ) {   // bit 1: c*r - s*i, c*i + s*r; bit 0: + and -
-                const uint32_t m = e << (31 - s);
-                v = Cx<T>{A::add(C.r, flip_sign(P.i, m)), A::add(C.i, flip_sign(P.r, ~m))};
-            } else {
-                v = Cx<T>{A::sub(C.r, P.i), A::add(C.i, P.r)};
-            }
+            v = turn<K == KRZ>(g, m, v);
         }
     }
 }
 
-template <class T, int S>
-__device__ __forceinline__ void swap_slots12(Slots<T, S>& x) {
-    const Cx<T> y = x.v[S == 4 ? 1 : 0];
-    x.v[S == 4 ? 1 : 0] = x.v[S == 4 ? 2 : 0];
-    x.v[S == 4 ? 2 : 0] = y;
-    x.pm = (x.pm & 9u) | ((x.pm & 2u) << 1) | ((x.pm & 4u) >> 1);
-}
-
 // The gates of a pass on the unit a warp holds; uid is the unit's base index. Absent slots hold
 // +-0, which no gate makes present (sqc_pass_dev.cuh).
-template <class T, int S>
-__device__ __forceinline__ void run_unit(const UGates<T>& sg, const GateDesc* __restrict__ gates, uint32_t ng,
+// `heads` says where each gate acts (UnitHead): the gates' own in shared memory, or the kernel's
+// parameters, where the whole warp reads them as one.
+template <class T, int S, class Heads>
+__device__ __forceinline__ void run_unit(const Heads& heads, const UGates<T>& sg, const GateDesc* __restrict__ gates, uint32_t ng,
                                          uint32_t uid, int lane, Slots<T, S>& x, bool& touched,
                                          const PruneBits& pb, unsigned long long& upd) {
-    unsigned n = __popc(x.pm);
 #pragma unroll 1
     for (uint32_t gi = 0; gi < ng; ++gi) {
         const UGate<T>& g = sg.g[gi];
-        const uint4 head = *reinterpret_cast<const uint4*>(&g);   // om, ov, loc, weight
-        upd += (unsigned long long)n * head.w;
-        if ((uid & head.x) != head.y) continue;   // a control outside the unit excludes all of it
+        const UnitHead head = heads[gi];
+        upd += (unsigned long long)x.n * head.weight;
+        if ((uid & head.om) != head.ov) continue;   // a control outside the unit excludes all of it
         const uint32_t w = (uint32_t)(int)sg.lw[gi][lane];
-        const uint32_t loc = head.z;
+        const uint32_t loc = head.loc;
         const GateDesc* gd = gates + gi;
         touched = true;
-        const bool exchange = S == 4 && (loc & kLocPair3);   // dimension 2: exchange slots around the pair code
-        if (exchange) swap_slots12<T, S>(x);
-        if ((loc >> kLocOp) < UO_Z) {
-            switch (loc >> kLocOp) {
-            case UO_X_PAIR: swap_pair<T, KX, S>(w, x); break;
-            case UO_X_SHFL: swap_shfl<T, KX, S>(loc, w, x); break;
-            case UO_Y_PAIR: swap_pair<T, KY, S>(w, x); break;
-            case UO_Y_SHFL: swap_shfl<T, KY, S>(loc, w, x); break;
-            case UO_H_PAIR: branch_pair<T, KH, S>(g, gd, w, x, pb); break;
-            case UO_H_SHFL: branch_shfl<T, KH, S>(g, gd, loc, w, x, pb); break;
-            case UO_RX_PAIR: branch_pair<T, KRX, S>(g, gd, w, x, pb); break;
-            case UO_RX_SHFL: branch_shfl<T, KRX, S>(g, gd, loc, w, x, pb); break;
-            case UO_RY_PAIR: branch_pair<T, KRY, S>(g, gd, w, x, pb); break;
-            case UO_RY_SHFL: branch_shfl<T, KRY, S>(g, gd, loc, w, x, pb); break;
-            case UO_U_PAIR: branch_pair<T, KU, S>(g, gd, w, x, pb); break;
-            default: branch_shfl<T, KU, S>(g, gd, loc, w, x, pb); break;
-            }
-            if (exchange) swap_slots12<T, S>(x);
-            n = __popc(x.pm);
-        } else {
-            const unsigned act = w & 15u;
-            const unsigned e = ((w >> 4) & 15u) ^ (((uid >> ((loc >> kLocBit) & 31u)) & 1u) && !(loc & kLocLane) ? act : 0u);
-            switch (loc >> kLocOp) {
-            case UO_Z: diag<T, KZ, S>(g, e, act, x); break;
-            case UO_S: diag<T, KS, S>(g, e, act, x); break;
-            case UO_SDG: diag<T, KSDG, S>(g, e, act, x); break;
-            case UO_YPH: diag<T, KYPH, S>(g, e, act, x); break;
-            case UO_RZ: diag<T, KRZ, S>(g, e, act, x); break;
-            default: diag<T, KPHASE, S>(g, e, act, x); break;
-            }
+        const unsigned act = w & 15u;
+        // diagonal gates: slots with logical target bit 1, the target's bit of the unit's base applied
+        auto ones = [&]() {
+            return ((w >> 4) & 15u) ^ (((uid >> ((loc >> kLocBit) & 31u)) & 1u) && !(loc & kLocLane) ? act : 0u);
+        };
+        switch (loc >> kLocOp) {
+        case UO_X_PAIR: swap_pair<T, KX, S, 1, false>(w, x); break;
+        case UO_X_SHFL: swap_shfl<T, KX, S, false>(loc, w, x); break;
+        case UO_ALL + UO_X_PAIR: swap_pair<T, KX, S, 1, true>(w, x); break;
+        case UO_ALL + UO_X_SHFL: swap_shfl<T, KX, S, true>(loc, w, x); break;
+        case UO_PAIR3 + UO_X_PAIR:
+            if constexpr (S == 4) swap_pair<T, KX, S, 2, false>(w, x);
+            break;
+        case UO_ALL3 + UO_X_PAIR:
+            if constexpr (S == 4) swap_pair<T, KX, S, 2, true>(w, x);
+            break;
+        case UO_Y_PAIR: swap_pair<T, KY, S, 1, false>(w, x); break;
+        case UO_Y_SHFL: swap_shfl<T, KY, S, false>(loc, w, x); break;
+        case UO_ALL + UO_Y_PAIR: swap_pair<T, KY, S, 1, true>(w, x); break;
+        case UO_ALL + UO_Y_SHFL: swap_shfl<T, KY, S, true>(loc, w, x); break;
+        case UO_PAIR3 + UO_Y_PAIR:
+            if constexpr (S == 4) swap_pair<T, KY, S, 2, false>(w, x);
+            break;
+        case UO_ALL3 + UO_Y_PAIR:
+            if constexpr (S == 4) swap_pair<T, KY, S, 2, true>(w, x);
+            break;
+        case UO_H_PAIR: branch_pair<T, KH, S, 1, false>(g, gd, w, x, pb); break;
+        case UO_H_SHFL: branch_shfl<T, KH, S, false>(g, gd, loc, w, x, pb); break;
+        case UO_ALL + UO_H_PAIR: branch_pair<T, KH, S, 1, true>(g, gd, w, x, pb); break;
+        case UO_ALL + UO_H_SHFL: branch_shfl<T, KH, S, true>(g, gd, loc, w, x, pb); break;
+        case UO_PAIR3 + UO_H_PAIR:
+            if constexpr (S == 4) branch_pair<T, KH, S, 2, false>(g, gd, w, x, pb);
+            break;
+        case UO_ALL3 + UO_H_PAIR:
+            if constexpr (S == 4) branch_pair<T, KH, S, 2, true>(g, gd, w, x, pb);
+            break;
+        case UO_RX_PAIR: branch_pair<T, KRX, S, 1, false>(g, gd, w, x, pb); break;
+        case UO_RX_SHFL: branch_shfl<T, KRX, S, false>(g, gd, loc, w, x, pb); break;
+        case UO_ALL + UO_RX_PAIR: branch_pair<T, KRX, S, 1, true>(g, gd, w, x, pb); break;
+        case UO_ALL + UO_RX_SHFL: branch_shfl<T, KRX, S, true>(g, gd, loc, w, x, pb); break;
+        case UO_PAIR3 + UO_RX_PAIR:
+            if constexpr (S == 4) branch_pair<T, KRX, S, 2, false>(g, gd, w, x, pb);
+            break;
+        case UO_ALL3 + UO_RX_PAIR:
+            if constexpr (S == 4) branch_pair<T, KRX, S, 2, true>(g, gd, w, x, pb);
+            break;
+        case UO_RY_PAIR: branch_pair<T, KRY, S, 1, false>(g, gd, w, x, pb); break;
+        case UO_RY_SHFL: branch_shfl<T, KRY, S, false>(g, gd, loc, w, x, pb); break;
+        case UO_ALL + UO_RY_PAIR: branch_pair<T, KRY, S, 1, true>(g, gd, w, x, pb); break;
+        case UO_ALL + UO_RY_SHFL: branch_shfl<T, KRY, S, true>(g, gd, loc, w, x, pb); break;
+        case UO_PAIR3 + UO_RY_PAIR:
+            if constexpr (S == 4) branch_pair<T, KRY, S, 2, false>(g, gd, w, x, pb);
+            break;
+        case UO_ALL3 + UO_RY_PAIR:
+            if constexpr (S == 4) branch_pair<T, KRY, S, 2, true>(g, gd, w, x, pb);
+            break;
+        case UO_U_PAIR: branch_pair<T, KU, S, 1, false>(g, gd, w, x, pb); break;
+        case UO_U_SHFL: branch_shfl<T, KU, S, false>(g, gd, loc, w, x, pb); break;
+        case UO_ALL + UO_U_PAIR: branch_pair<T, KU, S, 1, true>(g, gd, w, x, pb); break;
+        case UO_ALL + UO_U_SHFL: branch_shfl<T, KU, S, true>(g, gd, loc, w, x, pb); break;
+        case UO_PAIR3 + UO_U_PAIR:
+            if constexpr (S == 4) branch_pair<T, KU, S, 2, false>(g, gd, w, x, pb);
+            break;
+        case UO_ALL3 + UO_U_PAIR:
+            if constexpr (S == 4) branch_pair<T, KU, S, 2, true>(g, gd, w, x, pb);
+            break;
+        case UO_Z: diag<T, KZ, S>(g, ones(), act, x); break;
+        case UO_S: diag<T, KS, S>(g, ones(), act, x); break;
+        case UO_SDG: diag<T, KSDG, S>(g, ones(), act, x); break;
+        case UO_YPH: diag<T, KYPH, S>(g, ones(), act, x); break;
+        case UO_RZ: diag<T, KRZ, S>(g, ones(), act, x); break;
+        case UO_PHASE: diag<T, KPHASE, S>(g, ones(), act, x); break;
+        default: __builtin_unreachable();
         }
     }
 }
@@ -420,34 +591,54 @@ __device__ __forceinline__ UnitPass unit_pass(uint32_t dn, uint32_t d0, uint32_t
 // (t's map is read through mq: a pass over many circuits leaves it in memory.)
 // One unit: load, apply the gates, write back. Absent buckets are created (header, keys, list
 // entry) when a key of theirs becomes present; the unit is this warp's alone, so plain stores do.
-template <class T, int DIMS>
+template <class T, int DIMS, class Heads>
 __device__ __forceinline__ void do_unit(const TableDev& t, const uint8_t* mq, Ctl* ctl, unsigned ep, const UnitPass& up, unsigned base,
-                                        const UGates<T>& sg, const GateDesc* gates, uint32_t ng, int lane,
+                                        const Heads& heads, const UGates<T>& sg, const GateDesc* gates, uint32_t ng, int lane,
                                         const PruneBits& pb, unsigned long long& cnt_nnz, unsigned long long& cnt_empty,
                                         unsigned long long& upd) {
     constexpr int S = 1 << (DIMS - 1);
     const int j = lane & 15;
     const unsigned b0 = base | ((unsigned)(lane >> 4) << up.dim[1]);
     unsigned bk[S];
-    uint2 h[S];
     Slots<T, S> x;
+    // lane k < 2^DIMS reads member k's header; a unit whose buckets are all live and full (every unit,
+    // in a state that fills its span) needs nothing more of them
+    constexpr unsigned kMembers = 1u << DIMS;
+    uint2 hk = make_uint2(ep, 0xFFFFu);
+    if (lane < (int)kMembers) {
+        unsigned b = base;
+#pragma unroll
+        for (int d = 0; d < DIMS; ++d) b |= (((unsigned)lane >> d) & 1u) << up.dim[d];
+        hk = __ldcg(reinterpret_cast<const uint2*>(&t.hdr[b].epoch));
+    }
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         bk[s] = b0 | ((s & 1) ? 1u << up.dim[0] : 0u) | ((s & 2) ? 1u << up.dim[2] : 0u);
-        h[s] = *reinterpret_cast<const uint2*>(&t.hdr[bk[s]].epoch);
-        const typename AmpT<T>::V a = reinterpret_cast<const typename AmpT<T>::V*>(t.amps)[(size_t)bk[s] * kSlots + j];
+        const typename AmpT<T>::V a =
+            __ldcg(reinterpret_cast<const typename AmpT<T>::V*>(t.amps) + (size_t)bk[s] * kSlots + j);
         x.v[s] = Cx<T>{a.x, a.y};
     }
-    x.pm = 0;
+    uint2 h[S];
+    const bool full = __all_sync(kFull, hk.x == ep && hk.y == 0xFFFFu);
+    x.pm = (1u << S) - 1u;
+    if (!full) {
+        x.pm = 0;
 #pragma unroll
-    for (int s = 0; s < S; ++s) {
-        const bool p = h[s].x == ep && ((h[s].y >> j) & 1u);
-        x.pm |= (unsigned)p << s;
-        x.v[s] = pick(p, x.v[s], czero<T>());
+        for (int s = 0; s < S; ++s) {
+            const int m = (s & 1) | ((lane >> 4) << 1) | ((s & 2) << 1);
+            h[s] = make_uint2(__shfl_sync(kFull, hk.x, m), __shfl_sync(kFull, hk.y, m));
+            const bool p = h[s].x == ep && ((h[s].y >> j) & 1u);
+            x.pm |= (unsigned)p << s;
+            x.v[s] = pick(p, x.v[s], czero<T>());
+        }
+    } else {
+#pragma unroll
+        for (int s = 0; s < S; ++s) h[s] = make_uint2(ep, 0xFFFFu);
     }
     bool touched = false;
     const unsigned pm0 = x.pm;
-    if (__any_sync(kFull, pm0 != 0)) run_unit<T, S>(sg, gates, ng, base, lane, x, touched, pb, upd);
+    x.n = __popc(pm0);
+    if (full || __any_sync(kFull, pm0 != 0)) run_unit<T, S>(heads, sg, gates, ng, base, lane, x, touched, pb, upd);
     const unsigned pm = x.pm;
     cnt_nnz += __popc(pm);
 #pragma unroll
@@ -489,7 +680,7 @@ __device__ __forceinline__ void do_unit(const TableDev& t, const uint8_t* mq, Ct
             for (int s = 0; s < S; ++s)
                 if ((fresh >> s) & 1u) t.list[at++] = bk[s];
         }
-    } else {
+    } else if (!full) {
 #pragma unroll
         for (int s = 0; s < S; ++s)
             if (j == 0 && h[s].x == ep && h[s].y == 0) cnt_empty += 1;
@@ -497,14 +688,13 @@ __device__ __forceinline__ void do_unit(const TableDev& t, const uint8_t* mq, Ct
 }
 
 // Units [u0, u1) step `stride` of a table whose live buckets fill it.
-template <class T, int DIMS>
+template <class T, int DIMS, class Heads>
 __device__ __forceinline__ void walk_units(const TableDev& t, const uint8_t* mq, Ctl* ctl, unsigned ep, const UnitPass& up,
-                                           unsigned long long u0, unsigned long long u1, unsigned long long stride,
-                                           const UGates<T>& sg, const GateDesc* gates, uint32_t ng, int lane,
+                                           unsigned u0, unsigned u1, unsigned stride, const Heads& heads, const UGates<T>& sg, const GateDesc* gates, uint32_t ng, int lane,
                                            const PruneBits& pb, unsigned long long& cnt_nnz,
                                            unsigned long long& cnt_empty, unsigned long long& upd) {
-    for (unsigned long long u = u0; u < u1; u += stride)
-        do_unit<T, DIMS>(t, mq, ctl, ep, up, unit_base<DIMS>((unsigned)u, up.lo), sg, gates, ng, lane, pb, cnt_nnz, cnt_empty,
+    for (unsigned u = u0; u < u1; u += stride)   // (at most 2^29 units: no wrap)
+        do_unit<T, DIMS>(t, mq, ctl, ep, up, unit_base<DIMS>(u, up.lo), heads, sg, gates, ng, lane, pb, cnt_nnz, cnt_empty,
                          upd);
 }
 
@@ -512,9 +702,9 @@ __device__ __forceinline__ void walk_units(const TableDev& t, const uint8_t* mq,
 // the mapped ones: lane l takes entry e0 + l; the unit belongs to its live member of smallest index
 // (members a pass creates are made by the unit's owner, after its own check), found by reading
 // the headers of the smaller members.
-template <class T, int DIMS>
+template <class T, int DIMS, class Heads>
 __device__ __forceinline__ void walk_entries(const TableDev& t, const uint8_t* mq, Ctl* ctl, unsigned ep, const UnitPass& up,
-                                             unsigned long long e0, unsigned long long n, const UGates<T>& sg,
+                                             unsigned long long e0, unsigned long long n, const Heads& heads, const UGates<T>& sg,
                                              const GateDesc* gates, uint32_t ng, int lane, const PruneBits& pb,
                                              unsigned long long& cnt_nnz, unsigned long long& cnt_empty,
                                              unsigned long long& upd) {
@@ -542,7 +732,7 @@ __device__ __forceinline__ void walk_entries(const TableDev& t, const uint8_t* m
     while (todo) {
         const int l = __ffs(todo) - 1;
         todo &= todo - 1;
-        do_unit<T, DIMS>(t, mq, ctl, ep, up, __shfl_sync(kFull, base, l), sg, gates, ng, lane, pb, cnt_nnz, cnt_empty, upd);
+        do_unit<T, DIMS>(t, mq, ctl, ep, up, __shfl_sync(kFull, base, l), heads, sg, gates, ng, lane, pb, cnt_nnz, cnt_empty, upd);
     }
 }
 

@@ -249,3 +249,24 @@ def test_key_ordered_readout(nq, k, precision):
     assert_identical(st.state(drop_negligible=True), tuple(x[keep] for x in full))
     assert np.isin(st.sample(200, seed=3), full[0]).all()
     st.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k,depth", [(14, 300), (17, 900)])
+def test_first_run_of_a_full_state_is_mapped(k, depth):
+    """A new state whose keys fill their span grows a mapped table (its refused passes are replayed)
+    however many branching gates the circuit has, and the next run of it does the same work."""
+    from sparqc_gb300.engine import State
+    g = circuits.random_circuit(30, k, depth, 2, circuits.SplitMix64(k), kinds=KINDS)
+    st, o = State(30), SparseOracle()
+    o.apply(g)
+    st.apply(g)
+    first = st.state(sorted=True)
+    passes = st.stats()["passes"]
+    assert st.stats()["replays"] > 0
+    st.set_zero()
+    st.apply(g)
+    assert_identical(first, o.state(sorted=True))
+    assert_identical(st.state(sorted=True), first)
+    assert st.stats()["passes"] == 2 * passes
+    st.close()
