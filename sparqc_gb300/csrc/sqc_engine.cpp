@@ -269,6 +269,7 @@ int Engine::set_zero() {
     list_hint_ = 1;
     key_hint_ = 1;
     fresh_ = true;
+    clean_ = false;
     mapped_ = true;
     map_.clear();
     int rc;
@@ -317,6 +318,7 @@ int Engine::set_state(const uint64_t* keys, const double* re, const double* im, 
     }
     int rc;
     if ((rc = cuda(cudaStreamSynchronize(stream_), "sync"))) return rc;
+    clean_ = false;
     pending_.clear();
     log_.clear();
     passes_.clear();
@@ -388,6 +390,7 @@ int Engine::apply(const sqc_gate* gates, uint64_t n) {
 int Engine::flush(bool hold_last) {
     if (pending_.empty()) return SQC_OK;
     const size_t n = pending_.size();
+    clean_ = false;
     int rc;
     if (desc_used_ + n > desc_cap_) {
         std::vector<sqc_gate> keep;
@@ -748,6 +751,7 @@ int Engine::sync() {
             if (ctl_host_->list_n > 4096 && ctl_host_->empty_groups * 2 > ctl_host_->list_n) {
                 if ((rc = rebuild(tab_.nb, mapped_))) return rc;
             }
+            clean_ = true;
             return SQC_OK;
         }
         if (st != ST_GROW) {
@@ -896,7 +900,7 @@ int Engine::take_unapplied(std::vector<sqc_gate>* rest) {
 }
 
 int Engine::nnz(uint64_t* out) {
-    int rc = sync();
+    int rc = settled();
     if (rc) return rc;
     *out = ctl_host_->nnz;
     return SQC_OK;
@@ -1009,7 +1013,7 @@ int Engine::ensure_cum(size_t n) {
 // (actual keys); *got receives their number (also when it exceeds the arrays).
 int Engine::readout_to_device(uint64_t mask, uint64_t value, bool drop_negl, unsigned long long* got, bool wait,
                               bool* ordered) {
-    int rc = sync();
+    int rc = settled();
     if (rc) return rc;
     const bool ranked = mapped_ && rank_worth(map_.n, ctl_host_->nnz);
     if (ordered) *ordered = ranked;
@@ -1122,7 +1126,7 @@ int Engine::load(const char* path) {
 
 int Engine::probability(uint64_t mask, uint64_t value, double* p) {
     if (!p) return fail(SQC_ERR_ARG, "null output");
-    int rc = sync();
+    int rc = settled();
     if (rc) return rc;
     if ((rc = cuda(cudaMemsetAsync(sums_, 0, sizeof(ExactSums), stream_), "memset")) ||
         (rc = cuda(launch_pattern_prob(dev(), ctl_, list_hint_, dbl_, mask, value ^ (plan_.frame & mask), sums_, sms_,
@@ -1150,6 +1154,7 @@ int Engine::measure(uint32_t qubit, double u, int* outcome, double* p1) {
     if (!(kept > 0.0)) return fail(SQC_ERR_STATE, "measurement outcome of probability zero");
     const unsigned long long bit = 1ULL << qubit;
     const unsigned long long val = out ? bit : 0ULL;
+    clean_ = false;
     if ((rc = cuda(launch_collapse(dev(), ctl_, list_hint_, dbl_, bit, val ^ (plan_.frame & bit), 1.0 / std::sqrt(kept),
                                    sms_, stream_),
                    "collapse")))
@@ -1203,7 +1208,7 @@ int Engine::sample(uint64_t shots, uint64_t seed, uint64_t* keys) {
 }
 
 int Engine::norm2(double* out) {
-    int rc = sync();
+    int rc = settled();
     if (rc) return rc;
     if ((rc = cuda(cudaMemsetAsync(sums_, 0, sizeof(ExactSums), stream_), "memset"))) return rc;
     if ((rc = cuda(launch_norm(dev(), ctl_, list_hint_, dbl_, sums_, sms_, stream_), "norm"))) return rc;

@@ -55,6 +55,9 @@ public:
     // feeds a circuit in slices keeps the passes it would get from the whole circuit.
     int flush(bool hold_last = false);
     int sync();
+    // sync() for the questions put to a state: nothing to wait for when no gate was queued or launched,
+    // and the state not reset, since the last one (the control block's mirror is then current)
+    int settled() { return clean_ && pending_.empty() ? 0 : sync(); }
     int nnz(uint64_t* out);
     int get_state(uint64_t* keys, double* re, double* im, uint64_t cap, uint64_t* n, uint32_t flags);
     // Readout into page-locked host arrays that completes while later work on the state runs:
@@ -160,6 +163,7 @@ private:
     unsigned long long list_hint_ = 1;
     unsigned long long key_hint_ = 1;   // keys the state holds after the launched passes, at most
     bool fresh_ = true;                 // |0...0>, no pass launched yet
+    bool clean_ = false;                // see settled()
     PruneBits prune_{};
 
     Planner plan_;              // after every queued gate

@@ -56,14 +56,21 @@ __device__ __forceinline__ void exact_add_prod(unsigned long long (&acc)[kSumChu
     }
 }
 
-// Add a warp's accumulators into the global sum (every lane calls it).
+// Add a block's accumulators into the global sum (every thread calls it, once per call site). The
+// warps meet in shared memory first: ten words are added to by the whole grid, and with an addition
+// per warp those, one after the other at the same ten addresses, took most of the kernel.
 __device__ __forceinline__ void exact_flush(unsigned long long (&acc)[kSumChunks], unsigned long long* out) {
+    __shared__ unsigned long long block[kSumChunks];
+    if (threadIdx.x < kSumChunks) block[threadIdx.x] = 0;
+    __syncthreads();
 #pragma unroll
     for (int i = 0; i < kSumChunks; ++i) {
         unsigned long long v = acc[i];
         for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0 && v) atomicAdd(out + i, v);
+        if ((threadIdx.x & 31) == 0 && v) atomicAdd(block + i, v);
     }
+    __syncthreads();
+    if (threadIdx.x < kSumChunks && block[threadIdx.x]) atomicAdd(out + threadIdx.x, block[threadIdx.x]);
 }
 #endif
 
