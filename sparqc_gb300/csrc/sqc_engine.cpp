@@ -30,6 +30,7 @@ constexpr unsigned long long kMapSpan = 16;
 // gigabyte, so that a state growing one qubit at a time is not rebuilt at every one; then twice.
 constexpr unsigned long long kMapRoomy = 1ULL << 21;
 constexpr unsigned long long kHashRoomy = 1ULL << 17;   // 55 MB
+constexpr uint32_t kRunMapFp64 = 18, kRunMapFp32 = 17;   // mapped bits up to which passes go out in runs (sqc_pass.cu: run_kernel)
 constexpr uint32_t kNoMap = 63;            // Span::dn of a pass whose bits no table maps: always refused
 
 bool map_worth(uint32_t dn, unsigned long long groups) {
@@ -492,7 +493,7 @@ int Engine::flush(bool hold_last) {
         return rc;
     cudaEvent_t ev_prev = nullptr;
     if (time_passes_ && (rc = record_event(&ev_prev))) return rc;
-    // a tiny state runs the flush's passes in one single-block launch (tiny_kernel): the live
+    // a tiny hashed state runs the flush's passes in one single-block launch (tiny_kernel): the live
     // buckets every pass may reach stay few enough that launches would cost more than the work
     {
         unsigned long long h = list_hint_, hmax = list_hint_;
@@ -501,11 +502,7 @@ int Engine::flush(bool hold_last) {
                 h = std::min<unsigned long long>({tab_.nb, h << sp.nx, h + sp.keys, group_bound(after[sp.g1 - 1], nq_)});
             hmax = std::max(hmax, h);
         }
-        if (mapped_) {   // unit passes enumerate the mapped bits' span
-            hmax = 1;
-            for (const Span& sp : spans) hmax = std::max(hmax, 1ULL << sp.dn);
-        }
-        if (spans.size() >= 2 && tiny_table(tab_.nb) && hmax <= kTinyMaxList) {
+        if (!mapped_ && spans.size() >= 2 && tiny_table(tab_.nb) && hmax <= kTinyMaxList) {
             TinyPass* ht = h_tiny_ + desc_used_;
             bool any_pair = false;
             for (size_t k = 0; k < spans.size(); ++k) {
@@ -518,9 +515,7 @@ int Engine::flush(bool hold_last) {
                 q.q2 = sp.q2;
                 q.q3 = sp.q3;
                 q.keys_fixed = sp.fixed ? 1u : 0u;
-                q.dn = sp.dn;
-                for (int i = 0; i < 3; ++i) q.dim[i] = sp.dim[i];
-                q.dim[3] = 0;
+                q.pad = 0;
                 q.grow_bound = group_bound(after[sp.g1 - 1], nq_);
                 q.key_bound = sp.keys;
                 any_pair = any_pair || sp.nx > 0;
@@ -528,8 +523,7 @@ int Engine::flush(bool hold_last) {
             if ((rc = cuda(cudaMemcpyAsync(d_tiny_ + desc_used_, ht, spans.size() * sizeof(TinyPass),
                                            cudaMemcpyHostToDevice, stream_), "H2D tiny passes")))
                 return rc;
-            if ((mapped_ ? launch_tiny_units(a, d_tiny_ + desc_used_, (uint32_t)spans.size(), dbl_, stream_)
-                         : launch_tiny(a, d_tiny_ + desc_used_, (uint32_t)spans.size(), dbl_, stream_)) < 0)
+            if (launch_tiny(a, d_tiny_ + desc_used_, (uint32_t)spans.size(), dbl_, stream_) < 0)
                 return launch_failed("tiny passes");
             if (time_passes_) {
                 cudaEvent_t ev = nullptr;
@@ -550,8 +544,48 @@ int Engine::flush(bool hold_last) {
             return SQC_OK;
         }
     }
-    for (const Span& sp : spans) {
-        const size_t i = sp.g1;
+    auto record = [&](const Span& sp) {
+        passes_pair_ += sp.nx > 0 ? 1 : 0;
+        passes_.push_back(PassRec{snap_log_, snap_plan_, sp.map0, sp.dn, sp.nx, sp.keys});
+        snap_log_ = src[sp.g1 - 1] + 1;
+        snap_plan_ = after[sp.g1 - 1];
+        ++passes_run_;
+        if (sp.nx) list_hint_ = std::min(tab_.nb, grown(sp.nx, group_bound(after[sp.g1 - 1], nq_), sp.keys));
+        key_hint_ = sp.keys;
+    };
+    RunArgs run;
+    for (size_t s = 0; s < spans.size();) {
+        const Span& sp = spans[s];
+        // consecutive passes of a small or middle mapped state go out in one launch
+        size_t e = s, words = 0;
+        while (mapped_ && !time_passes_ && e < spans.size() && spans[e].dn <= (dbl_ ? kRunMapFp64 : kRunMapFp32) &&
+               (1ULL << spans[e].dn) <= a.max_groups && words + 1 + spans[e].g1 - spans[e].g0 <= kRunWords) {
+            words += 1 + spans[e].g1 - spans[e].g0;
+            ++e;
+        }
+        if (e - s >= 2) {
+            run.t = a.t;
+            run.ctl = a.ctl;
+            run.gates = a.gates;
+            run.prune = a.prune;
+            run.amp_bytes = a.amp_bytes;
+            run.np = (uint32_t)(e - s);
+            run.tag = run_tag_;
+            run_tag_ += run.np;
+            UnitHead* w = run.words;
+            for (; s < e; ++s) {
+                const Span& r = spans[s];
+                *w++ = UnitHead{(uint32_t)(r.g1 - r.g0) | (r.fixed ? kRunFixed : 0u) | (r.nx ? kRunPair : 0u) | (r.dn << 16),
+                                r.dim[0] | (r.dim[1] << 8) | (r.dim[2] << 16), (uint32_t)r.g0, 0u};
+                for (size_t k = r.g0; k < r.g1; ++k) *w++ = UnitHead{hd[k].om, hd[k].ov, hd[k].loc, hd[k].pad + 1u};
+                record(r);
+            }
+            const int nl = launch_unit_run(run, dims, spans[e - 1].dn, dbl_, sms_, stream_);
+            if (nl < 0) return launch_failed("gate passes");
+            launches_ += (uint64_t)nl;
+            continue;
+        }
+        ++s;
         a.g0 = (uint32_t)sp.g0;
         a.g1 = (uint32_t)sp.g1;
         a.nx = sp.nx;
@@ -559,35 +593,28 @@ int Engine::flush(bool hold_last) {
         a.q2 = sp.q2;
         a.q3 = sp.q3;
         a.keys_fixed = sp.fixed ? 1u : 0u;
-        a.grow_bound = group_bound(after[i - 1], nq_);
+        a.grow_bound = group_bound(after[sp.g1 - 1], nq_);
         a.key_bound = sp.keys;
         if (!mapped_ && sp.nx && grown(sp.nx, a.grow_bound, sp.keys) > a.max_groups) {
             if ((rc = make_room(sp.nx, a.grow_bound, sp.keys))) return rc;
             a.t = dev();
             a.max_groups = max_groups();
         }
-        if (sp.nx) list_hint_ = std::min(tab_.nb, grown(sp.nx, a.grow_bound, sp.keys));
-        key_hint_ = sp.keys;
+        const unsigned long long hint = sp.nx ? std::min(tab_.nb, grown(sp.nx, a.grow_bound, sp.keys)) : list_hint_;
         a.dn = sp.dn;
         for (int d = 0; d < 3; ++d) a.dim[d] = sp.dim[d];
         if (mapped_)
             for (size_t k = sp.g0; k < sp.g1; ++k) a.heads[k - sp.g0] = UnitHead{hd[k].om, hd[k].ov, hd[k].loc, hd[k].pad + 1u};
-        const int nl = mapped_ ? launch_unit_pass(a, dbl_, sms_, stream_)
-                               : launch_pass(a, list_hint_, dbl_, sms_, stream_);
+        const int nl = mapped_ ? launch_unit_pass(a, dbl_, sms_, stream_) : launch_pass(a, hint, dbl_, sms_, stream_);
         if (nl < 0) return launch_failed("gate pass");
-        const bool pair = sp.nx > 0;
         if (time_passes_) {
             cudaEvent_t ev = nullptr;
             if ((rc = record_event(&ev))) return rc;
-            timed_.push_back(TimedPass{ev_prev, ev, pair});
+            timed_.push_back(TimedPass{ev_prev, ev, sp.nx > 0});
             ev_prev = ev;
         }
-        passes_pair_ += pair ? 1 : 0;
-        passes_.push_back(PassRec{snap_log_, snap_plan_, sp.map0, sp.dn, sp.nx, sp.keys});
-        snap_log_ = src[i - 1] + 1;
-        snap_plan_ = after[i - 1];
+        record(sp);
         launches_ += (uint64_t)nl;
-        ++passes_run_;
         // a mapped pass the table is too small for refuses, and so would every later one: they
         // are queued again, with it, when the table has grown
         if (mapped_ && (1ULL << sp.dn) > a.max_groups) break;
@@ -777,6 +804,7 @@ int Engine::rebuild(unsigned long long nb_new, bool mapped) {
     epochs_ = 1;
     c.status = 0;
     c.done = 0;
+    c.bar = 0;
     c.seq = 0;
     c.list_n = 0;
     c.list_tail = 0;

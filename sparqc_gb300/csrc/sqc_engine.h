@@ -192,6 +192,7 @@ private:
     void* d_cum_tmp_ = nullptr;
     size_t cum_cap_ = 0, cum_tmp_bytes_ = 0;
 
+    uint32_t run_tag_ = 1;          // RunArgs.tag of the next run
     uint64_t gates_applied_ = 0, passes_run_ = 0, launches_ = 0, replays_ = 0, rebuilds_ = 0;
     uint64_t passes_pair_ = 0;
 

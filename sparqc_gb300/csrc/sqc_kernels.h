@@ -18,10 +18,10 @@ int launch_pass(const PassArgs& a, unsigned long long list_hint, bool dbl, int s
 bool tiny_table(unsigned long long buckets);
 // The passes (device array of np records; a's per-pass fields are ignored) in one launch.
 int launch_tiny(const PassArgs& a, const TinyPass* passes, uint32_t np, bool dbl, cudaStream_t st);
-// A pass over a mapped table (sqc_unit.cuh; a.dn, a.dims and a.dim set), and the passes of a flush on
-// a tiny one in a single launch. FP32 units have three dimensions, FP64 units two or three.
+// A pass over a mapped table (sqc_unit.cuh; a.dn, a.dims and a.dim set), and a run of such passes in
+// one launch (dn: mapped bits of the last). FP32 units have three dimensions, FP64 units two or three.
 int launch_unit_pass(const PassArgs& a, bool dbl, int sms, cudaStream_t st);
-int launch_tiny_units(const PassArgs& a, const TinyPass* passes, uint32_t np, bool dbl, cudaStream_t st);
+int launch_unit_run(const RunArgs& a, uint32_t dims, uint32_t dn, bool dbl, int sms, cudaStream_t st);
 cudaError_t launch_set_zero(const TableDev& t, Ctl* ctl, bool dbl, cudaStream_t st);
 // Load n entries; a stored key is the entry's key ^ frame.
 cudaError_t launch_set_state(const unsigned long long* keys, const double* re, const double* im,

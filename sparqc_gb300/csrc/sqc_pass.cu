@@ -227,49 +227,145 @@ __global__ void __launch_bounds__(kThreads, UnitOcc<T, DIMS>::kMin) unit_kernel(
     finish_pass(ctl, cnt_nnz, cnt_empty, upd, nnz_in, a.keys_fixed != 0, a.nx > 0, a.amp_bytes);
 }
 
-// The passes of a flush on a tiny mapped table, one block, one launch (as tiny_kernel below).
+// ---- a run of unit passes in one launch ----------------------------------------------------------
+// Small and middle states spend most of a pass on its edges: a launch of its own waits for the
+// previous pass's last block, publishes the pass through three dependent atomics and reads its
+// gates and the control block before the first unit. A run keeps its blocks for all its passes
+// (a cooperative launch: every block is resident) and meets at a counter between them, with the
+// next pass's gates staged while it waits. No pass of a run refuses (the host ends a run before one
+// that would), and all that a pass publishes is linear in its counts, so each thread adds
+// its own up and the last block to finish publishes the whole run.
+struct ParamHeads {   // the heads in the parameter bank from word o on
+    const RunArgs& a;
+    uint32_t o;
+    __device__ __forceinline__ UnitHead operator[](uint32_t i) const { return a.words[o + i]; }
+};
+
+template <class T>
+__device__ __forceinline__ void stage_run(UGates<T>& sg, const RunArgs& a, uint32_t o) {
+    const uint32_t ng = a.words[o].om & 0xFFu;
+    const GateDesc* gates = a.gates + a.words[o].loc;
+    for (uint32_t i = threadIdx.x; i < ng; i += blockDim.x) stage_ugate(sg.g + i, gates + i);
+    for (uint32_t i = threadIdx.x; i < ng * 32u; i += blockDim.x)
+        sg.lw[i >> 5][i & 31u] = short_word(lane_word(a.words[o + 1 + (i >> 5)].loc, i & 31u));
+}
+
+constexpr unsigned kMaxPolls = 1u << 22;   // a few seconds: far longer than any pass of a run
+
 template <class T, int DIMS>
-__global__ void __launch_bounds__(kThreads) tiny_unit_kernel(PassArgs a, const TinyPass* __restrict__ tp, uint32_t np) {
-    __shared__ UGates<T> sg;
-    __shared__ unsigned long long red[3][kThreads / 32];
+__global__ void __launch_bounds__(kThreads, UnitOcc<T, DIMS>::kMin) run_kernel(const __grid_constant__ RunArgs a) {
+    __shared__ UGates<T> sg[2];
+    __shared__ unsigned long long acc[3][kThreads];   // each thread's own: amp updates, bytes, bytes of pair passes
+    __shared__ unsigned long long red[5], n_sh;
+    __shared__ int stop, last;
     Ctl* ctl = a.ctl;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (*(volatile unsigned int*)&ctl->status) return;
-    const unsigned ep = *(volatile unsigned int*)&ctl->epoch;
-    unsigned long long nnz_in = *(volatile unsigned long long*)&ctl->nnz;
-    for (uint32_t p = 0; p < np; ++p) {
-        const TinyPass q = tp[p];
-        if ((1ULL << q.dn) > a.max_groups) {   // refuse before touching the state
-            if (threadIdx.x == 0) atomicCAS(&ctl->status, 0u, (unsigned)ST_GROW);
-            return;
+    const unsigned ep = ctl->epoch;
+    unsigned long long n = *(volatile unsigned long long*)&ctl->list_n;   // live buckets, at least
+    const unsigned long long moved = 8ULL + a.amp_bytes, fixed = 8ULL + 2ULL * a.amp_bytes;
+    {
+        const uint32_t f = a.words[0].om;
+        const unsigned long long in = blockIdx.x == 0 && threadIdx.x == 0 ? *(volatile unsigned long long*)&ctl->nnz : 0;
+        acc[0][threadIdx.x] = 0;
+        acc[1][threadIdx.x] = in * (f & kRunFixed ? fixed : moved);
+        acc[2][threadIdx.x] = f & kRunPair ? in * (f & kRunFixed ? fixed : moved) : 0;
+        if (threadIdx.x < 5) red[threadIdx.x] = 0;
+        if (threadIdx.x == 0) stop = 0;
+    }
+    const int lane = threadIdx.x & 31;
+    // a pass of fewer units than warps spreads them over the blocks
+    const unsigned w = __shfl_sync(kFull, threadIdx.x >> 5, 0) * gridDim.x + blockIdx.x;
+    const unsigned nw = gridDim.x * (blockDim.x >> 5);
+    stage_run<T>(sg[0], a, 0);
+    __syncthreads();
+    uint32_t o = 0;
+    unsigned long long cnt_nnz, cnt_empty;
+    for (uint32_t p = 0;; ++p) {
+        const UnitHead rec = a.words[o];
+        const uint32_t ng = rec.om & 0xFFu, dn = rec.om >> 16;
+        const UnitPass up = unit_pass<DIMS>(dn, rec.ov & 0xFFu, (rec.ov >> 8) & 0xFFu, (rec.ov >> 16) & 0xFFu);
+        const ParamHeads heads{a, o + 1};
+        const GateDesc* gates = a.gates + rec.loc;
+        unsigned long long upd = 0;
+        cnt_nnz = cnt_empty = 0;
+        if (walk_list(n, dn)) {
+            for (unsigned long long e0 = w * 32ULL; e0 < n; e0 += nw * 32ULL)
+                walk_entries<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, e0, n, heads, sg[p & 1], gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+        } else {
+            walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, nw, heads, sg[p & 1], gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
         }
-        stage_ugates<T>(sg, a.gates, q.g0, q.g1);
-        const UnitPass up = unit_pass<DIMS>(q.dn, q.dim[0], q.dim[1], q.dim[2]);
-        unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
-        walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, kThreads / 32, SharedHeads<T>{sg.g}, sg, a.gates + q.g0, q.g1 - q.g0, lane, a.prune,
-                            cnt_nnz, cnt_empty, upd);
-        cnt_nnz = warp_sum(cnt_nnz);
-        cnt_empty = warp_sum(cnt_empty);
-        upd = warp_sum(upd);
-        if (lane == 0) { red[0][w] = cnt_nnz; red[1][w] = cnt_empty; red[2][w] = upd; }
+        o += 1 + ng;
+        const bool end = p + 1 == a.np;
+        const uint32_t f = rec.om, g = end ? 0u : a.words[o].om;
+        const unsigned long long out = f & kRunFixed ? 0 : moved, in = end ? 0 : g & kRunFixed ? fixed : moved;
+        acc[0][threadIdx.x] += upd;
+        acc[1][threadIdx.x] += cnt_nnz * (out + in);
+        acc[2][threadIdx.x] += cnt_nnz * ((f & kRunPair ? out : 0) + (g & kRunPair ? in : 0));
+        if (end) break;
+        // every block's pass is done before any block's next one; whether the next pass walks the list
+        // (and needs its exact length) follows from what every block knows
+        const bool list = walk_list(n, g >> 16);
+        const uint32_t tag = a.tag + p;
         __syncthreads();
-        unsigned long long tn = 0;   // every thread knows the pass's key count
-        for (int i = 0; i < kThreads / 32; ++i) tn += red[0][i];
-        if (threadIdx.x == 0) {
-            unsigned long long te = 0, tu = 0;
-            for (int i = 0; i < kThreads / 32; ++i) { te += red[1][i]; tu += red[2][i]; }
-            ctl->nnz = tn;
-            ctl->empty_groups = te;
-            ctl->list_n = *(volatile unsigned long long*)&ctl->list_tail;
-            ctl->amp_updates += tu;
-            const unsigned long long ab = q.keys_fixed ? nnz_in * (8ULL + 2ULL * a.amp_bytes)
-                                                       : (nnz_in + tn) * (8ULL + a.amp_bytes);
-            ctl->alg_bytes += ab;
-            if (q.nx > 0) ctl->alg_bytes_pair += ab;
-            ctl->seq += 1;
+        if (gridDim.x == 1) {
+            if (threadIdx.x == 0 && list) n_sh = *(volatile unsigned long long*)&ctl->list_tail;
+            stage_run<T>(sg[(p + 1) & 1], a, o);
+        } else {
+            if (threadIdx.x == 0) {
+                __threadfence();
+                const unsigned prev = atomicAdd(&ctl->bar, 1u);
+                if (list && prev + 1 == gridDim.x * (p + 1)) {   // all are here and none goes on: the length is exact
+                    __threadfence();
+                    const unsigned long long len = *(volatile unsigned long long*)&ctl->list_tail;
+                    atomicExch(&ctl->bar_len, ((unsigned long long)tag << 32) | len);
+                }
+            }
+            stage_run<T>(sg[(p + 1) & 1], a, o);
+            if (threadIdx.x == 0) {
+                unsigned left = kMaxPolls;
+                if (list) {
+                    unsigned long long v;
+                    while ((uint32_t)((v = *(volatile unsigned long long*)&ctl->bar_len) >> 32) != tag && --left) {}
+                    n_sh = v & 0xFFFFFFFFULL;
+                } else {
+                    while (*(volatile unsigned int*)&ctl->bar < gridDim.x * (p + 1) && --left) {}
+                }
+                if (!left) {
+                    atomicCAS(&ctl->status, 0u, (unsigned)ST_TIMEOUT);
+                    stop = 1;
+                }
+                __threadfence();
+            }
         }
-        nnz_in = tn;
-        __syncthreads();   // the pass is published, and red and sg are free, before the next one
+        __syncthreads();
+        if (stop) return;
+        if (list) n = n_sh;
+    }
+    // publish the run
+    const unsigned long long v[5] = {warp_sum(cnt_nnz), warp_sum(cnt_empty), warp_sum(acc[0][threadIdx.x]),
+                                     warp_sum(acc[1][threadIdx.x]), warp_sum(acc[2][threadIdx.x])};
+    if (lane == 0)
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+            if (v[i]) atomicAdd(&red[i], v[i]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (red[0]) atomicAdd(&ctl->acc_nnz, red[0]);
+        if (red[1]) atomicAdd(&ctl->acc_empty, red[1]);
+        if (red[2]) atomicAdd(&ctl->amp_updates, red[2]);
+        if (red[3]) atomicAdd(&ctl->alg_bytes, red[3]);
+        if (red[4]) atomicAdd(&ctl->alg_bytes_pair, red[4]);
+        __threadfence();
+        last = atomicAdd(&ctl->bar, 1u) + 1 == gridDim.x * (gridDim.x == 1 ? 1u : a.np);
+        if (last) {
+            __threadfence();
+            ctl->nnz = atomicExch(&ctl->acc_nnz, 0ULL);
+            ctl->empty_groups = atomicExch(&ctl->acc_empty, 0ULL);
+            ctl->list_n = *(volatile unsigned long long*)&ctl->list_tail;
+            ctl->seq += a.np;
+            ctl->bar = 0;
+            __threadfence();
+        }
     }
 }
 
@@ -752,6 +848,28 @@ cudaError_t launch_unit(const PassArgs& a, int sms, cudaStream_t st) {
     return launch_dep(unit_kernel<T, DIMS>, grid, kThreads, 0, a, st);
 }
 
+// A run's blocks: a warp per unit of its largest pass, at most one resident wave. Few units get blocks
+// of four warps, one for each scheduler of an SM, on more SMs.
+template <class T, int DIMS>
+cudaError_t launch_run(const RunArgs& a, uint32_t dn, int sms, cudaStream_t st) {
+    static int resident = 0;
+    if (!resident) resident = occupancy(run_kernel<T, DIMS>, kThreads, 0);
+    const unsigned long long units = std::max<unsigned long long>(1, (1ULL << dn) >> DIMS);
+    const int threads = units <= 4ULL * (unsigned long long)sms ? 128 : kThreads;
+    const unsigned long long wave = (unsigned long long)sms * resident;
+    const int grid = (int)std::max<unsigned long long>(1, std::min<unsigned long long>(wave, (units + threads / 32 - 1) / (threads / 32)));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = grid > 1 ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, run_kernel<T, DIMS>, a);
+}
+
 template <class T, int NX>
 cudaError_t launch_staged(const PassArgs& a, int grid, cudaStream_t st) {
     staged_kernel<T, NX><<<grid, kStagedThreads, staged_smem<T, NX>(), st>>>(a);
@@ -769,17 +887,15 @@ int launch_tiny(const PassArgs& a, const TinyPass* passes, uint32_t np, bool dbl
     return cudaGetLastError() == cudaSuccess ? 1 : -1;
 }
 
-int launch_tiny_units(const PassArgs& a, const TinyPass* passes, uint32_t np, bool dbl, cudaStream_t st) {
-    if (a.t.mask + 1 > kTinyMaxBuckets) return -1;
-    if (!dbl) tiny_unit_kernel<float, 3><<<1, kThreads, 0, st>>>(a, passes, np);
-    else if (a.dims == 3) tiny_unit_kernel<double, 3><<<1, kThreads, 0, st>>>(a, passes, np);
-    else tiny_unit_kernel<double, 2><<<1, kThreads, 0, st>>>(a, passes, np);
-    return cudaGetLastError() == cudaSuccess ? 1 : -1;
-}
-
 int launch_unit_pass(const PassArgs& a, bool dbl, int sms, cudaStream_t st) {
     const cudaError_t e = !dbl ? launch_unit<float, 3>(a, sms, st)
                           : a.dims == 3 ? launch_unit<double, 3>(a, sms, st) : launch_unit<double, 2>(a, sms, st);
+    return e == cudaSuccess ? 1 : -1;
+}
+
+int launch_unit_run(const RunArgs& a, uint32_t dims, uint32_t dn, bool dbl, int sms, cudaStream_t st) {
+    const cudaError_t e = !dbl ? launch_run<float, 3>(a, dn, sms, st)
+                          : dims == 3 ? launch_run<double, 3>(a, dn, sms, st) : launch_run<double, 2>(a, dn, sms, st);
     return e == cudaSuccess ? 1 : -1;
 }
 

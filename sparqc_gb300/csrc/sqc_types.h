@@ -66,7 +66,7 @@ struct Ctl {
     unsigned int epoch;             // live-bucket epoch of the table
     unsigned int status;            // Status; nonzero stops every later pass until the host repairs
     unsigned int done;              // blocks finished in the running pass
-    unsigned int pad0;
+    unsigned int bar;               // blocks that have met between the passes of a run (0 outside one)
     unsigned long long seq;         // passes completed since the last reset
     unsigned long long nnz;         // keys held
     unsigned long long list_n;      // live buckets (list entries) committed at the last pass end
@@ -81,6 +81,7 @@ struct Ctl {
     unsigned long long acc_max;     // bit pattern of a non-negative double (max |a-b|)
     unsigned long long work;        // list entries handed out in the running pass (0 between passes)
     unsigned long long units_n;     // owned units the running pass's resolve kernel wrote (0 between passes)
+    unsigned long long bar_len;     // a run's live buckets before a pass that walks the list, tagged with the pass
 };
 
 // Gate descriptor with host-resolved coefficients (std::cos/std::sin on the host, so the
@@ -158,9 +159,8 @@ struct alignas(16) UnitHead {
 
 // One pass of a single-launch run over a tiny table (tiny_kernel): what PassArgs says per pass.
 struct TinyPass {
-    uint32_t g0, g1, nx, q1, q2, q3, keys_fixed, dn;
+    uint32_t g0, g1, nx, q1, q2, q3, keys_fixed, pad;
     unsigned long long grow_bound;
-    uint32_t dim[4];        // unit passes: bucket bits of the unit's dimensions (dim[3] unused)
     unsigned long long key_bound;
 };
 
@@ -185,6 +185,23 @@ struct PassArgs {
     // 3) and the bucket bit of each dimension
     uint32_t dn, dims, dim[3];
     UnitHead heads[kMaxRun];   // unit passes: those of the pass's gates (read from the parameter bank)
+};
+
+// A run of unit passes in one launch (run_kernel). words holds the passes one after another: a
+// record (om: gates in bits 0..7, the flags below, mapped bits after the pass from bit 16; ov: the bucket
+// bits of the unit's dimensions, a byte each; loc: the pass's first gate), then the heads of
+// its gates. All of it is read from the parameter bank.
+constexpr uint32_t kRunWords = 496;        // 8 KB of parameters
+constexpr uint32_t kRunFixed = 1u << 8;    // every gate is diagonal
+constexpr uint32_t kRunPair = 1u << 9;     // the pass pairs groups
+struct RunArgs {
+    TableDev t;
+    Ctl* ctl;
+    const GateDesc* gates;
+    PruneBits prune;
+    uint32_t np, amp_bytes;
+    uint32_t tag;              // of the run's first pass: passes of an engine have different ones
+    UnitHead words[kRunWords];
 };
 
 }  // namespace sqc

@@ -712,7 +712,7 @@ __device__ __forceinline__ void walk_entries(const TableDev& t, const uint8_t* m
     unsigned base = 0;
     bool own = false;
     if (e0 + lane < n) {
-        const unsigned b = t.list[e0 + lane];
+        const unsigned b = __ldcg(t.list + e0 + lane);   // (an earlier pass of the same launch may have written it)
         int idx = 0;
         base = b;
 #pragma unroll

@@ -270,3 +270,48 @@ def test_first_run_of_a_full_state_is_mapped(k, depth):
     assert_identical(st.state(sorted=True), first)
     assert st.stats()["passes"] == 2 * passes
     st.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("nq,k,depth", [(8, 5, 60), (12, 9, 200), (16, 12, 700), (18, 16, 300), (24, 20, 120), (24, 23, 60)])
+def test_runs_of_passes_equal_single_passes(nq, k, depth, precision):
+    """The passes of a flush in one launch leave what a launch each leaves (timed passes are launched
+    one by one): keys, amplitudes, counts; one block, several, a full wave, and states too large."""
+    from sparqc_gb300 import engine
+    g = circuits.random_circuit(nq, k, depth, 3, circuits.SplitMix64(circuits.stream_seed("runs", nq * 100 + k)))
+    one = engine.State(nq, precision=precision, time_passes=True)
+    run = engine.State(nq, precision=precision)
+    for st in (one, run):
+        st.apply(g)
+        st.sync()
+    a, b = one.stats(), run.stats()
+    for f in ("passes", "amp_updates", "alg_bytes", "alg_bytes_pair", "passes_pair", "replays"):
+        assert a[f] == b[f], f
+    assert_identical(run.state(), one.state())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("keys", [40, 300, 1500])
+def test_runs_that_walk_the_list(keys, precision):
+    """Few live buckets among the mapped ones: every pass of a run walks the list, whose length
+    changes from pass to pass; with 1500 keys later passes walk every unit."""
+    from sparqc_gb300 import engine
+    rng = np.random.default_rng(keys)
+    key = np.unique(rng.integers(0, 1 << 16, keys, dtype=np.uint64))
+    amp = rng.standard_normal((2, key.size)) / np.sqrt(key.size)
+    c = circuits.SplitMix64(circuits.stream_seed("list", keys))
+    g = [(G.X, 4 + int(c.next() % 12), [int(c.next() % 4)], 0.0) if i % 5 else
+         (G.RY, int(c.next() % 16), [(int(c.next() % 3) + 13)], 0.4) for i in range(80)]
+    g = G.gate_array([(a, t, [q for q in ctl if q != t], th) for a, t, ctl, th in g])
+    states = []
+    for timed in (True, False):
+        st = engine.State(16, precision=precision, time_passes=timed)
+        st.set_state(key, amp[0], amp[1])
+        st.apply(g)
+        st.sync()
+        states.append((st.state(), st.stats()))
+    (sa, a), (sb, b) = states
+    assert [a[f] for f in ("passes", "amp_updates", "alg_bytes")] == [b[f] for f in ("passes", "amp_updates", "alg_bytes")]
+    assert_identical(sb, sa)
