@@ -17,7 +17,6 @@ namespace {
 
 constexpr unsigned long long kMinBuckets = 64;
 constexpr size_t kFlushAt = 1024;          // queued gates that trigger a launch
-constexpr unsigned long long kTinyMaxList = 256;   // live buckets up to which a flush is one launch
 constexpr size_t kDescInitial = 1 << 13;   // descriptors held between verified syncs
 constexpr unsigned long long kEpochRestart = 0xFFFFFF00ULL;   // epochs before the headers are cleared
 constexpr double kMaxLoad = 0.9;           // live buckets a pair pass may leave behind
@@ -29,8 +28,12 @@ constexpr unsigned long long kMapSpan = 16;
 // Buckets a grown mapped table has beyond its span: eight times as many while that is under a
 // gigabyte, so that a state growing one qubit at a time is not rebuilt at every one; then twice.
 constexpr unsigned long long kMapRoomy = 1ULL << 21;
+constexpr double kHashLoad = 0.35;          // ... and a hashed table stays below while memory allows: lookups of absent
+                                            // groups probe to the first free bucket (2^17 keys of logic, 82 passes:
+                                            // 0.9 15.7 ms, 0.7 9.7, 0.5 8.4, 0.35 6.9, 0.25 7.5 with more rebuilds)
 constexpr unsigned long long kHashRoomy = 1ULL << 17;   // 55 MB
 constexpr uint32_t kRunMapFp64 = 18, kRunMapFp32 = 17;   // mapped bits up to which passes go out in runs (sqc_pass.cu: run_kernel)
+constexpr unsigned long long kRunMaxList = 1ULL << 17;   // ... and live buckets of a hashed one
 constexpr uint32_t kNoMap = 63;            // Span::dn of a pass whose bits no table maps: always refused
 
 bool map_worth(uint32_t dn, unsigned long long groups) {
@@ -61,8 +64,6 @@ Engine::~Engine() {
     if (sums_host_) cudaFreeHost(sums_host_);
     if (d_desc_) cudaFree(d_desc_);
     if (h_desc_) cudaFreeHost(h_desc_);
-    if (d_tiny_) cudaFree(d_tiny_);
-    if (h_tiny_) cudaFreeHost(h_tiny_);
     if (d_rk_) cudaFree(d_rk_);   // one allocation with d_rr_ and d_ri_
     rank_.release();
     if (d_cum_) cudaFree(d_cum_);
@@ -93,9 +94,11 @@ int Engine::launch_failed(const char* what) {
 }
 
 size_t Engine::bucket_bytes() const {
-    return sizeof(Header) + kSlots * sizeof(unsigned long long) + kSlots * (dbl_ ? 16 : 8) + sizeof(unsigned) +
-           sizeof(Unit);
+    return sizeof(Header) + kSlots * sizeof(unsigned long long) + kSlots * (dbl_ ? 16 : 8) + sizeof(unsigned);
 }
+
+// Groups up to which a hashed table is kept as it is.
+unsigned long long Engine::roomy_groups() const { return (unsigned long long)(hash_load_ * (double)tab_.nb); }
 
 unsigned long long Engine::max_groups() const { return (unsigned long long)(kMaxLoad * (double)tab_.nb); }
 
@@ -188,7 +191,6 @@ int Engine::alloc_table(unsigned long long nb, HostTable* out) {
     t.keys = reinterpret_cast<unsigned long long*>(base += nb * sizeof(Header));
     t.amps = base += nb * kSlots * sizeof(unsigned long long);
     t.list = reinterpret_cast<unsigned*>(base += nb * kSlots * (dbl_ ? 16 : 8));
-    t.units = reinterpret_cast<Unit*>(base += nb * sizeof(unsigned));
     if ((rc = cuda(cudaMemsetAsync(t.hdr, 0, nb * sizeof(Header), stream_), "cudaMemset(hdr)"))) {
         free_table(&t);
         return rc;
@@ -208,7 +210,6 @@ TableDev Engine::dev() const {
     d.keys = tab_.keys;
     d.amps = tab_.amps;
     d.list = tab_.list;
-    d.units = tab_.units;
     d.mask = tab_.nb - 1;
     d.map_on = 0;
     d.map_n = 0;
@@ -221,19 +222,13 @@ int Engine::ensure_desc(size_t n) {
     const size_t cap = std::max(n, desc_cap_ * 2);
     if (d_desc_) cudaFree(d_desc_);
     if (h_desc_) cudaFreeHost(h_desc_);
-    if (d_tiny_) cudaFree(d_tiny_);
-    if (h_tiny_) cudaFreeHost(h_tiny_);
     d_desc_ = nullptr;
     h_desc_ = nullptr;
-    d_tiny_ = nullptr;
-    h_tiny_ = nullptr;
     desc_cap_ = 0;
     int rc;
     if ((rc = cuda(cudaMalloc(&d_desc_, cap * sizeof(GateDesc)), "cudaMalloc(desc)"))) return rc;
     if ((rc = cuda(cudaMallocHost(&h_desc_, cap * sizeof(GateDesc)), "cudaMallocHost(desc)"))) return rc;
     // tiny-launch pass records, indexed like the descriptors (a flush has no more passes than gates)
-    if ((rc = cuda(cudaMalloc(&d_tiny_, cap * sizeof(TinyPass)), "cudaMalloc(tiny)"))) return rc;
-    if ((rc = cuda(cudaMallocHost(&h_tiny_, cap * sizeof(TinyPass)), "cudaMallocHost(tiny)"))) return rc;
     desc_cap_ = cap;
     return SQC_OK;
 }
@@ -439,10 +434,36 @@ int Engine::flush(bool hold_last) {
         unsigned long long keys;     // keys after the pass, at most
     };
     std::vector<Span> spans;
-    split_passes(hd, nd, max_run_, max_nx_,
-                 [&](size_t g0, size_t g1, uint32_t nx, uint32_t q1, uint32_t q2, uint32_t q3, bool fixed) {
-                     spans.push_back(Span{g0, g1, nx, q1, q2, q3, fixed, 0, 0, {0, 0, 0}, 0});
-                 });
+    // mapped tables pair up to max_nx_ qubits >= 4 a pass, hashed ones two of any (columns)
+    auto split = [&] {
+        spans.clear();
+        split_passes(hd, nd, max_run_, mapped_ ? max_nx_ : std::min(max_nx_, 2u),
+                     [&](size_t g0, size_t g1, uint32_t, uint32_t q1, uint32_t q2, uint32_t q3, bool fixed) {
+                         uint32_t nx = 0;   // qubits that pair groups
+                         for (uint32_t q : {q1, q2, q3}) nx += q != kNoQubit && q >= (uint32_t)kSlotBits ? 1 : 0;
+                         spans.push_back(Span{g0, g1, nx, q1, q2, q3, fixed, 0, 0, {0, 0, 0}, 0});
+                     }, !mapped_);
+        unsigned long long keys = key_hint_;   // a branching gate at most doubles them
+        for (Span& sp : spans) {
+            for (size_t i = sp.g0; i < sp.g1; ++i)
+                if (is_branch_kind(hd[i].kind)) keys = std::min(keys * 2, kKeysUnknown);
+            sp.keys = keys;
+        }
+    };
+    split();
+    if (fresh_ && mapped_) {
+        // a state that will spread too thinly for any map starts hashed: |0...0> lies in bucket 0
+        // either way, so nothing moves
+        GroupMap m;
+        for (const Span& sp : spans) {
+            const bool fits = m.extend(after[sp.g1 - 1].kmask, nq_);
+            if (fits && ((1ULL << m.n) <= max_groups() || map_worth(m.n, sp.keys))) continue;
+            mapped_ = false;
+            a.t = dev();
+            split();
+            break;
+        }
+    }
     if (hold_last && spans.size() >= 2) {
         // the last pass's gates, and the host-resolved gates around them, go back to the queue;
         // the planner returns to its state after the last device gate that is launched
@@ -457,29 +478,13 @@ int Engine::flush(bool hold_last) {
     // how each pass applies its gates: by place in its units (mapped tables; the map grows with
     // the bits its gates make differ) or by key (hashed ones)
     const uint32_t dims = dbl_ && max_nx_ < 3 ? 2u : 3u;
-    unsigned long long keys = key_hint_;   // a branching gate at most doubles them
-    for (Span& sp : spans) {
-        for (size_t i = sp.g0; i < sp.g1; ++i)
-            if (is_branch_kind(hd[i].kind)) keys = std::min(keys * 2, kKeysUnknown);
-        sp.keys = keys;
-    }
-    if (fresh_ && mapped_) {
-        // a state that will spread too thinly for any map starts hashed: |0...0> lies in bucket 0
-        // either way, so nothing moves
-        GroupMap m;
-        for (const Span& sp : spans) {
-            const bool fits = m.extend(after[sp.g1 - 1].kmask, nq_);
-            if (fits && ((1ULL << m.n) <= max_groups() || map_worth(m.n, sp.keys))) continue;
-            mapped_ = false;
-            a.t = dev();
-            break;
-        }
-    }
     fresh_ = fresh_ && spans.empty();
     for (Span& sp : spans) {
         const uint32_t q[3] = {sp.q1, sp.q2, sp.q3};
-        encode_pass(hd, sp.g0, sp.g1, sp.q1, sp.q3);
-        if (!mapped_) continue;
+        if (!mapped_) {
+            encode_column_pass(hd, sp.g0, sp.g1, q, sp.dim);
+            continue;
+        }
         sp.map0 = map_.n;
         sp.dn = kNoMap;   // more bits than a table maps: the pass refuses, and the state is hashed then
         if (!map_.extend(after[sp.g1 - 1].kmask, nq_)) continue;
@@ -493,57 +498,6 @@ int Engine::flush(bool hold_last) {
         return rc;
     cudaEvent_t ev_prev = nullptr;
     if (time_passes_ && (rc = record_event(&ev_prev))) return rc;
-    // a tiny hashed state runs the flush's passes in one single-block launch (tiny_kernel): the live
-    // buckets every pass may reach stay few enough that launches would cost more than the work
-    {
-        unsigned long long h = list_hint_, hmax = list_hint_;
-        for (const Span& sp : spans) {
-            if (sp.nx)
-                h = std::min<unsigned long long>({tab_.nb, h << sp.nx, h + sp.keys, group_bound(after[sp.g1 - 1], nq_)});
-            hmax = std::max(hmax, h);
-        }
-        if (!mapped_ && spans.size() >= 2 && tiny_table(tab_.nb) && hmax <= kTinyMaxList) {
-            TinyPass* ht = h_tiny_ + desc_used_;
-            bool any_pair = false;
-            for (size_t k = 0; k < spans.size(); ++k) {
-                const Span& sp = spans[k];
-                TinyPass& q = ht[k];
-                q.g0 = (uint32_t)sp.g0;
-                q.g1 = (uint32_t)sp.g1;
-                q.nx = sp.nx;
-                q.q1 = sp.q1;
-                q.q2 = sp.q2;
-                q.q3 = sp.q3;
-                q.keys_fixed = sp.fixed ? 1u : 0u;
-                q.pad = 0;
-                q.grow_bound = group_bound(after[sp.g1 - 1], nq_);
-                q.key_bound = sp.keys;
-                any_pair = any_pair || sp.nx > 0;
-            }
-            if ((rc = cuda(cudaMemcpyAsync(d_tiny_ + desc_used_, ht, spans.size() * sizeof(TinyPass),
-                                           cudaMemcpyHostToDevice, stream_), "H2D tiny passes")))
-                return rc;
-            if (launch_tiny(a, d_tiny_ + desc_used_, (uint32_t)spans.size(), dbl_, stream_) < 0)
-                return launch_failed("tiny passes");
-            if (time_passes_) {
-                cudaEvent_t ev = nullptr;
-                if ((rc = record_event(&ev))) return rc;
-                timed_.push_back(TimedPass{ev_prev, ev, any_pair});
-            }
-            for (const Span& sp : spans) {
-                passes_pair_ += sp.nx > 0 ? 1 : 0;
-                passes_.push_back(PassRec{snap_log_, snap_plan_, sp.map0, sp.dn, sp.nx, sp.keys});
-                snap_log_ = src[sp.g1 - 1] + 1;
-                snap_plan_ = after[sp.g1 - 1];
-                ++passes_run_;
-            }
-            ++launches_;
-            list_hint_ = h;
-            key_hint_ = keys;
-            desc_used_ += nd;
-            return SQC_OK;
-        }
-    }
     auto record = [&](const Span& sp) {
         passes_pair_ += sp.nx > 0 ? 1 : 0;
         passes_.push_back(PassRec{snap_log_, snap_plan_, sp.map0, sp.dn, sp.nx, sp.keys});
@@ -556,11 +510,23 @@ int Engine::flush(bool hold_last) {
     RunArgs run;
     for (size_t s = 0; s < spans.size();) {
         const Span& sp = spans[s];
-        // consecutive passes of a small or middle mapped state go out in one launch
+        // consecutive passes of a small or middle state go out in one launch, up to one that the table is
+        // known or may turn out to be too small for
         size_t e = s, words = 0;
-        while (mapped_ && !time_passes_ && e < spans.size() && spans[e].dn <= (dbl_ ? kRunMapFp64 : kRunMapFp32) &&
-               (1ULL << spans[e].dn) <= a.max_groups && words + 1 + spans[e].g1 - spans[e].g0 <= kRunWords) {
-            words += 1 + spans[e].g1 - spans[e].g0;
+        unsigned long long items = list_hint_;
+        while (!time_passes_ && e < spans.size()) {
+            const Span& r = spans[e];
+            const size_t w = mapped_ ? 1 + r.g1 - r.g0 : 2;
+            if (words + w > kRunWords) break;
+            if (mapped_) {
+                if (r.dn > (dbl_ ? kRunMapFp64 : kRunMapFp32) || (1ULL << r.dn) > a.max_groups) break;
+                items = std::max(1ULL, (1ULL << r.dn) >> dims);
+            } else if (r.nx) {
+                const unsigned long long h = std::min({group_bound(after[r.g1 - 1], nq_), items << r.nx, items + r.keys});
+                if (h > roomy_groups() || h > kRunMaxList) break;
+                items = h;
+            }
+            words += w;
             ++e;
         }
         if (e - s >= 2) {
@@ -569,18 +535,25 @@ int Engine::flush(bool hold_last) {
             run.gates = a.gates;
             run.prune = a.prune;
             run.amp_bytes = a.amp_bytes;
+            run.max_groups = a.max_groups;
             run.np = (uint32_t)(e - s);
             run.tag = run_tag_;
             run_tag_ += run.np;
             UnitHead* w = run.words;
             for (; s < e; ++s) {
                 const Span& r = spans[s];
-                *w++ = UnitHead{(uint32_t)(r.g1 - r.g0) | (r.fixed ? kRunFixed : 0u) | (r.nx ? kRunPair : 0u) | (r.dn << 16),
+                *w++ = UnitHead{(uint32_t)(r.g1 - r.g0) | (r.fixed ? kRunFixed : 0u) | (r.nx ? kRunPair : 0u) |
+                                    ((mapped_ ? r.dn : r.nx) << 16),
                                 r.dim[0] | (r.dim[1] << 8) | (r.dim[2] << 16), (uint32_t)r.g0, 0u};
-                for (size_t k = r.g0; k < r.g1; ++k) *w++ = UnitHead{hd[k].om, hd[k].ov, hd[k].loc, hd[k].pad + 1u};
+                if (mapped_) {
+                    for (size_t k = r.g0; k < r.g1; ++k) *w++ = UnitHead{hd[k].om, hd[k].ov, hd[k].loc, hd[k].pad + 1u};
+                } else {
+                    const unsigned long long bounds[2] = {group_bound(after[r.g1 - 1], nq_), r.keys};
+                    std::memcpy(w++, bounds, sizeof bounds);
+                }
                 record(r);
             }
-            const int nl = launch_unit_run(run, dims, spans[e - 1].dn, dbl_, sms_, stream_);
+            const int nl = launch_run_passes(run, dims, items, dbl_, sms_, stream_);
             if (nl < 0) return launch_failed("gate passes");
             launches_ += (uint64_t)nl;
             continue;
@@ -589,13 +562,10 @@ int Engine::flush(bool hold_last) {
         a.g0 = (uint32_t)sp.g0;
         a.g1 = (uint32_t)sp.g1;
         a.nx = sp.nx;
-        a.q1 = sp.q1;
-        a.q2 = sp.q2;
-        a.q3 = sp.q3;
         a.keys_fixed = sp.fixed ? 1u : 0u;
         a.grow_bound = group_bound(after[sp.g1 - 1], nq_);
         a.key_bound = sp.keys;
-        if (!mapped_ && sp.nx && grown(sp.nx, a.grow_bound, sp.keys) > a.max_groups) {
+        if (!mapped_ && sp.nx && grown(sp.nx, a.grow_bound, sp.keys) > roomy_groups()) {
             if ((rc = make_room(sp.nx, a.grow_bound, sp.keys))) return rc;
             a.t = dev();
             a.max_groups = max_groups();
@@ -605,7 +575,7 @@ int Engine::flush(bool hold_last) {
         for (int d = 0; d < 3; ++d) a.dim[d] = sp.dim[d];
         if (mapped_)
             for (size_t k = sp.g0; k < sp.g1; ++k) a.heads[k - sp.g0] = UnitHead{hd[k].om, hd[k].ov, hd[k].loc, hd[k].pad + 1u};
-        const int nl = mapped_ ? launch_unit_pass(a, dbl_, sms_, stream_) : launch_pass(a, hint, dbl_, sms_, stream_);
+        const int nl = mapped_ ? launch_unit_pass(a, dbl_, sms_, stream_) : launch_hash_pass(a, hint, dbl_, sms_, stream_);
         if (nl < 0) return launch_failed("gate pass");
         if (time_passes_) {
             cudaEvent_t ev = nullptr;
@@ -638,7 +608,7 @@ unsigned long long Engine::hashed_size(unsigned long long groups, uint32_t nx, u
     const double by_keys = (double)groups + 4.0 * (double)keys;
     const double one_pass = std::min((double)groups * (double)(1u << nx), (double)groups + (double)keys);
     const double want = std::max(one_pass, std::min(room, by_keys));
-    const unsigned long long nb = std::max(kMinBuckets, pow2_at_least((unsigned long long)std::ceil(want / kMaxLoad)));
+    const unsigned long long nb = std::max(kMinBuckets, pow2_at_least((unsigned long long)std::ceil(want / kHashLoad)));
     return std::max(nb, std::min(nb * 32, kHashRoomy));
 }
 
@@ -650,11 +620,16 @@ int Engine::make_room(uint32_t nx, unsigned long long bound, unsigned long long 
     if ((rc = read_ctl())) return rc;
     if (ctl_host_->status != ST_OK) return SQC_OK;   // an earlier pass refused or failed: sync() deals with it
     list_hint_ = std::max<unsigned long long>(ctl_host_->list_n, 1);
-    if (grown(nx, bound, keys) <= max_groups()) return SQC_OK;
+    if (grown(nx, bound, keys) <= roomy_groups()) return SQC_OK;
     const unsigned long long groups = ctl_host_->list_n - std::min(ctl_host_->list_n, ctl_host_->empty_groups);
-    const unsigned long long nb = std::max(tab_.nb, hashed_size(groups, nx, keys));
-    if ((double)nb * bucket_bytes() > (double)budget_) return SQC_OK;   // the pass refuses; sync() decides
+    unsigned long long nb = std::max(tab_.nb, hashed_size(groups, nx, keys));
+    while (nb > tab_.nb && (double)nb * bucket_bytes() > (double)budget_) nb /= 2;
+    if (nb == tab_.nb && ctl_host_->empty_groups * 4 < ctl_host_->list_n) {   // as large as it gets: fill it up
+        hash_load_ = kMaxLoad;
+        return SQC_OK;   // a pass that still does not fit refuses; sync() decides
+    }
     if ((rc = rebuild(nb, false))) return rc;
+    if (grown(nx, bound, keys) > roomy_groups()) hash_load_ = kMaxLoad;
     passes_.clear();   // all verified: later ones count from here
     return SQC_OK;
 }
@@ -795,6 +770,7 @@ int Engine::sync() {
 // Copy the live, non-empty buckets into a new table of nb_new buckets. The control block
 // must be in sync with the device (read_ctl) and no pass may be in flight.
 int Engine::rebuild(unsigned long long nb_new, bool mapped) {
+    hash_load_ = kHashLoad;
     HostTable nt;
     int rc;
     if ((rc = alloc_table(nb_new, &nt))) return rc;
@@ -810,13 +786,11 @@ int Engine::rebuild(unsigned long long nb_new, bool mapped) {
     c.list_tail = 0;
     c.empty_groups = 0;
     c.acc_nnz = c.acc_empty = c.acc_upd = 0;
-    c.work = 0;
-    c.units_n = 0;
     std::memcpy(ctl_host_, &c, sizeof c);
     if ((rc = cuda(cudaMemcpyAsync(ctl_, ctl_host_, sizeof(Ctl), cudaMemcpyHostToDevice, stream_), "H2D ctl")))
         return rc;
     TableDev nd;
-    nd.hdr = nt.hdr; nd.keys = nt.keys; nd.amps = nt.amps; nd.list = nt.list; nd.units = nt.units;
+    nd.hdr = nt.hdr; nd.keys = nt.keys; nd.amps = nt.amps; nd.list = nt.list;
     nd.mask = nt.nb - 1;
     nd.map_on = 0;
     nd.map_n = 0;
@@ -1188,7 +1162,7 @@ int Engine::measure(uint32_t qubit, double u, int* outcome, double* p1) {
                    "collapse")))
         return rc;
     launches_ += 2;
-    if (mapped_) {   // the kept keys are the buckets' presence masks now
+    {   // the kept keys are the buckets' presence masks now
         if ((rc = cuda(launch_refresh_masks(dev(), ctl_, list_hint_, sms_, stream_), "refresh masks"))) return rc;
         ++launches_;
     }

@@ -21,7 +21,6 @@ struct HostTable {
     unsigned long long* keys = nullptr;
     void* amps = nullptr;
     unsigned int* list = nullptr;
-    Unit* units = nullptr;
     unsigned long long nb = 0;
 };
 
@@ -127,6 +126,7 @@ private:
     int record_event(cudaEvent_t* out);
     void harvest_events();
     unsigned long long max_groups() const;
+    unsigned long long roomy_groups() const;
 
     int device_ = 0;
     int sms_ = 1;
@@ -177,8 +177,6 @@ private:
 
     GateDesc* d_desc_ = nullptr;
     GateDesc* h_desc_ = nullptr;
-    TinyPass* d_tiny_ = nullptr;    // pass records of single-launch flushes (tiny states)
-    TinyPass* h_tiny_ = nullptr;
     size_t desc_cap_ = 0, desc_used_ = 0;
 
     unsigned long long* d_rk_ = nullptr;
@@ -192,6 +190,7 @@ private:
     void* d_cum_tmp_ = nullptr;
     size_t cum_cap_ = 0, cum_tmp_bytes_ = 0;
 
+    double hash_load_ = 0.35;       // load up to which a hashed table stays as it is
     uint32_t run_tag_ = 1;          // RunArgs.tag of the next run
     uint64_t gates_applied_ = 0, passes_run_ = 0, launches_ = 0, replays_ = 0, rebuilds_ = 0;
     uint64_t passes_pair_ = 0;

@@ -126,7 +126,6 @@ extern "C" int sqc_apply_fixed(uint32_t nq, const uint64_t* keys_in, const doubl
     t.keys = reinterpret_cast<unsigned long long*>(b + kOffKeys);
     t.amps = b + kOffAmps;
     t.list = reinterpret_cast<unsigned*>(b + kOffList);
-    t.units = nullptr;    // small tables take the direct pass, which needs neither
     t.mask = kFixedBuckets - 1;
     t.map_on = 0;         // the scratch table is hashed
     t.map_n = 0;
@@ -154,25 +153,28 @@ extern "C" int sqc_apply_fixed(uint32_t nq, const uint64_t* keys_in, const doubl
                                                      outside, ctl);
         if (cudaGetLastError() != cudaSuccess) return SQC_ERR_CUDA;
     }
-    // same pass split as the engine with one cross-group qubit per pass: one cross-group gate,
-    // then a stream run; each pass's gates are encoded before the descriptors are uploaded
+    // passes that pair across one qubit; each pass's gates are encoded before the descriptors are uploaded
     struct Span {
-        uint32_t g0, g1, q1;
+        uint32_t g0, g1, dim[3];
         bool pair, fixed;
     };
     Span spans[kFixedMaxGates];
     size_t ns = 0, i = 0;
     while (i < n_gates) {
         const size_t start = i;
-        auto streamable = [&](size_t k) { return hd[k].target < (uint32_t)kSlotBits || diag_kind(hd[k].kind); };
-        const bool pair = !streamable(i);
-        if (pair) ++i;
-        while (i < n_gates && i - start < (size_t)kMaxRun && streamable(i)) ++i;
+        uint32_t pairing = kNoQubit;
+        for (; i < n_gates && i - start < (size_t)kMaxRun; ++i) {
+            if (diag_kind(hd[i].kind) || hd[i].target == pairing) continue;
+            if (pairing != kNoQubit) break;
+            pairing = hd[i].target;
+        }
+        const bool pair = pairing != kNoQubit && pairing >= (uint32_t)kSlotBits;
         bool fixed = true;
         for (size_t k = start; k < i; ++k) fixed = fixed && diag_kind(hd[k].kind);
-        const uint32_t q1 = pair ? hd[start].target : kNoQubit;
-        encode_pass(hd, start, i, q1);
-        spans[ns++] = Span{(uint32_t)start, (uint32_t)i, q1, pair, fixed};
+        const uint32_t q[2] = {pairing, kNoQubit};
+        Span& sp = spans[ns++];
+        sp = Span{(uint32_t)start, (uint32_t)i, {0, 0, 0}, pair, fixed};
+        encode_column_pass(hd, start, i, q, sp.dim);
     }
     if (n_gates && cudaMemcpyAsync(d_desc, hd, n_gates * sizeof(GateDesc), cudaMemcpyHostToDevice, st) != cudaSuccess)
         return SQC_ERR_CUDA;
@@ -193,13 +195,12 @@ extern "C" int sqc_apply_fixed(uint32_t nq, const uint64_t* keys_in, const doubl
         a.g0 = spans[k].g0;
         a.g1 = spans[k].g1;
         a.nx = spans[k].pair ? 1u : 0u;
-        a.q1 = spans[k].q1;
-        a.q2 = kNoQubit;
-        a.q3 = kNoQubit;
+        a.dims = 2;
+        for (int d = 0; d < 3; ++d) a.dim[d] = spans[k].dim[d];
         a.grow_bound = ~0ULL;
         a.key_bound = kKeysUnknown;
         a.keys_fixed = spans[k].fixed ? 1u : 0u;
-        if (launch_pass(a, kFixedBuckets, true, sms, st) < 0) return SQC_ERR_CUDA;
+        if (launch_hash_pass(a, kFixedBuckets, true, sms, st) < 0) return SQC_ERR_CUDA;
     }
     if (launch_readout(t, ctl, kFixedBuckets, 0ULL, true, reinterpret_cast<unsigned long long*>(keys_out), re_out,
                        im_out, cap_out, false, a.prune, sms, st) != cudaSuccess)

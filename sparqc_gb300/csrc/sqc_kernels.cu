@@ -54,8 +54,6 @@ __global__ void set_zero_kernel(TableDev t, Ctl* ctl, int dbl) {
         ctl->status = 0;
         ctl->done = 0;
         ctl->bar = 0;
-        ctl->work = 0;
-        ctl->units_n = 0;
         ctl->acc_nnz = ctl->acc_empty = ctl->acc_upd = 0;
         ctl->seq = 0;
         ctl->amp_updates = 0;
@@ -70,7 +68,7 @@ __global__ void set_zero_kernel(TableDev t, Ctl* ctl, int dbl) {
         const size_t s = (size_t)b * kSlots + lane;
         t.keys[s] = lane == 0 ? 0ULL : empty_key(lane);
         if (lane == 0) {
-            if (t.map_on) t.hdr[b].aux = 1u;   // presence mask: slot 0
+            t.hdr[b].aux = 1u;   // presence mask: slot 0
             if (dbl) reinterpret_cast<double2*>(t.amps)[s] = make_double2(1.0, 0.0);
             else reinterpret_cast<float2*>(t.amps)[s] = make_float2(1.0f, 0.0f);
         }
@@ -90,8 +88,6 @@ __global__ void set_state_begin_kernel(Ctl* ctl) {
     ctl->status = 0;
     ctl->done = 0;
     ctl->bar = 0;
-    ctl->work = 0;
-    ctl->units_n = 0;
     ctl->acc_nnz = ctl->acc_empty = ctl->acc_upd = 0;
     ctl->seq = 0;
     ctl->amp_updates = 0;
@@ -150,7 +146,7 @@ __global__ void set_state_end_kernel(Ctl* ctl, unsigned long long n) {
     ctl->nnz = n;
 }
 
-// Presence masks of a mapped table's listed buckets, from their keys (a half-warp per bucket).
+// Presence masks of a table's listed buckets, from their keys (a half-warp per bucket).
 __global__ void refresh_masks_kernel(TableDev t, Ctl* ctl) {
     const unsigned long long n = ctl->list_tail;
     const int lane = threadIdx.x & 31, j = lane & 15;
@@ -341,7 +337,7 @@ __global__ void rehash_kernel(TableDev told, unsigned long long n_old, TableDev 
         if (keep && j == 0) nbk = claim_group(tnew, ep_new, load_hdr(told.hdr + b).group, &ctl->status, &created);
         nbk = (long long)shfl64((unsigned long long)nbk, half << 4);
         const long long fresh = (keep && j == 0 && nbk >= 0) ? nbk : -1;
-        if (fresh >= 0 && tnew.map_on) tnew.hdr[fresh].aux = mine;
+        if (fresh >= 0) tnew.hdr[fresh].aux = mine;
         if (keep && nbk >= 0) {
             const size_t d = (size_t)nbk * kSlots + j;
             tnew.keys[d] = k;
@@ -384,7 +380,7 @@ cudaError_t launch_set_state(const unsigned long long* keys, const double* re, c
         set_state_claim_kernel<<<ge, kThreads, 0, st>>>(keys, n, frame, t, ctl);
         set_state_clear_kernel<<<grid_for(n * kSlots, kThreads, sms), kThreads, 0, st>>>(t, ctl);
         set_state_fill_kernel<<<ge, kThreads, 0, st>>>(keys, re, im, n, frame, t, ctl, dbl ? 1 : 0);
-        if (t.map_on) refresh_masks_kernel<<<grid_for(n, kThreads / 16, sms), kThreads, 0, st>>>(t, ctl);
+        refresh_masks_kernel<<<grid_for(n, kThreads / 16, sms), kThreads, 0, st>>>(t, ctl);
     }
     set_state_end_kernel<<<1, 1, 0, st>>>(ctl, n);
     return cudaGetLastError();

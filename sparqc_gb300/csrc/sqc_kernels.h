@@ -10,24 +10,19 @@
 
 namespace sqc {
 
-// One gate pass (sqc_pass.cu): the direct kernel (tables up to 2^20 buckets), or the resolve
-// kernel (pair and quad passes) and the staged kernel. Returns the number of kernels launched,
-// or -1 when a launch failed.
-int launch_pass(const PassArgs& a, unsigned long long list_hint, bool dbl, int sms, cudaStream_t st);
-// Tables small enough for tiny_kernel: every pass of a flush in one single-block launch.
-bool tiny_table(unsigned long long buckets);
-// The passes (device array of np records; a's per-pass fields are ignored) in one launch.
-int launch_tiny(const PassArgs& a, const TinyPass* passes, uint32_t np, bool dbl, cudaStream_t st);
-// A pass over a mapped table (sqc_unit.cuh; a.dn, a.dims and a.dim set), and a run of such passes in
-// one launch (dn: mapped bits of the last). FP32 units have three dimensions, FP64 units two or three.
+// One gate pass (sqc_pass.cu) over a mapped table (a.dn, a.dims and a.dim set) or a hashed one (a.dims,
+// a.dim and the bounds set). Returns the number of kernels launched, or -1 when a launch failed.
 int launch_unit_pass(const PassArgs& a, bool dbl, int sms, cudaStream_t st);
-int launch_unit_run(const RunArgs& a, uint32_t dims, uint32_t dn, bool dbl, int sms, cudaStream_t st);
+int launch_hash_pass(const PassArgs& a, unsigned long long list_hint, bool dbl, int sms, cudaStream_t st);
+// A run of passes in one launch; items: units (mapped tables) or live buckets (hashed ones) of the
+// largest pass, at most. FP32 units have three dimensions, FP64 units two or three.
+int launch_run_passes(const RunArgs& a, uint32_t dims, unsigned long long items, bool dbl, int sms, cudaStream_t st);
 cudaError_t launch_set_zero(const TableDev& t, Ctl* ctl, bool dbl, cudaStream_t st);
 // Load n entries; a stored key is the entry's key ^ frame.
 cudaError_t launch_set_state(const unsigned long long* keys, const double* re, const double* im,
                              unsigned long long n, unsigned long long frame, const TableDev& t, Ctl* ctl, bool dbl,
                              int sms, cudaStream_t st);
-// Recompute the presence masks (Header.aux) of a mapped table's listed buckets from their keys.
+// Recompute the presence masks (Header.aux) of a table's listed buckets from their keys.
 cudaError_t launch_refresh_masks(const TableDev& t, Ctl* ctl, unsigned long long list_hint, int sms, cudaStream_t st);
 // Readout of the present entries whose stored key k has (k & smask) == sval (all by default).
 cudaError_t launch_readout(const TableDev& t, Ctl* ctl, unsigned long long list_hint, unsigned long long frame,

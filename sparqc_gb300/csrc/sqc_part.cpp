@@ -227,8 +227,7 @@ int PartState::init(uint32_t nq, const sqc_hash_table_parameters* params, const 
     sqc_default_options(&o);
     if (opt) o = *opt;
     if (device_bytes) {   // the first table within the cap too
-        const uint64_t bucket = sizeof(Header) + kSlots * (8 + (o.precision == SQC_FP32 ? 8 : 16)) + sizeof(unsigned) +
-                                sizeof(Unit);   // as the engine counts a bucket
+        const uint64_t bucket = sizeof(Header) + kSlots * (8 + (o.precision == SQC_FP32 ? 8 : 16)) + sizeof(unsigned);   // as the engine counts a bucket
         uint64_t nb = 64;
         while (nb < 1024 && (nb * 2) * bucket <= device_bytes) nb *= 2;
         if (!o.initial_buckets || o.initial_buckets > nb) o.initial_buckets = nb;

@@ -121,6 +121,24 @@ bool GroupMap::extend(unsigned long long kmask, uint32_t nq) {
     return true;
 }
 
+// The op code of a gate kind (pairing kinds: on slots 0-1 and 2-3).
+static uint32_t unit_op(uint32_t kind) {
+    switch (kind) {
+    case KX: return UO_X_PAIR;
+    case KY: return UO_Y_PAIR;
+    case KH: return UO_H_PAIR;
+    case KRX: return UO_RX_PAIR;
+    case KRY: return UO_RY_PAIR;
+    case KU: return UO_U_PAIR;
+    case KZ: return UO_Z;
+    case KS: return UO_S;
+    case KSDG: return UO_SDG;
+    case KYPH: return UO_YPH;
+    case KRZ: return UO_RZ;
+    default: return UO_PHASE;   // Phase, T, Tdg
+    }
+}
+
 void encode_unit_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[3], const GroupMap& map, uint32_t dims,
                       uint32_t dim[3]) {
     // the cross-group qubit with the fewest gates goes to the lane dimension (1), whose gates
@@ -197,28 +215,40 @@ void encode_unit_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[3], co
             if (((s ^ sval) & smask) == 0) slots |= 1u << s;
             if ((slot_bit != kNoQubit && ((s >> slot_bit) & 1u)) != flip) bits |= 1u << s;
         }
-        uint32_t op;
         const uint32_t shfl = lane_bit != kNoQubit ? 1u : 0u;
-        switch (g.kind) {
-        case KX: op = UO_X_PAIR + shfl; break;
-        case KY: op = UO_Y_PAIR + shfl; break;
-        case KH: op = UO_H_PAIR + shfl; break;
-        case KRX: op = UO_RX_PAIR + shfl; break;
-        case KRY: op = UO_RY_PAIR + shfl; break;
-        case KU: op = UO_U_PAIR + shfl; break;
-        case KZ: op = UO_Z; break;
-        case KS: op = UO_S; break;
-        case KSDG: op = UO_SDG; break;
-        case KYPH: op = UO_YPH; break;
-        case KRZ: op = UO_RZ; break;
-        default: op = UO_PHASE; break;   // Phase, T, Tdg
-        }
+        uint32_t op = unit_op(g.kind) + (pairs ? shfl : 0u);
         const bool all = pairs && !lmask && !smask;   // no controls inside the unit
         if (pairs && (all || pair3)) op += all ? (pair3 ? UO_ALL3 : UO_ALL) : UO_PAIR3;
         const uint32_t tb = lane_bit != kNoQubit ? lane_bit : slot_bit != kNoQubit ? kMaxMapBits : outer;
         g.loc = lmask | (lval << kLocLaneVal) | (slots << kLocSlots) | (bits << kLocSlotBit) | (tb << kLocBit) |
                 (shfl ? kLocLane : 0u) | (flip ? kLocFlip : 0u) |
                 (op << kLocOp);
+    }
+}
+
+void encode_column_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[2], uint32_t dim[3]) {
+    for (int i = 0; i < 2; ++i) dim[i] = q[i] == kNoQubit ? 64u : q[i];
+    dim[2] = 64u;
+    for (size_t k = g0; k < g1; ++k) {
+        GateDesc& g = d[k];
+        g.om = g.ov = 0;
+        uint32_t smask = 0, sval = 0, slot_bit = kNoQubit;
+        for (uint32_t i = 0; i < 2; ++i) {
+            if (q[i] == kNoQubit) continue;
+            if (g.target == q[i]) slot_bit = i;
+            if (!((g.ctrl >> q[i]) & 1ULL)) continue;
+            smask |= 1u << i;
+            sval |= (uint32_t)((g.cval >> q[i]) & 1ULL) << i;
+        }
+        const bool flip = (g.flip & kOpFlip) != 0, pairs = is_branch_kind(g.kind) || is_swap_kind(g.kind);
+        uint32_t slots = 0, bits = 0;
+        for (uint32_t s = 0; s < 4; ++s) {
+            if (((s ^ sval) & smask) == 0) slots |= 1u << s;
+            if ((slot_bit != kNoQubit && ((s >> slot_bit) & 1u)) != flip) bits |= 1u << s;
+        }
+        const uint32_t op = unit_op(g.kind) + (pairs && slot_bit == 1 ? UO_PAIR3 : 0u);
+        g.loc = (slots << kLocSlots) | (bits << kLocSlotBit) | (slot_bit != kNoQubit ? kLocLane : 0u) |
+                ((g.target & 31u) << kLocBit) | (g.target >= 32u ? kLocHigh : 0u) | (flip ? kLocFlip : 0u) | (op << kLocOp);
     }
 }
 

@@ -49,15 +49,16 @@ bool plan_gate(Planner& p, const sqc_gate& g, GateDesc* out);
 // max_nx (<= 3) distinct qubits; streamable gates may sit anywhere in it. Passes are cut
 // greedily. f(g0, g1, nx, q1, q2, q3, keys_fixed) is called per pass, q1..q3 the cross-group
 // qubits in order of first use (kNoQubit when absent).
+// With columns, gates on the low four qubits pair too (passes over hashed tables).
 template <class F>
-void split_passes(const GateDesc* d, size_t n, size_t max_run, uint32_t max_nx, F&& f) {
+void split_passes(const GateDesc* d, size_t n, size_t max_run, uint32_t max_nx, F&& f, bool columns = false) {
     size_t i = 0;
     while (i < n) {
         const size_t start = i;
         uint32_t q[3] = {kNoQubit, kNoQubit, kNoQubit};
         uint32_t nx = 0;
         while (i < n && i - start < max_run) {
-            if (!streamable(d[i])) {
+            if (columns ? !is_diag_kind(d[i].kind) : !streamable(d[i])) {
                 const uint32_t t = d[i].target;
                 if (t != q[0] && t != q[1] && t != q[2]) {
                     if (nx >= max_nx || nx >= 3) break;
@@ -106,6 +107,11 @@ struct GroupMap {
 // mapped. Dimensions without a cross-group qubit take the lowest free bucket bits.
 void encode_unit_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[3], const GroupMap& map, uint32_t dims,
                       uint32_t dim[3]);
+
+// The same for a pass over a hashed table, whose columns (sqc_unit.cuh) are the keys that differ in its
+// pairing qubits q[0..1], any qubits (split_passes with columns; kNoQubit when absent); dim gets them,
+// 64 for an absent one.
+void encode_column_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[2], uint32_t dim[3]);
 
 // An order of gates g[0..n) that passes fuse better, as a permutation: perm[i] is the index of
 // the i-th gate to apply. Passes are built greedily from the first gate not yet placed: a gate

@@ -171,7 +171,7 @@ int Server::submit(const sqc_circuit_desc* c, uint64_t* id) {
 
 // Device bytes of a solo circuit's engine tables (sized so they never grow).
 size_t Server::solo_bytes(const Request& r) const {
-    const size_t per = sizeof(Header) + kSlots * 8 + kSlots * (dbl_ ? 16 : 8) + 4 + sizeof(Unit);
+    const size_t per = sizeof(Header) + kSlots * 8 + kSlots * (dbl_ ? 16 : 8) + 4;
     return (size_t)r.nb * per;
 }
 

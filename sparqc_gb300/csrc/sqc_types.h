@@ -27,25 +27,15 @@ enum Kind : uint32_t { KX = 0, KY, KZ, KH, KPHASE, KRZ, KRX, KRY, KS, KSDG, KT, 
 struct alignas(16) Header {
     unsigned long long group;   // key >> 4 of the bucket's keys
     unsigned int epoch;         // live iff equal to the state's epoch
-    unsigned int aux;           // 0
+    unsigned int aux;           // presence mask: bit j is set iff key (group << 4) | j is held
 };
 
-// One unit of a pass that pairs groups, resolved before the pass. With cross-group qubits
-// q1, q2, q3 (masks m1 = 1 << (q1 - 4), ...; a pair pass has q1 only, a quad pass q1 and q2),
-// the unit is the set of groups G0 | i0*m1 | i1*m2 | i2*m3 with G0 having those stored bits 0;
-// b[i0 + 2*i1 + 4*i2] is the bucket of member (i0, i1, i2), kNoBucket when the group is absent.
-// Pair passes use b[0..1], quad passes b[0..3], octet passes b[0..7].
-constexpr unsigned kNoBucket = 0xFFFFFFFFu;
-struct alignas(16) Unit {
-    unsigned long long G0;
-    unsigned int b[8];
-};
+constexpr unsigned kNoBucket = 0xFFFFFFFFu;   // no bucket: the group is absent
 
 // Where a group's bucket is. A *mapped* table addresses groups directly: bucket bit i is group
 // bit map_q[i], for the map_n group bits that may differ between keys (in the order they began
 // to); every other bit of a stored group is 0, so the address is exact and no probing is needed.
-// Header.aux then holds the bucket's presence mask. A *hashed* table (map_on 0) probes linearly
-// from a hash of the group, and Header.aux is 0.
+// A *hashed* table (map_on 0) probes linearly from a hash of the group.
 constexpr uint32_t kMaxMapBits = 31;
 
 struct TableDev {
@@ -53,7 +43,6 @@ struct TableDev {
     unsigned long long* keys;
     void* amps;
     unsigned int* list;         // live buckets, in claim order
-    Unit* units;                // owned units of a pair or quad pass, compacted by the resolve kernel
     unsigned long long mask;    // nb - 1
     uint32_t map_on;            // 1: mapped, 0: hashed
     uint32_t map_n;             // mapped group bits
@@ -79,17 +68,13 @@ struct Ctl {
     unsigned long long out_count;   // readout counter
     double acc[6];                  // reductions: norm, compare
     unsigned long long acc_max;     // bit pattern of a non-negative double (max |a-b|)
-    unsigned long long work;        // list entries handed out in the running pass (0 between passes)
-    unsigned long long units_n;     // owned units the running pass's resolve kernel wrote (0 between passes)
     unsigned long long bar_len;     // a run's live buckets before a pass that walks the list, tagged with the pass
 };
 
 // Gate descriptor with host-resolved coefficients (std::cos/std::sin on the host, so the
 // device and the CPU oracle use identical values) in the stored-key frame: the gate acts on
 // a stored key s iff (s & ctrl) == cval, and the member's logical target bit is
-// ((s >> target) & 1) ^ flip. The first 32 bytes (kind .. pad) are read as two 16-byte
-// vectors, hence the alignment. `flip` holds the frame flip in bit 0 and, once the gate's
-// pass is known, how that pass applies it (kOp* bits, set by encode_pass on the host).
+// ((s >> target) & 1) ^ flip.
 struct alignas(16) GateDesc {
     uint32_t kind, target;
     unsigned long long ctrl, cval;
@@ -98,9 +83,9 @@ struct alignas(16) GateDesc {
     double m[8];          // u: m00, m01, m10, m11 as (re, im)
     float cf, sf;         // float copies for FP32 states
     float mf[8];
-    // how a unit pass (sqc_unit.cuh) applies the gate, set by encode_unit_pass on the host: the
-    // unit's base index u satisfies the controls outside the unit iff (u & om) == ov; loc holds
-    // the rest (kLoc* fields)
+    // how its pass (sqc_unit.cuh) applies the gate, set by encode_unit_pass on the host: in a mapped
+    // table the unit's base bucket u satisfies the controls outside the unit iff (u & om) == ov (in a
+    // hashed one the column's key is tested against ctrl and cval); loc holds the rest (kLoc* fields)
     uint32_t om, ov, loc, pad2;
 };
 
@@ -111,6 +96,7 @@ constexpr uint32_t kLocSlotBit = 14;       // bits 14..17: diagonal gates: logic
 constexpr uint32_t kLocBit = 18;           // bits 18..22: the target's bit of the lane index or of the unit's base (31: none)
 constexpr uint32_t kLocLane = 1u << 23;    // ... of the lane index
 constexpr uint32_t kLocFlip = 1u << 24;    // the stored frame flips the target bit (pairing gates)
+constexpr uint32_t kLocHigh = 1u << 25;    // hashed tables: kLocBit counts from bit 32 of the column's key
 constexpr uint32_t kLocOp = 26;            // bits 26..31: UOp
 // Pairing gates come as their controls inside the unit ask, on slots 0-1 and 2-3 or (UO_PAIR3) 0-2 and
 // 1-3, and, when they have none there (every lane and slot takes part), straight through (UO_ALL,
@@ -123,7 +109,7 @@ enum UOp : uint32_t {
     UO_PAIR3 = 31   // + 0, 2, .., 10: the same with controls inside the unit
 };
 
-// GateDesc.flip bits.
+// GateDesc.flip bits: the frame's flip, and what encode_pass says of a gate by kind and qubits.
 constexpr uint32_t kOpFlip = 1u << 0;      // the stored frame flips the target bit
 constexpr uint32_t kOpPair = 1u << 1;      // pairs the a and b slots (first cross-group qubit)
 constexpr uint32_t kOpShfl = 1u << 2;      // partner slot in lane ^ (1 << off_log2)
@@ -157,40 +143,31 @@ struct alignas(16) UnitHead {
     uint32_t om, ov, loc, weight;
 };
 
-// One pass of a single-launch run over a tiny table (tiny_kernel): what PassArgs says per pass.
-struct TinyPass {
-    uint32_t g0, g1, nx, q1, q2, q3, keys_fixed, pad;
-    unsigned long long grow_bound;
-    unsigned long long key_bound;
-};
-
 struct PassArgs {
     TableDev t;
     Ctl* ctl;
     const GateDesc* gates;
     uint32_t g0, g1;        // gate range [g0, g1) of this pass
-    uint32_t nx;            // cross-group qubits of the pass: 0 (stream), 1 (pair) or 2 (quad)
+    uint32_t nx;            // cross-group qubits of the pass
     uint32_t keys_fixed;    // 1: every gate of the pass is diagonal (no key changes)
     uint32_t amp_bytes;     // 16 (FP64) or 8 (FP32)
-    uint32_t credit;        // gates resolved on the host just before this pass (identity or
-                            // relabel): each is credited with this pass's input key count
     unsigned long long max_groups;   // a pass that pairs groups refuses to start when its groups could
                                      // exceed this: min(grow_bound, n << nx, n + key_bound) > max_groups
     PruneBits prune;
-    uint32_t q1, q2, q3;             // the cross-group qubits (kNoQubit when absent)
     unsigned long long grow_bound;   // groups the state can hold after the pass, at most
     unsigned long long key_bound;    // keys it can hold after the pass, at most: a pass makes no more
                                      // groups than that (hashed tables; at most kKeysUnknown)
-    // unit passes (mapped tables): mapped bits in use after the pass, dimensions of a unit (2 or
-    // 3) and the bucket bit of each dimension
+    // mapped bits in use after the pass (mapped tables), dimensions of a unit (2 or 3) and the bucket
+    // bit (mapped) or qubit (hashed; 64: none) of each dimension
     uint32_t dn, dims, dim[3];
-    UnitHead heads[kMaxRun];   // unit passes: those of the pass's gates (read from the parameter bank)
+    UnitHead heads[kMaxRun];   // mapped tables: those of the pass's gates (read from the parameter bank)
 };
 
-// A run of unit passes in one launch (run_kernel). words holds the passes one after another: a
-// record (om: gates in bits 0..7, the flags below, mapped bits after the pass from bit 16; ov: the bucket
-// bits of the unit's dimensions, a byte each; loc: the pass's first gate), then the heads of
-// its gates. All of it is read from the parameter bank.
+// A run of passes in one launch (run_kernel). words holds the passes one after another: a record (om:
+// gates in bits 0..7, the flags below, from bit 16 the mapped bits after the pass or, in a hashed
+// table, its cross-group qubits; ov: the dimensions' bits, a byte each; loc: the pass's
+// first gate), then the heads of its gates (mapped) or grow_bound and key_bound (hashed; PassArgs).
+// All of it is read from the parameter bank.
 constexpr uint32_t kRunWords = 496;        // 8 KB of parameters
 constexpr uint32_t kRunFixed = 1u << 8;    // every gate is diagonal
 constexpr uint32_t kRunPair = 1u << 9;     // the pass pairs groups
@@ -201,6 +178,7 @@ struct RunArgs {
     PruneBits prune;
     uint32_t np, amp_bytes;
     uint32_t tag;              // of the run's first pass: passes of an engine have different ones
+    unsigned long long max_groups;   // hashed tables: as in PassArgs
     UnitHead words[kRunWords];
 };
 

@@ -16,10 +16,36 @@
 // presence changes: FP32 16.5 bytes per key and pass instead of 32.
 #pragma once
 #include "sqc_dmul.cuh"
-#include "sqc_pass_dev.cuh"
+#include "sqc_device.cuh"
 
 namespace sqc {
 namespace {
+
+template <class T> struct AmpT;
+template <> struct AmpT<double> { using V = double2; };
+template <> struct AmpT<float> { using V = float2; };
+
+template <class T> __device__ __forceinline__ Cx<T> czero() { return Cx<T>{T(0), T(0)}; }
+
+__device__ __forceinline__ unsigned long long umin64(unsigned long long a, unsigned long long b) { return a < b ? a : b; }
+
+template <class T>
+__device__ __forceinline__ void store_amp(void* amps, size_t s, Cx<T> a) {
+    typename AmpT<T>::V v;
+    v.x = a.r;
+    v.y = a.i;
+    reinterpret_cast<typename AmpT<T>::V*>(amps)[s] = v;
+}
+
+template <class T>
+__device__ __forceinline__ Cx<T> pick(bool c, Cx<T> x, Cx<T> y) {
+    return Cx<T>{c ? x.r : y.r, c ? x.i : y.i};
+}
+
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
+    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(kFull, v, o);
+    return v;
+}
 
 // A pass's gate in shared memory: the first 16 bytes say where it acts, then the coefficients.
 template <class T> struct UGate;
@@ -466,7 +492,7 @@ __device__ __forceinline__ void diag(const UGate<T>& g, unsigned e, unsigned act
 }
 
 // The gates of a pass on the unit a warp holds; uid is the unit's base index. Absent slots hold
-// +-0, which no gate makes present (sqc_pass_dev.cuh).
+// +-0, and the prune threshold is positive: no gate makes a slot present out of absent ones.
 // `heads` says where each gate acts (UnitHead): the gates' own in shared memory, or the kernel's
 // parameters, where the whole warp reads them as one.
 template <class T, int S, class Heads>
@@ -741,6 +767,296 @@ __device__ __forceinline__ void walk_entries(const TableDev& t, const uint8_t* m
 // pass), a list entry its ownership check.
 __device__ __forceinline__ bool walk_list(unsigned long long list_n, uint32_t dn) {
     return dn >= 6 && list_n < (1ULL << (dn - 3));
+}
+
+// ---- hashed tables -------------------------------------------------------------------------------
+// Keys too thin for a map: most groups hold one key among their 16 slots, and a warp per unit would
+// run every gate on lanes without one. A pass here pairs keys across at most two qubits, the low four
+// included, and splits its units into columns: the four keys that differ in those qubits, all in
+// one lane, so gates need no exchange between lanes and 32 columns of any units run together. A warp takes
+// a piece of the live list. Each lane looks up the members of one entry's unit and settles
+// whether the entry owns it; the presence masks (Header.aux) come with the lookups. The columns of the
+// owned units that hold a key are then dealt to the lanes, 32 at a time; only amplitudes of
+// present keys are read. Controls and diagonal targets outside the column are tested per lane.
+// 2^17 keys in FP64, one or two to a group: 285 us a pass with a warp per unit (and 335 us by pairs of
+// slots with their keys), see hash_kernel for this form.
+constexpr int kColumn = 4;   // keys of a column
+
+// A pass's gate in shared memory.
+template <class T> struct HGates {
+    UGate<T> g[kMaxRun];
+    unsigned long long om[kMaxRun], ov[kMaxRun];   // controls outside the column
+};
+
+// Where a pass's two qubits lie: group masks, or slot masks of the low four (both 0: no such qubit).
+struct HashDims {
+    unsigned long long gm[2], keys;   // keys: both as key bits
+    unsigned lm[2];
+    unsigned groups, valid;           // column bits that change the group, that exist
+};
+__device__ __forceinline__ HashDims hash_dims(uint32_t d0, uint32_t d1) {
+    HashDims r;
+    const uint32_t d[2] = {d0, d1};
+    r.keys = 0;
+    r.groups = r.valid = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        r.gm[i] = d[i] >= (uint32_t)kSlotBits && d[i] < 64u ? 1ULL << (d[i] - kSlotBits) : 0ULL;
+        r.lm[i] = d[i] < (uint32_t)kSlotBits ? 1u << d[i] : 0u;
+        if (d[i] < 64u) r.keys |= 1ULL << d[i];
+        if (r.gm[i]) r.groups |= 1u << i;
+        if (d[i] < 64u) r.valid |= 1u << i;
+    }
+    return r;
+}
+
+// Copy ng gates into shared memory for a pass with pairing qubits dk (key bits); no barrier.
+template <class T>
+__device__ __forceinline__ void stage_hgates(HGates<T>& sg, const GateDesc* __restrict__ gates, uint32_t ng, unsigned long long dk) {
+    for (uint32_t i = threadIdx.x; i < ng; i += blockDim.x) {
+        const GateDesc* g = gates + i;
+        stage_ugate(sg.g + i, g);
+        const unsigned long long om = __ldg(&g->ctrl) & ~dk;
+        sg.om[i] = om;
+        sg.ov[i] = __ldg(&g->cval) & om;
+    }
+}
+
+// A warp's piece of a pass: per list entry the members of its unit (bucket, kNoBucket when absent, and
+// presence mask before the pass), their masks now, and the columns that hold keys (entry << 4 | slot).
+struct HashWork {
+    uint2 m[32][4];
+    unsigned now[32][4];
+    unsigned short cols[512];
+};
+
+// The gates of a pass on one column a lane; kb is the column's key with the pass's qubits 0.
+template <class T>
+__device__ __forceinline__ void run_columns(const HGates<T>& sg, const GateDesc* __restrict__ gates, uint32_t ng, unsigned long long kb,
+                                            bool on, Slots<T, kColumn>& x, bool& touched, const PruneBits& pb,
+                                            unsigned long long& upd) {
+#pragma unroll 1
+    for (uint32_t gi = 0; gi < ng; ++gi) {
+        const UGate<T>& g = sg.g[gi];
+        upd += (unsigned long long)x.n * g.weight;
+        const uint32_t loc = g.loc;
+        const bool acts = on && (kb & sg.om[gi]) == sg.ov[gi];
+        if (!__any_sync(kFull, acts)) continue;
+        touched = touched || acts;
+        const GateDesc* gd = gates + gi;
+        const unsigned act = acts ? (loc >> kLocSlots) & 15u : 0u;
+        const uint32_t w = act | (loc & kLocFlip ? 0x80000000u : 0u);   // pairing gates: slots, logical bit of the first
+        auto ones = [&]() {   // diagonal gates: slots with logical target bit 1
+            const uint32_t word = loc & kLocHigh ? (uint32_t)(kb >> 32) : (uint32_t)kb;
+            const bool at = !(loc & kLocLane) && ((word >> ((loc >> kLocBit) & 31u)) & 1u);
+            return (((loc >> kLocSlotBit) & 15u) ^ (at ? 15u : 0u)) & act;
+        };
+        switch (loc >> kLocOp) {
+        case UO_X_PAIR: swap_pair<T, KX, kColumn, 1, false>(w, x); break;
+        case UO_PAIR3 + UO_X_PAIR: swap_pair<T, KX, kColumn, 2, false>(w, x); break;
+        case UO_Y_PAIR: swap_pair<T, KY, kColumn, 1, false>(w, x); break;
+        case UO_PAIR3 + UO_Y_PAIR: swap_pair<T, KY, kColumn, 2, false>(w, x); break;
+        case UO_H_PAIR: branch_pair<T, KH, kColumn, 1, false>(g, gd, w, x, pb); break;
+        case UO_PAIR3 + UO_H_PAIR: branch_pair<T, KH, kColumn, 2, false>(g, gd, w, x, pb); break;
+        case UO_RX_PAIR: branch_pair<T, KRX, kColumn, 1, false>(g, gd, w, x, pb); break;
+        case UO_PAIR3 + UO_RX_PAIR: branch_pair<T, KRX, kColumn, 2, false>(g, gd, w, x, pb); break;
+        case UO_RY_PAIR: branch_pair<T, KRY, kColumn, 1, false>(g, gd, w, x, pb); break;
+        case UO_PAIR3 + UO_RY_PAIR: branch_pair<T, KRY, kColumn, 2, false>(g, gd, w, x, pb); break;
+        case UO_U_PAIR: branch_pair<T, KU, kColumn, 1, false>(g, gd, w, x, pb); break;
+        case UO_PAIR3 + UO_U_PAIR: branch_pair<T, KU, kColumn, 2, false>(g, gd, w, x, pb); break;
+        case UO_Z: diag<T, KZ, kColumn>(g, ones(), act, x); break;
+        case UO_S: diag<T, KS, kColumn>(g, ones(), act, x); break;
+        case UO_SDG: diag<T, KSDG, kColumn>(g, ones(), act, x); break;
+        case UO_YPH: diag<T, KYPH, kColumn>(g, ones(), act, x); break;
+        case UO_RZ: diag<T, KRZ, kColumn>(g, ones(), act, x); break;
+        case UO_PHASE: diag<T, KPHASE, kColumn>(g, ones(), act, x); break;
+        default: __builtin_unreachable();
+        }
+    }
+}
+
+// The units of list entries [e0, e1) (at most 32). An entry owns its unit when it is the live member of
+// smallest index (the reference's pair rule, emulator/device/device_table_FC.cuh:62-110, lifted to
+// groups; members a pass creates are made by the unit's owner, after its own check).
+template <class T>
+__device__ __forceinline__ void walk_hashed(const TableDev& t, Ctl* ctl, unsigned ep, const HashDims& dm, unsigned long long e0,
+                                            unsigned long long e1, HashWork& wk, const HGates<T>& sg, const GateDesc* gates,
+                                            uint32_t ng, int lane, const PruneBits& pb, unsigned long long& cnt_nnz,
+                                            unsigned long long& cnt_empty, unsigned long long& upd) {
+    unsigned long long base = 0;
+    bool owns = false;
+    unsigned cols = 0;
+    auto member = [&](unsigned long long G0, int k) { return G0 | ((k & 1) ? dm.gm[0] : 0ULL) | ((k & 2) ? dm.gm[1] : 0ULL); };
+    if (e0 + lane < e1) {
+        const unsigned b = __ldcg(t.list + e0 + lane);   // (an earlier pass of the same launch may have written it)
+        const Header own = load_hdr_cg(t.hdr + b);
+        const int idx = ((own.group & dm.gm[0]) ? 1 : 0) | ((own.group & dm.gm[1]) ? 2 : 0);
+        base = own.group & ~(dm.gm[0] | dm.gm[1]);
+        Header h[4];
+        unsigned at[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {   // the first probes of all members together
+            h[k].epoch = ep + 1;
+            at[k] = b;
+            if (k != idx && (k & ~dm.groups) == 0) {
+                at[k] = (unsigned)(mix64(member(base, k)) & t.mask);
+                h[k] = load_hdr_cg(t.hdr + at[k]);
+            }
+        }
+        owns = true;
+        unsigned any = own.aux;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            uint2 m = make_uint2(kNoBucket, 0u);
+            if (k == idx) {
+                m = make_uint2(b, own.aux);
+            } else if (h[k].epoch == ep) {
+                const unsigned long long G = member(base, k);
+                Header c = h[k];
+                unsigned long long p = at[k];
+                for (uint32_t i = 1; i < kMaxProbe && c.epoch == ep && c.group != G; ++i) {
+                    p = (p + 1) & t.mask;
+                    c = load_hdr_cg(t.hdr + p);
+                }
+                if (c.epoch == ep && c.group == G) {
+                    m = make_uint2((unsigned)p, c.aux);
+                    if (k < idx) owns = false;
+                    any |= c.aux;
+                }
+            }
+            wk.m[lane][k] = m;
+            wk.now[lane][k] = m.y;
+        }
+        if (owns) {   // its columns: slots with the pass's low qubits 0
+            cols = any;
+#pragma unroll
+            for (int d = 0; d < 2; ++d) {
+                const unsigned q = dm.lm[d];
+                if (q) cols = (cols | (cols >> q)) & (q == 1 ? 0x5555u : q == 2 ? 0x3333u : q == 4 ? 0x0F0Fu : 0x00FFu);
+            }
+        }
+    }
+    unsigned upto = __popc(cols);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_up_sync(kFull, upto, o);
+        if (lane >= o) upto += v;
+    }
+    const unsigned total = __shfl_sync(kFull, upto, 31);
+    {
+        unsigned at = upto - __popc(cols);
+        for (unsigned c = cols; c; c &= c - 1) wk.cols[at++] = (unsigned short)((lane << 4) | (__ffs(c) - 1));
+    }
+    __syncwarp();
+    unsigned fresh = 0;   // members of this lane's entry that the pass has made
+    for (unsigned c0 = 0; c0 < total; c0 += 32) {
+        const bool on = c0 + lane < total;
+        const unsigned id = on ? wk.cols[c0 + lane] : 0u;
+        const int l = (int)(id >> 4);
+        const unsigned j0 = id & 15u;
+        const unsigned long long G0 = shfl64(base, l);
+        Slots<T, kColumn> x;
+        x.pm = 0;
+#pragma unroll
+        for (int s = 0; s < kColumn; ++s) {
+            const unsigned j = j0 | ((s & 1) ? dm.lm[0] : 0u) | ((s & 2) ? dm.lm[1] : 0u);
+            const uint2 m = wk.m[l][s & dm.groups];
+            const bool p = on && (s & ~dm.valid) == 0 && ((m.y >> j) & 1u);
+            x.pm |= (unsigned)p << s;
+            x.v[s] = czero<T>();
+            if (p) {
+                const typename AmpT<T>::V a = __ldcg(reinterpret_cast<const typename AmpT<T>::V*>(t.amps) + (size_t)m.x * kSlots + j);
+                x.v[s] = Cx<T>{a.x, a.y};
+            }
+        }
+        bool touched = false;
+        const unsigned pm0 = x.pm;
+        x.n = __popc(pm0);
+        run_columns<T>(sg, gates, ng, (G0 << kSlotBits) | j0, on, x, touched, pb, upd);
+        const unsigned pm = x.pm;
+        cnt_nnz += __popc(pm);
+        bool absent = false;
+#pragma unroll
+        for (int s = 0; s < kColumn; ++s) {
+            if (!(((pm ^ pm0) >> s) & 1u)) continue;
+            const unsigned j = j0 | ((s & 1) ? dm.lm[0] : 0u) | ((s & 2) ? dm.lm[1] : 0u);
+            if ((pm >> s) & 1u) {
+                atomicOr(&wk.now[l][s & dm.groups], 1u << j);
+                absent = absent || wk.m[l][s & dm.groups].x == kNoBucket;
+            } else {
+                atomicAnd(&wk.now[l][s & dm.groups], ~(1u << j));
+            }
+        }
+        if (__any_sync(kFull, absent)) {   // groups that appear: claimed by the lane of their unit's entry
+            __syncwarp();
+            if (owns) {
+#pragma unroll 1
+                for (int k = 0; k < 4; ++k) {
+                    if (wk.m[lane][k].x != kNoBucket || wk.now[lane][k] == 0) continue;
+                    bool created;
+                    const long long nb = claim_group(t, ep, member(base, k), &ctl->status, &created);
+                    if (nb < 0) continue;
+                    wk.m[lane][k].x = (unsigned)nb;
+                    fresh |= 1u << k;
+                    ulonglong2* keys = reinterpret_cast<ulonglong2*>(t.keys + (size_t)nb * kSlots);
+#pragma unroll
+                    for (int j = 0; j < kSlots; j += 2) keys[j / 2] = make_ulonglong2(empty_key(j), empty_key(j + 1));
+                }
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int s = 0; s < kColumn; ++s) {
+            const bool p = (pm >> s) & 1u, moved = ((pm ^ pm0) >> s) & 1u;
+            if (!moved && !(p && touched)) continue;
+            const unsigned j = j0 | ((s & 1) ? dm.lm[0] : 0u) | ((s & 2) ? dm.lm[1] : 0u);
+            const unsigned b = wk.m[l][s & dm.groups].x;
+            if (b == kNoBucket) continue;   // (the table is full: the pass has failed)
+            if (p) store_amp<T>(t.amps, (size_t)b * kSlots + j, x.v[s]);
+            if (moved) t.keys[(size_t)b * kSlots + j] = p ? (member(G0, s & (int)dm.groups) << kSlotBits) | j : empty_key((int)j);
+        }
+    }
+    __syncwarp();
+    // masks that changed, and the buckets made: those go to the list together, with one addition to its
+    // length (every warp adds to it)
+    if (owns) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint2 m = wk.m[lane][k];
+            if (m.x == kNoBucket) continue;
+            const unsigned now = wk.now[lane][k];
+            if (now != m.y) t.hdr[m.x].aux = now;
+            if (now == 0) cnt_empty += 1;
+        }
+    }
+    if (__any_sync(kFull, fresh != 0)) {
+        const unsigned made = __popc(fresh);
+        unsigned sum = made;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned v = __shfl_up_sync(kFull, sum, o);
+            if (lane >= o) sum += v;
+        }
+        unsigned long long at = 0;
+        if (lane == 31) at = atomicAdd(&ctl->list_tail, (unsigned long long)sum);
+        at = shfl64(at, 31) + (sum - made);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if ((fresh >> k) & 1u) t.list[at++] = wk.m[lane][k].x;
+    }
+    __syncwarp();
+}
+
+// A hashed pass's share of a warp: entries are dealt out in pieces of up to 32, as many to every warp
+// (a piece is a chain of dependent loads, so few entries take small pieces rather than several).
+template <class T>
+__device__ __forceinline__ void walk_hashed_all(const TableDev& t, Ctl* ctl, unsigned ep, const HashDims& dm, unsigned long long n,
+                                                unsigned w, unsigned nw, HashWork& wk, const HGates<T>& sg,
+                                                const GateDesc* gates, uint32_t ng, int lane, const PruneBits& pb,
+                                                unsigned long long& cnt_nnz, unsigned long long& cnt_empty, unsigned long long& upd) {
+    const unsigned long long rounds = (n + nw * 32ULL - 1) / (nw * 32ULL), piece = rounds ? (n + nw * rounds - 1) / (nw * rounds) : 1;
+    for (unsigned long long e0 = w * piece; e0 < n; e0 += nw * piece)
+        walk_hashed<T>(t, ctl, ep, dm, e0, umin64(e0 + piece, n), wk, sg, gates, ng, lane, pb, cnt_nnz, cnt_empty, upd);
 }
 
 }  // namespace

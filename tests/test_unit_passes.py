@@ -315,3 +315,29 @@ def test_runs_that_walk_the_list(keys, precision):
     (sa, a), (sb, b) = states
     assert [a[f] for f in ("passes", "amp_updates", "alg_bytes")] == [b[f] for f in ("passes", "amp_updates", "alg_bytes")]
     assert_identical(sb, sa)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("cross", [0, 1])
+@pytest.mark.parametrize("keys", [1, 31, 700, 20000])
+def test_column_passes(keys, cross, precision):
+    """Keys spread over 64 qubits (hashed tables): passes whose two pairing qubits are low, high or one of
+    each, passes with none, controls on many qubits, inside the column and out, diagonal targets in
+    either half of the key; groups that appear and that empty."""
+    rng = np.random.default_rng(keys)
+    spread = np.uint64(0xFEDCBA9876543210)
+    key = np.unique(np.concatenate([rng.integers(0, 1 << 63, keys, dtype=np.uint64) * np.uint64(2) + np.uint64(keys & 1),
+                                    np.array([0, 0xFFFFFFFFFFFFFFFF, int(spread)][: 1 if keys == 1 else 3], np.uint64)]))
+    amp = rng.standard_normal((2, key.size))
+    c = circuits.SplitMix64(circuits.stream_seed("columns", keys))
+    pick = lambda n: c.next() % n
+    gs = []
+    for i in range(48):
+        t = [pick(4), 4 + pick(28), 32 + pick(32), 63, 35, 36][i % 6]
+        ctl = tuple({q for q in [pick(4), pick(64), 35, 3][: pick(5)] if q != t})
+        if i % 12 == 7:
+            ctl = tuple(q for q in range(20, 60) if q != t)
+        group = KINDS[pick(3)]
+        gs.append((group[pick(len(group))], t, ctl, 0.3 + 0.1 * i) if i % 8 else (G.X, t, ctl[:1], 0.0))
+    _both(64, G.gate_array(gs[: 48 if keys < 20000 else 14]), precision, max_cross_qubits=cross, init=(key, amp[0], amp[1]))
