@@ -97,8 +97,9 @@ __global__ void __launch_bounds__(kThreads, UnitOcc<T, DIMS>::kMin) unit_kernel(
     const GateDesc* gates = a.gates + a.g0;
     unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
     if (walk_list(n, a.dn)) {
-        for (unsigned long long e0 = w * 32ULL; e0 < n; e0 += nw * 32ULL)
-            walk_entries<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, e0, n, a.heads, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+        const unsigned long long piece = list_piece(n, nw);
+        for (unsigned long long e0 = w * piece; e0 < n; e0 += nw * piece)
+            walk_entries<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, e0, umin64(e0 + piece, n), a.heads, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
     } else {
         walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, nw, a.heads, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
     }
@@ -226,8 +227,9 @@ __global__ void __launch_bounds__(kThreads, HASHED ? kHashBlocks : UnitOcc<T, DI
             const ParamHeads heads{a, o + 1};
             cnt_nnz = cnt_empty = 0;
             if (walk_list(n, dn)) {
-                for (unsigned long long e0 = w * 32ULL; e0 < n; e0 += nw * 32ULL)
-                    walk_entries<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, e0, n, heads, sg[p & 1], gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+                const unsigned long long piece = list_piece(n, nw);
+                for (unsigned long long e0 = w * piece; e0 < n; e0 += nw * piece)
+                    walk_entries<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, e0, umin64(e0 + piece, n), heads, sg[p & 1], gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
             } else {
                 walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, nw, heads, sg[p & 1], gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
             }

@@ -724,20 +724,28 @@ __device__ __forceinline__ void walk_units(const TableDev& t, const uint8_t* mq,
                          upd);
 }
 
-// The units of list entries [e0, e0 + 32) below n, for tables whose live buckets are few among
+// List entries a warp takes at a time, for n entries and nw warps: up to 32, as many pieces to every warp.
+// Few entries make small pieces: the units of a piece run one after another in a mapped pass (2^11
+// keys, FP32: 27 -> 5 us a pass), and a piece is a chain of dependent loads in any.
+__device__ __forceinline__ unsigned long long list_piece(unsigned long long n, unsigned nw) {
+    const unsigned long long rounds = (n + nw * 32ULL - 1) / (nw * 32ULL);
+    return rounds ? (n + nw * rounds - 1) / (nw * rounds) : 1;
+}
+
+// The units of list entries [e0, e1) (at most 32), for tables whose live buckets are few among
 // the mapped ones: lane l takes entry e0 + l; the unit belongs to its live member of smallest index
 // (members a pass creates are made by the unit's owner, after its own check), found by reading
 // the headers of the smaller members.
 template <class T, int DIMS, class Heads>
 __device__ __forceinline__ void walk_entries(const TableDev& t, const uint8_t* mq, Ctl* ctl, unsigned ep, const UnitPass& up,
-                                             unsigned long long e0, unsigned long long n, const Heads& heads, const UGates<T>& sg,
+                                             unsigned long long e0, unsigned long long e1, const Heads& heads, const UGates<T>& sg,
                                              const GateDesc* gates, uint32_t ng, int lane, const PruneBits& pb,
                                              unsigned long long& cnt_nnz, unsigned long long& cnt_empty,
                                              unsigned long long& upd) {
     constexpr int K = 1 << DIMS;
     unsigned base = 0;
     bool own = false;
-    if (e0 + lane < n) {
+    if (e0 + lane < e1) {
         const unsigned b = __ldcg(t.list + e0 + lane);   // (an earlier pass of the same launch may have written it)
         int idx = 0;
         base = b;
@@ -1047,14 +1055,13 @@ __device__ __forceinline__ void walk_hashed(const TableDev& t, Ctl* ctl, unsigne
     __syncwarp();
 }
 
-// A hashed pass's share of a warp: entries are dealt out in pieces of up to 32, as many to every warp
-// (a piece is a chain of dependent loads, so few entries take small pieces rather than several).
+// A hashed pass's share of a warp.
 template <class T>
 __device__ __forceinline__ void walk_hashed_all(const TableDev& t, Ctl* ctl, unsigned ep, const HashDims& dm, unsigned long long n,
                                                 unsigned w, unsigned nw, HashWork& wk, const HGates<T>& sg,
                                                 const GateDesc* gates, uint32_t ng, int lane, const PruneBits& pb,
                                                 unsigned long long& cnt_nnz, unsigned long long& cnt_empty, unsigned long long& upd) {
-    const unsigned long long rounds = (n + nw * 32ULL - 1) / (nw * 32ULL), piece = rounds ? (n + nw * rounds - 1) / (nw * rounds) : 1;
+    const unsigned long long piece = list_piece(n, nw);
     for (unsigned long long e0 = w * piece; e0 < n; e0 += nw * piece)
         walk_hashed<T>(t, ctl, ep, dm, e0, umin64(e0 + piece, n), wk, sg, gates, ng, lane, pb, cnt_nnz, cnt_empty, upd);
 }
