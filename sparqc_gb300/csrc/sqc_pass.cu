@@ -107,10 +107,11 @@ __global__ void __launch_bounds__(kThreads, UnitOcc<T, DIMS>::kMin) unit_kernel(
 }
 
 // ---- pass over a hashed table -----------------------------------------------------------------------
-constexpr int kHashBlocks = 3;   // resident blocks per SM asked for
+// resident blocks per SM asked for (FP64 at four: 2% slower; FP32 at three: 4% slower)
+template <class T> constexpr int kHashBlocks = sizeof(T) == 8 ? 3 : 4;
 
 template <class T>
-__global__ void __launch_bounds__(kThreads, kHashBlocks) hash_kernel(const __grid_constant__ PassArgs a) {
+__global__ void __launch_bounds__(kThreads, kHashBlocks<T>) hash_kernel(const __grid_constant__ PassArgs a) {
     __shared__ HGates<T> sg;
     __shared__ HashWork wk[kThreads / 32];
     const HashDims dm = hash_dims(a.dim[0], a.dim[1]);
@@ -176,7 +177,7 @@ template <class T, bool HASHED> struct RunGates { using G = UGates<T>; };
 template <class T> struct RunGates<T, true> { using G = HGates<T>; };
 
 template <class T, int DIMS, bool HASHED>
-__global__ void __launch_bounds__(kThreads, HASHED ? kHashBlocks : UnitOcc<T, DIMS>::kMin) run_kernel(const __grid_constant__ RunArgs a) {
+__global__ void __launch_bounds__(kThreads, HASHED ? kHashBlocks<T> : UnitOcc<T, DIMS>::kMin) run_kernel(const __grid_constant__ RunArgs a) {
     __shared__ typename RunGates<T, HASHED>::G sg[2];
     __shared__ HashWork wk[HASHED ? kThreads / 32 : 1];
     __shared__ unsigned long long acc[3][kThreads];   // each thread's own: amp updates, bytes, bytes of pair passes
