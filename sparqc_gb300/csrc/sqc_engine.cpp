@@ -122,10 +122,8 @@ int Engine::init(uint32_t nq, const sqc_hash_table_parameters* params, const sqc
     lf_ = o.load_factor;
     max_run_ = o.max_fused_gates ? std::min<uint32_t>(o.max_fused_gates, kMaxRun) : kMaxRun;
     if (o.max_cross_qubits > 3) return fail(SQC_ERR_ARG, "max_cross_qubits must be 0, 1, 2 or 3");
-    // default: three for FP32 (octet passes measured 14% faster on the 40-qubit workload), two
-    // for FP64 (octet passes hold four slots per lane, which halves the FP64 kernels' occupancy:
-    // the direct kernel ran 10% slower on the 40-qubit workload; on the 64-qubit workload the
-    // staged kernel gained 1.4% from the fewer passes, with 36% fewer bytes moved per circuit)
+    // default: three for FP32; two for FP64, whose units of eight buckets double the registers of a lane
+    // (three: 1000 gates on 2^20 keys 3.81 -> 4.39 ms, 500 on 2^24 27.2 -> 32.8 ms)
     max_nx_ = o.max_cross_qubits ? o.max_cross_qubits : (o.precision == SQC_FP32 ? 3 : 2);
     time_passes_ = o.time_passes != 0;
     dev_upd_only_ = o.device_updates_only != 0;
@@ -477,7 +475,13 @@ int Engine::flush(bool hold_last) {
     }
     // how each pass applies its gates: by place in its units (mapped tables; the map grows with
     // the bits its gates make differ) or by key (hashed ones)
-    const uint32_t dims = dbl_ && max_nx_ < 3 ? 2u : 3u;
+    uint32_t dims = dbl_ && max_nx_ < 3 ? 2u : 3u;
+    if (mapped_ && !spans.empty()) {
+        // at most two mapped bits: a third dimension would only double the slots of the one warp (keys of
+        // six qubits, FP32, 343 gates: 86 -> 67 us)
+        GroupMap m = map_;
+        if (m.extend(after[spans.back().g1 - 1].kmask, nq_) && m.n <= 2) dims = 2;
+    }
     fresh_ = fresh_ && spans.empty();
     for (Span& sp : spans) {
         const uint32_t q[3] = {sp.q1, sp.q2, sp.q3};

@@ -15,7 +15,7 @@ namespace sqc {
 int launch_unit_pass(const PassArgs& a, bool dbl, int sms, cudaStream_t st);
 int launch_hash_pass(const PassArgs& a, unsigned long long list_hint, bool dbl, int sms, cudaStream_t st);
 // A run of passes in one launch; items: units (mapped tables) or live buckets (hashed ones) of the
-// largest pass, at most. FP32 units have three dimensions, FP64 units two or three.
+// largest pass, at most. Units have two or three dimensions.
 int launch_run_passes(const RunArgs& a, uint32_t dims, unsigned long long items, bool dbl, int sms, cudaStream_t st);
 cudaError_t launch_set_zero(const TableDev& t, Ctl* ctl, bool dbl, cudaStream_t st);
 // Load n entries; a stored key is the entry's key ^ frame.

@@ -394,7 +394,7 @@ cudaError_t launch_run(const RunArgs& a, unsigned long long items, int sms, cuda
 }  // namespace
 
 int launch_unit_pass(const PassArgs& a, bool dbl, int sms, cudaStream_t st) {
-    const cudaError_t e = !dbl ? launch_unit<float, 3>(a, sms, st)
+    const cudaError_t e = !dbl ? (a.dims == 3 ? launch_unit<float, 3>(a, sms, st) : launch_unit<float, 2>(a, sms, st))
                           : a.dims == 3 ? launch_unit<double, 3>(a, sms, st) : launch_unit<double, 2>(a, sms, st);
     return e == cudaSuccess ? 1 : -1;
 }
@@ -407,7 +407,7 @@ int launch_hash_pass(const PassArgs& a, unsigned long long list_hint, bool dbl, 
 int launch_run_passes(const RunArgs& a, uint32_t dims, unsigned long long items, bool dbl, int sms, cudaStream_t st) {
     cudaError_t e;
     if (a.t.map_on)
-        e = !dbl ? launch_run<float, 3, false>(a, items, sms, st)
+        e = !dbl ? (dims == 3 ? launch_run<float, 3, false>(a, items, sms, st) : launch_run<float, 2, false>(a, items, sms, st))
             : dims == 3 ? launch_run<double, 3, false>(a, items, sms, st) : launch_run<double, 2, false>(a, items, sms, st);
     else
         e = dbl ? launch_run<double, 2, true>(a, items, sms, st) : launch_run<float, 2, true>(a, items, sms, st);
