@@ -300,17 +300,16 @@ typedef struct sqc_batch_options {
     void* stream;              /* cudaStream_t; NULL = the batch creates its own */
     double prune_threshold;    /* > 0, default 1e-14 */
     double load_factor;        /* groups per bucket of a slice at the group bound, (0, 0.45]; default 0.45 */
-    uint32_t min_chunk;        /* list entries a warp takes at once, a multiple of 4; default 8 */
+    uint32_t min_chunk;        /* smallest share of a pass a block takes at once, in list entries, a
+                                  multiple of 4; default 8 */
     uint32_t blocks_per_sm;    /* persistent blocks per SM, 0 = as many as fit */
     uint64_t memory_budget;    /* bytes of device memory the batch may hold, 0 = 98% of the device */
     uint32_t use_graph;        /* 1: sqc_batch_run replays a captured CUDA graph */
     uint32_t idle_limit_us;    /* a warp of the persistent kernel that finds no work for this long
                                   ends the run, which then fails with SQC_ERR_STATE (every wait in
                                   the kernel is bounded); 0 = 2 s */
-    uint32_t threads_per_unit; /* threads that hold one unit of a pass pairing 16-key groups: 16 (a
-                                  pair of groups per half-warp: one qubit >= 4 per pass) or 32 (a
-                                  quad per warp: two qubits >= 4 per pass); 0 = 32. Results do not
-                                  depend on it; sqc_batch_autotune picks it */
+    uint32_t threads_per_unit; /* 16: passes pair 16-key groups across one qubit >= 4; 32: across two (FP64) or three (FP32);
+                                  0 = 32. Results do not depend on it; sqc_batch_autotune picks it */
     uint32_t schedule_gates;   /* 1: each circuit is applied in the order sqc_schedule_gates gives it
                                   for two cross-group qubits per pass (whatever threads_per_unit),
                                   as sqc_options.schedule_gates; 0 (default): the order given */

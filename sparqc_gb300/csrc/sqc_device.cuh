@@ -1,12 +1,13 @@
 // Device-side layout and arithmetic of the sparse statevector table.
 //
 // Table layout (one table per state, updated in place by every pass):
-//   hdr [nb]          16-byte bucket headers {group, epoch, aux}
+//   hdr [nb]          16-byte bucket headers {group, epoch, presence mask}
 //   keys[nb * 16]     64-bit stored keys, 16 per bucket (128 bytes)
 //   amps[nb * 16]     amplitudes, double2 (FP64) or float2 (FP32), same slot order
 //   list[nb]          indices of the live buckets, in claim order
 // A bucket holds the keys of one group G = key >> 4 at slot key & 15. Buckets are found by
-// linear probing from mix(G) & (nb - 1). A bucket is live iff hdr.epoch equals the state's
+// their mapped bits, or in hashed tables by linear probing from mix64(G) & (nb - 1) (sqc_types.h,
+// TableDev). A bucket is live iff hdr.epoch equals the state's
 // epoch, so a reset only bumps the epoch. A slot is occupied iff the low 4 bits of its
 // stored key equal the slot index; empty slots hold EMPTY(j) = 0xFFFF...F0 | (15 - j).
 // Live buckets are never freed between resets: a group whose keys are all pruned stays as an
@@ -171,27 +172,7 @@ __device__ __forceinline__ float neg(float x) {
     return __int_as_float(v);
 }
 
-// Gate descriptors are read-only for a whole launch and read by every warp for every slot it
-// holds, while the table streams through the same L1: descriptor loads are marked to stay in L1
-// (evict_last), so the table's traffic does not push them out to L2 between uses.
-__device__ __forceinline__ uint4 ld_desc4(const void* p) {
-    uint4 v;
-    asm("ld.global.nc.L1::evict_last.v4.u32 {%0, %1, %2, %3}, [%4];"
-        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ double ld_desc(const double* p) {
-    double v;
-    asm("ld.global.nc.L1::evict_last.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ float ld_desc(const float* p) {
-    float v;
-    asm("ld.global.nc.L1::evict_last.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-
-// Programmatic dependent launch. Direct passes are launched with programmatic stream
+// Programmatic dependent launch. Single passes are launched with programmatic stream
 // serialization, so the next pass's blocks may be placed on the SMs while the running pass
 // drains. Such a kernel first waits until the previous grid in the stream has completed and
 // its writes are visible (a no-op without that launch attribute), and then lets the next pass
@@ -199,88 +180,6 @@ __device__ __forceinline__ float ld_desc(const float* p) {
 // resident by then, so nothing waits on a block that cannot be placed.
 __device__ __forceinline__ void wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_next_grid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// A gate's (c, s) pair copied to shared memory, with its descriptor for the U matrix.
-template <class T> struct SmemCoef {
-    T c, s;
-    const GateDesc* g;
-};
-
-// Coefficients are read through a pointer to the (L1-resident, warp-broadcast) descriptor, or
-// from the pair a pass staged in shared memory.
-template <class T> struct Coef;
-template <> struct Coef<double> {
-    __device__ static __forceinline__ double c(const GateDesc* g) { return ld_desc(&g->c); }
-    __device__ static __forceinline__ double s(const GateDesc* g) { return ld_desc(&g->s); }
-    __device__ static __forceinline__ double m(const GateDesc* g, int i) { return ld_desc(&g->m[i]); }
-    __device__ static __forceinline__ double c(const SmemCoef<double>& k) { return k.c; }
-    __device__ static __forceinline__ double s(const SmemCoef<double>& k) { return k.s; }
-    __device__ static __forceinline__ double m(const SmemCoef<double>& k, int i) { return ld_desc(&k.g->m[i]); }
-};
-template <> struct Coef<float> {
-    __device__ static __forceinline__ float c(const GateDesc* g) { return ld_desc(&g->cf); }
-    __device__ static __forceinline__ float s(const GateDesc* g) { return ld_desc(&g->sf); }
-    __device__ static __forceinline__ float m(const GateDesc* g, int i) { return ld_desc(&g->mf[i]); }
-    __device__ static __forceinline__ float c(const SmemCoef<float>& k) { return k.c; }
-    __device__ static __forceinline__ float s(const SmemCoef<float>& k) { return k.s; }
-    __device__ static __forceinline__ float m(const SmemCoef<float>& k, int i) { return ld_desc(&k.g->mf[i]); }
-};
-
-// Branching update seen from one member of a pair, for gate kind K: a = own amplitude,
-// b = partner amplitude, bit = own logical target bit. Each form rounds exactly like the
-// reference's pair formula for that member (a + (-b) == a - b and (-s)*x == -(s*x) hold
-// exactly in IEEE arithmetic):
-//   H : bit 0 -> f*(v0 + v1),             bit 1 -> f*(v0 - v1)
-//   Rx: c*own + s*(i-rotated partner)      (symmetric in the two members)
-//   Ry: bit 0 -> c*v0 - s*v1,             bit 1 -> c*v1 + s*v0
-//   U : self term first, then partner term, fused multiply-add chain (no reference form).
-template <class T, uint32_t K, class G>
-__device__ __forceinline__ Cx<T> branch_update(const G& g, bool bit, Cx<T> a, Cx<T> b) {
-    using A = Arith<T>;
-    Cx<T> o;
-    if constexpr (K == KH) {
-        const T f = Coef<T>::c(g);
-        const Cx<T> x = bit ? b : a;
-        const Cx<T> y = bit ? Cx<T>{neg(a.r), neg(a.i)} : b;
-        o.r = A::mul(f, A::add(x.r, y.r));
-        o.i = A::mul(f, A::add(x.i, y.i));
-    } else if constexpr (K == KRX) {
-        const T c = Coef<T>::c(g), s = Coef<T>::s(g);
-        o.r = A::add(A::mul(c, a.r), A::mul(s, b.i));
-        o.i = A::sub(A::mul(c, a.i), A::mul(s, b.r));
-    } else if constexpr (K == KRY) {
-        const T c = Coef<T>::c(g), s0 = Coef<T>::s(g);
-        const T s = bit ? s0 : neg(s0);
-        o.r = A::add(A::mul(c, a.r), A::mul(s, b.r));
-        o.i = A::add(A::mul(c, a.i), A::mul(s, b.i));
-    } else {  // KU
-        const T m00r = Coef<T>::m(g, 0), m00i = Coef<T>::m(g, 1), m01r = Coef<T>::m(g, 2), m01i = Coef<T>::m(g, 3);
-        const T m10r = Coef<T>::m(g, 4), m10i = Coef<T>::m(g, 5), m11r = Coef<T>::m(g, 6), m11i = Coef<T>::m(g, 7);
-        const T msr = bit ? m11r : m00r, msi = bit ? m11i : m00i;
-        const T mor = bit ? m10r : m01r, moi = bit ? m10i : m01i;
-        o.r = A::fma(neg(moi), b.i, A::fma(mor, b.r, A::fma(neg(msi), a.i, A::mul(msr, a.r))));
-        o.i = A::fma(moi, b.r, A::fma(mor, b.i, A::fma(msi, a.r, A::mul(msr, a.i))));
-    }
-    return o;
-}
-
-// Diagonal update of one amplitude for gate kind K (reference: z_core, phase_core, rz_core).
-template <class T, uint32_t K, class G>
-__device__ __forceinline__ Cx<T> diag_update(const G& g, bool bit, Cx<T> a) {
-    using A = Arith<T>;
-    if constexpr (K == KZ) return bit ? Cx<T>{neg(a.r), neg(a.i)} : a;
-    else if constexpr (K == KS) return bit ? Cx<T>{neg(a.i), a.r} : a;
-    else if constexpr (K == KSDG) return bit ? Cx<T>{a.i, neg(a.r)} : a;
-    else if constexpr (K == KYPH) return bit ? Cx<T>{neg(a.i), a.r} : Cx<T>{a.i, neg(a.r)};
-    else if constexpr (K == KRZ) {
-        const T c = Coef<T>::c(g), s0 = Coef<T>::s(g);
-        const T s = bit ? s0 : neg(s0);   // bit 0: conj(a)*v0, bit 1: a*v1
-        return Cx<T>{A::sub(A::mul(c, a.r), A::mul(s, a.i)), A::add(A::mul(c, a.i), A::mul(s, a.r))};
-    } else {  // KPHASE, KT, KTDG: only bit-1 amplitudes change (callers skip bit 0)
-        const T c = Coef<T>::c(g), s = Coef<T>::s(g);
-        return Cx<T>{A::sub(A::mul(c, a.r), A::mul(s, a.i)), A::add(A::mul(c, a.i), A::mul(s, a.r))};
-    }
-}
 
 // Swap update for gate kind K: the amplitude arriving from the partner (reference: x_core,
 // y_core).
@@ -311,22 +210,5 @@ __device__ __forceinline__ bool negligible(Cx<float> v, const PruneBits& t) {
     const float f = __int_as_float((int)t.f);
     return fabsf(v.r) <= f && fabsf(v.i) <= f;
 }
-
-// ---- asynchronous global -> shared copies (sm_80+ PTX) ----------------------------------
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-// Asynchronous 16-byte global -> shared copy (both addresses 16-byte aligned), L2 only.
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-
-// Close the thread's current group of cp.async copies.
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-
-// Wait until at most N of the thread's committed cp.async groups are still in flight.
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 }  // namespace sqc

@@ -153,7 +153,7 @@ extern "C" int sqc_apply_fixed(uint32_t nq, const uint64_t* keys_in, const doubl
                                                      outside, ctl);
         if (cudaGetLastError() != cudaSuccess) return SQC_ERR_CUDA;
     }
-    // passes that pair across one qubit; each pass's gates are encoded before the descriptors are uploaded
+    // passes of at most one gate that pairs groups; each pass's gates are encoded before the descriptors are uploaded
     struct Span {
         uint32_t g0, g1, dim[3];
         bool pair, fixed;
@@ -162,16 +162,19 @@ extern "C" int sqc_apply_fixed(uint32_t nq, const uint64_t* keys_in, const doubl
     size_t ns = 0, i = 0;
     while (i < n_gates) {
         const size_t start = i;
-        uint32_t pairing = kNoQubit;
+        // a gate that pairs groups begins a pass: each is checked against the scratch table's room
+        uint32_t q[2] = {kNoQubit, kNoQubit};
+        const bool pair = !diag_kind(hd[i].kind) && hd[i].target >= (uint32_t)kSlotBits;
         for (; i < n_gates && i - start < (size_t)kMaxRun; ++i) {
-            if (diag_kind(hd[i].kind) || hd[i].target == pairing) continue;
-            if (pairing != kNoQubit) break;
-            pairing = hd[i].target;
+            const uint32_t t = hd[i].target;
+            if (diag_kind(hd[i].kind)) continue;
+            if (t >= (uint32_t)kSlotBits && i != start) break;
+            if (t == q[0] || t == q[1]) continue;
+            if (q[1] != kNoQubit) break;
+            q[q[0] == kNoQubit ? 0 : 1] = t;
         }
-        const bool pair = pairing != kNoQubit && pairing >= (uint32_t)kSlotBits;
         bool fixed = true;
         for (size_t k = start; k < i; ++k) fixed = fixed && diag_kind(hd[k].kind);
-        const uint32_t q[2] = {pairing, kNoQubit};
         Span& sp = spans[ns++];
         sp = Span{(uint32_t)start, (uint32_t)i, {0, 0, 0}, pair, fixed};
         encode_column_pass(hd, start, i, q, sp.dim);

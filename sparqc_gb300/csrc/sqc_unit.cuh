@@ -223,8 +223,12 @@ __device__ __forceinline__ Cx<T> shfl_cx(Cx<T> a, int off) {
 }
 
 // ---- one gate on the slots a lane holds ---------------------------------------------------------
-// Formulas and rounding are branch_update's, swap_update's and diag_update's (sqc_device.cuh): an
-// Rx, Ry, Rz or Phase result is C + P', C = c * own, P' the s-product of the own or the partner
+// Every result rounds as the reference's pair formula for that member (emulator/device/device_data.cuh:159-319):
+//   H : bit 0 -> f*(v0 + v1),             bit 1 -> f*(v0 - v1)
+//   Rx: c*own + s*(i-rotated partner)      (symmetric in the two members)
+//   Ry: bit 0 -> c*v0 - s*v1,             bit 1 -> c*v1 + s*v0
+//   U : self term first, then partner term, fused multiply-add chain (no reference form).
+// An Rx, Ry, Rz or Phase result is C + P', C = c * own, P' the s-product of the own or the partner
 // amplitude with its sign flipped and its components exchanged as the kind asks (a - b and a + (-b),
 // (-s) * x and -(s * x), and (-1) * a + b and b - a, round alike).
 template <class T, int S> struct Slots {
