@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kThreads, UnitOcc<T, DIMS>::kMin) unit_kernel(
         for (unsigned long long e0 = w * piece; e0 < n; e0 += nw * piece)
             walk_entries<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, e0, umin64(e0 + piece, n), a.heads, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
     } else {
-        walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, nw, a.heads, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+        walk_all_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, nw, a.heads, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
     }
     finish_pass(ctl, cnt_nnz, cnt_empty, upd, nnz_in, a.keys_fixed != 0, a.nx > 0, a.amp_bytes);
 }
@@ -232,7 +232,11 @@ __global__ void __launch_bounds__(kThreads, HASHED ? kHashBlocks<T> : UnitOcc<T,
                 for (unsigned long long e0 = w * piece; e0 < n; e0 += nw * piece)
                     walk_entries<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, e0, umin64(e0 + piece, n), heads, sg[p & 1], gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
             } else {
-                walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, nw, heads, sg[p & 1], gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+                // (FP32 runs have four rounds at most, and no registers to spare for turning the deal)
+                if constexpr (sizeof(T) == 4)
+                    walk_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, up.units, nw, heads, sg[p & 1], gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+                else
+                    walk_all_units<T, DIMS>(a.t, a.t.map_q, ctl, ep, up, w, nw, heads, sg[p & 1], gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
             }
             o += 1 + ng;
         }
