@@ -238,23 +238,19 @@ def profile_block(prof, name):
 def pass_roofline(s0, s1, alg_step, alg_pair_step, steps, dev_ms, peak, measured, precision, profile_name):
     """Roofline of the dominant gate-pass kernel over steps whose passes are timed one by one.
 
-    Every pass is bracketed by CUDA events on the engine's stream (time_passes); pair passes
-    (one direct_kernel<T, true> launch, or resolve_kernel + staged_kernel<T, true> on large
-    tables) and stream passes (direct/staged_kernel<T, false>) are timed apart. achieved =
-    the kind's algorithmic bytes (device counter) / its event time.
+    Every pass is one launch, bracketed by CUDA events on the engine's stream (time_passes);
+    passes that pair groups and those that do not are timed apart. achieved = the kind's
+    algorithmic bytes (device counter) / its event time.
     """
     t_pair = (s1["pass_ns_pair"] - s0["pass_ns_pair"]) / 1e9
     t_stream = (s1["pass_ns_stream"] - s0["pass_ns_stream"]) / 1e9
     n_pair = (s1["passes_pair"] - s0["passes_pair"]) / steps
     n_all = (s1["passes"] - s0["passes"]) / steps
-    staged = s1["buckets"] > (1 << 20)
-    T = "double" if precision == 64 else "float"
-    nx = "1|2|3" if precision == 32 else "1|2"   # FP32 passes pair across up to three high qubits
+    kernel = "unit_kernel<double, 2>" if precision == 64 else "unit_kernel<float, 3>"
     kinds = {
-        "pair": {"kernel": (f"resolve_kernel<{nx}> + staged_kernel<{T}, {nx}>" if staged
-                            else f"direct_kernel<{T}, {nx}>") + " (passes pairing 16-key groups)",
+        "pair": {"kernel": kernel + " (passes pairing 16-key groups)",
                  "bytes": alg_pair_step * steps, "t": t_pair, "passes": n_pair},
-        "stream": {"kernel": f"staged_kernel<{T}, 0>" if staged else f"direct_kernel<{T}, 0>",
+        "stream": {"kernel": kernel + " (other passes)",
                    "bytes": (alg_step - alg_pair_step) * steps, "t": t_stream, "passes": n_all - n_pair},
     }
     dom = max(kinds, key=lambda k: kinds[k]["t"])
@@ -264,7 +260,7 @@ def pass_roofline(s0, s1, alg_step, alg_pair_step, steps, dev_ms, peak, measured
     out = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
            "traffic": (prof["traffic_bytes_per_launch"] * prof.get("traffic_scale", 1.0)
                        if "traffic_bytes_per_launch" in prof else None), "kernel": d["kernel"],
-           "launches_per_step": d["passes"] * (2 if (staged and dom == "pair") else 1),
+           "launches_per_step": d["passes"],
            "alg_bytes_per_pass": d["bytes"] / steps / max(d["passes"], 1),
            "avg_pass_us": 1e6 * d["t"] / steps / max(d["passes"], 1),
            "share_of_step_time": d["t"] * 1e3 / dev_ms if dev_ms > 0 else None,
@@ -281,12 +277,12 @@ def pass_roofline(s0, s1, alg_step, alg_pair_step, steps, dev_ms, peak, measured
     return out
 
 
-def profile_for(args, staged):
+def profile_for(args):
     """Name of the committed ncu summary of this workload's dominant pass kernel."""
     prec = f"fp{args.precision}"
     if args.workload == "c4":
         return f"batch_run_kernel_c4_{prec}"
-    return f"{'staged' if staged else 'direct'}_kernel_{args.workload}_{prec}"
+    return f"unit_kernel_{args.workload}_{prec}"
 
 
 def host_numa(device):
@@ -589,7 +585,7 @@ def run_gpu(args):
     peaks = measured_peaks()
     peak = peaks["hbm_gbs"] if peaks else 6800.0
     roofline = pass_roofline(r0, r1, alg_per_step, alg_pair_step, args.steps, dev_ms_t, peak, peaks is not None,
-                             args.precision, profile_for(args, s1["buckets"] > (1 << 20)))
+                             args.precision, profile_for(args))
     roofline["pass_timing"] = ("per-pass CUDA events over the same number of further steps of the same circuit "
                                "(events between passes stop the launch overlap of the measured steps)")
     roofline["ms_per_step_with_pass_events"] = dev_ms_t / args.steps

@@ -226,7 +226,6 @@ int Engine::ensure_desc(size_t n) {
     int rc;
     if ((rc = cuda(cudaMalloc(&d_desc_, cap * sizeof(GateDesc)), "cudaMalloc(desc)"))) return rc;
     if ((rc = cuda(cudaMallocHost(&h_desc_, cap * sizeof(GateDesc)), "cudaMallocHost(desc)"))) return rc;
-    // tiny-launch pass records, indexed like the descriptors (a flush has no more passes than gates)
     desc_cap_ = cap;
     return SQC_OK;
 }
