@@ -383,7 +383,6 @@ int Engine::apply(const sqc_gate* gates, uint64_t n) {
 int Engine::flush(bool hold_last) {
     if (pending_.empty()) return SQC_OK;
     const size_t n = pending_.size();
-    clean_ = false;
     int rc;
     if (desc_used_ + n > desc_cap_) {
         std::vector<sqc_gate> keep;
@@ -395,6 +394,7 @@ int Engine::flush(bool hold_last) {
         pending_.swap(keep);
         if ((rc = ensure_desc(n))) return rc;
     }
+    clean_ = false;   // (after the sync above, which sets it)
     const size_t log_base = log_.size();
     log_.insert(log_.end(), pending_.begin(), pending_.end());
     GateDesc* hd = h_desc_ + desc_used_;

@@ -341,3 +341,20 @@ def test_column_passes(keys, cross, precision):
         group = KINDS[pick(3)]
         gs.append((group[pick(len(group))], t, ctl, 0.3 + 0.1 * i) if i % 8 else (G.X, t, ctl[:1], 0.0))
     _both(64, G.gate_array(gs[: 48 if keys < 20000 else 14]), precision, max_cross_qubits=cross, init=(key, amp[0], amp[1]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k,buckets", [(10, 1024), (14, 64)])
+def test_questions_after_one_long_call(k, buckets):
+    """More gates in one call than the engine's descriptors hold: the state, its key count and its norm
+    are the whole circuit's, asked for without a sync."""
+    from sparqc_gb300.engine import State
+    g = circuits.random_circuit(20, k, 9000, 2, circuits.SplitMix64(k), kinds=KINDS)
+    st, o = State(20, initial_buckets=buckets), SparseOracle()
+    o.apply(g)
+    st.apply(g)
+    want = o.state(sorted=True)
+    assert st.nnz() == want[0].size
+    assert abs(st.norm2() - float((want[1] ** 2 + want[2] ** 2).sum())) < 1e-9
+    assert_identical(st.state(sorted=True), want)
+    st.close()
