@@ -83,7 +83,9 @@ int Engine::fail(int code, const std::string& msg) {
 int Engine::cuda(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return SQC_OK;
     err = std::string(what) + ": " + cudaGetErrorString(e);
-    return e == cudaErrorMemoryAllocation ? SQC_ERR_OOM : SQC_ERR_CUDA;
+    if (e != cudaErrorMemoryAllocation) return SQC_ERR_CUDA;
+    cudaGetLastError();   // reported here: the next launch must not find it
+    return SQC_ERR_OOM;
 }
 
 // A launcher reported a failed launch: its error, or a generic one when the runtime holds none.
@@ -481,6 +483,7 @@ int Engine::flush(bool hold_last) {
         GroupMap m = map_;
         if (m.extend(after[spans.back().g1 - 1].kmask, nq_) && m.n <= 2) dims = 2;
     }
+    const bool was_fresh = fresh_;
     fresh_ = fresh_ && spans.empty();
     for (Span& sp : spans) {
         const uint32_t q[3] = {sp.q1, sp.q2, sp.q3};
@@ -496,12 +499,26 @@ int Engine::flush(bool hold_last) {
     }
     if (mapped_) map_.store(&a.t);   // a pass uses the first dn of the mapped bits
     a.dims = dims;
+    size_t launched = 0;   // passes of this flush
+    // The flush cannot go on: the gates after the last launched pass go back to the queue, with the
+    // planner and the map as that pass left them, so that nothing is lost if the caller goes on.
+    auto put_back = [&](int rc_) {
+        pending_.insert(pending_.begin(), log_.begin() + (std::ptrdiff_t)snap_log_, log_.end());
+        gates_applied_ -= log_.size() - snap_log_;
+        log_.resize(snap_log_);
+        plan_ = snap_plan_;
+        if (mapped_ && launched < spans.size()) map_.n = spans[launched].map0;
+        fresh_ = was_fresh && !launched;
+        desc_used_ += nd;   // the launched passes read theirs
+        return rc_;
+    };
     if ((rc = cuda(cudaMemcpyAsync(d_desc_ + desc_used_, hd, nd * sizeof(GateDesc), cudaMemcpyHostToDevice, stream_),
                    "H2D gate descriptors")))
-        return rc;
+        return put_back(rc);
     cudaEvent_t ev_prev = nullptr;
-    if (time_passes_ && (rc = record_event(&ev_prev))) return rc;
+    if (time_passes_ && (rc = record_event(&ev_prev))) return put_back(rc);
     auto record = [&](const Span& sp) {
+        ++launched;
         passes_pair_ += sp.nx > 0 ? 1 : 0;
         passes_.push_back(PassRec{snap_log_, snap_plan_, sp.map0, sp.dn, sp.nx, sp.keys});
         snap_log_ = src[sp.g1 - 1] + 1;
@@ -543,8 +560,8 @@ int Engine::flush(bool hold_last) {
             run.tag = run_tag_;
             run_tag_ += run.np;
             UnitHead* w = run.words;
-            for (; s < e; ++s) {
-                const Span& r = spans[s];
+            for (size_t i = s; i < e; ++i) {
+                const Span& r = spans[i];
                 *w++ = UnitHead{(uint32_t)(r.g1 - r.g0) | (r.fixed ? kRunFixed : 0u) | (r.nx ? kRunPair : 0u) |
                                     ((mapped_ ? r.dn : r.nx) << 16),
                                 r.dim[0] | (r.dim[1] << 8) | (r.dim[2] << 16), (uint32_t)r.g0, 0u};
@@ -554,10 +571,10 @@ int Engine::flush(bool hold_last) {
                     const unsigned long long bounds[2] = {group_bound(after[r.g1 - 1], nq_), r.keys};
                     std::memcpy(w++, bounds, sizeof bounds);
                 }
-                record(r);
             }
             const int nl = launch_run_passes(run, dims, items, dbl_, sms_, stream_);
-            if (nl < 0) return launch_failed("gate passes");
+            if (nl < 0) return put_back(launch_failed("gate passes"));
+            for (; s < e; ++s) record(spans[s]);
             launches_ += (uint64_t)nl;
             continue;
         }
@@ -569,7 +586,7 @@ int Engine::flush(bool hold_last) {
         a.grow_bound = group_bound(after[sp.g1 - 1], nq_);
         a.key_bound = sp.keys;
         if (!mapped_ && sp.nx && grown(sp.nx, a.grow_bound, sp.keys) > roomy_groups()) {
-            if ((rc = make_room(sp.nx, a.grow_bound, sp.keys))) return rc;
+            if ((rc = make_room(sp.nx, a.grow_bound, sp.keys))) return put_back(rc);
             a.t = dev();
             a.max_groups = max_groups();
         }
@@ -579,15 +596,15 @@ int Engine::flush(bool hold_last) {
         if (mapped_)
             for (size_t k = sp.g0; k < sp.g1; ++k) a.heads[k - sp.g0] = UnitHead{hd[k].om, hd[k].ov, hd[k].loc, hd[k].pad + 1u};
         const int nl = mapped_ ? launch_unit_pass(a, dbl_, sms_, stream_) : launch_hash_pass(a, hint, dbl_, sms_, stream_);
-        if (nl < 0) return launch_failed("gate pass");
+        if (nl < 0) return put_back(launch_failed("gate pass"));
+        record(sp);
+        launches_ += (uint64_t)nl;
         if (time_passes_) {
             cudaEvent_t ev = nullptr;
-            if ((rc = record_event(&ev))) return rc;
+            if ((rc = record_event(&ev))) return put_back(rc);
             timed_.push_back(TimedPass{ev_prev, ev, sp.nx > 0});
             ev_prev = ev;
         }
-        record(sp);
-        launches_ += (uint64_t)nl;
         // a mapped pass the table is too small for refuses, and so would every later one: they
         // are queued again, with it, when the table has grown
         if (mapped_ && (1ULL << sp.dn) > a.max_groups) break;
@@ -631,7 +648,13 @@ int Engine::make_room(uint32_t nx, unsigned long long bound, unsigned long long 
         hash_load_ = kMaxLoad;
         return SQC_OK;   // a pass that still does not fit refuses; sync() decides
     }
-    if ((rc = rebuild(nb, false))) return rc;
+    // no memory for it: the present table fills up, and a pass that does not fit refuses
+    rc = rebuild(nb, false);
+    if (rc == SQC_ERR_OOM || rc == SQC_ERR_BUDGET) {
+        hash_load_ = kMaxLoad;
+        return SQC_OK;
+    }
+    if (rc) return rc;
     if (grown(nx, bound, keys) > roomy_groups()) hash_load_ = kMaxLoad;
     passes_.clear();   // all verified: later ones count from here
     return SQC_OK;

@@ -34,7 +34,9 @@ struct Device {
     size_t total = (size_t)284 << 30;            // bytes of the device
     size_t big_limit = 0;                        // allocations of at least this many bytes fail (0: none)
     int fail_big = 0;                            // ... while this is positive
+    int fail_copies = 0;                         // copies to the device that fail
     long bad = 0;                                // accesses outside an allocation, misuse of events
+    cudaError_t last = cudaSuccess;              // what cudaGetLastError answers, once
     long syncs = 0, passes = 0, runs = 0;
     bool capturing = false;
     std::vector<long> events;                    // time of each event's last record, 0: never
@@ -182,8 +184,8 @@ void sqc_default_options(sqc_options* o) {
 cudaError_t cudaMalloc(void** p, size_t n) {
     using namespace fake;
     *p = nullptr;
-    if (dev.held + n > dev.total) return cudaErrorMemoryAllocation;
-    if (dev.big_limit && n >= dev.big_limit && dev.fail_big > 0) { --dev.fail_big; return cudaErrorMemoryAllocation; }
+    if (dev.held + n > dev.total) return dev.last = cudaErrorMemoryAllocation;
+    if (dev.big_limit && n >= dev.big_limit && dev.fail_big > 0) { --dev.fail_big; return dev.last = cudaErrorMemoryAllocation; }
     // a range that is not backed is only an address
     static unsigned char* next = reinterpret_cast<unsigned char*>(1ULL << 60);
     unsigned char* q = n <= kBacked ? (unsigned char*)std::calloc(1, n) : next;
@@ -216,6 +218,7 @@ cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) {
 }
 cudaError_t cudaMemset(void* p, int v, size_t n) { return cudaMemsetAsync(p, v, n, nullptr); }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) {
+    if (k == cudaMemcpyHostToDevice && fake::dev.fail_copies > 0) { --fake::dev.fail_copies; return cudaErrorUnknown; }
     if (!fake::dev.inside(k == cudaMemcpyHostToDevice ? d : s, n)) { ++fake::dev.bad; return cudaSuccess; }
     std::memcpy(d, s, n);
     return cudaSuccess;
@@ -246,7 +249,11 @@ cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t a, cudaEvent_t b) {
     *ms = (float)(y - x);
     return cudaSuccess;
 }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+    const cudaError_t e = fake::dev.last;
+    fake::dev.last = cudaSuccess;
+    return e;
+}
 cudaError_t cudaPeekAtLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "error"; }
 cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
@@ -256,7 +263,7 @@ cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { *f = fake::dev.total - fake::
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) { a->type = cudaMemoryTypeHost; return cudaSuccess; }
 }
 
-// ---- launchers ----
+// ---- launchers (as theirs do, they answer with the last error) ----
 namespace sqc {
 using namespace fake;
 
@@ -268,7 +275,7 @@ cudaError_t launch_set_zero(const TableDev&, Ctl* ctl, bool, cudaStream_t) {
     st.amp = {{0, 1.0}};
     st.live = {0};
     ctl->nnz = ctl->list_n = ctl->list_tail = 1;
-    return cudaSuccess;
+    return cudaGetLastError();
 }
 cudaError_t launch_set_state(const unsigned long long* keys, const double* re, const double* im, unsigned long long n,
                              unsigned long long frame, const TableDev&, Ctl* ctl, bool, int, cudaStream_t) {
@@ -282,7 +289,7 @@ cudaError_t launch_set_state(const unsigned long long* keys, const double* re, c
     }
     ctl->nnz = n;
     ctl->list_n = ctl->list_tail = st.live.size();
-    return cudaSuccess;
+    return cudaGetLastError();
 }
 int launch_unit_pass(const PassArgs& a, bool, int, cudaStream_t) {
     fake::pass(a.ctl, a.gates, a.g0, a.g1, a.prune, (1ULL << a.dn) > a.max_groups);
@@ -309,7 +316,7 @@ int launch_run_passes(const RunArgs& a, uint32_t, unsigned long long, bool, int,
     }
     return 1;
 }
-cudaError_t launch_refresh_masks(const TableDev&, Ctl*, unsigned long long, int, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_refresh_masks(const TableDev&, Ctl*, unsigned long long, int, cudaStream_t) { return cudaGetLastError(); }
 static void emit(const TableDev&, Ctl* ctl, unsigned long long frame, unsigned long long* ok, double* re, double* im,
                  unsigned long long cap, unsigned long long smask, unsigned long long sval) {
     std::vector<std::pair<unsigned long long, Amp>> out;
@@ -327,7 +334,7 @@ cudaError_t launch_readout(const TableDev& t, Ctl* ctl, unsigned long long, unsi
                            unsigned long long* ok, double* re, double* im, unsigned long long cap, bool, PruneBits, int,
                            cudaStream_t, unsigned long long smask, unsigned long long sval) {
     emit(t, ctl, frame, ok, re, im, cap, smask, sval);
-    return cudaSuccess;
+    return cudaGetLastError();
 }
 RankJob rank_job(const TableDev& t, const Ctl* ctl, unsigned long long frame, unsigned long long, unsigned long long) {
     RankJob j;
@@ -337,18 +344,18 @@ RankJob rank_job(const TableDev& t, const Ctl* ctl, unsigned long long frame, un
     j.frame = frame;
     return j;
 }
-cudaError_t RankScratch::need(size_t, size_t) { return cudaSuccess; }
+cudaError_t RankScratch::need(size_t, size_t) { return cudaGetLastError(); }
 void RankScratch::release() {}
 cudaError_t launch_ranked(const RankJob& one, const RankJob*, uint32_t, unsigned long long, unsigned long long*, bool,
                           unsigned long long* k, double* re, double* im, unsigned long long cap, bool, PruneBits,
                           unsigned long long*, unsigned long long*, cudaStream_t) {
     emit(one.t, const_cast<Ctl*>(one.ctl), one.frame, k, re, im, cap, 0, 0);
-    return cudaSuccess;
+    return cudaGetLastError();
 }
-cudaError_t launch_norm(const TableDev&, Ctl*, unsigned long long, bool, ExactSums*, int, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_norm(const TableDev&, Ctl*, unsigned long long, bool, ExactSums*, int, cudaStream_t) { return cudaGetLastError(); }
 cudaError_t launch_compare(const TableDev&, const Ctl*, unsigned long long, bool, const TableDev&, const Ctl*, unsigned long long,
-                           bool, unsigned long long, Ctl*, ExactSums*, int, cudaStream_t) { return cudaSuccess; }
-cudaError_t measure_fp64_rate(int, double*) { return cudaSuccess; }
+                           bool, unsigned long long, Ctl*, ExactSums*, int, cudaStream_t) { return cudaGetLastError(); }
+cudaError_t measure_fp64_rate(int, double*) { return cudaGetLastError(); }
 // The rebuild drops groups without keys; a hashed table takes at most what its buckets hold.
 cudaError_t launch_rehash(const TableDev&, unsigned long long, const TableDev& nt, unsigned, int, Ctl* ctl, int, cudaStream_t) {
     State& st = fake::dev.state[ctl];
@@ -356,21 +363,21 @@ cudaError_t launch_rehash(const TableDev&, unsigned long long, const TableDev& n
     for (auto& kv : st.amp) st.live.insert(kv.first >> kSlotBits);
     ctl->list_tail = st.live.size();
     if (st.live.size() > nt.mask + 1) ctl->status = ST_TABLE_FULL;
-    return cudaSuccess;
+    return cudaGetLastError();
 }
 cudaError_t launch_pattern_prob(const TableDev&, Ctl*, unsigned long long, bool, unsigned long long, unsigned long long, ExactSums*,
-                                int, cudaStream_t) { return cudaSuccess; }
+                                int, cudaStream_t) { return cudaGetLastError(); }
 cudaError_t launch_collapse(const TableDev&, Ctl*, unsigned long long, bool, unsigned long long, unsigned long long, double, int,
-                            cudaStream_t) { return cudaSuccess; }
+                            cudaStream_t) { return cudaGetLastError(); }
 size_t sort_scratch_bytes(unsigned long long) { return 256; }
 cudaError_t sort_entries(SortBuffers& b, unsigned long long n, uint32_t, bool, int, cudaStream_t) {
     std::memcpy(b.keys_out, b.keys_in, n * 8);   // (emit writes in key order)
     std::memcpy(b.re_out, b.re_in, n * 8);
     std::memcpy(b.im_out, b.im_in, n * 8);
-    return cudaSuccess;
+    return cudaGetLastError();
 }
 size_t cumulate_scratch_bytes(unsigned long long) { return 256; }
-cudaError_t cumulate(const double*, const double*, double*, unsigned long long, void*, size_t, int, cudaStream_t) { return cudaSuccess; }
+cudaError_t cumulate(const double*, const double*, double*, unsigned long long, void*, size_t, int, cudaStream_t) { return cudaGetLastError(); }
 cudaError_t launch_sample(const unsigned long long*, const double*, unsigned long long, unsigned long long, unsigned long long,
-                          unsigned long long*, int, cudaStream_t) { return cudaSuccess; }
+                          unsigned long long*, int, cudaStream_t) { return cudaGetLastError(); }
 }  // namespace sqc

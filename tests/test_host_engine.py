@@ -74,3 +74,55 @@ def test_questions_after_more_gates_than_descriptors(engine_objects, tmp_path, b
         CHECK(holds(e, expected(g)));
     }
     """ % (buckets, pieces))
+
+
+THIN = """
+    // few keys over many qubits: a state no map is worth, which outgrows its hashed table
+    std::vector<sqc_gate> g;
+    for (uint32_t q = 0; q < 6; ++q) g.push_back(gate(KH, q));
+    for (uint32_t i = 0; i < 26; ++i) g.push_back(gate(KX, 6 + i, 1ULL << (i % 6)));
+    for (uint32_t i = 0; i < 6; ++i) g.push_back(gate(KRY, 8 + 3 * i, 0, 0.7));
+"""
+
+
+@pytest.mark.parametrize("lasting", [1, 2, 1000000])
+def test_allocation_failure_in_a_flush_loses_no_gate(engine_objects, tmp_path, lasting):
+    """The table cannot be enlarged while a flush is launching (one failed allocation, two, all of them):
+    a call may say so, but the gates stay, and the state is the whole circuit's once there is memory."""
+    run(engine_objects, tmp_path, THIN + """
+    Engine e;
+    sqc_options o;
+    sqc_default_options(&o);
+    o.initial_buckets = 64;
+    make(e, 60, &o);
+    dev.big_limit = 64 * e.bucket_bytes_now();
+    dev.fail_big = %d;
+    CHECK(e.apply(g.data(), g.size()) == SQC_OK);
+    const int a = e.flush(), b = e.sync();
+    CHECK(a == SQC_OK || a == SQC_ERR_OOM);
+    CHECK(b == SQC_OK || b == SQC_ERR_OOM);
+    if (%d > 1000) {
+        CHECK(b == SQC_ERR_OOM);
+        CHECK(e.sync() == SQC_ERR_OOM);   // it stays an error while there is no memory
+        uint64_t n = 0;
+        CHECK(e.nnz(&n) == SQC_ERR_OOM);
+    }
+    dev.fail_big = 0;
+    CHECK(holds(e, expected(g)));
+    sqc_stats st;
+    e.stats(&st);
+    CHECK(st.gates_applied == g.size());
+    """ % (lasting, lasting))
+
+
+def test_failed_copy_in_a_flush_loses_no_gate(engine_objects, tmp_path):
+    """A flush that cannot upload its descriptors queues its gates again."""
+    run(engine_objects, tmp_path, THIN + """
+    Engine e;
+    make(e, 60);
+    CHECK(e.apply(g.data(), 10) == SQC_OK && e.flush() == SQC_OK);
+    dev.fail_copies = 1;
+    CHECK(e.apply(g.data() + 10, g.size() - 10) == SQC_OK);
+    CHECK(e.flush() == SQC_ERR_CUDA);
+    CHECK(holds(e, expected(g)));
+    """)
