@@ -354,7 +354,7 @@ def test_questions_after_one_long_call(k, buckets):
     o.apply(g)
     st.apply(g)
     want = o.state(sorted=True)
-    assert st.nnz() == want[0].size
+    assert st.nnz == want[0].size
     assert abs(st.norm2() - float((want[1] ** 2 + want[2] ** 2).sum())) < 1e-9
     assert_identical(st.state(sorted=True), want)
     st.close()
