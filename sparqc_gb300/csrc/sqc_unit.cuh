@@ -274,17 +274,17 @@ __device__ __forceinline__ void pair_results(const UGate<float>& g, const GateDe
     }
 }
 
-__device__ __forceinline__ bool is_zero(double x) {   // no FP64 compare
-    return (((uint32_t)__double2hiint(x) & 0x7FFFFFFFu) | (uint32_t)__double2loint(x)) == 0;
-}
+// Whether x is finite and its high word not 0: adding +-0 to it then changes nothing (no FP64 compare).
+__device__ __forceinline__ bool plain(double x) { return ((uint32_t)__double2hiint(x) & 0x7FFFFFFFu) - 1u < 0x7FEFFFFFu; }
 // U's chain for one member. `uniform`: its logical bit is the whole warp's; the bit-0 row's own
-// coefficient is real, and its imaginary terms add +-0, which changes nothing unless the sum so far
-// is itself 0: two of the chain's eight FP64 instructions are spared.
+// coefficient is real, and its imaginary terms are 0 * a part of a: they add +-0, and two of the chain's
+// eight FP64 instructions are spared, unless a part is infinite or NaN (the sum so far, a part
+// times a coefficient of at most 1, then is too) or the sum so far is 0.
 __device__ __forceinline__ Cx<double> u_update(const GateDesc* gd, bool bit, bool uniform, Cx<double> a, Cx<double> b) {
     auto m = [&](int i) { return __ldg(&gd->m[i]); };
     const double msr = bit ? m(6) : m(0), mor = bit ? m(4) : m(2), moi = bit ? m(5) : m(3);
     double r = __dmul_rn(msr, a.r), i = __dmul_rn(msr, a.i);
-    if (!uniform || bit || is_zero(r) || is_zero(i)) {
+    if (!uniform || bit || !plain(r) || !plain(i)) {
         const double msi = bit ? m(7) : m(1);
         r = __fma_rn(neg(msi), a.i, r);
         i = __fma_rn(msi, a.r, i);

@@ -358,3 +358,37 @@ def test_questions_after_one_long_call(k, buckets):
     assert abs(st.norm2() - float((want[1] ** 2 + want[2] ** 2).sum())) < 1e-9
     assert_identical(st.state(sorted=True), want)
     st.close()
+
+
+def _same(got, want):
+    """Equal keys, and equal parts where neither is NaN; NaN in the same places."""
+    assert np.array_equal(got[0], want[0])
+    for a, b in zip(got[1:], want[1:]):
+        assert np.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("hashed", [False, True])
+@pytest.mark.parametrize("kind", [G.U, G.H, G.RX, G.RY])
+def test_infinite_and_nan_amplitudes(kind, hashed, precision):
+    """Infinite and NaN parts follow the formulas wherever the pass puts the target: in a slot of the lane,
+    in another lane (the second of two such qubits), in the bucket, in a column."""
+    from sparqc_gb300.engine import State
+    rng = np.random.default_rng(11)
+    nq = 60 if hashed else 9
+    keys = np.unique(rng.integers(0, 1 << nq, 300, dtype=np.uint64)) if hashed else np.arange(1 << nq, dtype=np.uint64)
+    for qubits in ((7,), (5, 6), (6, 5, 4), (2,), (1, 8)):
+        a = rng.standard_normal((2, keys.size))
+        odd = rng.choice(keys.size, 24, replace=False)
+        a[0, odd[:12]] = np.array([np.inf, -np.inf, np.nan, 0.0] * 3)
+        a[1, odd[6:18]] = np.array([np.inf, -np.inf, np.nan, 0.0] * 3)
+        gs = G.gate_array([(kind, q, ((q + 3) % nq,) if i else (), 0.9 + i, 0.4, 1.1) if kind == G.U else
+                           (kind, q, (), 0.9 + i) for i, q in enumerate(qubits)])
+        st, o = State(nq, precision=precision), SparseOracle(precision)
+        st.set_state(keys, a[0], a[1])
+        o.set_state(keys, a[0], a[1])
+        st.apply(gs)
+        o.apply(gs)
+        _same(st.state(sorted=True), o.state(sorted=True))
+        st.close()
