@@ -90,6 +90,7 @@ const char* plan_circuit(uint32_t nq, const sqc_gate* gates, uint64_t n, uint32_
                          const uint32_t q[3] = {q1, q2, q3};
                          uint32_t dim[3];
                          encode_unit_pass(c.desc.data(), g0, g1, q, c.map, dims, dim);
+                         c.odd = c.odd || odd_pass(c.desc.data(), g0, g1);
                          b.dn = (uint8_t)c.map.n;
                          for (int i = 0; i < 3; ++i) b.dim[i] = (uint8_t)dim[i];
                      }
@@ -211,6 +212,8 @@ int Batch::plan_and_upload() {
             return fail(SQC_ERR_ARG, "circuit " + std::to_string(i) + ": " + why);
     }
     plans_.swap(plans);
+    odd_ = false;
+    for (const CircuitPlan& c : plans_) odd_ = odd_ || c.odd;
     ran_ = synced_ = false;
     // descriptors and passes, concatenated
     size_t nd = 0, np = 0;
@@ -364,14 +367,14 @@ int Batch::run() {
     if (use_graph_) {
         if (!graph_exec_) {
             if ((rc = cuda(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "begin capture"))) return rc;
-            const cudaError_t le = launch_batch(args(), dbl_, grid(), (int)blocks_per_sm_, 0, stream_);
+            const cudaError_t le = launch_batch(args(), dbl_, grid(), (int)blocks_per_sm_, odd_, 0, stream_);
             const cudaError_t ce = cudaStreamEndCapture(stream_, &graph_);
             if ((rc = cuda(le, "batch launch (capture)")) || (rc = cuda(ce, "end capture"))) return rc;
             if ((rc = cuda(cudaGraphInstantiate(&graph_exec_, graph_, 0), "graph instantiate"))) return rc;
         }
         if ((rc = cuda(cudaGraphLaunch(graph_exec_, stream_), "graph launch"))) return rc;
     } else {
-        if ((rc = cuda(launch_batch(args(), dbl_, grid(), (int)blocks_per_sm_, 0, stream_), "batch launch"))) return rc;
+        if ((rc = cuda(launch_batch(args(), dbl_, grid(), (int)blocks_per_sm_, odd_, 0, stream_), "batch launch"))) return rc;
     }
     if ((rc = cuda(cudaEventRecord(ev1_, stream_), "event"))) return rc;
     launches_ += 2;

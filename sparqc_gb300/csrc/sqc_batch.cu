@@ -182,7 +182,7 @@ __device__ bool find_chunk(const BatchArgs& a, unsigned c, int lane, Claim* out)
 // on with the next pass's chunk 0, so a circuit that fits one chunk runs like a tiny state, one
 // barrier between passes. (A warp per chunk of two units, each with its own staged copy: 128
 // circuits FP32 9.6 ms, 256 circuits FP64 35 ms.)
-// MINB: blocks per SM the register allocation is sized for.
+// MINB: blocks per SM the register allocation is sized for; 1: circuits may have UO_ODD gates.
 template <class T, int MINB>
 __global__ void __launch_bounds__(kBatchThreads, MINB) batch_run_kernel(BatchArgs a) {
     constexpr int DIMS = (int)(sizeof(T) == 8 ? kBatchDims64 : kBatchDims32);
@@ -240,9 +240,9 @@ __global__ void __launch_bounds__(kBatchThreads, MINB) batch_run_kernel(BatchArg
         unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
         if (walk_list(n, bp.dn)) {
             for (unsigned long long i = ib + w; i < ie; i += kBatchWarps)
-                walk_entries<T, DIMS>(t, C.t.map_q, ctl, ep, up, i * 32, n, SharedHeads<T>{sg.g}, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+                walk_entries<T, DIMS>(t, C.t.map_q, ctl, ep, up, i * 32, n, SharedHeads<T, MINB == 1>{sg.g}, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
         } else {
-            walk_units<T, DIMS>(t, C.t.map_q, ctl, ep, up, (unsigned)(ib + w), (unsigned)ie, kBatchWarps, SharedHeads<T>{sg.g}, sg, gates, ng, lane, a.prune, cnt_nnz,
+            walk_units<T, DIMS>(t, C.t.map_q, ctl, ep, up, (unsigned)(ib + w), (unsigned)ie, kBatchWarps, SharedHeads<T, MINB == 1>{sg.g}, sg, gates, ng, lane, a.prune, cnt_nnz,
                              cnt_empty, upd);
         }
         cnt_nnz = warp_sum(cnt_nnz);
@@ -394,9 +394,10 @@ int batch_residency(bool dbl, int blocks_per_sm) {
     return c;
 }
 
-cudaError_t launch_batch(const BatchArgs& a, bool dbl, int grid, int blocks_per_sm, unsigned long long deadline_ns,
+cudaError_t launch_batch(const BatchArgs& a, bool dbl, int grid, int blocks_per_sm, bool odd, unsigned long long deadline_ns,
                          cudaStream_t st) {
     batch_begin_kernel<<<1, 1024, 0, st>>>(a, deadline_ns);
+    if (odd) return dbl ? launch_run<double, 1>(a, grid, st) : launch_run<float, 1>(a, grid, st);
     const bool v3 = blocks_per_sm == 0 || blocks_per_sm >= 3;
     if (dbl) return v3 ? launch_run<double, 3>(a, grid, st) : launch_run<double, 2>(a, grid, st);
     return v3 ? launch_run<float, 3>(a, grid, st) : launch_run<float, 2>(a, grid, st);

@@ -21,8 +21,9 @@ namespace sqc {
 
 // Blocks per SM that fit for the kernel variant chosen by blocks_per_sm (0: as many as fit).
 int batch_residency(bool dbl, int blocks_per_sm);
-// The begin kernel and the persistent kernel on `grid` blocks.
-cudaError_t launch_batch(const BatchArgs& a, bool dbl, int grid, int blocks_per_sm, unsigned long long deadline_ns,
+// The begin kernel and the persistent kernel on `grid` blocks; odd: a circuit has a gate with a coefficient that
+// is not finite.
+cudaError_t launch_batch(const BatchArgs& a, bool dbl, int grid, int blocks_per_sm, bool odd, unsigned long long deadline_ns,
                          cudaStream_t st);
 
 // Bytes of a table slice of nb buckets (header, keys, amplitudes, list; 256-byte aligned parts).
@@ -42,6 +43,7 @@ struct CircuitPlan {
     GroupMap map;                  // group bits its table is mapped by
     unsigned long long bound = 1;  // groups the circuit can ever hold
     uint64_t n_gates = 0;
+    bool odd = false;              // a gate has a coefficient that is not finite
 };
 
 // Plan a circuit from |0...0>. Returns nullptr or the reason it cannot be batched.
@@ -108,6 +110,7 @@ private:
     std::vector<CircuitPlan> plans_;
     std::vector<uint32_t> nqs_;                  // the prepared circuits, kept for re-planning
     std::vector<std::vector<sqc_gate>> gates_;   // as applied (schedule_gates order when sched_)
+    bool odd_ = false;                           // a circuit's plan is odd
     bool sched_ = false;
     uint32_t max_nx_ = 2;                        // qubits >= 4 a pass may pair across: 1 (pair units) or 2 (quads)
     std::vector<unsigned long long> nb_;

@@ -537,7 +537,7 @@ int Engine::flush(bool hold_last) {
         while (!time_passes_ && e < spans.size()) {
             const Span& r = spans[e];
             const size_t w = mapped_ ? 1 + r.g1 - r.g0 : 2;
-            if (words + w > kRunWords) break;
+            if (words + w > kRunWords || odd_pass(hd, r.g0, r.g1)) break;
             if (mapped_) {
                 if (r.dn > (dbl_ ? kRunMapFp64 : kRunMapFp32) || (1ULL << r.dn) > a.max_groups) break;
                 items = std::max(1ULL, (1ULL << r.dn) >> dims);
@@ -583,6 +583,7 @@ int Engine::flush(bool hold_last) {
         a.g1 = (uint32_t)sp.g1;
         a.nx = sp.nx;
         a.keys_fixed = sp.fixed ? 1u : 0u;
+        a.odd = odd_pass(hd, sp.g0, sp.g1) ? 1u : 0u;
         a.grow_bound = group_bound(after[sp.g1 - 1], nq_);
         a.key_bound = sp.keys;
         if (!mapped_ && sp.nx && grown(sp.nx, a.grow_bound, sp.keys) > roomy_groups()) {

@@ -203,6 +203,7 @@ extern "C" int sqc_apply_fixed(uint32_t nq, const uint64_t* keys_in, const doubl
         a.grow_bound = ~0ULL;
         a.key_bound = kKeysUnknown;
         a.keys_fixed = spans[k].fixed ? 1u : 0u;
+        a.odd = odd_pass(hd, a.g0, a.g1) ? 1u : 0u;
         if (launch_hash_pass(a, kFixedBuckets, true, sms, st) < 0) return SQC_ERR_CUDA;
     }
     if (launch_readout(t, ctl, kFixedBuckets, 0ULL, true, reinterpret_cast<unsigned long long*>(keys_out), re_out,

@@ -121,6 +121,13 @@ bool GroupMap::extend(unsigned long long kmask, uint32_t nq) {
     return true;
 }
 
+// Whether a coefficient is not finite (an angle was infinite or NaN).
+static bool odd_gate(const GateDesc& g) {
+    bool odd = !std::isfinite(g.c) || !std::isfinite(g.s);
+    for (double m : g.m) odd = odd || !std::isfinite(m);
+    return odd;
+}
+
 // The op code of a gate kind (pairing kinds: on slots 0-1 and 2-3).
 static uint32_t unit_op(uint32_t kind) {
     switch (kind) {
@@ -219,6 +226,7 @@ void encode_unit_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[3], co
         uint32_t op = unit_op(g.kind) + (pairs ? shfl : 0u);
         const bool all = pairs && !lmask && !smask;   // no controls inside the unit
         if (pairs && (all || pair3)) op += all ? (pair3 ? UO_ALL3 : UO_ALL) : UO_PAIR3;
+        if (odd_gate(g)) op = UO_ODD + (pair3 ? 2u : pairs ? shfl : 0u);
         const uint32_t tb = lane_bit != kNoQubit ? lane_bit : slot_bit != kNoQubit ? kMaxMapBits : outer;
         g.loc = lmask | (lval << kLocLaneVal) | (slots << kLocSlots) | (bits << kLocSlotBit) | (tb << kLocBit) |
                 (shfl ? kLocLane : 0u) | (flip ? kLocFlip : 0u) |
@@ -246,7 +254,8 @@ void encode_column_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[2], 
             if (((s ^ sval) & smask) == 0) slots |= 1u << s;
             if ((slot_bit != kNoQubit && ((s >> slot_bit) & 1u)) != flip) bits |= 1u << s;
         }
-        const uint32_t op = unit_op(g.kind) + (pairs && slot_bit == 1 ? UO_PAIR3 : 0u);
+        const bool pair3 = pairs && slot_bit == 1;
+        const uint32_t op = odd_gate(g) ? UO_ODD + (pair3 ? 2u : 0u) : unit_op(g.kind) + (pair3 ? UO_PAIR3 : 0u);
         g.loc = (slots << kLocSlots) | (bits << kLocSlotBit) | (slot_bit != kNoQubit ? kLocLane : 0u) |
                 ((g.target & 31u) << kLocBit) | (g.target >= 32u ? kLocHigh : 0u) | (flip ? kLocFlip : 0u) | (op << kLocOp);
     }

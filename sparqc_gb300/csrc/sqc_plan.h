@@ -113,6 +113,13 @@ void encode_unit_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[3], co
 // 64 for an absent one.
 void encode_column_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[2], uint32_t dim[3]);
 
+// Whether an encoded pass has a gate with a coefficient that is not finite.
+inline bool odd_pass(const GateDesc* d, size_t g0, size_t g1) {
+    for (size_t k = g0; k < g1; ++k)
+        if (d[k].loc >> kLocOp >= UO_ODD) return true;
+    return false;
+}
+
 // An order of gates g[0..n) that passes fuse better, as a permutation: perm[i] is the index of
 // the i-th gate to apply. Passes are built greedily from the first gate not yet placed: a gate
 // within the next `window` joins the pass when it commutes with every gate it moves ahead of

@@ -331,8 +331,11 @@ int Server::step(uint32_t* finished) {
     if (!any && solo_.empty()) return cuda(cudaStreamSynchronize(stream_), "sync");
     const uint32_t n = n_used_;
     if ((rc = cuda(cudaEventRecord(ev0_, stream_), "event"))) return rc;
-    for (uint32_t s = 0; s < n; ++s)   // the requests this launch runs, for its retirement
+    bool odd = false;
+    for (uint32_t s = 0; s < n; ++s) {   // the requests this launch runs, for its retirement
         in_rid_[s] = slot_req_[s] && reqs_.at(slot_req_[s]).state == SQC_REQ_RUNNING ? slot_req_[s] : 0;
+        odd = odd || (in_rid_[s] && reqs_.at(in_rid_[s]).plan.odd);
+    }
     if (any) {
         // the small circuits: one time slice of the persistent kernel over the resident slots
         std::memcpy(stg_circ_, h_circ_, n * sizeof(BCirc));
@@ -345,7 +348,7 @@ int Server::step(uint32_t* finished) {
             return rc;
         const int grid = sms_ * batch_residency(dbl_, 0);
         const unsigned long long slice_ns = (unsigned long long)(slice_ms_ * 1e6);
-        if ((rc = cuda(launch_batch(args(n), dbl_, grid, 0, slice_ns, stream_), "batch launch")) ||
+        if ((rc = cuda(launch_batch(args(n), dbl_, grid, 0, odd, slice_ns, stream_), "batch launch")) ||
             (rc = cuda(cudaMemcpyAsync(h_sched_, d_sched_, n * sizeof(BSched), cudaMemcpyDeviceToHost, stream_), "D2H")) ||
             (rc = cuda(cudaMemcpyAsync(h_ctl_, d_ctl_, n * sizeof(Ctl), cudaMemcpyDeviceToHost, stream_), "D2H")) ||
             (rc = cuda(cudaMemcpyAsync(h_bctl_, d_bctl_, sizeof(BatchCtl), cudaMemcpyDeviceToHost, stream_), "D2H")))

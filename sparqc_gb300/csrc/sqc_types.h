@@ -106,7 +106,8 @@ enum UOp : uint32_t {
     UO_RY_SHFL, UO_U_PAIR, UO_U_SHFL, UO_Z, UO_S, UO_SDG, UO_YPH, UO_RZ, UO_PHASE,
     UO_ALL = 18,    // + 0..11: the forms above
     UO_ALL3 = 30,   // + 0, 2, .., 10: UO_X_PAIR .. UO_U_PAIR on dimension 2
-    UO_PAIR3 = 31   // + 0, 2, .., 10: the same with controls inside the unit
+    UO_PAIR3 = 31,  // + 0, 2, .., 10: the same with controls inside the unit
+    UO_ODD = 61     // a gate with a coefficient that is not finite; + 1: pairs lanes, + 2: on dimension 2
 };
 
 // GateDesc.flip bits: the frame's flip, and what encode_pass says of a gate by kind and qubits.
@@ -160,6 +161,7 @@ struct PassArgs {
     // mapped bits in use after the pass (mapped tables), dimensions of a unit (2 or 3) and the bucket
     // bit (mapped) or qubit (hashed; 64: none) of each dimension
     uint32_t dn, dims, dim[3];
+    uint32_t odd;           // 1: a gate is UO_ODD (never in a run)
     UnitHead heads[kMaxRun];   // mapped tables: those of the pass's gates (read from the parameter bank)
 };
 

@@ -112,14 +112,17 @@ __device__ __forceinline__ uint32_t lane_word(uint32_t loc, uint32_t lane) {
 
 __device__ __forceinline__ int16_t short_word(uint32_t w) { return (int16_t)((w & 0xFFu) | ((w >> 16) & 0x8000u)); }
 
-// A pass's heads read from its gates in shared memory.
-template <class T> struct SharedHeads {
+// A pass's heads read from its gates in shared memory. ODD: some may be UO_ODD gates.
+template <class T, bool ODD = false> struct SharedHeads {
     const UGate<T>* g;
     __device__ __forceinline__ UnitHead operator[](uint32_t i) const {
         const uint4 h = *reinterpret_cast<const uint4*>(g + i);   // om, ov, loc, weight
         return UnitHead{h.x, h.y, h.z, h.w};
     }
 };
+
+template <class Heads> constexpr bool kOddHeads = false;
+template <class T> constexpr bool kOddHeads<SharedHeads<T, true>> = true;
 
 // The gates of a pass in shared memory: the gates, and their lane words.
 template <class T> struct UGates {
@@ -495,6 +498,62 @@ __device__ __forceinline__ void diag(const UGate<T>& g, unsigned e, unsigned act
     }
 }
 
+// A gate with a coefficient that is not finite (an infinite or NaN angle). The forms above run absent
+// slots along, as products of 0 are 0; here they would become NaN, and pairs without keys would get some. So
+// presence is looked at: every pair with a key follows the formula, all others stay absent and 0.
+// Only U can have finite rows beside others; every other result of such a gate is NaN. Passes with such
+// a gate go to kernels of their own: as one more case in the ordinary ones, it cost FP32 passes 8 to 20% in
+// spilled registers, though it never ran.
+template <class T> __device__ __forceinline__ T u_coef(const GateDesc* gd, int i);
+template <> __device__ __forceinline__ double u_coef<double>(const GateDesc* gd, int i) { return __ldg(&gd->m[i]); }
+template <> __device__ __forceinline__ float u_coef<float>(const GateDesc* gd, int i) { return __ldg(&gd->mf[i]); }
+template <class T, int S>
+__device__ __forceinline__ Slots<T, S> odd_gate(const GateDesc* gd, uint32_t loc, uint32_t w, unsigned ones, Slots<T, S> x, PruneBits pb) {
+    using A = Arith<T>;
+    const uint32_t kind = __ldg(&gd->kind), form = (loc >> kLocOp) - UO_ODD;
+    const T nan = (T)__int_as_float(0x7FC00000);
+    const unsigned act = w & ((1u << S) - 1u);
+    if (!branch_kind(kind)) {   // Rz, Phase
+        const unsigned on = (kind == KRZ ? act : ones) & x.pm;
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+            if ((on >> s) & 1u) x.v[s] = Cx<T>{nan, nan};
+        return x;
+    }
+    Cx<T> b[S];   // the partners
+    unsigned pp;
+    if (form == 1) {
+        const int off = 1 << ((loc >> kLocBit) & 31u);
+        pp = __shfl_xor_sync(kFull, x.pm, off);
+#pragma unroll
+        for (int s = 0; s < S; ++s) b[s] = shfl_cx(x.v[s], off);
+    } else {
+        const bool far = S == 4 && form == 2;
+        pp = far ? (x.pm << 2) | (x.pm >> 2) : ((x.pm & 5u) << 1) | ((x.pm >> 1) & 5u);
+#pragma unroll
+        for (int s = 0; s < S; ++s) b[s] = pick(far, x.v[s ^ (S == 4 ? 2 : 1)], x.v[s ^ 1]);
+    }
+    const unsigned any = (x.pm | pp) & act;
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        if (!((any >> s) & 1u)) continue;
+        Cx<T> o{nan, nan};
+        if (kind == KU) {
+            const bool bit = ((w >> 31) != 0) != (form != 1 && (s & (form == 2 ? 2 : 1)));
+            const int own = bit ? 6 : 0, mix = bit ? 4 : 2;
+            const T sr = u_coef<T>(gd, own), si = u_coef<T>(gd, own + 1), mr = u_coef<T>(gd, mix), mi = u_coef<T>(gd, mix + 1);
+            const Cx<T> a = x.v[s], c = b[s];
+            o.r = A::fma(neg(mi), c.i, A::fma(mr, c.r, A::fma(neg(si), a.i, A::mul(sr, a.r))));
+            o.i = A::fma(mi, c.r, A::fma(mr, c.i, A::fma(si, a.r, A::mul(sr, a.i))));
+        }
+        const bool keep = !negligible(o, pb);
+        x.v[s] = pick(keep, o, czero<T>());
+        x.pm = (x.pm & ~(1u << s)) | ((unsigned)keep << s);
+    }
+    x.n = __popc(x.pm);
+    return x;
+}
+
 // The gates of a pass on the unit a warp holds; uid is the unit's base index. Absent slots hold
 // +-0, and the prune threshold is positive: no gate makes a slot present out of absent ones.
 // `heads` says where each gate acts (UnitHead): the gates' own in shared memory, or the kernel's
@@ -585,7 +644,9 @@ __device__ __forceinline__ void run_unit(const Heads& heads, const UGates<T>& sg
         case UO_YPH: diag<T, KYPH, S>(g, ones(), act, x); break;
         case UO_RZ: diag<T, KRZ, S>(g, ones(), act, x); break;
         case UO_PHASE: diag<T, KPHASE, S>(g, ones(), act, x); break;
-        default: __builtin_unreachable();
+        default:
+            if constexpr (kOddHeads<Heads>) x = odd_gate<T, S>(gd, loc, w, ones(), x, pb);
+            else __builtin_unreachable();
         }
     }
 }
@@ -862,8 +923,9 @@ struct HashWork {
     unsigned short cols[512];
 };
 
-// The gates of a pass on one column a lane; kb is the column's key with the pass's qubits 0.
-template <class T>
+// The gates of a pass on one column a lane; kb is the column's key with the pass's qubits 0. ODD: some may be
+// UO_ODD gates.
+template <class T, bool ODD>
 __device__ __forceinline__ void run_columns(const HGates<T>& sg, const GateDesc* __restrict__ gates, uint32_t ng, unsigned long long kb,
                                             bool on, Slots<T, kColumn>& x, bool& touched, const PruneBits& pb,
                                             unsigned long long& upd) {
@@ -902,7 +964,9 @@ __device__ __forceinline__ void run_columns(const HGates<T>& sg, const GateDesc*
         case UO_YPH: diag<T, KYPH, kColumn>(g, ones(), act, x); break;
         case UO_RZ: diag<T, KRZ, kColumn>(g, ones(), act, x); break;
         case UO_PHASE: diag<T, KPHASE, kColumn>(g, ones(), act, x); break;
-        default: __builtin_unreachable();
+        default:
+            if constexpr (ODD) x = odd_gate<T, kColumn>(gd, loc, w, ones(), x, pb);
+            else __builtin_unreachable();
         }
     }
 }
@@ -910,7 +974,7 @@ __device__ __forceinline__ void run_columns(const HGates<T>& sg, const GateDesc*
 // The units of list entries [e0, e1) (at most 32). An entry owns its unit when it is the live member of
 // smallest index (the reference's pair rule, emulator/device/device_table_FC.cuh:62-110, lifted to
 // groups; members a pass creates are made by the unit's owner, after its own check).
-template <class T>
+template <class T, bool ODD>
 __device__ __forceinline__ void walk_hashed(const TableDev& t, Ctl* ctl, unsigned ep, const HashDims& dm, unsigned long long e0,
                                             unsigned long long e1, HashWork& wk, const HGates<T>& sg, const GateDesc* gates,
                                             uint32_t ng, int lane, const PruneBits& pb, unsigned long long& cnt_nnz,
@@ -1004,7 +1068,7 @@ __device__ __forceinline__ void walk_hashed(const TableDev& t, Ctl* ctl, unsigne
         bool touched = false;
         const unsigned pm0 = x.pm;
         x.n = __popc(pm0);
-        run_columns<T>(sg, gates, ng, (G0 << kSlotBits) | j0, on, x, touched, pb, upd);
+        run_columns<T, ODD>(sg, gates, ng, (G0 << kSlotBits) | j0, on, x, touched, pb, upd);
         const unsigned pm = x.pm;
         cnt_nnz += __popc(pm);
         bool absent = false;
@@ -1080,14 +1144,14 @@ __device__ __forceinline__ void walk_hashed(const TableDev& t, Ctl* ctl, unsigne
 }
 
 // A hashed pass's share of a warp.
-template <class T>
+template <class T, bool ODD = false>
 __device__ __forceinline__ void walk_hashed_all(const TableDev& t, Ctl* ctl, unsigned ep, const HashDims& dm, unsigned long long n,
                                                 unsigned w, unsigned nw, HashWork& wk, const HGates<T>& sg,
                                                 const GateDesc* gates, uint32_t ng, int lane, const PruneBits& pb,
                                                 unsigned long long& cnt_nnz, unsigned long long& cnt_empty, unsigned long long& upd) {
     const unsigned long long piece = list_piece(n, nw);
     for (unsigned long long e0 = w * piece; e0 < n; e0 += nw * piece)
-        walk_hashed<T>(t, ctl, ep, dm, e0, umin64(e0 + piece, n), wk, sg, gates, ng, lane, pb, cnt_nnz, cnt_empty, upd);
+        walk_hashed<T, ODD>(t, ctl, ep, dm, e0, umin64(e0 + piece, n), wk, sg, gates, ng, lane, pb, cnt_nnz, cnt_empty, upd);
 }
 
 }  // namespace

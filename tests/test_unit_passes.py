@@ -392,3 +392,35 @@ def test_infinite_and_nan_amplitudes(kind, hashed, precision):
         o.apply(gs)
         _same(st.state(sorted=True), o.state(sorted=True))
         st.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("where", ["mapped", "hashed", "batch"])
+@pytest.mark.parametrize("gate", [(G.RX, np.nan), (G.RY, np.inf), (G.RZ, -np.inf), (G.PHASE, np.nan), (G.U, np.nan, 0.3, 0.2),
+                                  (G.U, 0.7, np.nan, 0.2), (G.U, 0.7, 0.3, np.inf)])
+def test_angles_that_are_not_finite(gate, where, precision):
+    """A NaN or infinite angle turns amplitudes to NaN; it makes no key out of pairs that hold none, and
+    absent keys stay 0 for the gates that follow."""
+    from sparqc_gb300.engine import Batch, State
+    nq, prefix = (60, 5) if where == "hashed" else (9, 5)
+    spread = [8 * q + 3 for q in range(prefix)] if where == "hashed" else [0, 2, 4, 5, 8]
+    first = [(G.H, q) for q in spread] + [(G.X, (q + 5) % nq, (q,)) for q in spread]
+    for qubits in ((6,), (5, 6), (6, 5, 4), (1,), (3, 7)):
+        odd = [(gate[0], q, ((q + 2) % 9,) if i else ()) + gate[1:] for i, q in enumerate(qubits)]
+        after = [(G.H, (qubits[0] + 1) % 9), (G.RY, (qubits[0] + 2) % 9, (), 0.4), (G.X, qubits[0], ((qubits[0] + 4) % 9,))]
+        gs = G.gate_array(first + odd + after)
+        o = SparseOracle(precision)
+        o.apply(gs)
+        if where == "batch":
+            st = Batch(precision=precision)
+            st.prepare([(nq, gs)])
+            st.run()
+            st.sync()
+            got = st.state(0)
+        else:
+            st = State(nq, precision=precision)
+            st.apply(gs)
+            got = st.state(sorted=True)
+        _same(got, o.state(sorted=True))
+        st.close()
