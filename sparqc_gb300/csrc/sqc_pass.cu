@@ -7,6 +7,7 @@
 // (such groups are beyond the entries the pass walks). Pruning follows the reference
 // (emulator/device/device_data.cuh:108-156): branching gates drop negligible outputs, swap
 // and diagonal gates keep every key.
+#include "sqc_meet.h"
 #include "sqc_pass.cuh"
 
 namespace sqc {
@@ -45,8 +46,6 @@ __device__ __forceinline__ void stage_run(UGates<T>& sg, const RunArgs& a, uint3
     for (uint32_t i = threadIdx.x; i < ng * 32u; i += blockDim.x)
         sg.lw[i >> 5][i & 31u] = short_word(lane_word(a.words[o + 1 + (i >> 5)].loc, i & 31u));
 }
-
-constexpr unsigned kMaxPolls = 1u << 22;   // a few seconds: far longer than any pass of a run
 
 template <class T, bool HASHED> struct RunGates { using G = UGates<T>; };
 template <class T> struct RunGates<T, true> { using G = HGates<T>; };
@@ -142,18 +141,17 @@ __global__ void __launch_bounds__(kThreads, HASHED ? kHashBlocks<T> : UnitOcc<T,
             }
             stage_run<T>(sg[(p + 1) & 1], a, o);
             if (threadIdx.x == 0) {
-                unsigned left = kMaxPolls;
+                auto status = [&] { return *(volatile unsigned int*)&ctl->status; };
+                Meet met;
                 if (list) {
                     unsigned long long v;
-                    while ((uint32_t)((v = *(volatile unsigned long long*)&ctl->bar_len) >> 32) != tag && --left) {}
+                    met = wait_meeting<HASHED>([&] { return (uint32_t)((v = *(volatile unsigned long long*)&ctl->bar_len) >> 32) == tag; }, status);
                     n_sh = v & 0xFFFFFFFFULL;
                 } else {
-                    while (*(volatile unsigned int*)&ctl->bar < gridDim.x * (p + 1) && --left) {}
+                    met = wait_meeting<HASHED>([&] { return *(volatile unsigned int*)&ctl->bar >= gridDim.x * (p + 1); }, status);
                 }
-                if (!left) {
-                    atomicCAS(&ctl->status, 0u, (unsigned)ST_TIMEOUT);
-                    stop = 1;
-                }
+                if (met == MEET_TIMEOUT) atomicCAS(&ctl->status, 0u, (unsigned)ST_TIMEOUT);
+                stop = met != MEET_OK;
                 __threadfence();
             }
         }

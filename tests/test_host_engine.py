@@ -126,3 +126,38 @@ def test_failed_copy_in_a_flush_loses_no_gate(engine_objects, tmp_path):
     CHECK(e.flush() == SQC_ERR_CUDA);
     CHECK(holds(e, expected(g)));
     """)
+
+
+def test_meeting_wait_ends_when_the_state_has_failed(tmp_path):
+    """The wait of a run's blocks at a meeting (sqc_meet.h): over when the others are there, soon over when the
+    state has failed (a block that saw that at its start never comes), and bounded."""
+    src = tmp_path / "meet.cpp"
+    src.write_text(r"""
+#include <cstdio>
+#include <initializer_list>
+#include "sqc_meet.h"
+using namespace sqc;
+static int fails = 0;
+#define CHECK(c) do { if (!(c)) { std::printf("FAIL line %d: %s\n", __LINE__, #c); ++fails; } } while (0)
+template <bool LOOK = true>
+static Meet wait(unsigned long met_at, unsigned long failed_at, unsigned long* polls) {
+    unsigned long n = 0;
+    const Meet m = wait_meeting<LOOK>([&] { return ++n >= met_at; }, [&] { return n >= failed_at ? ST_TABLE_FULL : ST_OK; });
+    *polls = n;
+    return m;
+}
+int main() {
+    const unsigned long never = ~0UL;
+    unsigned long n;
+    for (unsigned long at : {1UL, 2UL, 63UL, 64UL, 65UL, 1000UL, (unsigned long)kMaxPolls}) CHECK(wait(at, never, &n) == MEET_OK && n == at);
+    CHECK(wait(1, 0, &n) == MEET_OK);
+    for (unsigned long at : {0UL, 1UL, 64UL, 65UL, 100000UL}) CHECK(wait(never, at, &n) == MEET_FAILED && n <= at + kStatusPolls);
+    CHECK(wait(never, never, &n) == MEET_TIMEOUT && n == kMaxPolls);
+    CHECK(wait<false>(1000, 0, &n) == MEET_OK && n == 1000);
+    CHECK(wait<false>(never, never, &n) == MEET_TIMEOUT && n == kMaxPolls);
+    std::printf("fails=%d\n", fails);
+}
+""")
+    exe = tmp_path / "meet"
+    subprocess.run(["g++", *FLAGS, str(src), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)], capture_output=True, text=True).stdout == "fails=0\n"
