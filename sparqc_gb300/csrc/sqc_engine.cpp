@@ -545,6 +545,8 @@ int Engine::flush(bool hold_last) {
                 const unsigned long long h = std::min({group_bound(after[r.g1 - 1], nq_), items << r.nx, items + r.keys});
                 if (h > roomy_groups() || h > kRunMaxList) break;
                 items = h;
+            } else if (items > kRunMaxList) {
+                break;
             }
             words += w;
             ++e;

@@ -161,3 +161,24 @@ int main() {
     exe = tmp_path / "meet"
     subprocess.run(["g++", *FLAGS, str(src), "-o", str(exe)], check=True)
     assert subprocess.run([str(exe)], capture_output=True, text=True).stdout == "fails=0\n"
+
+
+@pytest.mark.parametrize("groups,runs", [(1 << 17, 1), ((1 << 17) + 1, 0)])
+def test_large_hashed_states_make_no_runs(engine_objects, tmp_path, groups, runs):
+    """Passes go out in one launch while the state has at most 2^17 live buckets, whatever gates they hold."""
+    run(engine_objects, tmp_path, """
+    Engine e;
+    sqc_options o;
+    sqc_default_options(&o);
+    o.max_fused_gates = 2;
+    make(e, 60, &o);
+    const size_t n = %d;
+    std::vector<uint64_t> k(n);
+    std::vector<double> r(n, 0.001), i(n, 0.0);
+    for (size_t j = 0; j < n; ++j) k[j] = (j * 0x9E3779B97F4A7C15ULL) >> 4 & ~15ULL;
+    CHECK(e.set_state(k.data(), r.data(), i.data(), n) == SQC_OK);
+    std::vector<sqc_gate> g;
+    for (int j = 0; j < 5; ++j) g.push_back(gate(KT, 59 - j, 1ULL << (10 + j)));
+    CHECK(e.apply(g.data(), g.size()) == SQC_OK && e.sync() == SQC_OK);
+    CHECK(dev.passes == 3 && dev.runs == %d);
+    """ % (groups, runs))
