@@ -589,7 +589,15 @@ int Engine::flush(bool hold_last) {
         a.grow_bound = group_bound(after[sp.g1 - 1], nq_);
         a.key_bound = sp.keys;
         if (!mapped_ && sp.nx && grown(sp.nx, a.grow_bound, sp.keys) > roomy_groups()) {
-            if ((rc = make_room(sp.nx, a.grow_bound, sp.keys))) return put_back(rc);
+            // (it reads the events of the passes timed so far, and recycles them: the next pass begins at a
+            // new one, after the wait and the rebuild)
+            const bool mine = timed_.empty() || timed_.back().after != ev_prev;
+            rc = make_room(sp.nx, a.grow_bound, sp.keys);
+            if (time_passes_) {
+                if (mine) ev_free_.push_back(ev_prev);
+                if (!rc) rc = record_event(&ev_prev);
+            }
+            if (rc) return put_back(rc);
             a.t = dev();
             a.max_groups = max_groups();
         }

@@ -182,3 +182,26 @@ def test_large_hashed_states_make_no_runs(engine_objects, tmp_path, groups, runs
     CHECK(e.apply(g.data(), g.size()) == SQC_OK && e.sync() == SQC_OK);
     CHECK(dev.passes == 3 && dev.runs == %d);
     """ % (groups, runs))
+
+
+def test_timed_passes_of_a_table_that_is_enlarged(engine_objects, tmp_path):
+    """Enlarging a table between two passes reads the events of the passes before it: every later pass
+    still spans from an event of its own to the next."""
+    run(engine_objects, tmp_path, THIN + """
+    Engine e;
+    sqc_options o;
+    sqc_default_options(&o);
+    o.initial_buckets = 64;
+    o.time_passes = 1;
+    make(e, 60, &o);
+    for (int k = 0; k < 3; ++k) {
+        CHECK(e.set_zero() == SQC_OK);
+        CHECK(e.apply(g.data(), g.size()) == SQC_OK);
+        CHECK(holds(e, expected(g)));
+    }
+    sqc_stats st;
+    e.stats(&st);
+    // one tick of the fake clock per pass, and none for what lies between two
+    CHECK(st.pass_ns_pair + st.pass_ns_stream == (unsigned long long)dev.passes * 1000000ULL);
+    CHECK(st.buckets > 64);
+    """)
