@@ -559,8 +559,6 @@ int Engine::flush(bool hold_last) {
             run.amp_bytes = a.amp_bytes;
             run.max_groups = a.max_groups;
             run.np = (uint32_t)(e - s);
-            run.tag = run_tag_;
-            run_tag_ += run.np;
             UnitHead* w = run.words;
             for (size_t i = s; i < e; ++i) {
                 const Span& r = spans[i];
@@ -818,6 +816,7 @@ int Engine::rebuild(unsigned long long nb_new, bool mapped) {
     c.status = 0;
     c.done = 0;
     c.bar = 0;
+    c.bar_len = 0;
     c.seq = 0;
     c.list_n = 0;
     c.list_tail = 0;

@@ -191,7 +191,6 @@ private:
     size_t cum_cap_ = 0, cum_tmp_bytes_ = 0;
 
     double hash_load_ = 0.35;       // load up to which a hashed table stays as it is
-    uint32_t run_tag_ = 1;          // RunArgs.tag of the next run
     uint64_t gates_applied_ = 0, passes_run_ = 0, launches_ = 0, replays_ = 0, rebuilds_ = 0;
     uint64_t passes_pair_ = 0;
 

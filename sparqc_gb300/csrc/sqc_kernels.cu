@@ -54,6 +54,7 @@ __global__ void set_zero_kernel(TableDev t, Ctl* ctl, int dbl) {
         ctl->status = 0;
         ctl->done = 0;
         ctl->bar = 0;
+        ctl->bar_len = 0;
         ctl->acc_nnz = ctl->acc_empty = ctl->acc_upd = 0;
         ctl->seq = 0;
         ctl->amp_updates = 0;
@@ -88,6 +89,7 @@ __global__ void set_state_begin_kernel(Ctl* ctl) {
     ctl->status = 0;
     ctl->done = 0;
     ctl->bar = 0;
+    ctl->bar_len = 0;
     ctl->acc_nnz = ctl->acc_empty = ctl->acc_upd = 0;
     ctl->seq = 0;
     ctl->amp_updates = 0;

@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kThreads, HASHED ? kHashBlocks<T> : UnitOcc<T,
         // every block's pass is done before any block's next one; whether the next pass walks the list
         // (and needs its exact length; a hashed one always does) follows from what every block knows
         const bool list = HASHED || walk_list(n, g >> 16);
-        const uint32_t tag = a.tag + p;
+        const uint32_t tag = p + 1;
         __syncthreads();
         if (gridDim.x == 1) {
             if (threadIdx.x == 0 && list) n_sh = *(volatile unsigned long long*)&ctl->list_tail;
@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(kThreads, HASHED ? kHashBlocks<T> : UnitOcc<T,
                 if (refused) ctl->status = ST_GROW;
             }
             ctl->bar = 0;
+            ctl->bar_len = 0;   // (a recorded run may come again)
             __threadfence();
         }
     }

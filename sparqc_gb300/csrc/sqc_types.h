@@ -69,6 +69,7 @@ struct Ctl {
     double acc[6];                  // reductions: norm, compare
     unsigned long long acc_max;     // bit pattern of a non-negative double (max |a-b|)
     unsigned long long bar_len;     // a run's live buckets before a pass that walks the list, tagged with the pass
+                                    // (0 outside a run)
 };
 
 // Gate descriptor with host-resolved coefficients (std::cos/std::sin on the host, so the
@@ -179,7 +180,6 @@ struct RunArgs {
     const GateDesc* gates;
     PruneBits prune;
     uint32_t np, amp_bytes;
-    uint32_t tag;              // of the run's first pass: passes of an engine have different ones
     unsigned long long max_groups;   // hashed tables: as in PassArgs
     UnitHead words[kRunWords];
 };

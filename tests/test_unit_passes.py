@@ -424,3 +424,36 @@ def test_angles_that_are_not_finite(gate, where, precision):
             got = st.state(sorted=True)
         _same(got, o.state(sorted=True))
         st.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("keys", [40, 300])
+def test_recorded_runs_replay(keys, precision):
+    """Passes recorded on the caller's stream into a CUDA graph (two passes that walk the list, in one
+    launch) do the same again at every replay: their meeting does not take the last replay's for its own."""
+    import torch
+    from sparqc_gb300.engine import State
+    rng = np.random.default_rng(keys)
+    key = np.unique(rng.integers(0, 1 << 16, keys, dtype=np.uint64))
+    amp = rng.standard_normal((2, key.size)) / np.sqrt(key.size)
+    gs = G.gate_array([(G.X, 4, (9,)), (G.RZ, 10, (2,), 0.4), (G.X, 5, (4, 11)), (G.RY, 6, (7, 12, 15), 0.3), (G.X, 8, (6,))]
+                      if precision == 64 else
+                      [(G.X, 4, (9,)), (G.X, 5, (4, 11)), (G.X, 10, (13,)), (G.RY, 6, (7, 12, 15), 0.3), (G.X, 8, (6,))])
+    s = torch.cuda.Stream()
+    st, o = State(16, precision=precision, initial_buckets=1 << 13, stream=s.cuda_stream), SparseOracle(precision)
+    st.set_state(key, amp[0], amp[1])
+    o.set_state(key, amp[0], amp[1])
+    st.apply(gs)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s, capture_error_mode="thread_local"):
+        st.flush()
+    with torch.cuda.stream(s):
+        for _ in range(50):
+            graph.replay()
+    for _ in range(50):
+        o.apply(gs)
+    s.synchronize()
+    assert st.stats()["passes"] == 2
+    assert_identical(st.state(sorted=True), o.state(sorted=True))
+    st.close()
