@@ -586,7 +586,7 @@ int Engine::flush(bool hold_last) {
         a.odd = odd_pass(hd, sp.g0, sp.g1) ? 1u : 0u;
         a.grow_bound = group_bound(after[sp.g1 - 1], nq_);
         a.key_bound = sp.keys;
-        if (!mapped_ && sp.nx && grown(sp.nx, a.grow_bound, sp.keys) > roomy_groups()) {
+        if (!mapped_ && sp.nx && grown(sp.nx, a.grow_bound, sp.keys) > roomy_groups() && !recording()) {
             // (it reads the events of the passes timed so far, and recycles them: the next pass begins at a
             // new one, after the wait and the rebuild)
             const bool mine = timed_.empty() || timed_.back().after != ev_prev;
@@ -667,6 +667,13 @@ int Engine::make_room(uint32_t nx, unsigned long long bound, unsigned long long 
     if (grown(nx, bound, keys) > roomy_groups()) hash_load_ = kMaxLoad;
     passes_.clear();   // all verified: later ones count from here
     return SQC_OK;
+}
+
+// Whether the stream's work is being recorded into a graph: nothing can be waited for then, and a pass
+// without room refuses when it is replayed.
+bool Engine::recording() const {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream_, &s) == cudaSuccess && s == cudaStreamCaptureStatusActive;
 }
 
 int Engine::read_sums() {

@@ -110,6 +110,7 @@ private:
     unsigned long long grown(uint32_t nx, unsigned long long bound, unsigned long long keys) const;
     unsigned long long hashed_size(unsigned long long groups, uint32_t nx, unsigned long long keys);
     int make_room(uint32_t nx, unsigned long long bound, unsigned long long keys);
+    bool recording() const;
     int repair(size_t failed_pass);
     int ensure_desc(size_t n);
     int ensure_readout(size_t n);

@@ -205,3 +205,22 @@ def test_timed_passes_of_a_table_that_is_enlarged(engine_objects, tmp_path):
     CHECK(st.pass_ns_pair + st.pass_ns_stream == (unsigned long long)dev.passes * 1000000ULL);
     CHECK(st.buckets > 64);
     """)
+
+
+def test_flush_waits_for_nothing_while_recording(engine_objects, tmp_path):
+    """A flush whose launches are recorded into a graph does not stop to enlarge the table: the passes are
+    recorded, one without room refuses when it runs, and the next sync repairs that."""
+    run(engine_objects, tmp_path, THIN + """
+    Engine e;
+    sqc_options o;
+    sqc_default_options(&o);
+    o.initial_buckets = 64;
+    make(e, 60, &o);
+    CHECK(e.apply(g.data(), g.size()) == SQC_OK);
+    dev.capturing = true;
+    const long before = dev.syncs;
+    CHECK(e.flush() == SQC_OK);
+    CHECK(dev.syncs == before);
+    dev.capturing = false;
+    CHECK(holds(e, expected(g)));
+    """)
