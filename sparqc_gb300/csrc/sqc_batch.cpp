@@ -7,6 +7,7 @@
 #include <cstring>
 #include <numeric>
 
+#include "sqc_devmem.h"
 #include "sqc_kernels.h"
 
 namespace sqc {
@@ -164,7 +165,7 @@ int Batch::init(const sqc_batch_options* opt) {
         own_stream_ = true;
     }
     if ((rc = cuda(cudaEventCreate(&ev0_), "event")) || (rc = cuda(cudaEventCreate(&ev1_), "event"))) return rc;
-    if ((rc = cuda(cudaMalloc(&d_bctl_, sizeof(BatchCtl)), "cudaMalloc(bctl)"))) return rc;
+    if ((rc = cuda(device_alloc(&d_bctl_, sizeof(BatchCtl)), "cudaMalloc(bctl)"))) return rc;
     if ((rc = cuda(cudaMemset(d_bctl_, 0, sizeof(BatchCtl)), "cudaMemset"))) return rc;
     if ((rc = cuda(cudaMallocHost(&h_bctl_, sizeof(BatchCtl)), "cudaMallocHost"))) return rc;
     return SQC_OK;
@@ -222,14 +223,14 @@ int Batch::plan_and_upload() {
         if (d_desc_) cudaFree(d_desc_);
         d_desc_ = nullptr;
         desc_cap_ = 0;
-        if ((rc = cuda(cudaMalloc(&d_desc_, std::max<size_t>(nd, 1) * sizeof(GateDesc)), "cudaMalloc(desc)"))) return rc;
+        if ((rc = cuda(device_alloc(&d_desc_, std::max<size_t>(nd, 1) * sizeof(GateDesc)), "cudaMalloc(desc)"))) return rc;
         desc_cap_ = std::max<size_t>(nd, 1);
     }
     if (np > pass_cap_) {
         if (d_pass_) cudaFree(d_pass_);
         d_pass_ = nullptr;
         pass_cap_ = 0;
-        if ((rc = cuda(cudaMalloc(&d_pass_, std::max<size_t>(np, 1) * sizeof(BPass)), "cudaMalloc(passes)"))) return rc;
+        if ((rc = cuda(device_alloc(&d_pass_, std::max<size_t>(np, 1) * sizeof(BPass)), "cudaMalloc(passes)"))) return rc;
         pass_cap_ = std::max<size_t>(np, 1);
     }
     if (n > circ_cap_) {
@@ -239,12 +240,12 @@ int Batch::plan_and_upload() {
         d_circ_ = nullptr; d_ctl_ = nullptr; d_sched_ = nullptr; d_words_ = nullptr; d_cmd_ = nullptr; d_limit_ = nullptr;
         h_ctl_ = nullptr;
         circ_cap_ = 0;
-        if ((rc = cuda(cudaMalloc(&d_circ_, n * sizeof(BCirc)), "cudaMalloc")) ||
-            (rc = cuda(cudaMalloc(&d_ctl_, n * sizeof(Ctl)), "cudaMalloc")) ||
-            (rc = cuda(cudaMalloc(&d_sched_, n * sizeof(BSched)), "cudaMalloc")) ||
-            (rc = cuda(cudaMalloc(&d_words_, n * sizeof(unsigned long long)), "cudaMalloc")) ||
-            (rc = cuda(cudaMalloc(&d_cmd_, n * sizeof(unsigned)), "cudaMalloc")) ||
-            (rc = cuda(cudaMalloc(&d_limit_, n * sizeof(unsigned)), "cudaMalloc")) ||
+        if ((rc = cuda(device_alloc(&d_circ_, n * sizeof(BCirc)), "cudaMalloc")) ||
+            (rc = cuda(device_alloc(&d_ctl_, n * sizeof(Ctl)), "cudaMalloc")) ||
+            (rc = cuda(device_alloc(&d_sched_, n * sizeof(BSched)), "cudaMalloc")) ||
+            (rc = cuda(device_alloc(&d_words_, n * sizeof(unsigned long long)), "cudaMalloc")) ||
+            (rc = cuda(device_alloc(&d_cmd_, n * sizeof(unsigned)), "cudaMalloc")) ||
+            (rc = cuda(device_alloc(&d_limit_, n * sizeof(unsigned)), "cudaMalloc")) ||
             (rc = cuda(cudaMallocHost(&h_ctl_, n * sizeof(Ctl)), "cudaMallocHost")))
             return rc;
         circ_cap_ = n;
@@ -293,7 +294,7 @@ int Batch::layout() {
         if (pool_) cudaFree(pool_);
         pool_ = nullptr;
         pool_cap_ = 0;
-        if ((rc = cuda(cudaMalloc(&pool_, total), "cudaMalloc(pool)"))) return rc;
+        if ((rc = cuda(device_alloc(&pool_, total), "cudaMalloc(pool)"))) return rc;
         pool_cap_ = total;
     }
     pool_used_ = total;
@@ -431,9 +432,9 @@ int Batch::ensure_readout(size_t n) {
     for (void* p : {(void*)d_rk_, (void*)d_rr_, (void*)d_ri_}) if (p) cudaFree(p);
     d_rk_ = nullptr; d_rr_ = nullptr; d_ri_ = nullptr; rcap_ = 0;
     int rc;
-    if ((rc = cuda(cudaMalloc(&d_rk_, cap * 8), "cudaMalloc(readout)")) ||
-        (rc = cuda(cudaMalloc(&d_rr_, cap * 8), "cudaMalloc(readout)")) ||
-        (rc = cuda(cudaMalloc(&d_ri_, cap * 8), "cudaMalloc(readout)")))
+    if ((rc = cuda(device_alloc(&d_rk_, cap * 8), "cudaMalloc(readout)")) ||
+        (rc = cuda(device_alloc(&d_rr_, cap * 8), "cudaMalloc(readout)")) ||
+        (rc = cuda(device_alloc(&d_ri_, cap * 8), "cudaMalloc(readout)")))
         return rc;
     rcap_ = cap;
     return SQC_OK;

@@ -8,6 +8,7 @@
 #include <cstring>
 #include <numeric>
 
+#include "sqc_devmem.h"
 #include "sqc_exact.cuh"
 #include "sqc_kernels.h"
 
@@ -57,7 +58,7 @@ Engine::~Engine() {
     if (ev_copied_) cudaEventDestroy(ev_copied_);
     if (h_async_n_) cudaFreeHost(h_async_n_);
     free_table(&tab_);
-    free_table(&spare_);
+    spare_drop(this);
     if (ctl_) cudaFree(ctl_);
     if (ctl_host_) cudaFreeHost(ctl_host_);
     if (sums_) cudaFree(sums_);
@@ -140,6 +141,7 @@ int Engine::init(uint32_t nq, const sqc_hash_table_parameters* params, const sqc
     size_t free_b = 0, total_b = 0;
     if ((rc = cuda(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo"))) return rc;
     budget_ = (size_t)((1.0 - reserve) * (double)total_b);
+    spare_limit_ = total_b / 8;
 
     if (o.stream) {
         stream_ = (cudaStream_t)o.stream;
@@ -153,10 +155,10 @@ int Engine::init(uint32_t nq, const sqc_hash_table_parameters* params, const sqc
     if ((double)tf >= thr_) tf = std::nextafter(tf, 0.0f);
     std::memcpy(&prune_.f, &tf, sizeof(float));
 
-    if ((rc = cuda(cudaMalloc(&ctl_, sizeof(Ctl)), "cudaMalloc(ctl)"))) return rc;
+    if ((rc = cuda(device_alloc(&ctl_, sizeof(Ctl)), "cudaMalloc(ctl)"))) return rc;
     if ((rc = cuda(cudaMemset(ctl_, 0, sizeof(Ctl)), "cudaMemset(ctl)"))) return rc;
     if ((rc = cuda(cudaMallocHost(&ctl_host_, sizeof(Ctl)), "cudaMallocHost(ctl)"))) return rc;
-    if ((rc = cuda(cudaMalloc(&sums_, sizeof(ExactSums)), "cudaMalloc(sums)"))) return rc;
+    if ((rc = cuda(device_alloc(&sums_, sizeof(ExactSums)), "cudaMalloc(sums)"))) return rc;
     if ((rc = cuda(cudaMallocHost(&sums_host_, sizeof(ExactSums)), "cudaMallocHost(sums)"))) return rc;
     std::memset(ctl_host_, 0, sizeof(Ctl));
     if ((rc = ensure_desc(kDescInitial))) return rc;
@@ -170,33 +172,32 @@ int Engine::init(uint32_t nq, const sqc_hash_table_parameters* params, const sqc
 int Engine::alloc_table(unsigned long long nb, HostTable* out) {
     if ((double)nb * bucket_bytes() > (double)budget_)
         return fail(SQC_ERR_BUDGET, "table memory would exceed the HBM budget");
-    HostTable t;
-    t.nb = nb;
     int rc;
-    if (spare_.nb == nb) {
-        t = spare_;
-        spare_ = HostTable();
-        if ((rc = cuda(cudaMemsetAsync(t.hdr, 0, nb * sizeof(Header), stream_), "cudaMemset(hdr)"))) {
-            free_table(&t);
-            return rc;
-        }
-        *out = t;
-        return SQC_OK;
+    const size_t bytes = nb * bucket_bytes();
+    void* base = spare_take(this, bytes);   // (one of this size was rebuilt from: the last but one table)
+    if (!base) {
+        spare_drop(this);   // of another size: its memory may be needed
+        if ((rc = cuda(device_alloc(&base, bytes), "cudaMalloc(table)"))) return rc;
     }
-    free_table(&spare_);   // of another size: its memory may be needed
-    // one allocation: nb is at least 64, so every array starts on a 256-byte boundary
-    unsigned char* base = nullptr;
-    if ((rc = cuda(cudaMalloc(&base, nb * bucket_bytes()), "cudaMalloc(table)"))) return rc;
-    t.hdr = reinterpret_cast<Header*>(base);
-    t.keys = reinterpret_cast<unsigned long long*>(base += nb * sizeof(Header));
-    t.amps = base += nb * kSlots * sizeof(unsigned long long);
-    t.list = reinterpret_cast<unsigned*>(base += nb * kSlots * (dbl_ ? 16 : 8));
+    HostTable t = table_at(base, nb);
     if ((rc = cuda(cudaMemsetAsync(t.hdr, 0, nb * sizeof(Header), stream_), "cudaMemset(hdr)"))) {
         free_table(&t);
         return rc;
     }
     *out = t;
     return SQC_OK;
+}
+
+// The arrays of a table in its one allocation: nb is at least 64, so every one starts on a 256-byte boundary.
+HostTable Engine::table_at(void* at, unsigned long long nb) const {
+    unsigned char* base = static_cast<unsigned char*>(at);
+    HostTable t;
+    t.nb = nb;
+    t.hdr = reinterpret_cast<Header*>(base);
+    t.keys = reinterpret_cast<unsigned long long*>(base += nb * sizeof(Header));
+    t.amps = base += nb * kSlots * sizeof(unsigned long long);
+    t.list = reinterpret_cast<unsigned*>(base += nb * kSlots * (dbl_ ? 16 : 8));
+    return t;
 }
 
 void Engine::free_table(HostTable* t) {
@@ -226,7 +227,7 @@ int Engine::ensure_desc(size_t n) {
     h_desc_ = nullptr;
     desc_cap_ = 0;
     int rc;
-    if ((rc = cuda(cudaMalloc(&d_desc_, cap * sizeof(GateDesc)), "cudaMalloc(desc)"))) return rc;
+    if ((rc = cuda(device_alloc(&d_desc_, cap * sizeof(GateDesc)), "cudaMalloc(desc)"))) return rc;
     if ((rc = cuda(cudaMallocHost(&h_desc_, cap * sizeof(GateDesc)), "cudaMallocHost(desc)"))) return rc;
     desc_cap_ = cap;
     return SQC_OK;
@@ -242,7 +243,7 @@ int Engine::ensure_readout(size_t n) {
     if (d_rk_) cudaFree(d_rk_);
     d_rk_ = nullptr; d_rr_ = nullptr; d_ri_ = nullptr; rcap_ = 0;
     int rc;
-    if ((rc = cuda(cudaMalloc(&d_rk_, cap * 24), "cudaMalloc(readout)"))) return rc;
+    if ((rc = cuda(device_alloc(&d_rk_, cap * 24), "cudaMalloc(readout)"))) return rc;
     d_rr_ = reinterpret_cast<double*>(d_rk_ + cap);
     d_ri_ = d_rr_ + cap;
     rcap_ = cap;
@@ -851,8 +852,7 @@ int Engine::rebuild(unsigned long long nb_new, bool mapped) {
         (rc = cuda(cudaStreamSynchronize(stream_), "sync")))
         return rc;
     if (!mapped && !mapped_ && (double)(tab_.nb + nb_new) * bucket_bytes() <= (double)budget_) {
-        free_table(&spare_);
-        spare_ = tab_;
+        spare_put(this, tab_.hdr, tab_.nb * bucket_bytes(), spare_limit_);
         tab_ = HostTable();
     }
     free_table(&tab_);
@@ -961,13 +961,13 @@ int Engine::ensure_sort(size_t n) {
     sort_cap_ = 0;
     const size_t tmp = sort_scratch_bytes(cap);
     int rc;
-    if ((rc = cuda(cudaMalloc(&sort_.keys_out, cap * 8), "cudaMalloc(sort)")) ||
-        (rc = cuda(cudaMalloc(&sort_.re_out, cap * 8), "cudaMalloc(sort)")) ||
-        (rc = cuda(cudaMalloc(&sort_.im_out, cap * 8), "cudaMalloc(sort)")) ||
-        (rc = cuda(cudaMalloc(&sort_.idx_in, cap * 4), "cudaMalloc(sort)")) ||
-        (rc = cuda(cudaMalloc(&sort_.idx_out, cap * 4), "cudaMalloc(sort)")) ||
-        (rc = cuda(cudaMalloc(&sort_.cum, cap * 8), "cudaMalloc(sort)")) ||
-        (rc = cuda(cudaMalloc(&sort_.tmp, tmp), "cudaMalloc(sort)")))
+    if ((rc = cuda(device_alloc(&sort_.keys_out, cap * 8), "cudaMalloc(sort)")) ||
+        (rc = cuda(device_alloc(&sort_.re_out, cap * 8), "cudaMalloc(sort)")) ||
+        (rc = cuda(device_alloc(&sort_.im_out, cap * 8), "cudaMalloc(sort)")) ||
+        (rc = cuda(device_alloc(&sort_.idx_in, cap * 4), "cudaMalloc(sort)")) ||
+        (rc = cuda(device_alloc(&sort_.idx_out, cap * 4), "cudaMalloc(sort)")) ||
+        (rc = cuda(device_alloc(&sort_.cum, cap * 8), "cudaMalloc(sort)")) ||
+        (rc = cuda(device_alloc(&sort_.tmp, tmp), "cudaMalloc(sort)")))
         return rc;
     sort_.tmp_bytes = tmp;
     sort_cap_ = cap;
@@ -1047,8 +1047,8 @@ int Engine::ensure_cum(size_t n) {
     d_cum_ = nullptr; d_cum_tmp_ = nullptr; cum_cap_ = 0;
     cum_tmp_bytes_ = cumulate_scratch_bytes(cap);
     int rc;
-    if ((rc = cuda(cudaMalloc(&d_cum_, cap * 8), "cudaMalloc(cumulative)")) ||
-        (rc = cuda(cudaMalloc(&d_cum_tmp_, cum_tmp_bytes_), "cudaMalloc(cumulative)")))
+    if ((rc = cuda(device_alloc(&d_cum_, cap * 8), "cudaMalloc(cumulative)")) ||
+        (rc = cuda(device_alloc(&d_cum_tmp_, cum_tmp_bytes_), "cudaMalloc(cumulative)")))
         return rc;
     cum_cap_ = cap;
     return SQC_OK;
@@ -1306,7 +1306,7 @@ int Engine::stats(sqc_stats* out) {
     out->passes = passes_run_;
     out->kernel_launches = launches_;
     out->buckets = tab_.nb;
-    out->table_bytes = (uint64_t)(tab_.nb * bucket_bytes());
+    out->table_bytes = (uint64_t)(tab_.nb * bucket_bytes() + spare_bytes(this));
     out->replays = replays_;
     out->amp_updates = (ctl_host_ ? ctl_host_->amp_updates : 0) + host_upd_;
     out->alg_bytes = ctl_host_ ? ctl_host_->alg_bytes : 0;

@@ -104,6 +104,7 @@ private:
     size_t bucket_bytes() const;
     int alloc_table(unsigned long long nb, HostTable* out);
     void free_table(HostTable* t);
+    HostTable table_at(void* base, unsigned long long nb) const;
     TableDev dev() const;
     int rebuild(unsigned long long nb_new, bool mapped);
     // hashed tables: groups after a pass, at most; buckets for a state; room for the next pass
@@ -149,11 +150,11 @@ private:
     uint32_t max_run_ = kMaxRun;
     uint32_t max_nx_ = 2;        // cross-group qubits per pass at most
     size_t budget_ = 0;
+    size_t spare_limit_ = 0;     // kept tables of all states (sqc_devmem.h): an eighth of the device
     cudaStream_t stream_ = nullptr;
     bool own_stream_ = false;
 
     HostTable tab_;
-    HostTable spare_;           // the table the last rebuild left, for the next one (hashed tables)
     GroupMap map_;              // mapped group bits, when mapped_
     bool mapped_ = true;        // the table is mapped (sqc_types.h, TableDev), else hashed
     Ctl* ctl_ = nullptr;        // device

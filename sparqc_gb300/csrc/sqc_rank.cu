@@ -4,6 +4,7 @@
 // 16 bytes per header and 16 (FP64) per key, writes 24 per key: bound by HBM (2^25 keys FP64:
 // against a list readout, a 64-bit radix sort of key-index pairs and a gather).
 #include "sqc_rank.h"
+#include "sqc_devmem.h"
 #include "sqc_device.cuh"
 
 #include <algorithm>
@@ -176,7 +177,7 @@ cudaError_t RankScratch::need(size_t ntiles, size_t njobs) {
         if (tiles) cudaFree(tiles);
         tiles = nullptr;
         tiles_cap = 0;
-        const cudaError_t e = cudaMalloc(&tiles, ntiles * sizeof(unsigned long long));
+        const cudaError_t e = device_alloc(&tiles, ntiles * sizeof(unsigned long long));
         if (e != cudaSuccess) return e;
         tiles_cap = ntiles;
     }
@@ -186,8 +187,8 @@ cudaError_t RankScratch::need(size_t ntiles, size_t njobs) {
         jobs = nullptr;
         counts = nullptr;
         jobs_cap = 0;
-        cudaError_t e = cudaMalloc(&jobs, njobs * sizeof(RankJob));
-        if (e == cudaSuccess) e = cudaMalloc(&counts, (njobs + 1) * sizeof(unsigned long long));
+        cudaError_t e = device_alloc(&jobs, njobs * sizeof(RankJob));
+        if (e == cudaSuccess) e = device_alloc(&counts, (njobs + 1) * sizeof(unsigned long long));
         if (e != cudaSuccess) return e;
         jobs_cap = njobs;
     }

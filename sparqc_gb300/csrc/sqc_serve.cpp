@@ -6,6 +6,7 @@
 #include <cstring>
 #include <numeric>
 
+#include "sqc_devmem.h"
 #include "sqc_kernels.h"
 
 namespace sqc {
@@ -84,6 +85,7 @@ int Server::init(const sqc_server_options* opt) {
     if ((rc = cuda(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo"))) return rc;
     const size_t total_budget = o.memory_budget ? (size_t)o.memory_budget
                                                 : (size_t)std::min(kDefaultBudget, 0.9 * (double)total_b);
+    if (total_budget > free_b && spare_drop_all() && (rc = cuda(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo"))) return rc;
     if (total_budget > free_b) return fail(SQC_ERR_BUDGET, "memory budget exceeds the free device memory");
     // the slice pool takes the budget but the share kept for solo circuits' own tables
     solo_cap_ = solo_min_groups_ == ~0ULL ? 0 : (size_t)((double)total_budget * o.solo_share_pct / 100.0);
@@ -95,14 +97,14 @@ int Server::init(const sqc_server_options* opt) {
         own_stream_ = true;
     }
     const size_t n = max_slots_;
-    if ((rc = cuda(cudaMalloc(&pool_, budget), "cudaMalloc(pool)")) ||
-        (rc = cuda(cudaMalloc(&d_circ_, n * sizeof(BCirc)), "cudaMalloc")) ||
-        (rc = cuda(cudaMalloc(&d_ctl_, n * sizeof(Ctl)), "cudaMalloc")) ||
-        (rc = cuda(cudaMalloc(&d_sched_, n * sizeof(BSched)), "cudaMalloc")) ||
-        (rc = cuda(cudaMalloc(&d_words_, n * sizeof(unsigned long long)), "cudaMalloc")) ||
-        (rc = cuda(cudaMalloc(&d_cmd_, n * sizeof(unsigned)), "cudaMalloc")) ||
-        (rc = cuda(cudaMalloc(&d_limit_, n * sizeof(unsigned)), "cudaMalloc")) ||
-        (rc = cuda(cudaMalloc(&d_bctl_, sizeof(BatchCtl)), "cudaMalloc")) ||
+    if ((rc = cuda(device_alloc(&pool_, budget), "cudaMalloc(pool)")) ||
+        (rc = cuda(device_alloc(&d_circ_, n * sizeof(BCirc)), "cudaMalloc")) ||
+        (rc = cuda(device_alloc(&d_ctl_, n * sizeof(Ctl)), "cudaMalloc")) ||
+        (rc = cuda(device_alloc(&d_sched_, n * sizeof(BSched)), "cudaMalloc")) ||
+        (rc = cuda(device_alloc(&d_words_, n * sizeof(unsigned long long)), "cudaMalloc")) ||
+        (rc = cuda(device_alloc(&d_cmd_, n * sizeof(unsigned)), "cudaMalloc")) ||
+        (rc = cuda(device_alloc(&d_limit_, n * sizeof(unsigned)), "cudaMalloc")) ||
+        (rc = cuda(device_alloc(&d_bctl_, sizeof(BatchCtl)), "cudaMalloc")) ||
         (rc = cuda(cudaMallocHost(&h_circ_, n * sizeof(BCirc)), "cudaMallocHost")) ||
         (rc = cuda(cudaMallocHost(&h_ctl_, n * sizeof(Ctl)), "cudaMallocHost")) ||
         (rc = cuda(cudaMallocHost(&h_sched_, n * sizeof(BSched)), "cudaMallocHost")) ||
@@ -511,9 +513,9 @@ int Server::get_state(uint64_t id, uint64_t* keys, double* re, double* im, uint6
         const size_t c = std::max<size_t>(have, 1024);
         for (void* p : {(void*)d_rk_, (void*)d_rr_, (void*)d_ri_}) if (p) cudaFree(p);
         d_rk_ = nullptr; d_rr_ = nullptr; d_ri_ = nullptr; rcap_ = 0;
-        if ((rc = cuda(cudaMalloc(&d_rk_, c * 8), "cudaMalloc(readout)")) ||
-            (rc = cuda(cudaMalloc(&d_rr_, c * 8), "cudaMalloc(readout)")) ||
-            (rc = cuda(cudaMalloc(&d_ri_, c * 8), "cudaMalloc(readout)")))
+        if ((rc = cuda(device_alloc(&d_rk_, c * 8), "cudaMalloc(readout)")) ||
+            (rc = cuda(device_alloc(&d_rr_, c * 8), "cudaMalloc(readout)")) ||
+            (rc = cuda(device_alloc(&d_ri_, c * 8), "cudaMalloc(readout)")))
             return rc;
         rcap_ = c;
     }

@@ -24,7 +24,7 @@ def _cuda_include():
 def engine_objects(tmp_path_factory):
     out = tmp_path_factory.mktemp("host_engine")
     objs = []
-    for src in ("sqc_engine.cpp", "sqc_plan.cpp"):
+    for src in ("sqc_engine.cpp", "sqc_plan.cpp", "sqc_devmem.cpp"):
         obj = out / (src + ".o")
         subprocess.run(["g++", *FLAGS, *_cuda_include(), "-c", os.path.join(CSRC, src), "-o", str(obj)], check=True)
         objs.append(str(obj))
@@ -223,4 +223,49 @@ def test_flush_waits_for_nothing_while_recording(engine_objects, tmp_path):
     CHECK(dev.syncs == before);
     dev.capturing = false;
     CHECK(holds(e, expected(g)));
+    """)
+
+
+MOVES = """
+    // 2^10 keys that move about: the groups they leave fill the table, which is rebuilt again and again
+    std::vector<sqc_gate> g;
+    for (uint32_t q = 0; q < 10; ++q) g.push_back(gate(KH, q));
+    for (uint32_t i = 0; i < 200; ++i) g.push_back(gate(KX, 10 + i % 40, 1ULL << (i % 10) | 1ULL << ((i * i + 3 * i + 1) % 10)));
+"""
+
+
+def test_kept_tables_are_counted_and_given_back(engine_objects, tmp_path):
+    """The table a rebuild leaves is kept for the next one: it is in the state's bytes, another state's
+    allocation gets its memory when there is no other, and so does this state's own."""
+    run(engine_objects, tmp_path, MOVES + """
+    auto buffers = [](size_t held, const sqc_stats& st) { return held - (size_t)st.table_bytes; };
+    sqc_options o;
+    sqc_default_options(&o);
+    o.initial_buckets = 1 << 12;
+    Engine a;
+    make(a, 60, &o);
+    sqc_stats st;
+    a.stats(&st);
+    const size_t other = buffers(dev.held, st);
+    size_t kept = 0;
+    for (int k = 0; k < 3; ++k) {
+        CHECK(a.set_zero() == SQC_OK && a.apply(g.data(), g.size()) == SQC_OK && a.sync() == SQC_OK);
+        a.stats(&st);
+        kept = (size_t)st.table_bytes - (size_t)st.buckets * a.bucket_bytes_now();
+        CHECK(buffers(dev.held, st) == other);   // (no readout yet)
+    }
+    CHECK(kept > 0);
+    dev.total = dev.held + (4 << 20);   // (another state's small buffers)
+    {
+        Engine b;
+        o.initial_buckets = kept / a.bucket_bytes_now();
+        make(b, 60, &o);
+        a.stats(&st);
+        CHECK(st.table_bytes == st.buckets * a.bucket_bytes_now());
+        dev.total = dev.held + (4 << 20);
+    }
+    CHECK(holds(a, expected(g)));
+    dev.total = (size_t)284 << 30;
+    CHECK(a.set_zero() == SQC_OK && a.apply(g.data(), g.size()) == SQC_OK);
+    CHECK(holds(a, expected(g)));
     """)
