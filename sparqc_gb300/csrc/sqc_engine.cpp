@@ -32,7 +32,10 @@ constexpr unsigned long long kMapRoomy = 1ULL << 21;
 constexpr double kHashLoad = 0.35;          // ... and a hashed table stays below while memory allows: lookups of absent
                                             // groups probe to the first free bucket (2^17 keys of logic, 82 passes:
                                             // 0.9 15.7 ms, 0.7 9.7, 0.5 8.4, 0.35 6.9, 0.25 7.5 with more rebuilds)
-constexpr unsigned long long kHashRoomy = 1ULL << 17;   // 55 MB
+constexpr unsigned long long kHashRoomy = 1ULL << 17;   // buckets (53 MB) a small hashed table gets at most beyond its need
+constexpr unsigned long long kRoomyKey = 32;            // ... with 32 to 64 to a key
+constexpr int kRoomyShare = 16;            // a hashed table takes more than it needs up to this part of the budget
+constexpr int kThinShare = 4;              // ... and a map of more than eight times its groups (three new bits) up to this one
 constexpr uint32_t kRunMapFp64 = 18, kRunMapFp32 = 17;   // mapped bits up to which passes go out in runs (sqc_pass.cu: run_kernel)
 constexpr unsigned long long kRunMaxList = 1ULL << 17;   // ... and live buckets of a hashed one
 constexpr uint32_t kNoMap = 63;            // Span::dn of a pass whose bits no table maps: always refused
@@ -631,15 +634,19 @@ unsigned long long Engine::grown(uint32_t nx, unsigned long long bound, unsigned
 
 // Buckets of a hashed table of `groups` groups: room for a pass, and for several that empty as many
 // groups as they make (keys that move leave their groups behind, live and empty, until the table is
-// rebuilt): eight times the groups, or every group the keys could make in four passes; small tables
-// far more, so that a short circuit needs no rebuild at all.
+// rebuilt): eight times the groups, or every group the keys could make in four passes, at a load of 0.35;
+// small tables 32 to 64 buckets to a key (up to 53 MB), so that short circuits need few rebuilds. Past a sixteenth of the budget memory
+// counts for more than time: room for a pass, or four times the groups, up to a load of 0.9.
 unsigned long long Engine::hashed_size(unsigned long long groups, uint32_t nx, unsigned long long keys) {
     const double room = std::max((double)groups * (double)std::max(8u, 1u << nx), 0.0);
     const double by_keys = (double)groups + 4.0 * (double)keys;
     const double one_pass = std::min((double)groups * (double)(1u << nx), (double)groups + (double)keys);
     const double want = std::max(one_pass, std::min(room, by_keys));
-    const unsigned long long nb = std::max(kMinBuckets, pow2_at_least((unsigned long long)std::ceil(want / kHashLoad)));
-    return std::max(nb, std::min(nb * 32, kHashRoomy));
+    unsigned long long nb = std::max(kMinBuckets, pow2_at_least((unsigned long long)std::ceil(want / kHashLoad)));
+    nb = std::max(nb, std::min(pow2_at_least(kRoomyKey * ctl_host_->nnz + 1), kHashRoomy));
+    const unsigned long long lean = pow2_at_least((unsigned long long)std::ceil(std::max(one_pass, 4.0 * (double)groups) / kMaxLoad));
+    while (nb > std::max(lean, kMinBuckets) && (double)nb * bucket_bytes() > (double)budget_ / kRoomyShare) nb /= 2;
+    return nb;
 }
 
 // Before a pass that might not fit a hashed table by what the host knows: look at the exact list
@@ -658,8 +665,9 @@ int Engine::make_room(uint32_t nx, unsigned long long bound, unsigned long long 
         hash_load_ = kMaxLoad;
         return SQC_OK;   // a pass that still does not fit refuses; sync() decides
     }
-    // no memory for it: the present table fills up, and a pass that does not fit refuses
+    // no memory for it: a smaller one, or the present table fills up, and a pass that does not fit refuses
     rc = rebuild(nb, false);
+    while (rc == SQC_ERR_OOM && nb / 2 > tab_.nb) rc = rebuild(nb /= 2, false);
     if (rc == SQC_ERR_OOM || rc == SQC_ERR_BUDGET) {
         hash_load_ = kMaxLoad;
         return SQC_OK;
@@ -873,19 +881,20 @@ int Engine::repair(size_t k) {
     // groups that still hold keys: the rebuild drops the others
     const unsigned long long groups = ctl_host_->list_n - std::min(ctl_host_->list_n, ctl_host_->empty_groups);
     auto fits = [&](unsigned long long b) { return (double)b * bucket_bytes() <= (double)budget_; };
-    unsigned long long nb = 0;
-    bool mapped = false;
+    int rc = SQC_ERR_OOM;   // until a table was made
     if (mapped_) {
         map_.n = pr.map_n;
         if (map_worth(pr.dn, groups)) {
             const unsigned long long span = 1ULL << pr.dn;
-            nb = std::max(span * 8 <= kMapRoomy ? span * 8 : std::max(span * 2, kMapRoomy), kMinBuckets);
-            while (nb > 2 * span && !fits(nb)) nb /= 2;   // at most 0.9 full, like a hashed table
-            mapped = fits(nb);
+            const double least = 2.0 * (double)span * bucket_bytes();   // at most 0.9 full, like a hashed table
+            unsigned long long nb = std::max(span * 8 <= kMapRoomy ? span * 8 : std::max(span * 2, kMapRoomy), kMinBuckets);
+            if (span > 8 * groups && least > (double)budget_ / kThinShare) nb = 0;
+            for (; nb >= 2 * span && rc == SQC_ERR_OOM; nb /= 2)   // no memory: a smaller one
+                if (fits(nb)) rc = rebuild(nb, true);
         }
     }
-    if (!mapped) {
-        nb = hashed_size(groups, pr.nx, pr.keys);
+    if (rc == SQC_ERR_OOM) {
+        unsigned long long nb = hashed_size(groups, pr.nx, pr.keys);
         // a hashed table mostly of emptied groups has room once they are dropped; else it doubles
         if (!mapped_ && (nb > tab_.nb || groups * 2 > ctl_host_->list_n)) nb = std::max(nb, tab_.nb * 2);
         // near the budget, take the largest table that still fits (the pass may refuse again)
@@ -893,9 +902,11 @@ int Engine::repair(size_t k) {
         while (fits(fit * 2)) fit *= 2;
         if (nb > fit && (fit > tab_.nb || mapped_)) nb = fit;
         if ((double)groups > kMaxLoad * (double)nb) return fail(SQC_ERR_BUDGET, "table memory would exceed the HBM budget");
+        rc = rebuild(nb, false);
+        // no memory: a smaller one that holds the groups, and more than the present one
+        while (rc == SQC_ERR_OOM && (mapped_ || nb / 2 > tab_.nb) && (double)groups <= kMaxLoad * (double)(nb / 2)) rc = rebuild(nb /= 2, false);
     }
-    int rc;
-    if ((rc = rebuild(nb, mapped))) return rc;
+    if (rc) return rc;
     std::vector<sqc_gate> again(log_.begin() + (long)pr.log_begin, log_.end());
     replays_ += passes_.size() - k;
     passes_run_ -= passes_.size() - k;

@@ -269,3 +269,67 @@ def test_kept_tables_are_counted_and_given_back(engine_objects, tmp_path):
     CHECK(a.set_zero() == SQC_OK && a.apply(g.data(), g.size()) == SQC_OK);
     CHECK(holds(a, expected(g)));
     """)
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("keys", [16, 300])
+def test_small_sparse_states_stay_small(engine_objects, tmp_path, keys, precision):
+    """A few hundred keys over many qubits hold a few megabytes, tables kept for a rebuild included."""
+    run(engine_objects, tmp_path, """
+    Engine e;
+    sqc_options o;
+    sqc_default_options(&o);
+    o.precision = %d;
+    make(e, 60, &o);
+    std::vector<uint64_t> k(%d);
+    std::vector<double> r(k.size(), 0.05), i(k.size(), 0.0);
+    std::map<unsigned long long, Amp> start;
+    for (size_t j = 0; j < k.size(); ++j) start[k[j] = ((j + 1) * 0x9E3779B97F4A7C15ULL) >> 4] = Amp(0.05, 0.0);
+    CHECK(e.set_state(k.data(), r.data(), i.data(), k.size()) == SQC_OK);
+    std::vector<sqc_gate> g;
+    for (uint32_t j = 0; j < 12; ++j) g.push_back(gate(j %% 6 ? KX : KRY, 7 + 4 * j, j %% 6 ? 1ULL << j : 0, 0.7));
+    CHECK(e.apply(g.data(), g.size()) == SQC_OK);
+    CHECK(holds(e, expected(g, start)));
+    sqc_stats st;
+    e.stats(&st);
+    std::printf("bytes %%llu\\n", (unsigned long long)st.table_bytes);
+    CHECK(st.table_bytes <= (size_t)2 * 16384 * e.bucket_bytes_now());
+    """ % (precision, keys))
+
+
+@pytest.mark.parametrize("mb", [160, 40, 34, 30])
+def test_tables_grow_by_what_there_is(engine_objects, tmp_path, mb):
+    """2^12 keys in groups of their own on a device with little memory: the table that would be best does not
+    fit beside the old one, and a smaller one is taken."""
+    run(engine_objects, tmp_path, """
+    dev.total = (size_t)%d << 20;
+    Engine e;
+    sqc_options o;
+    sqc_default_options(&o);
+    o.initial_buckets = 64;
+    make(e, 60, &o);
+    std::vector<sqc_gate> g;
+    for (uint32_t q = 0; q < 12; ++q) g.push_back(gate(KH, q));
+    for (uint32_t q = 0; q < 12; ++q) g.push_back(gate(KX, 12 + 4 * q, 1ULL << q));
+    CHECK(e.apply(g.data(), g.size()) == SQC_OK);
+    CHECK(holds(e, expected(g)));
+    """ % mb)
+
+
+def test_thin_maps_take_a_share_of_the_device(engine_objects, tmp_path):
+    """2^14 groups that spread over 18 bits would be mapped by a table of half the device: they are hashed
+    instead, and the state takes an eighth of it."""
+    run(engine_objects, tmp_path, """
+    dev.total = (size_t)512 << 20;
+    Engine e;
+    make(e, 60);
+    std::vector<sqc_gate> g;
+    for (uint32_t q = 4; q < 18; ++q) g.push_back(gate(KH, q));
+    for (uint32_t q = 0; q < 4; ++q) g.push_back(gate(KX, 20 + 4 * q, 7ULL << (4 + 3 * q)));
+    CHECK(e.apply(g.data(), g.size()) == SQC_OK);
+    CHECK(holds(e, expected(g)));
+    sqc_stats st;
+    e.stats(&st);
+    std::printf("bytes %llu peak %zu\\n", (unsigned long long)st.table_bytes, dev.peak);
+    CHECK(st.table_bytes <= dev.total / 8 && dev.peak <= dev.total / 2);
+    """)
