@@ -101,6 +101,7 @@ __device__ __forceinline__ long long lookup_group(const TableDev& t, unsigned ep
         const Header h = load_hdr_cg(t.hdr + b);
         if (h.epoch != ep) return -1;
         if (h.group == G) return (long long)b;
+        if (t.map_on) return -1;   // the address is exact: a group with a bit outside the map is nowhere else
         b = (b + 1) & t.mask;
     }
     return -1;

@@ -457,3 +457,31 @@ def test_recorded_runs_replay(keys, precision):
     assert st.stats()["passes"] == 2
     assert_identical(st.state(sorted=True), o.state(sorted=True))
     st.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+def test_comparing_states_on_different_bits(precision):
+    """Two states whose keys differ in a bit neither maps share no key; telling that takes one look per key
+    in a dense table too, about what a comparison of equal states takes (16 times it: far below the
+    thousands of neighbours that a search would visit)."""
+    import time
+    from sparqc_gb300.engine import State
+    gs = [(G.RY, q, (), 0.3 + q) for q in range(18)]
+    a, b, c = State(40, precision=precision), State(40, precision=precision), State(40, precision=precision)
+    a.apply(G.gate_array(gs))
+    b.apply(G.gate_array(gs))
+    c.apply(G.gate_array(gs + [(G.X, 30)]))
+
+    def best(other):
+        t = []
+        for _ in range(5):
+            t0 = time.perf_counter()
+            r = a.compare(other)
+            t.append(time.perf_counter() - t0)
+        return r, min(t)
+
+    (same, t_same), (apart, t_apart) = best(b), best(c)
+    assert same[0] > 1 - 1e-6 and same[1] == 0.0
+    assert apart[0] == 0.0 and apart[1] > 0.0
+    assert t_apart < 16 * t_same
