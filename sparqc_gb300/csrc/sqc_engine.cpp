@@ -32,6 +32,8 @@ constexpr unsigned long long kMapRoomy = 1ULL << 21;
 constexpr double kHashLoad = 0.35;          // ... and a hashed table stays below while memory allows: lookups of absent
                                             // groups probe to the first free bucket (2^17 keys of logic, 82 passes:
                                             // 0.9 15.7 ms, 0.7 9.7, 0.5 8.4, 0.35 6.9, 0.25 7.5 with more rebuilds)
+constexpr unsigned long long kSmallTable = 1ULL << 16;  // up to here (26 MB, in the L2) lookups are cheap beside a rebuild
+constexpr double kSmallLoad = 0.6;
 constexpr unsigned long long kHashRoomy = 1ULL << 17;   // buckets (53 MB) a small hashed table gets at most beyond its need
 constexpr unsigned long long kRoomyKey = 32;            // ... with 32 to 64 to a key
 constexpr int kRoomyShare = 16;            // a hashed table takes more than it needs up to this part of the budget
@@ -433,19 +435,24 @@ int Engine::flush(bool hold_last) {
         size_t g0, g1;
         uint32_t nx, q1, q2, q3;
         bool fixed;
+        uint32_t slots;              // hashed tables: a slot pass's form, or 0
         uint32_t map0, dn, dim[3];   // mapped tables: mapped bits before and after, the units' dimensions
         unsigned long long keys;     // keys after the pass, at most
     };
     std::vector<Span> spans;
-    // mapped tables pair up to max_nx_ qubits >= 4 a pass, hashed ones two of any (columns)
     auto split = [&] {
         spans.clear();
-        split_passes(hd, nd, max_run_, mapped_ ? max_nx_ : std::min(max_nx_, 2u),
-                     [&](size_t g0, size_t g1, uint32_t, uint32_t q1, uint32_t q2, uint32_t q3, bool fixed) {
-                         uint32_t nx = 0;   // qubits that pair groups
-                         for (uint32_t q : {q1, q2, q3}) nx += q != kNoQubit && q >= (uint32_t)kSlotBits ? 1 : 0;
-                         spans.push_back(Span{g0, g1, nx, q1, q2, q3, fixed, 0, 0, {0, 0, 0}, 0});
-                     }, !mapped_);
+        auto add = [&](size_t g0, size_t g1, uint32_t slots, uint32_t q1, uint32_t q2, uint32_t q3, bool fixed) {
+            uint32_t nx = 0;   // qubits that pair groups
+            for (uint32_t q : {q1, q2, q3}) nx += q != kNoQubit && q >= (uint32_t)kSlotBits ? 1 : 0;
+            spans.push_back(Span{g0, g1, nx, q1, q2, q3, fixed, slots, 0, 0, {0, 0, 0}, 0});
+        };
+        if (mapped_)
+            split_passes(hd, nd, max_run_, max_nx_, [&](size_t g0, size_t g1, uint32_t, uint32_t q1, uint32_t q2, uint32_t q3, bool fixed) {
+                add(g0, g1, 0u, q1, q2, q3, fixed);
+            });
+        else
+            plan_hashed(hd, nd, max_run_, max_nx_, std::min(max_nx_, 2u), 3u, dbl_, list_hint_, std::min(key_hint_, 16 * list_hint_), add);
         unsigned long long keys = key_hint_;   // a branching gate at most doubles them
         for (Span& sp : spans) {
             for (size_t i = sp.g0; i < sp.g1; ++i)
@@ -492,7 +499,8 @@ int Engine::flush(bool hold_last) {
     for (Span& sp : spans) {
         const uint32_t q[3] = {sp.q1, sp.q2, sp.q3};
         if (!mapped_) {
-            encode_column_pass(hd, sp.g0, sp.g1, q, sp.dim);
+            if (sp.slots) encode_slot_pass(hd, sp.g0, sp.g1, sp.slots, q, sp.dim);
+            else encode_column_pass(hd, sp.g0, sp.g1, q, sp.dim);
             continue;
         }
         sp.map0 = map_.n;
@@ -541,7 +549,7 @@ int Engine::flush(bool hold_last) {
         while (!time_passes_ && e < spans.size()) {
             const Span& r = spans[e];
             const size_t w = mapped_ ? 1 + r.g1 - r.g0 : 2;
-            if (words + w > kRunWords || odd_pass(hd, r.g0, r.g1)) break;
+            if (words + w > kRunWords || r.slots || odd_pass(hd, r.g0, r.g1)) break;
             if (mapped_) {
                 if (r.dn > (dbl_ ? kRunMapFp64 : kRunMapFp32) || (1ULL << r.dn) > a.max_groups) break;
                 items = std::max(1ULL, (1ULL << r.dn) >> dims);
@@ -588,6 +596,7 @@ int Engine::flush(bool hold_last) {
         a.nx = sp.nx;
         a.keys_fixed = sp.fixed ? 1u : 0u;
         a.odd = odd_pass(hd, sp.g0, sp.g1) ? 1u : 0u;
+        a.slots = sp.slots;
         a.grow_bound = group_bound(after[sp.g1 - 1], nq_);
         a.key_bound = sp.keys;
         if (!mapped_ && sp.nx && grown(sp.nx, a.grow_bound, sp.keys) > roomy_groups() && !recording()) {
@@ -821,7 +830,7 @@ int Engine::sync() {
 // Copy the live, non-empty buckets into a new table of nb_new buckets. The control block
 // must be in sync with the device (read_ctl) and no pass may be in flight.
 int Engine::rebuild(unsigned long long nb_new, bool mapped) {
-    hash_load_ = kHashLoad;
+    hash_load_ = nb_new <= kSmallTable ? kSmallLoad : kHashLoad;
     HostTable nt;
     int rc;
     if ((rc = alloc_table(nb_new, &nt))) return rc;

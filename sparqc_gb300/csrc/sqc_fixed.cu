@@ -153,31 +153,25 @@ extern "C" int sqc_apply_fixed(uint32_t nq, const uint64_t* keys_in, const doubl
                                                      outside, ctl);
         if (cudaGetLastError() != cudaSuccess) return SQC_ERR_CUDA;
     }
-    // passes of at most one gate that pairs groups; each pass's gates are encoded before the descriptors are uploaded
+    // passes of at most one gate that pairs groups, at their beginning: each is checked against the scratch
+    // table's room; every pass's gates are encoded before the descriptors are uploaded
     struct Span {
         uint32_t g0, g1, dim[3];
         bool pair, fixed;
+        uint32_t slots;
     };
     Span spans[kFixedMaxGates];
-    size_t ns = 0, i = 0;
-    while (i < n_gates) {
-        const size_t start = i;
-        // a gate that pairs groups begins a pass: each is checked against the scratch table's room
-        uint32_t q[2] = {kNoQubit, kNoQubit};
-        const bool pair = !diag_kind(hd[i].kind) && hd[i].target >= (uint32_t)kSlotBits;
-        for (; i < n_gates && i - start < (size_t)kMaxRun; ++i) {
-            const uint32_t t = hd[i].target;
-            if (diag_kind(hd[i].kind)) continue;
-            if (t >= (uint32_t)kSlotBits && i != start) break;
-            if (t == q[0] || t == q[1]) continue;
-            if (q[1] != kNoQubit) break;
-            q[q[0] == kNoQubit ? 0 : 1] = t;
-        }
-        bool fixed = true;
-        for (size_t k = start; k < i; ++k) fixed = fixed && diag_kind(hd[k].kind);
-        Span& sp = spans[ns++];
-        sp = Span{(uint32_t)start, (uint32_t)i, {0, 0, 0}, pair, fixed};
-        encode_column_pass(hd, start, i, q, sp.dim);
+    size_t ns = 0;
+    for (size_t i = 0, e = 0; i < n_gates; i = e) {
+        auto pairs = [&](size_t k) { return !diag_kind(hd[k].kind) && hd[k].target >= (uint32_t)kSlotBits; };
+        for (e = i + 1; e < n_gates && !pairs(e);) ++e;
+        plan_hashed(hd + i, e - i, (size_t)kMaxRun, 1u, 2u, 2u, true, n_in, n_in, [&](size_t g0, size_t g1, uint32_t slots, uint32_t q1, uint32_t q2, uint32_t q3, bool fixed) {
+            Span& sp = spans[ns++];
+            sp = Span{(uint32_t)(i + g0), (uint32_t)(i + g1), {0, 0, 0}, g0 == 0 && pairs(i), fixed, slots};
+            const uint32_t q[3] = {q1, q2, q3};
+            if (slots) encode_slot_pass(hd, sp.g0, sp.g1, slots, q, sp.dim);
+            else encode_column_pass(hd, sp.g0, sp.g1, q, sp.dim);
+        });
     }
     if (n_gates && cudaMemcpyAsync(d_desc, hd, n_gates * sizeof(GateDesc), cudaMemcpyHostToDevice, st) != cudaSuccess)
         return SQC_ERR_CUDA;
@@ -204,6 +198,7 @@ extern "C" int sqc_apply_fixed(uint32_t nq, const uint64_t* keys_in, const doubl
         a.key_bound = kKeysUnknown;
         a.keys_fixed = spans[k].fixed ? 1u : 0u;
         a.odd = odd_pass(hd, a.g0, a.g1) ? 1u : 0u;
+        a.slots = spans[k].slots;
         if (launch_hash_pass(a, kFixedBuckets, true, sms, st) < 0) return SQC_ERR_CUDA;
     }
     if (launch_readout(t, ctl, kFixedBuckets, 0ULL, true, reinterpret_cast<unsigned long long*>(keys_out), re_out,

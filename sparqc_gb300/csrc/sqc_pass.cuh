@@ -141,6 +141,49 @@ __global__ void __launch_bounds__(kThreads, ODD ? 2 : kHashBlocks<T>) hash_kerne
     finish_pass(ctl, cnt_nnz, cnt_empty, upd, nnz_in, a.keys_fixed != 0, a.nx > 0, a.amp_bytes);
 }
 
+// A slot pass (walk_slots; S == kLowForm: walk_low). plain: FP64 products by the FP64 instruction. A few warps are not bound by its pipe
+// but by fetching code, and the integer products are 20 times as long.
+constexpr int kLowForm = 16;
+template <class T, int S, bool ODD>
+__global__ void __launch_bounds__(kThreads, ODD ? 2 : kHashBlocks<T>) slot_kernel(const __grid_constant__ PassArgs a) {
+    __shared__ HGates<T> sg;
+    __shared__ SlotWork wk[S == kLowForm ? 1 : kThreads / 32];
+    unsigned long long gm[3];
+    for (int i = 0; i < 3; ++i) gm[i] = a.dim[i] < 64u ? 1ULL << (a.dim[i] - kSlotBits) : 0ULL;
+    const uint32_t ng = a.g1 - a.g0;
+    const GateDesc* gates = a.gates + a.g0;
+    stage_hgates<T>(sg, gates, ng, S == kLowForm ? 3ULL : (gm[1] | gm[2]) << kSlotBits);   // no kernel writes the gates: staged while the previous pass drains
+    if constexpr (sizeof(T) == 8)
+        if (a.plain)
+            for (uint32_t i = threadIdx.x; i < ng; i += blockDim.x) sg.g[i].exact = 0;   // (the thread's own)
+    __syncthreads();
+    wait_prior_grid();
+    allow_next_grid();
+    Ctl* ctl = a.ctl;
+    if (*(volatile unsigned int*)&ctl->status) return;
+    const unsigned long long n = ctl->list_n;
+    if (could_overflow(n, a.nx, a.grow_bound, a.key_bound, a.max_groups)) {   // refuse before touching the state
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(&ctl->status, 0u, (unsigned)ST_GROW);
+        return;
+    }
+    const unsigned ep = ctl->epoch;
+    const unsigned long long nnz_in = ctl->nnz;
+    const int lane = threadIdx.x & 31;
+    const unsigned wid = __shfl_sync(kFull, threadIdx.x >> 5, 0), nw = gridDim.x * (kThreads / 32);
+    unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
+    unsigned long long piece = list_piece(n, nw);
+    if constexpr (S == kLowForm) {
+        piece = 8;
+        for (unsigned long long e0 = (wid * gridDim.x + blockIdx.x) * piece; e0 < n; e0 += nw * piece)
+            walk_low<T, ODD>(a.t, e0, umin64(e0 + piece, n), sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+    } else {
+        if (a.nx == 0) piece += piece & 1;   // (at most 32)
+        for (unsigned long long e0 = (wid * gridDim.x + blockIdx.x) * piece; e0 < n; e0 += nw * piece)
+            walk_slots<T, S, ODD>(a.t, ctl, ep, gm, a.nx, e0, umin64(e0 + piece, n), wk[wid], sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+    }
+    finish_pass(ctl, cnt_nnz, cnt_empty, upd, nnz_in, a.keys_fixed != 0, a.nx > 0, a.amp_bytes);
+}
+
 template <class K>
 int occupancy(K kernel, int threads) {
     int per_sm = 0;
@@ -193,9 +236,29 @@ int launch_unit_kernel(const PassArgs& a, bool dbl, int sms, cudaStream_t st) {
     return e == cudaSuccess ? 1 : -1;
 }
 
+template <class T, int S, bool ODD>
+cudaError_t launch_slots(const PassArgs& a, unsigned long long list_hint, int sms, cudaStream_t st) {
+    static int resident = 0;
+    if (!resident) resident = occupancy(slot_kernel<T, S, ODD>, kThreads);
+    // a warp per unit, or per two units of one group
+    const unsigned long long items = a.nx ? list_hint : (list_hint + 1) / 2;
+    PassArgs b = a;
+    b.plain = items <= 4ULL * (unsigned long long)sms;   // at most a warp to a scheduler
+    return launch_dep(slot_kernel<T, S, ODD>, grid_of(items, kThreads, sms, resident), b, st);
+}
+
+template <class T, bool ODD>
+cudaError_t launch_slots(const PassArgs& a, unsigned long long list_hint, int sms, cudaStream_t st) {
+    if constexpr (sizeof(T) == 4)
+        if (a.slots == 2) return launch_slots<T, kLowForm, ODD>(a, (list_hint + 3) / 4, sms, st);
+    return a.nx <= 1 ? launch_slots<T, 1, ODD>(a, list_hint, sms, st)
+           : a.nx == 2 ? launch_slots<T, 2, ODD>(a, list_hint, sms, st) : launch_slots<T, 4, ODD>(a, list_hint, sms, st);
+}
+
 template <bool ODD>
 int launch_hash_kernel(const PassArgs& a, unsigned long long list_hint, bool dbl, int sms, cudaStream_t st) {
-    const cudaError_t e = dbl ? launch_hash<double, ODD>(a, list_hint, sms, st) : launch_hash<float, ODD>(a, list_hint, sms, st);
+    const cudaError_t e = a.slots ? (dbl ? launch_slots<double, ODD>(a, list_hint, sms, st) : launch_slots<float, ODD>(a, list_hint, sms, st))
+                          : dbl ? launch_hash<double, ODD>(a, list_hint, sms, st) : launch_hash<float, ODD>(a, list_hint, sms, st);
     return e == cudaSuccess ? 1 : -1;
 }
 

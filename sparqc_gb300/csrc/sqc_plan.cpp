@@ -234,30 +234,48 @@ void encode_unit_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[3], co
     }
 }
 
+// One gate's place in a pass over a hashed table whose lanes hold the four keys that differ in qubits q0 and q1:
+// controls on them by slot, all others by key; op is the gate's op code (pairing gates on q0 or q1: with the
+// form on q1 added).
+static void encode_in_lane(GateDesc& g, uint32_t q0, uint32_t q1, uint32_t lane_bit) {
+    g.om = g.ov = 0;
+    const uint32_t q[2] = {q0, q1};   // (kNoQubit: none)
+    uint32_t smask = 0, sval = 0, slot_bit = kNoQubit;
+    for (uint32_t i = 0; i < 2; ++i) {
+        if (q[i] == kNoQubit) continue;
+        if (g.target == q[i]) slot_bit = i;
+        if (!((g.ctrl >> q[i]) & 1ULL)) continue;
+        smask |= 1u << i;
+        sval |= (uint32_t)((g.cval >> q[i]) & 1ULL) << i;
+    }
+    const bool flip = (g.flip & kOpFlip) != 0, pairs = is_branch_kind(g.kind) || is_swap_kind(g.kind);
+    uint32_t slots = 0, bits = 0;
+    for (uint32_t s = 0; s < 4; ++s) {
+        if (((s ^ sval) & smask) == 0) slots |= 1u << s;
+        if ((slot_bit != kNoQubit && ((s >> slot_bit) & 1u)) != flip) bits |= 1u << s;
+    }
+    const bool pair3 = pairs && slot_bit == 1, lanes = pairs && slot_bit == kNoQubit;
+    const uint32_t op = odd_gate(g) ? UO_ODD + (pair3 ? 2u : lanes ? 1u : 0u) : unit_op(g.kind) + (pair3 ? UO_PAIR3 : lanes ? 1u : 0u);
+    const uint32_t bit = lanes ? lane_bit : g.target & 31u;
+    g.loc = (slots << kLocSlots) | (bits << kLocSlotBit) | (slot_bit != kNoQubit ? kLocLane : 0u) | (bit << kLocBit) |
+            (!lanes && g.target >= 32u ? kLocHigh : 0u) | (flip ? kLocFlip : 0u) | (op << kLocOp);
+}
+
 void encode_column_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[2], uint32_t dim[3]) {
-    for (int i = 0; i < 2; ++i) dim[i] = q[i] == kNoQubit ? 64u : q[i];
+    dim[0] = q[0];
+    dim[1] = q[1];
     dim[2] = 64u;
+    for (int i = 0; i < 2; ++i)   // (2^16 groups of 16 keys, 24 diagonal gates, FP64: 747 us with one key to a column)
+        if (dim[i] == kNoQubit) dim[i] = dim[1 - i] == 0u ? 1u : 0u;
+    for (size_t k = g0; k < g1; ++k) encode_in_lane(d[k], dim[0], dim[1], 0);
+}
+
+void encode_slot_pass(GateDesc* d, size_t g0, size_t g1, uint32_t form, const uint32_t q[3], uint32_t dim[3]) {
+    for (int i = 0; i < 3; ++i) dim[i] = q[i] == kNoQubit ? 64u : q[i];
+    // lane bits: qubits 0 to 3, then the first cross-group one; the others are in a lane
     for (size_t k = g0; k < g1; ++k) {
-        GateDesc& g = d[k];
-        g.om = g.ov = 0;
-        uint32_t smask = 0, sval = 0, slot_bit = kNoQubit;
-        for (uint32_t i = 0; i < 2; ++i) {
-            if (q[i] == kNoQubit) continue;
-            if (g.target == q[i]) slot_bit = i;
-            if (!((g.ctrl >> q[i]) & 1ULL)) continue;
-            smask |= 1u << i;
-            sval |= (uint32_t)((g.cval >> q[i]) & 1ULL) << i;
-        }
-        const bool flip = (g.flip & kOpFlip) != 0, pairs = is_branch_kind(g.kind) || is_swap_kind(g.kind);
-        uint32_t slots = 0, bits = 0;
-        for (uint32_t s = 0; s < 4; ++s) {
-            if (((s ^ sval) & smask) == 0) slots |= 1u << s;
-            if ((slot_bit != kNoQubit && ((s >> slot_bit) & 1u)) != flip) bits |= 1u << s;
-        }
-        const bool pair3 = pairs && slot_bit == 1;
-        const uint32_t op = odd_gate(g) ? UO_ODD + (pair3 ? 2u : 0u) : unit_op(g.kind) + (pair3 ? UO_PAIR3 : 0u);
-        g.loc = (slots << kLocSlots) | (bits << kLocSlotBit) | (slot_bit != kNoQubit ? kLocLane : 0u) |
-                ((g.target & 31u) << kLocBit) | (g.target >= 32u ? kLocHigh : 0u) | (flip ? kLocFlip : 0u) | (op << kLocOp);
+        if (form == 2) encode_in_lane(d[k], 0, 1, d[k].target - 2);   // (lanes: qubits 2 and 3)
+        else encode_in_lane(d[k], q[1], q[2], std::min(d[k].target, 4u));
     }
 }
 

@@ -3,6 +3,7 @@
 // (coefficients on the host) and the split of a descriptor sequence into passes.
 #pragma once
 #include <cstddef>
+#include <algorithm>
 #include <cstdint>
 
 #include "../../include/sparqc.h"
@@ -109,9 +110,52 @@ void encode_unit_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[3], co
                       uint32_t dim[3]);
 
 // The same for a pass over a hashed table, whose columns (sqc_unit.cuh) are the keys that differ in its
-// pairing qubits q[0..1], any qubits (split_passes with columns; kNoQubit when absent); dim gets them,
-// 64 for an absent one.
+// pairing qubits q[0..1], any qubits (split_passes with columns; kNoQubit when absent: a low qubit takes its
+// place, so that a column always has four keys); dim gets them.
 void encode_column_pass(GateDesc* d, size_t g0, size_t g1, const uint32_t q[2], uint32_t dim[3]);
+
+// The same for a slot pass (walk_slots) with cross-group qubits q[0..2] (kNoQubit when absent); dim as above.
+// form 1: a slot to a lane (walk_slots), 2: four (walk_low; no cross-group qubits).
+void encode_slot_pass(GateDesc* d, size_t g0, size_t g1, uint32_t form, const uint32_t q[3], uint32_t dim[3]);
+
+// Passes of a descriptor sequence over a hashed table: column passes (split_passes with columns, at most `two`
+// (1 or 2) pairing qubits) or slot passes (at most max_nx cross-group qubits). A slot pass runs the absent slots
+// of its units along. It is taken where the state is small (groups) or its groups hold enough keys, those that
+// branching gates on low qubits will add among them, and it takes the gates of at least two column passes, or `spare`
+// when it needs lookups (a cross-group qubit); a pass that is one column pass either way where the state is small,
+// or FP64 groups hold enough keys. (us, start
+// of the sequence to its end, columns against slots: 24 gates on low qubits, FP64, 2^12 groups of 16 keys 169
+// and 57, 2^16 478 and 246; 36 gates on the low and two other qubits, 30000 groups of one key 1018 and 516; but a
+// million keys in groups of one or two, 60 gates, few branching: 7.4 ms and 14.)
+// f(g0, g1, form, q1, q2, q3, keys_fixed): form 0, a column pass and its pairing qubits, or a slot pass (encode_slot_pass)
+// and its cross-group ones.
+constexpr unsigned long long kSlotSmall = 1ULL << 15;   // groups of a small state
+template <class F>
+void plan_hashed(const GateDesc* d, size_t n, size_t max_run, uint32_t max_nx, uint32_t two, uint32_t spare, bool dbl,
+                 unsigned long long groups, unsigned long long keys, F&& f) {
+    for (size_t i = 0; i < n;) {
+        // the slot pass from here, and the column passes over the same gates
+        struct { size_t g1; uint32_t nx, q[3]; bool fixed; } slot{}, col{};
+        split_passes(d + i, std::min(n - i, max_run), max_run, max_nx, [&](size_t g0, size_t g1, uint32_t nx, uint32_t q1, uint32_t q2, uint32_t q3, bool fixed) {
+            if (g0 == 0) slot = {i + g1, nx, {q1, q2, q3}, fixed};
+        });
+        size_t cols = 0;
+        split_passes(d + i, slot.g1 - i, max_run, two, [&](size_t g0, size_t g1, uint32_t nx, uint32_t q1, uint32_t q2, uint32_t q3, bool fixed) {
+            if (g0 == 0) col = {i + g1, nx, {q1, q2, q3}, fixed};
+            ++cols;
+        }, true);
+        uint32_t low = 0;   // low qubits with a branching gate
+        for (size_t k = i; k < slot.g1; ++k)
+            if (is_branch_kind(d[k].kind) && d[k].target < (uint32_t)kSlotBits) low |= 1u << d[k].target;
+        const unsigned long long held = std::min(keys << __builtin_popcount(low), 16 * groups);   // (keys: at most 2^62)
+        const bool slots = slot.nx ? cols >= spare && (groups <= kSlotSmall || held >= 8 * groups)
+                                   : cols >= 2 ? groups <= kSlotSmall || held >= 4 * groups : groups <= kSlotSmall / 4 || (dbl && held >= 4 * groups);
+        const auto& p = slots ? slot : col;
+        const uint32_t form = !slots ? 0u : !dbl && !slot.nx && groups > kSlotSmall / 2 ? 2u : 1u;
+        f(i, p.g1, form, p.q[0], p.q[1], p.q[2], p.fixed);
+        i = p.g1;
+    }
+}
 
 // Whether an encoded pass has a gate with a coefficient that is not finite.
 inline bool odd_pass(const GateDesc* d, size_t g0, size_t g1) {

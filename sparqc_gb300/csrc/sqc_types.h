@@ -163,6 +163,9 @@ struct PassArgs {
     // bit (mapped) or qubit (hashed; 64: none) of each dimension
     uint32_t dn, dims, dim[3];
     uint32_t odd;           // 1: a gate is UO_ODD (never in a run)
+    uint32_t slots;         // 1: a slot pass (hashed tables; never in a run): dim holds its cross-group qubits;
+                            // 2: one without any, four slots to a lane (FP32)
+    uint32_t plain;         // slot passes: FP64 products by the FP64 instruction
     UnitHead heads[kMaxRun];   // mapped tables: those of the pass's gates (read from the parameter bank)
 };
 

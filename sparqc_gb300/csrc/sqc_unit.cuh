@@ -531,7 +531,7 @@ __device__ __forceinline__ Slots<T, S> odd_gate(const GateDesc* gd, uint32_t loc
         const bool far = S == 4 && form == 2;
         pp = far ? (x.pm << 2) | (x.pm >> 2) : ((x.pm & 5u) << 1) | ((x.pm >> 1) & 5u);
 #pragma unroll
-        for (int s = 0; s < S; ++s) b[s] = pick(far, x.v[s ^ (S == 4 ? 2 : 1)], x.v[s ^ 1]);
+        for (int s = 0; s < S; ++s) b[s] = S == 1 ? x.v[0] : pick(far, x.v[s ^ (S == 4 ? 2 : S - 1 & 1)], x.v[s ^ (S > 1)]);
     }
     const unsigned any = (x.pm | pp) & act;
 #pragma unroll
@@ -1152,6 +1152,284 @@ __device__ __forceinline__ void walk_hashed_all(const TableDev& t, Ctl* ctl, uns
     const unsigned long long piece = list_piece(n, nw);
     for (unsigned long long e0 = w * piece; e0 < n; e0 += nw * piece)
         walk_hashed<T, ODD>(t, ctl, ep, dm, e0, umin64(e0 + piece, n), wk, sg, gates, ng, lane, pb, cnt_nnz, cnt_empty, upd);
+}
+
+// ---- slot passes over hashed tables ---------------------------------------------------------------
+// A column pass pairs across two qubits. Gates that go back and forth between more of them, the four low ones
+// above all, would take a pass for every few gates; a slot pass takes any number on qubits 0..3 and on up to three
+// cross-group ones. Its units are whole: the 16 slots of each of the 2^nx groups that differ in the cross-group
+// qubits, a lane per slot. The first cross-group qubit is lane bit 4 (without one, a warp holds two units), the
+// next two pair the S = 1, 2 or 4 slots of a lane. Absent slots are run along: the host takes this form
+// where it spares column passes, or where a state is so small that lanes are idle anyway (plan_hashed).
+constexpr int kSlotMembers = 8;   // groups of a unit at most
+struct SlotWork {
+    uint2 m[32][kSlotMembers];    // as HashWork::m
+};
+
+// Op codes that pair the slots of a lane.
+constexpr unsigned long long kSlotLocal = (1ULL << UO_X_PAIR) | (1ULL << UO_Y_PAIR) | (1ULL << UO_H_PAIR) | (1ULL << UO_RX_PAIR) |
+                                          (1ULL << UO_RY_PAIR) | (1ULL << UO_U_PAIR) |
+                                          (1ULL << (UO_PAIR3 + UO_X_PAIR)) | (1ULL << (UO_PAIR3 + UO_Y_PAIR)) |
+                                          (1ULL << (UO_PAIR3 + UO_H_PAIR)) | (1ULL << (UO_PAIR3 + UO_RX_PAIR)) |
+                                          (1ULL << (UO_PAIR3 + UO_RY_PAIR)) | (1ULL << (UO_PAIR3 + UO_U_PAIR)) | (7ULL << UO_ODD);
+
+// The gates of a slot pass on the S slots of a lane; kb is the key of the lane's first slot.
+template <class T, int S, bool ODD>
+__device__ __forceinline__ void run_slots(const HGates<T>& sg, const GateDesc* __restrict__ gates, uint32_t ng, unsigned long long kb,
+                                          int lane, bool on, Slots<T, S>& x, bool& touched, const PruneBits& pb,
+                                          unsigned long long& upd) {
+#pragma unroll 1
+    for (uint32_t gi = 0; gi < ng; ++gi) {
+        const UGate<T>& g = sg.g[gi];
+        upd += (unsigned long long)x.n * g.weight;
+        const bool acts = on && (kb & sg.om[gi]) == sg.ov[gi];
+        // a slot that no acting lane has a key in stays absent, but for gates that pair the slots of a lane
+        unsigned live = 0;
+        if constexpr (S == 1) live = __any_sync(kFull, acts && x.pm) ? 1u : 0u;
+        else live = __reduce_or_sync(kFull, acts ? x.pm : 0u);
+        if (!live) continue;
+        uint32_t loc = g.loc;
+        if (S > 1 && !(kSlotLocal >> (loc >> kLocOp) & 1ULL)) loc &= ~((~live & 15u) << kLocSlots);
+        touched = touched || acts;
+        const GateDesc* gd = gates + gi;
+        const unsigned act = acts ? (loc >> kLocSlots) & 15u : 0u;
+        const uint32_t w = act | (loc & kLocFlip ? 0x80000000u : 0u);            // pairs of slots: the logical bit of the first
+        const uint32_t wl = w ^ (((uint32_t)lane >> ((loc >> kLocBit) & 31u)) << 31);   // pairs of lanes: that of the lane
+        auto ones = [&]() {   // diagonal gates: slots with logical target bit 1
+            const uint32_t word = loc & kLocHigh ? (uint32_t)(kb >> 32) : (uint32_t)kb;
+            const bool at = !(loc & kLocLane) && ((word >> ((loc >> kLocBit) & 31u)) & 1u);
+            return (((loc >> kLocSlotBit) & 15u) ^ (at ? 15u : 0u)) & act;
+        };
+        switch (loc >> kLocOp) {
+        case UO_X_SHFL: swap_shfl<T, KX, S, false>(loc, wl, x); break;
+        case UO_Y_SHFL: swap_shfl<T, KY, S, false>(loc, wl, x); break;
+        case UO_H_SHFL: branch_shfl<T, KH, S, false>(g, gd, loc, wl, x, pb); break;
+        case UO_RX_SHFL: branch_shfl<T, KRX, S, false>(g, gd, loc, wl, x, pb); break;
+        case UO_RY_SHFL: branch_shfl<T, KRY, S, false>(g, gd, loc, wl, x, pb); break;
+        case UO_U_SHFL: branch_shfl<T, KU, S, false>(g, gd, loc, wl, x, pb); break;
+        case UO_Z: diag<T, KZ, S>(g, ones(), act, x); break;
+        case UO_S: diag<T, KS, S>(g, ones(), act, x); break;
+        case UO_SDG: diag<T, KSDG, S>(g, ones(), act, x); break;
+        case UO_YPH: diag<T, KYPH, S>(g, ones(), act, x); break;
+        case UO_RZ: diag<T, KRZ, S>(g, ones(), act, x); break;
+        case UO_PHASE: diag<T, KPHASE, S>(g, ones(), act, x); break;
+        default:
+            if constexpr (ODD)
+                if (loc >> kLocOp >= UO_ODD) {
+                    x = odd_gate<T, S>(gd, loc, loc >> kLocOp == UO_ODD + 1 ? wl : w, ones(), x, pb);
+                    break;
+                }
+            if constexpr (S > 1) {
+                switch (loc >> kLocOp) {
+                case UO_X_PAIR: swap_pair<T, KX, S, 1, false>(w, x); break;
+                case UO_Y_PAIR: swap_pair<T, KY, S, 1, false>(w, x); break;
+                case UO_H_PAIR: branch_pair<T, KH, S, 1, false>(g, gd, w, x, pb); break;
+                case UO_RX_PAIR: branch_pair<T, KRX, S, 1, false>(g, gd, w, x, pb); break;
+                case UO_RY_PAIR: branch_pair<T, KRY, S, 1, false>(g, gd, w, x, pb); break;
+                case UO_U_PAIR: branch_pair<T, KU, S, 1, false>(g, gd, w, x, pb); break;
+                default:
+                    if constexpr (S == 4) {
+                        switch (loc >> kLocOp) {
+                        case UO_PAIR3 + UO_X_PAIR: swap_pair<T, KX, S, 2, false>(w, x); break;
+                        case UO_PAIR3 + UO_Y_PAIR: swap_pair<T, KY, S, 2, false>(w, x); break;
+                        case UO_PAIR3 + UO_H_PAIR: branch_pair<T, KH, S, 2, false>(g, gd, w, x, pb); break;
+                        case UO_PAIR3 + UO_RX_PAIR: branch_pair<T, KRX, S, 2, false>(g, gd, w, x, pb); break;
+                        case UO_PAIR3 + UO_RY_PAIR: branch_pair<T, KRY, S, 2, false>(g, gd, w, x, pb); break;
+                        case UO_PAIR3 + UO_U_PAIR: branch_pair<T, KU, S, 2, false>(g, gd, w, x, pb); break;
+                        default: __builtin_unreachable();
+                        }
+                    } else {
+                        __builtin_unreachable();
+                    }
+                }
+            } else {
+                __builtin_unreachable();
+            }
+        }
+    }
+}
+
+// The units of list entries [e0, e1) (at most 32) of a pass with cross-group bits gm (nx of them, S = 1 for
+// nx <= 1, else 2^(nx - 1)).
+template <class T, int S, bool ODD>
+__device__ __forceinline__ void walk_slots(const TableDev& t, Ctl* ctl, unsigned ep, const unsigned long long (&gm)[3], uint32_t nx,
+                                           unsigned long long e0, unsigned long long e1, SlotWork& wk, const HGates<T>& sg,
+                                           const GateDesc* gates, uint32_t ng, int lane, const PruneBits& pb,
+                                           unsigned long long& cnt_nnz, unsigned long long& cnt_empty, unsigned long long& upd) {
+    auto member = [&](unsigned long long G0, int k) {
+        return G0 | ((k & 1) ? gm[0] : 0ULL) | ((k & 2) ? gm[1] : 0ULL) | ((k & 4) ? gm[2] : 0ULL);
+    };
+    // a lane per entry: its unit's members, and whether it owns the unit (as in walk_hashed)
+    unsigned long long base = 0;
+    bool owns = false;
+    if (e0 + lane < e1) {
+        const unsigned b = __ldcg(t.list + e0 + lane);   // (an earlier pass of the same launch may have written it)
+        const Header own = load_hdr_cg(t.hdr + b);
+        const int idx = ((own.group & gm[0]) ? 1 : 0) | ((own.group & gm[1]) ? 2 : 0) | ((own.group & gm[2]) ? 4 : 0);
+        base = own.group & ~(gm[0] | gm[1] | gm[2]);
+        owns = true;
+        constexpr int kMost = S == 1 ? 2 : 2 * S;
+        Header h[kMost];
+        unsigned at[kMost];
+#pragma unroll
+        for (int k = 0; k < kMost; ++k) {   // the first probes of all members together
+            h[k].epoch = ep + 1;
+            at[k] = b;
+            if (k != idx && k < (1 << nx)) {
+                at[k] = (unsigned)(mix64(member(base, k)) & t.mask);
+                h[k] = load_hdr_cg(t.hdr + at[k]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kMost; ++k) {
+            uint2 m = make_uint2(kNoBucket, 0u);
+            if (k == idx) {
+                m = make_uint2(b, own.aux);
+            } else if (h[k].epoch == ep) {
+                const unsigned long long G = member(base, k);
+                Header c = h[k];
+                unsigned long long p = at[k];
+                for (uint32_t i = 1; i < kMaxProbe && c.epoch == ep && c.group != G; ++i) {
+                    p = (p + 1) & t.mask;
+                    c = load_hdr_cg(t.hdr + p);
+                }
+                if (c.epoch == ep && c.group == G) {
+                    m = make_uint2((unsigned)p, c.aux);
+                    if (k < idx) owns = false;
+                }
+            }
+            wk.m[lane][k] = m;
+        }
+    }
+    unsigned todo = __ballot_sync(kFull, owns);
+    __syncwarp();
+    const int half = lane >> 4, j = lane & 15;
+    while (todo) {
+        int l = __ffs(todo) - 1;   // the unit of the lane's half, or of the warp
+        todo &= todo - 1;
+        bool on = true;
+        if (S == 1 && nx == 0) {
+            const int second = todo ? __ffs(todo) - 1 : -1;
+            todo &= todo - 1;
+            on = half == 0 || second >= 0;
+            if (half && on) l = second;
+        }
+        const unsigned long long G0 = member(shfl64(base, l), S == 1 && nx == 0 ? 0 : half);
+        uint2 m[S];
+        Slots<T, S> x;
+        x.pm = 0;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            m[s] = on ? wk.m[l][(S == 1 && nx == 0 ? 0 : half) | (s << 1)] : make_uint2(kNoBucket, 0u);
+            const bool p = (m[s].y >> j) & 1u;
+            x.pm |= (unsigned)p << s;
+            x.v[s] = czero<T>();
+            if (p) {
+                const typename AmpT<T>::V a = __ldcg(reinterpret_cast<const typename AmpT<T>::V*>(t.amps) + (size_t)m[s].x * kSlots + j);
+                x.v[s] = Cx<T>{a.x, a.y};
+            }
+        }
+        bool touched = false;
+        const unsigned pm0 = x.pm;
+        x.n = __popc(pm0);
+        run_slots<T, S, ODD>(sg, gates, ng, (G0 << kSlotBits) | (unsigned)j, lane, on, x, touched, pb, upd);
+        const unsigned pm = x.pm;
+        cnt_nnz += __popc(pm);
+        // groups that appear, all claimed together: member s of a half by its lane s
+        unsigned now[S];
+        bool make = false;
+        unsigned long long mine = 0;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const unsigned bal = __ballot_sync(kFull, (pm >> s) & 1u);
+            now[s] = half ? bal >> 16 : bal & 0xFFFFu;
+            if (j == s) {
+                make = on && m[s].x == kNoBucket && now[s] != 0;
+                mine = member(G0, s << 1);
+            }
+        }
+        unsigned nb = kNoBucket;
+        if (__any_sync(kFull, make)) {
+            bool created = false;
+            if (make) {
+                const long long c = claim_group(t, ep, mine, &ctl->status, &created);
+                if (c >= 0) nb = (unsigned)c;
+            }
+            __syncwarp();
+            const unsigned got = __ballot_sync(kFull, created);
+            unsigned long long at = 0;
+            if (lane == 0 && got) at = atomicAdd(&ctl->list_tail, (unsigned long long)__popc(got));
+            at = shfl64(at, 0) + __popc(got & ((1u << lane) - 1u));
+            if (created) t.list[at] = nb;
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const unsigned made = __shfl_sync(kFull, nb, (lane & 16) | s);
+            const bool fresh = m[s].x == kNoBucket;
+            const unsigned b = fresh ? made : m[s].x;
+            if (b == kNoBucket) continue;   // absent, or the table is full: the pass has failed
+            const bool p = (pm >> s) & 1u, moved = ((pm ^ pm0) >> s) & 1u;
+            const size_t at = (size_t)b * kSlots + j;
+            if (p && (touched || moved)) store_amp<T>(t.amps, at, x.v[s]);
+            if (fresh || moved) t.keys[at] = p ? (member(G0, s << 1) << kSlotBits) | (unsigned)j : empty_key(j);
+            if (j == 0 && (fresh || now[s] != m[s].y)) t.hdr[b].aux = now[s];
+            if (j == 0 && now[s] == 0) cnt_empty += 1;
+        }
+    }
+    __syncwarp();
+}
+
+// The list entries [e0, e1) of a slot pass without cross-group qubits, four slots to a lane: qubits 0 and 1 in a
+// lane, 2 and 3 lane bits 0 and 1, eight groups to a warp. Decoding a gate then serves four slots. FP32 passes
+// over many groups are bound by that (2^16 groups of 16 keys, 24 gates: 108 us with a slot to a lane); FP64 ones
+// by the products, and small ones by the chain of a lane's slots.
+template <class T, bool ODD>
+__device__ __forceinline__ void walk_low(const TableDev& t, unsigned long long e0, unsigned long long e1, const HGates<T>& sg,
+                                         const GateDesc* gates, uint32_t ng, int lane, const PruneBits& pb,
+                                         unsigned long long& cnt_nnz, unsigned long long& cnt_empty, unsigned long long& upd) {
+    const int quarter = (lane & 3) * 4;
+    for (unsigned long long e = e0 + (lane >> 2); __any_sync(kFull, e < e1); e += 8) {
+        const bool on = e < e1;
+        unsigned b = 0;
+        Header h;
+        h.group = 0;
+        h.aux = 0;
+        if (on) {
+            b = __ldcg(t.list + e);   // (an earlier pass of the same launch may have written it)
+            h = load_hdr_cg(t.hdr + b);
+        }
+        const size_t at = (size_t)b * kSlots + quarter;
+        Slots<T, 4> x;
+        x.pm = (h.aux >> quarter) & 15u;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            x.v[s] = czero<T>();
+            if ((x.pm >> s) & 1u) {
+                const typename AmpT<T>::V a = __ldcg(reinterpret_cast<const typename AmpT<T>::V*>(t.amps) + at + s);
+                x.v[s] = Cx<T>{a.x, a.y};
+            }
+        }
+        bool touched = false;
+        const unsigned pm0 = x.pm;
+        x.n = __popc(pm0);
+        run_slots<T, 4, ODD>(sg, gates, ng, (h.group << kSlotBits) | (unsigned)quarter, lane, on, x, touched, pb, upd);
+        const unsigned pm = x.pm;
+        cnt_nnz += __popc(pm);
+        unsigned now = pm << quarter;
+        now |= __shfl_xor_sync(kFull, now, 1);
+        now |= __shfl_xor_sync(kFull, now, 2);
+        if (!on) continue;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const bool p = (pm >> s) & 1u, moved = ((pm ^ pm0) >> s) & 1u;
+            if (p && (touched || moved)) store_amp<T>(t.amps, at + s, x.v[s]);
+            if (moved) t.keys[at + s] = p ? (h.group << kSlotBits) | (unsigned)(quarter + s) : empty_key(quarter + s);
+        }
+        if (quarter == 0) {
+            if (now != h.aux) t.hdr[b].aux = now;
+            if (now == 0) cnt_empty += 1;
+        }
+    }
 }
 
 }  // namespace

@@ -485,3 +485,62 @@ def test_comparing_states_on_different_bits(precision):
     assert same[0] > 1 - 1e-6 and same[1] == 0.0
     assert apart[0] == 0.0 and apart[1] > 0.0
     assert t_apart < 16 * t_same
+
+
+def _slot_gates(cross, seed, n=40):
+    """Gates that go back and forth between the four low qubits and `cross` others, controls and phases anywhere."""
+    c = circuits.SplitMix64(circuits.stream_seed("slots", seed))
+    pick = lambda k: c.next() % k
+    pairing = [0, 1, 2, 3] + [20, 47, 5][:cross]
+    gs = []
+    for i in range(n):
+        group = KINDS[pick(3)]
+        diag = group is KINDS[0]
+        t = pick(64) if diag else pairing[pick(len(pairing))] if i >= len(pairing) else pairing[i]
+        ctl = tuple({q for q in [pick(4), pick(64), pairing[pick(len(pairing))], 63][: pick(5)] if q != t})
+        gs.append((group[pick(len(group))], t, ctl, 0.3 + 0.1 * i, 0.2, 0.7))
+    return G.gate_array(gs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("cross", [0, 1, 2, 3])
+@pytest.mark.parametrize("groups,per", [(1, 1), (1, 16), (31, 5), (33, 16), (700, 1), (3000, 12)])
+def test_slot_passes(groups, per, cross, precision):
+    """Hashed tables, gates on the low qubits and up to three others in turns: units of one to eight groups, one
+    to eight of them to a warp, with groups that appear and that empty; few passes for many gates."""
+    from sparqc_gb300.engine import State
+    rng = np.random.default_rng(groups * 100 + per)
+    g = np.unique(rng.integers(0, 1 << 59, groups, dtype=np.uint64)) * np.uint64(2) + np.uint64(1)
+    key = (g[:, None] << np.uint64(4)) + rng.permuted(np.tile(np.arange(16, dtype=np.uint64), (g.size, 1)), axis=1)[:, :per]
+    key = np.unique(np.concatenate([key.ravel(), np.array([0, 0xFFFFFFFFFFFFFFFF], np.uint64)]))
+    amp = rng.standard_normal((2, key.size))
+    gs = _slot_gates(cross, cross + groups)
+    _both(64, gs, precision, init=(key, amp[0], amp[1]))
+    st = State(64, precision=precision)
+    st.set_state(key, amp[0], amp[1])
+    st.apply(gs)
+    st.sync()
+    assert st.stats()["passes"] <= (1 if cross <= 2 or precision == 32 else 40)
+    st.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+def test_slot_passes_that_empty_groups_and_odd_angles(precision):
+    """A slot pass that moves every key of a group away, one with NaN angles in lanes and slots."""
+    key = (np.arange(200, dtype=np.uint64) * np.uint64(0x9E3779B97F4A7C15)) | np.uint64(1 << 20)
+    key = np.unique(key)
+    amp = np.random.default_rng(2).standard_normal((2, key.size))
+    move = [(G.X, 20, (q,)) for q in range(4)] + [(k, q, (20,)) for k in (G.Y, G.X) for q in range(4)] + [(G.X, 20, (63,)), (G.RY, 2), (G.RX, 1)]
+    _both(64, G.gate_array(move), precision, init=(key, amp[0], amp[1]))
+    from sparqc_gb300.engine import State
+    odd = [(G.RX, q, (33,), np.nan) for q in (0, 3, 20)] + [(G.U, 2, (40,), 0.4, np.inf, 0.1), (G.RZ, 3, (41,), np.nan), (G.U, 1, (50,), 0.4, 0.1, np.nan)]
+    gs = G.gate_array([(G.H, 0), (G.RY, 1, (), 0.4)] + odd + [(G.H, q) for q in (3, 2, 20, 1, 0)])
+    st, o = State(64, precision=precision), SparseOracle(precision)
+    st.set_state(key, amp[0], amp[1])
+    o.set_state(key, amp[0], amp[1])
+    st.apply(gs)
+    o.apply(gs)
+    _same(st.state(sorted=True), o.state(sorted=True))
+    st.close()
