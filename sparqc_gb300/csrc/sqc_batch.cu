@@ -44,10 +44,10 @@ __device__ __forceinline__ UnitPass units_of(const BPass& p) {
     return unit_pass<DIMS>(p.dn, p.dim[0], p.dim[1], p.dim[2]);
 }
 
-// Items of a pass: its units, or the list 32 entries at a time (walk_list).
+// Items of a pass: its units, or the list's entries (walk_list).
 template <int DIMS>
 __device__ __forceinline__ unsigned long long pass_items(const BPass& p, unsigned long long list_n) {
-    if (walk_list(list_n, p.dn)) return (list_n + 31) / 32;
+    if (walk_list(list_n, p.dn)) return list_n;
     return units_of<DIMS>(p).units;
 }
 __device__ __forceinline__ unsigned long long pass_items(const BPass& p, unsigned long long list_n, bool dbl) {
@@ -55,17 +55,25 @@ __device__ __forceinline__ unsigned long long pass_items(const BPass& p, unsigne
 }
 
 // Chunking of a pass over n items while `running` circuits share the GPU: items per chunk and the
-// chunk count. A chunk gives every warp of its block at least min_chunk's list entries (four to an
-// item); a pass has at most target_chunks chunks shared among the running circuits, but up to
-// kBusyChunks, so that a large circuit's passes still spread when many run (256 circuits, FP32:
-// 10.7 ms with the smallest chunks for all, 7.3 with four times as many entries).
-__device__ __forceinline__ void chunking(const BatchArgs& a, unsigned long long n, unsigned running, unsigned* chunk,
+// chunk count. A pass has at most target_chunks chunks shared among the running circuits. A chunk of units gives
+// every warp of its block at least min_chunk / 4 of them, and a pass of units up to kBusyChunks chunks, so that a large
+// circuit's passes still spread when many run (256 circuits, FP32: 10.7 ms with the smallest chunks
+// for all, 7.3 with four times as many entries). A chunk of list entries, whose units follow one another in a
+// warp, is at least min_chunk of them and a warp's share at most 32.
+__device__ __forceinline__ void chunking(const BatchArgs& a, unsigned long long n, bool list, unsigned running, unsigned* chunk,
                                          unsigned* total) {
     const unsigned share = a.target_chunks / (running ? running : 1u);
-    const unsigned target = share > kBusyChunks ? share : kBusyChunks;
-    unsigned long long c = (n + target - 1) / target;
-    const unsigned least = a.min_chunk / 4 * kBatchWarps;
-    if (c < least) c = least;
+    unsigned long long c;
+    if (list) {
+        c = share ? (n + share - 1) / share : n;
+        if (c > 32u * kBatchWarps) c = 32u * kBatchWarps;
+        if (c < a.min_chunk) c = a.min_chunk;
+    } else {
+        const unsigned target = share > kBusyChunks ? share : kBusyChunks;
+        c = (n + target - 1) / target;
+        const unsigned least = a.min_chunk / 4 * kBatchWarps;
+        if (c < least) c = least;
+    }
     *chunk = (unsigned)c;
     const unsigned long long t = (n + c - 1) / c;
     *total = (unsigned)(t ? t : 1);
@@ -114,7 +122,7 @@ __device__ __noinline__ bool finish_circuit_pass(const BatchArgs& a, unsigned c,
         atomicCAS(&ctl->status, 0u, (unsigned)ST_GROW);
         state = BS_FAILED;
     } else {
-        chunking(a, pass_items(nxp, n, a.amp_bytes == 16), *(volatile unsigned int*)&a.bctl->left, &chunk, &total);
+        chunking(a, pass_items(nxp, n, a.amp_bytes == 16), walk_list(n, nxp.dn), *(volatile unsigned int*)&a.bctl->left, &chunk, &total);
         if (next >= limit || (dl && globaltimer() > dl)) state = BS_PARKED;
     }
     const bool run = state == BS_RUN;
@@ -239,8 +247,10 @@ __global__ void __launch_bounds__(kBatchThreads, MINB) batch_run_kernel(BatchArg
         const uint32_t ng = bp.g1 - bp.g0;
         unsigned long long cnt_nnz = 0, cnt_empty = 0, upd = 0;
         if (walk_list(n, bp.dn)) {
-            for (unsigned long long i = ib + w; i < ie; i += kBatchWarps)
-                walk_entries<T, DIMS>(t, C.t.map_q, ctl, ep, up, i * 32, n, SharedHeads<T, MINB == 1>{sg.g}, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
+            const unsigned per = (unsigned)(ie - ib + kBatchWarps - 1) / kBatchWarps;   // as many to every warp
+            const unsigned long long we = umin64(ib + (w + 1) * per, ie);
+            for (unsigned long long e = ib + w * per; e < we; e += 32)
+                walk_entries<T, DIMS>(t, C.t.map_q, ctl, ep, up, e, umin64(e + 32, we), SharedHeads<T, MINB == 1>{sg.g}, sg, gates, ng, lane, a.prune, cnt_nnz, cnt_empty, upd);
         } else {
             walk_units<T, DIMS>(t, C.t.map_q, ctl, ep, up, (unsigned)(ib + w), (unsigned)ie, kBatchWarps, SharedHeads<T, MINB == 1>{sg.g}, sg, gates, ng, lane, a.prune, cnt_nnz,
                              cnt_empty, upd);
@@ -335,7 +345,8 @@ __global__ void batch_begin_kernel(BatchArgs a, unsigned long long deadline_ns) 
                 s->limit = lim;
                 s->done = 0;
                 unsigned chunk, total;
-                chunking(a, C.npasses ? pass_items(C.passes[0], 1, a.amp_bytes == 16) : 1, a.n, &chunk, &total);
+                chunking(a, C.npasses ? pass_items(C.passes[0], 1, a.amp_bytes == 16) : 1, C.npasses && walk_list(1, C.passes[0].dn), a.n,
+                         &chunk, &total);
                 s->chunk = chunk;
                 s->next_total = total;
                 const bool run = b >= 0 && C.npasses > 0 && lim > 0;

@@ -544,3 +544,46 @@ def test_slot_passes_that_empty_groups_and_odd_angles(precision):
     o.apply(gs)
     _same(st.state(sorted=True), o.state(sorted=True))
     st.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+def test_a_thin_circuit_of_a_batch_spreads_over_warps(precision):
+    """A circuit whose passes walk their list takes a batch about as long as a state of its own (three times it
+    at most; a warp for every 32 entries takes six times it)."""
+    import time
+    from sparqc_gb300.engine import Batch, State
+    c = circuits.SplitMix64(circuits.stream_seed("thin-batch"))
+    gs = [(G.H, q) for q in range(9)] + [(G.X, 9 + i, (i % 9, (i + 4) % 9)[: 1 + i % 2]) for i in range(14)]
+    for j in range(120):
+        t, a, b = 9 + c.next() % 14, c.next() % 23, c.next() % 23
+        gs.append((G.X, t, tuple({q for q in (a, b) if q != t})) if j % 4 else (G.RZ, t, tuple({a} - {t}), 0.3))
+    gs = G.gate_array(gs)
+    o = SparseOracle(precision)
+    o.apply(gs)
+    b = Batch(precision=precision)
+    b.prepare([(40, gs)])
+    st = State(40, precision=precision, initial_buckets=1 << 17)   # mapped, as the batch's slice
+
+    def best(f):
+        t = []
+        for _ in range(7):
+            t0 = time.perf_counter()
+            f()
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    def alone():
+        st.set_zero()
+        st.apply(gs)
+        st.sync()
+
+    def batch():
+        b.run()
+        b.sync()
+
+    t_alone, t_batch = best(alone), best(batch)
+    assert_identical(b.state(0), o.state(sorted=True))
+    assert t_batch < 3 * t_alone, (t_batch, t_alone)
+    b.close()
+    st.close()
