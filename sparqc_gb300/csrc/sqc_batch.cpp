@@ -102,6 +102,18 @@ const char* plan_circuit(uint32_t nq, const sqc_gate* gates, uint64_t n, uint32_
     return nullptr;
 }
 
+void sort_by_key(uint64_t* keys, double* re, double* im, uint64_t n) {
+    std::vector<uint64_t> idx(n), k(keys, keys + n);
+    std::vector<double> r(re, re + n), m(im, im + n);
+    std::iota(idx.begin(), idx.end(), (uint64_t)0);
+    std::sort(idx.begin(), idx.end(), [&](uint64_t x, uint64_t y) { return k[x] < k[y]; });
+    for (uint64_t i = 0; i < n; ++i) {
+        keys[i] = k[idx[i]];
+        re[i] = r[idx[i]];
+        im[i] = m[idx[i]];
+    }
+}
+
 Batch::~Batch() {
     if (stream_) cudaStreamSynchronize(stream_);
     drop_graph();
@@ -497,13 +509,21 @@ int Batch::get_state(uint32_t i, uint64_t* keys, double* re, double* im, uint64_
     const unsigned long long have = h_ctl_[i].nnz;
     if ((rc = ensure_readout(have))) return rc;
     Ctl* ctl = d_ctl_ + i;
-    const RankJob job = rank_job(tables_[i], ctl, plans_[i].end.frame, 0, 0);
-    if ((rc = cuda(rank_.need(job.tiles(), 0), "cudaMalloc(readout)")) ||
-        (rc = cuda(launch_ranked(job, nullptr, 1, job.tiles(), rank_.tiles, dbl_, d_rk_, d_rr_, d_ri_, rcap_,
-                                 (flags & SQC_READ_DROP_NEGLIGIBLE) != 0, prune_, &ctl->out_count, nullptr, stream_),
-                   "readout")))
+    const bool drop = (flags & SQC_READ_DROP_NEGLIGIBLE) != 0, ranked = rank_worth_unsorted(tables_[i].map_n, have);
+    if (ranked) {
+        const RankJob job = rank_job(tables_[i], ctl, plans_[i].end.frame, 0, 0);
+        if ((rc = cuda(rank_.need(job.tiles(), 0), "cudaMalloc(readout)")) ||
+            (rc = cuda(launch_ranked(job, nullptr, 1, job.tiles(), rank_.tiles, dbl_, d_rk_, d_rr_, d_ri_, rcap_, drop, prune_,
+                                     &ctl->out_count, nullptr, stream_),
+                       "readout")))
+            return rc;
+    } else if ((rc = cuda(cudaMemsetAsync(&ctl->out_count, 0, sizeof(unsigned long long), stream_), "memset")) ||
+               (rc = cuda(launch_readout(tables_[i], ctl, std::max<unsigned long long>(h_ctl_[i].list_n, 1), plans_[i].end.frame,
+                                         dbl_, d_rk_, d_rr_, d_ri_, rcap_, drop, prune_, sms_, stream_),
+                          "readout"))) {
         return rc;
-    launches_ += 3;
+    }
+    launches_ += ranked ? 3 : 1;
     unsigned long long got = 0;
     if ((rc = cuda(cudaMemcpyAsync(&got, &ctl->out_count, sizeof got, cudaMemcpyDeviceToHost, stream_), "D2H")) ||
         (rc = cuda(cudaStreamSynchronize(stream_), "sync")))
@@ -518,7 +538,8 @@ int Batch::get_state(uint32_t i, uint64_t* keys, double* re, double* im, uint64_
             (rc = cuda(cudaStreamSynchronize(stream_), "sync")))
             return rc;
     }
-    return SQC_OK;   // in key order, asked for or not
+    if (!ranked && (flags & SQC_READ_SORTED)) sort_by_key(keys, re, im, got);   // (a ranked one is in key order)
+    return SQC_OK;
 }
 
 int Batch::table_of(uint32_t i, TableDev* t, const Ctl** ctl, unsigned long long* hint, unsigned long long* frame,

@@ -50,6 +50,8 @@ struct CircuitPlan {
 // max_nx: cross-group qubits of a pass at most; dims: dimensions of the batch kernel's units.
 const char* plan_circuit(uint32_t nq, const sqc_gate* gates, uint64_t n, uint32_t max_run, uint32_t max_nx,
                          uint32_t dims, CircuitPlan* out);
+// Entries of a readout by key, on the host.
+void sort_by_key(uint64_t* keys, double* re, double* im, uint64_t n);
 // Dimensions of the batch kernel's units: three in FP32, two in FP64 (whose slots are twice as large).
 constexpr uint32_t kBatchDims64 = 2, kBatchDims32 = 3;
 inline uint32_t batch_dims(bool dbl) { return dbl ? kBatchDims64 : kBatchDims32; }

@@ -35,6 +35,12 @@ inline bool rank_worth(uint32_t n, unsigned long long nnz) {
     return (1ULL << n) <= (1ULL << 22) || (1ULL << n) <= 16 * nnz;
 }
 
+// The same for the batch's and the server's tables, whose list readouts are sorted on the host (one circuit of 600
+// keys, FP64: 2^18 headers 75 us, 2^20 93, by the list 76).
+inline bool rank_worth_unsorted(uint32_t n, unsigned long long nnz) {
+    return (1ULL << n) <= (1ULL << 18) || (1ULL << n) <= 256 * nnz;
+}
+
 // Device scratch of ranked readouts, grown as needed: a count per tile, and for several jobs the
 // jobs, their counts and the total.
 struct RankScratch {

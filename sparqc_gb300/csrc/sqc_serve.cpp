@@ -520,13 +520,21 @@ int Server::get_state(uint64_t id, uint64_t* keys, double* re, double* im, uint6
         rcap_ = c;
     }
     Ctl* ctl = d_ctl_ + r.slot;
-    const RankJob job = rank_job(r.table, ctl, r.plan.end.frame, 0, 0);
-    if ((rc = cuda(rank_.need(job.tiles(), 0), "cudaMalloc(readout)")) ||
-        (rc = cuda(launch_ranked(job, nullptr, 1, job.tiles(), rank_.tiles, dbl_, d_rk_, d_rr_, d_ri_, rcap_,
-                                 (flags & SQC_READ_DROP_NEGLIGIBLE) != 0, prune_, &ctl->out_count, nullptr, stream_),
-                   "readout")))
+    const bool drop = (flags & SQC_READ_DROP_NEGLIGIBLE) != 0, ranked = rank_worth_unsorted(r.table.map_n, have);
+    if (ranked) {
+        const RankJob job = rank_job(r.table, ctl, r.plan.end.frame, 0, 0);
+        if ((rc = cuda(rank_.need(job.tiles(), 0), "cudaMalloc(readout)")) ||
+            (rc = cuda(launch_ranked(job, nullptr, 1, job.tiles(), rank_.tiles, dbl_, d_rk_, d_rr_, d_ri_, rcap_, drop, prune_,
+                                     &ctl->out_count, nullptr, stream_),
+                       "readout")))
+            return rc;
+    } else if ((rc = cuda(cudaMemsetAsync(&ctl->out_count, 0, sizeof(unsigned long long), stream_), "memset")) ||
+               (rc = cuda(launch_readout(r.table, ctl, std::max<unsigned long long>(r.ctl.list_n, 1), r.plan.end.frame, dbl_, d_rk_,
+                                         d_rr_, d_ri_, rcap_, drop, prune_, sms_, stream_),
+                          "readout"))) {
         return rc;
-    launches_ += 3;
+    }
+    launches_ += ranked ? 3 : 1;
     unsigned long long got = 0;
     if ((rc = cuda(cudaMemcpyAsync(&got, &ctl->out_count, sizeof got, cudaMemcpyDeviceToHost, stream_), "D2H")) ||
         (rc = cuda(cudaStreamSynchronize(stream_), "sync")))
@@ -541,7 +549,8 @@ int Server::get_state(uint64_t id, uint64_t* keys, double* re, double* im, uint6
             (rc = cuda(cudaStreamSynchronize(stream_), "sync")))
             return rc;
     }
-    return SQC_OK;   // in key order, asked for or not
+    if (!ranked && (flags & SQC_READ_SORTED)) sort_by_key(keys, re, im, got);   // (a ranked one is in key order)
+    return SQC_OK;
 }
 
 int Server::table_of(uint64_t id, TableDev* t, const Ctl** ctl, unsigned long long* hint, unsigned long long* frame,

@@ -587,3 +587,33 @@ def test_a_thin_circuit_of_a_batch_spreads_over_warps(precision):
     assert t_batch < 3 * t_alone, (t_batch, t_alone)
     b.close()
     st.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+def test_readouts_of_thin_circuits_go_by_the_list(precision):
+    """A few keys among 2^20 mapped groups: a batch's and a server's readout visits the live buckets in one
+    launch, in key order when asked; with more keys, or fewer groups, it stays the ranked one (three)."""
+    from sparqc_gb300.engine import Batch, Server
+    thin = G.gate_array([(G.H, q) for q in range(4)] + [(G.X, 4 + i, (i % 4,)) for i in range(20)] + [(G.X, 7), (G.Y, 2)])
+    dense = G.gate_array([(G.H, q) for q in range(9)])
+    b, sv = Batch(precision=precision), Server(precision=precision, memory_budget=4 << 30)
+    b.prepare([(40, thin), (40, dense)])
+    b.run()
+    b.sync()
+    ids = [sv.submit(40, g) for g in (thin, dense)]
+    while any(sv.status(r)[0] != 2 for r in ids):
+        sv.step()
+    for i, (g, launches) in enumerate(((thin, 1), (dense, 3))):
+        o = SparseOracle(precision)
+        o.apply(g)
+        want = o.state(sorted=True)
+        for read, stats in ((lambda **k: b.state(i, **k), b.stats), (lambda **k: sv.state(ids[i], **k), sv.stats)):
+            before = stats()["kernel_launches"]
+            assert_identical(read(sorted=True), want)
+            assert stats()["kernel_launches"] == before + launches
+            got = read(sorted=False)
+            order = np.argsort(got[0])
+            assert_identical(tuple(x[order] for x in got), want)
+    b.close()
+    sv.close()
