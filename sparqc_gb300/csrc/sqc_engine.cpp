@@ -545,14 +545,18 @@ int Engine::flush(bool hold_last) {
         // consecutive passes of a small or middle state go out in one launch, up to one that the table is
         // known or may turn out to be too small for
         size_t e = s, words = 0;
-        unsigned long long items = list_hint_;
+        unsigned long long items = mapped_ ? 1 : list_hint_, live = list_hint_;
         while (!time_passes_ && e < spans.size()) {
             const Span& r = spans[e];
             const size_t w = mapped_ ? 1 + r.g1 - r.g0 : 2;
             if (words + w > kRunWords || r.slots || odd_pass(hd, r.g0, r.g1)) break;
             if (mapped_) {
                 if (r.dn > (dbl_ ? kRunMapFp64 : kRunMapFp32) || (1ULL << r.dn) > a.max_groups) break;
-                items = std::max(1ULL, (1ULL << r.dn) >> dims);
+                // a pass that is sure to walk its list needs no more warps than entries: a thin state's run then
+                // leaves the rest of the GPU to other streams, and its blocks meet sooner
+                if (r.nx) live = std::min({group_bound(after[r.g1 - 1], nq_), live << r.nx, live + r.keys});
+                const unsigned long long units = std::max(1ULL, (1ULL << r.dn) >> dims);
+                items = std::max(items, r.dn >= 6 && live < (1ULL << (r.dn - 3)) ? live : units);
             } else if (r.nx) {
                 const unsigned long long h = std::min({group_bound(after[r.g1 - 1], nq_), items << r.nx, items + r.keys});
                 if (h > roomy_groups() || h > kRunMaxList) break;

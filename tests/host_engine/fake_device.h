@@ -38,6 +38,7 @@ struct Device {
     long bad = 0;                                // accesses outside an allocation, misuse of events
     cudaError_t last = cudaSuccess;              // what cudaGetLastError answers, once
     long syncs = 0, passes = 0, runs = 0;
+    unsigned long long items = 0;                // most items a run was launched for
     bool capturing = false;
     std::vector<long> events;                    // time of each event's last record, 0: never
     long now = 0;
@@ -300,8 +301,9 @@ int launch_hash_pass(const PassArgs& a, unsigned long long, bool, int, cudaStrea
     fake::pass(a.ctl, a.gates, a.g0, a.g1, a.prune, overflow(a.ctl->list_n, a.nx, a.grow_bound, a.key_bound, a.max_groups));
     return 1;
 }
-int launch_run_passes(const RunArgs& a, uint32_t, unsigned long long, bool, int, cudaStream_t) {
+int launch_run_passes(const RunArgs& a, uint32_t, unsigned long long items, bool, int, cudaStream_t) {
     ++fake::dev.runs;
+    fake::dev.items = std::max(fake::dev.items, items);
     uint32_t o = 0;
     for (uint32_t p = 0; p < a.np; ++p) {
         const UnitHead r = a.words[o];

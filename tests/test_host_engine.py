@@ -333,3 +333,24 @@ def test_thin_maps_take_a_share_of_the_device(engine_objects, tmp_path):
     std::printf("bytes %llu peak %zu\\n", (unsigned long long)st.table_bytes, dev.peak);
     CHECK(st.table_bytes <= dev.total / 8 && dev.peak <= dev.total / 2);
     """)
+
+
+def test_runs_of_thin_mapped_states_take_few_blocks(engine_objects, tmp_path):
+    """A run whose passes walk the list is launched for the live buckets there can be, not for every unit of
+    the map; one whose passes walk the units for those."""
+    run(engine_objects, tmp_path, """
+    sqc_options o;
+    sqc_default_options(&o);
+    o.initial_buckets = 1 << 18;
+    for (uint32_t k : {4u, 14u}) {   // keys: 2^4, or 2^14 that fill the map
+        Engine e;
+        make(e, 40, &o);
+        dev.items = 0;
+        std::vector<sqc_gate> g;
+        for (uint32_t q = 0; q < k; ++q) g.push_back(gate(KH, 4 + q));
+        for (uint32_t q = k; q < 14; ++q) g.push_back(gate(KX, 4 + q, 1ULL << (4 + q % k)));
+        CHECK(e.apply(g.data(), g.size()) == SQC_OK && e.sync() == SQC_OK);
+        CHECK(dev.items == (k == 4 ? 16u * 6u : 1u << 12));
+        CHECK(holds(e, expected(g)));
+    }
+    """)
