@@ -463,6 +463,13 @@ int Batch::get_states(uint64_t* keys, double* re, double* im, uint64_t cap, uint
     }
     if (total) *total = off[nc];
     int rc;
+    if (nc == 1 && counts && !rank_worth_unsorted(tables_[0].map_n, off[1])) {
+        uint64_t n = 0;
+        rc = get_state(0, keys, re, im, cap, &n, flags);
+        if (total) *total = n;
+        if (!rc) counts[0] = n;
+        return rc;
+    }
     if ((rc = ensure_readout(off[nc]))) return rc;
     // every circuit's entries, in key order, one circuit after the other
     std::vector<RankJob> jobs(nc);

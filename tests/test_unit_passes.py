@@ -615,5 +615,13 @@ def test_readouts_of_thin_circuits_go_by_the_list(precision):
             got = read(sorted=False)
             order = np.argsort(got[0])
             assert_identical(tuple(x[order] for x in got), want)
+    b.prepare([(40, thin)])   # the only circuit of a batch, by the call that reads all
+    b.run()
+    b.sync()
+    before = b.stats()["kernel_launches"]
+    o = SparseOracle(precision)
+    o.apply(thin)
+    assert_identical(b.states(sorted=True)[0], o.state(sorted=True))
+    assert b.stats()["kernel_launches"] == before + 1
     b.close()
     sv.close()
