@@ -3,8 +3,8 @@
 // A batch holds up to a few thousand independent circuits, each with its own table slice
 // (the single-state layout of sqc_device.cuh, sized from the circuit's group bound), its own
 // control block (Ctl) and gate descriptors. One persistent kernel runs every circuit's
-// passes: a circuit's pass is cut into chunks of units (sqc_unit.cuh); any warp may take any chunk
-// of any circuit, and the warp that finishes the last chunk of a pass publishes it and opens
+// passes: a circuit's pass is cut into chunks of units (sqc_unit.cuh); any block may take any chunk
+// of any circuit, and the block that finishes the last chunk of a pass publishes it and opens
 // the circuit's next pass. Circuits never wait for one another.
 #pragma once
 #include <cstdint>
@@ -24,7 +24,7 @@ struct BPass {
 
 // A circuit of the batch (read-only while the kernel runs).
 struct BCirc {
-    TableDev t;                    // its table slice (units unused)
+    TableDev t;                    // its table slice
     const GateDesc* gates;
     const BPass* passes;
     uint32_t npasses;
@@ -44,7 +44,7 @@ enum BState : unsigned int { BS_IDLE = 0, BS_RUN = 1, BS_DONE = 2, BS_PARKED = 3
 
 struct alignas(32) BSched {
     unsigned int done;         // chunks finished in the current pass
-    unsigned int chunk;        // items (units, or 32 list entries each) per chunk in the current pass
+    unsigned int chunk;        // items (units, or list entries) per chunk in the current pass
     unsigned int next_total;   // chunks of the pass a parked circuit resumes with
     unsigned int state;        // BState
     unsigned int limit;        // the circuit parks before starting this pass
@@ -74,7 +74,7 @@ struct BatchArgs {
     const unsigned int* limit;      // begin kernel: pass limit per circuit
     uint32_t n;                     // circuits
     uint32_t amp_bytes;             // 16 (FP64) or 8 (FP32)
-    uint32_t min_chunk;             // list entries per chunk at least (a multiple of 4)
+    uint32_t min_chunk;             // list entries per chunk at least (a multiple of 4); a quarter as many units to a warp
     uint32_t target_chunks;         // chunks per pass at most, for large circuits
     PruneBits prune;
     unsigned long long idle_limit_ns;   // a warp that finds no work for this long records ST_TIMEOUT

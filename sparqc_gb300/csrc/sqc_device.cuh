@@ -191,10 +191,6 @@ __device__ __forceinline__ Cx<T> swap_update(bool bit, Cx<T> b) {
 }
 
 __host__ __device__ constexpr bool branch_kind(uint32_t k) { return k == KH || k == KRX || k == KRY || k == KU; }
-__host__ __device__ constexpr bool swap_kind(uint32_t k) { return k == KX || k == KY; }
-__host__ __device__ constexpr bool one_sided_kind(uint32_t k) {
-    return k == KZ || k == KS || k == KSDG || k == KPHASE || k == KT || k == KTDG;
-}
 
 // Prune rule of the reference (emulator/include/data_t.h:50-60): |re| < thr && |im| < thr,
 // decided in FP64. For doubles |x| < thr is compared on the bit patterns (non-negative

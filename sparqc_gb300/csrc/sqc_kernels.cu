@@ -19,31 +19,13 @@ __device__ __forceinline__ Cx<T> load_amp(const void* amps, size_t s) {
     const typename AmpT<T>::V v = reinterpret_cast<const typename AmpT<T>::V*>(amps)[s];
     return Cx<T>{v.x, v.y};
 }
-template <class T>
-__device__ __forceinline__ void store_amp(void* amps, size_t s, Cx<T> a) {
-    typename AmpT<T>::V v;
-    v.x = a.r;
-    v.y = a.i;
-    reinterpret_cast<typename AmpT<T>::V*>(amps)[s] = v;
-}
 __device__ __forceinline__ Cx<double> load_amp_any(const void* amps, size_t s, bool dbl) {
     if (dbl) { const double2 v = reinterpret_cast<const double2*>(amps)[s]; return Cx<double>{v.x, v.y}; }
     const float2 v = reinterpret_cast<const float2*>(amps)[s];
     return Cx<double>{(double)v.x, (double)v.y};
 }
 
-template <class T> __device__ __forceinline__ Cx<T> czero() { return Cx<T>{T(0), T(0)}; }
-
 __device__ __forceinline__ bool slot_present(unsigned long long key, int j) { return (int)(key & 15ULL) == j; }
-
-__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
-    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(kFull, v, o);
-    return v;
-}
-__device__ __forceinline__ double warp_sum(double v) {
-    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(kFull, v, o);
-    return v;
-}
 
 // |0...0>: new epoch (every bucket becomes free), claim group 0, store key 0 with amplitude 1.
 __global__ void set_zero_kernel(TableDev t, Ctl* ctl, int dbl) {

@@ -32,11 +32,6 @@ __device__ __forceinline__ Cx<T> amp_at(const void* amps, size_t s) {
     }
 }
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(kFull, v, o);
-    return v;
-}
-
 // sums->c[SUM_NORM] += sum of |a|^2 over present keys with (stored & smask) == sval, exactly.
 template <class T>
 __global__ void pattern_prob_kernel(TableDev t, Ctl* ctl, unsigned long long smask, unsigned long long sval,

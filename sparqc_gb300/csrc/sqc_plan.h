@@ -74,10 +74,9 @@ void split_passes(const GateDesc* d, size_t n, size_t max_run, uint32_t max_nx, 
     }
 }
 
-// Record in descriptors [g0, g1) -- one pass with cross-group qubits q1, q2, q3 (in order of
-// first use; kNoQubit when absent) -- how the pass applies each gate (GateDesc.flip kOp*
-// bits): gates on q1 and q3 pair slots held by the same lane, gates on q2 and on qubits 0..3
-// pair lanes (shuffles).
+// A summary of descriptors [g0, g1), one pass with cross-group qubits q1, q2, q3 (in order of first use;
+// kNoQubit when absent), by kind and qubits (GateDesc.flip kOp* bits): gates on q1 and q3 pair slots, gates on
+// q2 and on qubits 0..3 lanes. For checks of pass splits: how passes apply their gates is in om, ov and loc.
 void encode_pass(GateDesc* d, size_t g0, size_t g1, uint32_t q1, uint32_t q3 = kNoQubit);
 
 // The group bits a mapped table addresses its buckets by (TableDev::map_q): bucket bit i is group

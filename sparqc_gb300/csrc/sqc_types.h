@@ -111,7 +111,7 @@ enum UOp : uint32_t {
     UO_ODD = 61     // a gate with a coefficient that is not finite; + 1: pairs lanes, + 2: on dimension 2
 };
 
-// GateDesc.flip bits: the frame's flip, and what encode_pass says of a gate by kind and qubits.
+// GateDesc.flip bits: the frame's flip (the only one passes read), and encode_pass's summary of a gate.
 constexpr uint32_t kOpFlip = 1u << 0;      // the stored frame flips the target bit
 constexpr uint32_t kOpPair = 1u << 1;      // pairs the a and b slots (first cross-group qubit)
 constexpr uint32_t kOpShfl = 1u << 2;      // partner slot in lane ^ (1 << off_log2)

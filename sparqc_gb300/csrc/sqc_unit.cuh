@@ -210,16 +210,6 @@ __device__ __forceinline__ float flip_sign(float x, uint32_t m) {
     return __int_as_float(__float_as_int(x) ^ (int)(m & 0x80000000u));
 }
 
-// Whether a branching result is kept (negligible's complement). FP64 looks at the high words
-// first: the 64-bit compares otherwise issue on the FP64 pipe.
-__device__ __forceinline__ bool kept(Cx<float> v, const PruneBits& pb) { return !negligible(v, pb); }
-__device__ __forceinline__ bool kept(Cx<double> v, const PruneBits& pb) {
-    const uint32_t th = (uint32_t)(pb.d >> 32), tl = (uint32_t)pb.d;
-    const uint32_t r = (uint32_t)__double2hiint(v.r) & 0x7FFFFFFFu, i = (uint32_t)__double2hiint(v.i) & 0x7FFFFFFFu;
-    if (r > th || i > th) return true;
-    return (r == th && (uint32_t)__double2loint(v.r) >= tl) || (i == th && (uint32_t)__double2loint(v.i) >= tl);
-}
-
 template <class T>
 __device__ __forceinline__ Cx<T> shfl_cx(Cx<T> a, int off) {
     return Cx<T>{__shfl_xor_sync(kFull, a.r, off), __shfl_xor_sync(kFull, a.i, off)};
