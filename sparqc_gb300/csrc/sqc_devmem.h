@@ -2,8 +2,9 @@
 //
 // A rebuild of a hashed table leaves the old table, and circuits whose keys move are rebuilt several times:
 // the next rebuild takes the kept table instead of allocating (a million loaded keys, 60 gates: 8.3 ms, and
-// 15.2 with an allocation each time). Kept tables belong to the whole process: at most an eighth of a device
-// in all, the oldest freed first, and given back whenever an allocation of any state, batch or server on
+// 15.2 with an allocation each time). Kept tables belong to the whole process: at most a quarter of a device
+// in all (three such states, 13.6 GB each, run in turns 8.0-9.5 ms, with an eighth 14.5-15.3), the oldest freed first,
+// and given back whenever an allocation of any state, batch or server on
 // that device fails. A kept table is not in use by any stream (a rebuild ends with a wait).
 #pragma once
 #include <cstddef>

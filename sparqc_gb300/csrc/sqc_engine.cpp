@@ -146,7 +146,7 @@ int Engine::init(uint32_t nq, const sqc_hash_table_parameters* params, const sqc
     size_t free_b = 0, total_b = 0;
     if ((rc = cuda(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo"))) return rc;
     budget_ = (size_t)((1.0 - reserve) * (double)total_b);
-    spare_limit_ = total_b / 8;
+    spare_limit_ = total_b / 4;
 
     if (o.stream) {
         stream_ = (cudaStream_t)o.stream;

@@ -150,7 +150,7 @@ private:
     uint32_t max_run_ = kMaxRun;
     uint32_t max_nx_ = 2;        // cross-group qubits per pass at most
     size_t budget_ = 0;
-    size_t spare_limit_ = 0;     // kept tables of all states (sqc_devmem.h): an eighth of the device
+    size_t spare_limit_ = 0;     // kept tables of all states (sqc_devmem.h): a quarter of the device
     cudaStream_t stream_ = nullptr;
     bool own_stream_ = false;
 
