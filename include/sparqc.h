@@ -496,7 +496,8 @@ typedef struct sqc_stats {
     uint64_t passes;           /* device gate passes executed */
     uint64_t kernel_launches;  /* kernels launched by this handle */
     uint64_t buckets;          /* current buckets per table */
-    uint64_t table_bytes;      /* device bytes held by both tables */
+    uint64_t table_bytes;      /* device bytes of the table, and of one kept for its next rebuild (given
+                                  back when an allocation on the device fails) */
     uint64_t replays;          /* passes re-run after table growth */
     uint64_t amp_updates;      /* sum over gates of input nonzeros (only counted after sync) */
     uint64_t alg_bytes;        /* algorithmic bytes of the passes: (nnz_in + nnz_out) * (8 + A) per

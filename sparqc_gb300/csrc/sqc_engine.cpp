@@ -106,7 +106,9 @@ size_t Engine::bucket_bytes() const {
 }
 
 // Groups up to which a hashed table is kept as it is.
-unsigned long long Engine::roomy_groups() const { return (unsigned long long)(hash_load_ * (double)tab_.nb); }
+unsigned long long Engine::roomy_groups() const {
+    return (unsigned long long)((fill_up_ ? kMaxLoad : tab_.nb <= kSmallTable ? kSmallLoad : kHashLoad) * (double)tab_.nb);
+}
 
 unsigned long long Engine::max_groups() const { return (unsigned long long)(kMaxLoad * (double)tab_.nb); }
 
@@ -675,18 +677,18 @@ int Engine::make_room(uint32_t nx, unsigned long long bound, unsigned long long 
     unsigned long long nb = std::max(tab_.nb, hashed_size(groups, nx, keys));
     while (nb > tab_.nb && (double)nb * bucket_bytes() > (double)budget_) nb /= 2;
     if (nb == tab_.nb && ctl_host_->empty_groups * 4 < ctl_host_->list_n) {   // as large as it gets: fill it up
-        hash_load_ = kMaxLoad;
+        fill_up_ = true;
         return SQC_OK;   // a pass that still does not fit refuses; sync() decides
     }
     // no memory for it: a smaller one, or the present table fills up, and a pass that does not fit refuses
     rc = rebuild(nb, false);
     while (rc == SQC_ERR_OOM && nb / 2 > tab_.nb) rc = rebuild(nb /= 2, false);
     if (rc == SQC_ERR_OOM || rc == SQC_ERR_BUDGET) {
-        hash_load_ = kMaxLoad;
+        fill_up_ = true;
         return SQC_OK;
     }
     if (rc) return rc;
-    if (grown(nx, bound, keys) > roomy_groups()) hash_load_ = kMaxLoad;
+    if (grown(nx, bound, keys) > roomy_groups()) fill_up_ = true;
     passes_.clear();   // all verified: later ones count from here
     return SQC_OK;
 }
@@ -834,7 +836,7 @@ int Engine::sync() {
 // Copy the live, non-empty buckets into a new table of nb_new buckets. The control block
 // must be in sync with the device (read_ctl) and no pass may be in flight.
 int Engine::rebuild(unsigned long long nb_new, bool mapped) {
-    hash_load_ = nb_new <= kSmallTable ? kSmallLoad : kHashLoad;
+    fill_up_ = false;
     HostTable nt;
     int rc;
     if ((rc = alloc_table(nb_new, &nt))) return rc;

@@ -192,7 +192,7 @@ private:
     void* d_cum_tmp_ = nullptr;
     size_t cum_cap_ = 0, cum_tmp_bytes_ = 0;
 
-    double hash_load_ = 0.6;        // load up to which a hashed table stays as it is (a small one, at first)
+    bool fill_up_ = false;          // no larger table is to be had: this one is used up to its load limit
     uint64_t gates_applied_ = 0, passes_run_ = 0, launches_ = 0, replays_ = 0, rebuilds_ = 0;
     uint64_t passes_pair_ = 0;
 
