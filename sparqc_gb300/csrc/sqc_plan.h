@@ -124,8 +124,8 @@ void encode_slot_pass(GateDesc* d, size_t g0, size_t g1, uint32_t form, const ui
 // when it needs lookups (a cross-group qubit); a pass that is one column pass either way where the state is small,
 // or FP64 groups hold enough keys. (us, start
 // of the sequence to its end, columns against slots: 24 gates on low qubits, FP64, 2^12 groups of 16 keys 169
-// and 57, 2^16 478 and 246; 36 gates on the low and two other qubits, 30000 groups of one key 1018 and 516; but a
-// million keys in groups of one or two, 60 gates, few branching: 7.4 ms and 14.)
+// and 45, 2^16 478 and 255; 36 gates on the low and two other qubits, 2^11 groups of 16 keys 344 and 69, 30000 of one key
+// 1018 and 492; but a million keys in groups of one or two, 60 gates, few branching: 7.4 ms and 14.)
 // f(g0, g1, form, q1, q2, q3, keys_fixed): form 0, a column pass and its pairing qubits, or a slot pass (encode_slot_pass)
 // and its cross-group ones.
 constexpr unsigned long long kSlotSmall = 1ULL << 15;   // groups of a small state
